@@ -3,9 +3,9 @@
 //
 // One CTA takes two tiles of 128 rows, the rows being (token, query head) pairs of
 // the heads that share one key/value head (row r = token * G + head, G heads per
-// key/value head, G a divisor of 128; the second tile holds the next 128 / G
-// tokens), and walks the request's keys in blocks of 128; both tiles use each block
-// of K and V, which is brought in once:
+// key/value head; a tile holds the whole tokens that fit, 128 / G of them, and the
+// second tile the next ones), and walks the request's keys in blocks of 128; both
+// tiles use each block of K and V, which is brought in once:
 //   warp 0      TMA: the Q tiles once (3-D boxes over [token][head][64]), then per
 //               block the K and V pages through the block table (one box per page),
 //               into rings of three stages each, 128-byte swizzle;
@@ -160,7 +160,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     if (warp == 0) {
         if (live) {
             if (lane == 0) {
-                mbar_expect_tx(&sm.q_full, (tr[1].has ? 2 : 1) * TM * HD * 2);
+                mbar_expect_tx(&sm.q_full, (tr[1].has ? 2 : 1) * tok_per_tile * G * HD * 2);
                 tma_load_3d(sm.q[0], &map_q, 0, kvh * G, t_base + tr[0].tok0, &sm.q_full);
                 if (tr[1].has) tma_load_3d(sm.q[1], &map_q, 0, kvh * G, t_base + tr[1].tok0, &sm.q_full);
             }
@@ -251,7 +251,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int qt = warp & 3;                                      // quarter of the tile's rows = of tensor memory's lanes
         const int r = qt * 32 + lane;                                 // row of the tile = lane of tensor memory
         const int tok = tr[t].tok0 + r / G;                           // token within the portion
-        const bool row_ok = tok < q_len;
+        // where G is no divisor of 128 the rows behind the tile's last token are nobody's: their queries were never
+        // loaded, every score of theirs is masked and nothing of them is written
+        const bool row_ok = r < tok_per_tile * G && tok < q_len;
         const int pos = row_ok ? ctx + tok : -1;
         const int lo = first_key(pos, window, chunk);
         const uint32_t lane_base = tmem + ((uint32_t)(qt * 32) << 16);
@@ -389,15 +391,26 @@ CELLM_API int cellm_attention_tc_supports(int hd, int nh, int nkv, int page_size
     return page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128;
 }
 
+// Groups that do not divide 128 leave a tile's last rows empty (2 of 128 for G = 3, 32 at most here). They are taken where at
+// least three quarters of the rows are in use: with 24 heads over 8, 2,048 queries behind 8,192 keys, the layer takes 509 us
+// here and 813 us on the mma.sync kernel, a ratio that a quarter of a tile does not use up. `uneven`: 0 for the entry points
+// that take divisors only.
+static bool attention_tc_takes(int hd, int nh, int nkv, int page_size, int uneven) {
+    if (cellm_attention_tc_supports(hd, nh, nkv, page_size)) return true;
+    if (!uneven || hd != 64 || nkv <= 0 || nh <= 0 || nh % nkv || nh / nkv > 128) return false;
+    const int G = nh / nkv;
+    return 128 / G * G >= 96 && cellm_attention_tc_supports(hd, nkv, nkv, page_size);
+}
+
 // out, q: [T, nh*64] bf16; pools: one layer's [pages][nkv][page_size][64] bf16. n_tiles = sum over the
-// requests of ceil(q_len / (256 / (nh/nkv))): a CTA takes two tiles of 128 rows that share their keys.
+// requests of ceil(q_len / (2 * (128 / (nh/nkv)))): a CTA takes two tiles of 128 rows that share their keys.
 static int attention_tc_impl(void* out, const void* q, const void* k_pool, const void* v_pool,
                              const int* cu_seqlens, const int* ctx_lens, const int* block_table, int bt_stride,
                              int B, int T, int n_tiles, int num_pages, int page_size, int nh, int nkv, int hd,
                              float scale, int window, const float* sinks, const float* gate, long long gate_ld, int* err,
-                             cudaStream_t stream, int chunk = 0) {
+                             cudaStream_t stream, int chunk = 0, int uneven = 0) {
     if (T <= 0 || n_tiles <= 0) return CELLM_OK;
-    if (!cellm_attention_tc_supports(hd, nh, nkv, page_size) || scale <= 0.f) return CELLM_ERR_SIZE;
+    if (!attention_tc_takes(hd, nh, nkv, page_size, uneven) || scale <= 0.f) return CELLM_ERR_SIZE;
     if (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out) & 15) return CELLM_ERR_ALIGN;
     const int G = nh / nkv;
     CUtensorMap mq, mk, mv;
@@ -433,6 +446,15 @@ CELLM_API int cellm_attention_tc(void* out, const void* q, const void* k_pool, c
                                  float scale, int window, int* err, cudaStream_t stream) {
     return attention_tc_impl(out, q, k_pool, v_pool, cu_seqlens, ctx_lens, block_table, bt_stride, B, T, n_tiles, num_pages,
                              page_size, nh, nkv, hd, scale, window, nullptr, nullptr, 0, err, stream);
+}
+
+// The same for groups of heads that need not divide 128 (three quarters of a tile's rows must be in use).
+CELLM_API int cellm_attention_tc_uneven(void* out, const void* q, const void* k_pool, const void* v_pool,
+                                        const int* cu_seqlens, const int* ctx_lens, const int* block_table, int bt_stride,
+                                        int B, int T, int n_tiles, int num_pages, int page_size, int nh, int nkv, int hd,
+                                        float scale, int window, int* err, cudaStream_t stream) {
+    return attention_tc_impl(out, q, k_pool, v_pool, cu_seqlens, ctx_lens, block_table, bt_stride, B, T, n_tiles, num_pages,
+                             page_size, nh, nkv, hd, scale, window, nullptr, nullptr, 0, err, stream, 0, 1);
 }
 
 // The same with a sink per head in every row's denominator (`sinks` [nh], 32-bit; null: none) and an output gate (`gate`

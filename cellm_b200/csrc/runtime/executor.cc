@@ -639,13 +639,14 @@ void* Run::attend(const AttentionParams& L, const ExecItem& it, const void* q, v
         // prompt portions that fill the tcgen05 kernel's pairs of 128-row tiles and enough CTAs (below that the
         // mma.sync kernel with its split over the keys fills the GPU better)
         const i64 ps = it.page_size;
-        if (hd == 64 && G <= 128 && 128 % G == 0 && (ps == 8 || ps == 16 || ps == 32 || ps == 64 || ps == 128)) {
-            const i64 per_tile = 256 / G;
+        // groups that do not divide 128 leave rows of a tile empty: taken where three quarters of them are in use
+        if (hd == 64 && G <= 128 && 128 / G * G >= 96 && (ps == 8 || ps == 16 || ps == 32 || ps == 64 || ps == 128)) {
+            const i64 per_tile = 2 * (128 / G);
             i64 tc_tiles = 0;
             for (i64 b = 0; b < s.B; ++b) tc_tiles += ceil_div(s.q_lens[b], per_tile);
             const i64 min_ctas = p.tc_min_ctas < 0 ? p.sms / 8 : p.tc_min_ctas;
             if (tc_tiles * nkv >= min_ctas && (double)T >= p.tc_min_fill * (double)(tc_tiles * per_tile)) {
-                LAUNCH(fn<AttentionTcFn>(FN_ATTENTION_TC)(o, q, it.k, it.v, s.cu_seqlens, s.ctx_lens, it.block_table, (int)it.bt_stride,
+                LAUNCH(fn<AttentionTcFn>(128 % G == 0 ? FN_ATTENTION_TC : FN_ATTENTION_TC_UNEVEN)(o, q, it.k, it.v, s.cu_seqlens, s.ctx_lens, it.block_table, (int)it.bt_stride,
                                                       (int)s.B, (int)T, (int)tc_tiles, (int)it.num_pages, (int)ps, (int)nh, (int)nkv,
                                                       (int)hd, scale, (int)L.window, s.err, s.stream),
                    "attention_tc");

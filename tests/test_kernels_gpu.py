@@ -500,6 +500,45 @@ def test_attention_tc(ps, nh, nkv, window):
     assert e.item() == 0
 
 
+def portions_ctx(c, lens, ctxs, e):
+    from cellm_b200.parts import StepContext
+    zero = torch.zeros_like(c["pos"])
+    return StepContext(T=len(zero), B=len(lens), dtype=c["q"].dtype, device=torch.device(DEV), token_ids=zero, positions=c["pos"],
+                       seq_of_token=c["seq"], cu_seqlens=c["cu"], ctx_lens=c["ctx"], slot_ids=torch.arange(len(lens), dtype=torch.int32, device=DEV),
+                       err=e, q_lens=list(lens), ctx_lens_host=list(ctxs), max_q_len=max(lens), max_total_len=max(a + b for a, b in zip(lens, ctxs)))
+
+
+@pytest.mark.parametrize("ps,nh,nkv", [(16, 6, 2), (8, 5, 1), (128, 12, 2), (32, 7, 1), (64, 60, 2), (16, 21, 1), (16, 24, 8)])
+@pytest.mark.parametrize("window", [0, 33])
+def test_attention_takes_groups_that_do_not_divide_a_tile(monkeypatch, ps, nh, nkv, window):
+    """Groups of 3, 5, 6, 7, 21 and 30 heads a key/value head: a tile's last rows belong to nobody. Through the executor's
+    choice of kernel, against the oracle and against the mma.sync kernel that took these groups before; a group that
+    would leave more than a quarter of a tile empty (43) still goes there."""
+    from cellm_b200 import ops
+    from cellm_b200.ops.attention import attention_flash
+    from cellm_b200.runtime import program
+    monkeypatch.setitem(program.OPTIONS, "attention_tc_min_ctas", 0)
+    monkeypatch.setitem(program.OPTIONS, "attention_tc_min_fill", 0.0)
+    hd, lens, ctxs = 64, [170, 1, 33, 129], [0, 500, 59, 640]
+    c = paged_case(lens, ctxs, nh, nkv, hd, ps, torch.bfloat16, seed=6)
+    e = err_word()
+    ctx = portions_ctx(c, lens, ctxs, e)
+    name = "cellm_attention_tc" if 128 % (nh // nkv) == 0 else "cellm_attention_tc_uneven"
+    for scale in (hd ** -0.5, 1.0):
+        before = program.CALLS[name]
+        out = ops.attention(c["q"], c["kp"], c["vp"], ctx, c["bt"], nh, scale, window)
+        assert program.CALLS[name] == before + 1
+        close(out, attention_reference(c, nh, nkv, hd, scale, window), torch.bfloat16, f"scale {scale}")
+        flash = attention_flash(c["q"], c["kp"], c["vp"], c["cu"], c["ctx"], c["bt"], c["q_lens"], nh, scale, window, e)
+        both = 2 * tol(torch.bfloat16, flash.double())          # either is within its own bound of the oracle
+        assert float((out.double() - flash.double()).abs().max()) <= both
+    assert e.item() == 0
+    d = paged_case([40], [0], 43, 1, hd, 16, torch.bfloat16, seed=1)
+    before = program.CALLS["cellm_attention_flash"]
+    ops.attention(d["q"], d["kp"], d["vp"], portions_ctx(d, [40], [0], e), d["bt"], 43, 0.125, 0)
+    assert program.CALLS["cellm_attention_flash"] == before + 1
+
+
 def test_attention_tc_refuses_what_it_does_not_take():
     from cellm_b200.ops.attention import attention_tc, attention_tc_supports
     assert not attention_tc_supports(128, 4, 4, 16) and not attention_tc_supports(64, 6, 2, 16)
