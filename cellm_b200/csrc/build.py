@@ -45,6 +45,7 @@ LIBRARIES: dict[str, tuple[str, list[str], list[str]]] = {
     "attention_latent": ("nvcc", ["kernels/attention_latent.cu"], []),
     "attention_expanded": ("nvcc", ["kernels/attention_expanded.cu"], []),
     "decay_chunks": ("nvcc", ["kernels/decay_chunks.cu"], []),
+    "state_chunks": ("nvcc", ["kernels/state_chunks.cu"], []),
 }
 
 _loaded: dict[str, ctypes.CDLL] = {}

@@ -373,19 +373,27 @@ hgrn2_scan_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
 
 #define RECURRENT_MAX_DIM 512
 
-CELLM_API int cellm_hgrn2_scan(float* o_out, float* state, long long slot_stride, int n_slots, float* proj, long long ld,
-                               int col_q, int col_f, int col_v, const float* f_bias, const float* lower,
-                               const int* cu_seqlens, const int* slot_ids, int B, int T, int heads, int dim, int vd, int* err,
-                               cudaStream_t stream) {
-    if (B <= 0 || T <= 0) return CELLM_OK;
-    if (heads <= 0 || dim <= 0 || vd <= 0 || dim > RECURRENT_MAX_DIM) return CELLM_ERR_SIZE;
+CELLM_API int cellm_hgrn2_gates(float* proj, long long ld, int col_q, int col_f, const float* f_bias, const float* lower, int T, int heads,
+                                int dim, cudaStream_t stream) {
+    if (T <= 0) return CELLM_OK;
+    if (heads <= 0 || dim <= 0 || dim > RECURRENT_MAX_DIM) return CELLM_ERR_SIZE;
     const size_t total = (size_t)T * 2 * heads * dim;
     CELLM_RUN(hgrn2_gates_kernel, (unsigned)std::min<size_t>((total + 255) / 256, 148 * 16), 256, 0, stream, proj, ld, col_q, col_f, f_bias,
               lower, T, heads * dim);
+    return CELLM_OK;
+}
+
+// The walk over gated q and f; portions of more than max_len tokens (0: no such limit) are left alone (heads of up to 128 rows).
+CELLM_API int cellm_hgrn2_walk(float* o_out, float* state, long long slot_stride, int n_slots, const float* proj, long long ld, int col_q,
+                               int col_f, int col_v, const int* cu_seqlens, const int* slot_ids, int B, int heads, int dim, int vd,
+                               int max_len, int* err, cudaStream_t stream) {
+    if (B <= 0) return CELLM_OK;
+    if (heads <= 0 || dim <= 0 || vd <= 0 || dim > RECURRENT_MAX_DIM || (max_len > 0 && dim > 128)) return CELLM_ERR_SIZE;
     WalkVectors vec;
     for (int a = 0; a < 5; ++a) vec.p[a] = nullptr, vec.ld[a] = ld, vec.heads_per[a] = 1;
     vec.p[0] = proj + col_q, vec.p[1] = proj + col_f;
     vec.vec16 = dim % 4 == 0 && ld % 4 == 0 && aligned16(vec.p[0]) && aligned16(vec.p[1]);
+    if (max_len > 0) vec.max_len = max_len;
 #define HGRN2_WALK(D, R)                                                                                           \
     CELLM_RUN((state_walk_kernel<D, R, 0>), dim3(B, heads, (vd + WalkShape<D, R>::CPB - 1) / WalkShape<D, R>::CPB), WALK_THREADS, 0, stream, \
               o_out, state, slot_stride, n_slots, vec, (const float*)(proj + col_v), ld, (const float*)nullptr, cu_seqlens, slot_ids,  \
@@ -401,10 +409,21 @@ CELLM_API int cellm_hgrn2_scan(float* o_out, float* state, long long slot_stride
             if (e != cudaSuccess) return (int)e;
         }
         CELLM_RUN(hgrn2_scan_kernel, dim3(B, heads, (vd + 31) / 32), 32, big, stream, o_out, state, slot_stride, n_slots,
-                  (const float*)proj, ld, col_q, col_f, col_v, cu_seqlens, slot_ids, heads, dim, vd, err);
+                  proj, ld, col_q, col_f, col_v, cu_seqlens, slot_ids, heads, dim, vd, err);
     }
 #undef HGRN2_WALK
     return CELLM_OK;
+}
+
+CELLM_API int cellm_hgrn2_scan(float* o_out, float* state, long long slot_stride, int n_slots, float* proj, long long ld,
+                               int col_q, int col_f, int col_v, const float* f_bias, const float* lower,
+                               const int* cu_seqlens, const int* slot_ids, int B, int T, int heads, int dim, int vd, int* err,
+                               cudaStream_t stream) {
+    if (B <= 0 || T <= 0) return CELLM_OK;
+    if (heads <= 0 || dim <= 0 || vd <= 0 || dim > RECURRENT_MAX_DIM) return CELLM_ERR_SIZE;
+    const int e = cellm_hgrn2_gates(proj, ld, col_q, col_f, f_bias, lower, T, heads, dim, stream);
+    return e != CELLM_OK ? e : cellm_hgrn2_walk(o_out, state, slot_stride, n_slots, proj, ld, col_q, col_f, col_v, cu_seqlens, slot_ids, B,
+                                                heads, dim, vd, 0, err, stream);
 }
 
 // ------------------------------------------------------------------------------------------------ delta rule: inputs
@@ -536,19 +555,19 @@ delta_scan_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     }
 }
 
-
-
-CELLM_API int cellm_delta_scan(float* o_out, float* state, long long slot_stride, int n_slots, const float* qk, const float* v_in,
+// Portions of more than max_len tokens (0: no such limit) are left alone (heads of up to 128 rows).
+CELLM_API int cellm_delta_walk(float* o_out, float* state, long long slot_stride, int n_slots, const float* qk, const float* v_in,
                                const float* beta, const float* decay, const int* cu_seqlens, const int* slot_ids, int B,
-                               int heads, int kvh, int dim, int vd, int* err, cudaStream_t stream) {
+                               int heads, int kvh, int dim, int vd, int max_len, int* err, cudaStream_t stream) {
     if (B <= 0) return CELLM_OK;
-    if (heads <= 0 || kvh <= 0 || heads % kvh || dim <= 0 || vd <= 0 || dim > RECURRENT_MAX_DIM) return CELLM_ERR_SIZE;
+    if (heads <= 0 || kvh <= 0 || heads % kvh || dim <= 0 || vd <= 0 || dim > RECURRENT_MAX_DIM || (max_len > 0 && dim > 128)) return CELLM_ERR_SIZE;
     WalkVectors vec;
     for (int a = 0; a < 5; ++a) vec.p[a] = nullptr, vec.ld[a] = 0, vec.heads_per[a] = 1;
     vec.p[0] = qk, vec.p[1] = qk + (size_t)kvh * dim, vec.p[2] = decay;
     vec.ld[0] = vec.ld[1] = 2LL * kvh * dim, vec.ld[2] = (long long)heads * dim;
     vec.heads_per[0] = vec.heads_per[1] = heads / kvh, vec.heads_per[2] = 1;
     vec.vec16 = dim % 4 == 0 && aligned16(qk) && aligned16(decay);
+    if (max_len > 0) vec.max_len = max_len;
 #define DELTA_WALK(D, R)                                                                                           \
     CELLM_RUN((state_walk_kernel<D, R, 1>), dim3(B, heads, (vd + WalkShape<D, R>::CPB - 1) / WalkShape<D, R>::CPB), WALK_THREADS, 0, stream, \
               o_out, state, slot_stride, n_slots, vec, v_in, (long long)heads * vd, beta, cu_seqlens, slot_ids, heads, dim, vd, err)
@@ -567,6 +586,13 @@ CELLM_API int cellm_delta_scan(float* o_out, float* state, long long slot_stride
     }
 #undef DELTA_WALK
     return CELLM_OK;
+}
+
+CELLM_API int cellm_delta_scan(float* o_out, float* state, long long slot_stride, int n_slots, const float* qk, const float* v_in,
+                               const float* beta, const float* decay, const int* cu_seqlens, const int* slot_ids, int B,
+                               int heads, int kvh, int dim, int vd, int* err, cudaStream_t stream) {
+    return cellm_delta_walk(o_out, state, slot_stride, n_slots, qk, v_in, beta, decay, cu_seqlens, slot_ids, B, heads, kvh, dim, vd, 0,
+                            err, stream);
 }
 
 // ------------------------------------------------------------------------------------------------ generalized delta rule

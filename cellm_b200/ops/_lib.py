@@ -55,6 +55,9 @@ _SIGNATURES = {
         "cellm_sink_attn_prep": [P, P, P, P, L, I, P, P, I, P, L, I, P, P, F, P, I, P, I, P, P, P, P, P, I, I, I, I, I, I, I, I, P, I, P, P],
         "cellm_attention_plain_masked": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, P, F, I, P, L, I, P, P],
         "cellm_attention_plain_sink": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, P, P, I, I, P, P],
+        "cellm_hgrn2_gates": [P, L, I, I, P, P, I, I, I, P],
+        "cellm_hgrn2_walk": [P, P, L, I, P, L, I, I, I, P, P, I, I, I, I, I, P, P],
+        "cellm_delta_walk": [P, P, L, I, P, P, P, P, P, P, I, I, I, I, I, I, P, P],
         "cellm_hgrn2_scan": [P, P, L, I, P, L, I, I, I, P, P, P, P, I, I, I, I, I, P, P],
         "cellm_delta_prep": [P, P, P, P, P, L, I, I, P, I, P, L, I, P, L, P, P, P, P, P, I, I, I, I, I, F, P, P],
         "cellm_delta_scan": [P, P, L, I, P, P, P, P, P, P, I, I, I, I, I, P, P],
@@ -104,6 +107,11 @@ _SIGNATURES = {
         "cellm_attention_flash_sink": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, I, P, P, I, P, P, P],
         "cellm_attention_flash_chunked": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, I, P, P],
         "cellm_attention_flash_masked": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, I, I, P, P, L, P, P],
+    },
+    "state_chunks": {
+        "cellm_state_chunks_floats": [I, I, I],
+        "cellm_delta_chunks": [P, P, L, I, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P, P],
+        "cellm_hgrn2_chunks": [P, P, L, I, P, L, I, I, I, P, P, I, I, I, I, I, I, P, P, P],
     },
     "decay_chunks": {
         "cellm_decay_chunks": [P, P, L, I, P, L, P, L, P, L, P, L, P, L, P, P, I, I, I, I, I, I, I, P, P, P, P],

@@ -194,16 +194,50 @@ def attention_flash_masked(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: i
     return out
 
 
+# Portions of this many tokens and more run the recurrences with a decay per channel in chunks (heads of up to 128
+# rows). One portion, 16 heads, token by token against in chunks: the delta rule with states of 128 x 128 32 against 21 us
+# at 64 tokens, 25 against 21 at 48, 12 against 20 at 24 (two kernels in place of one); 915 against 217 at 2,048. HGRN2 with
+# 64 x 128 15 against 27 us at 64 tokens, 45 against 27 at 128; 627 against 177 at 2,048.
+DELTA_CHUNKS_FROM, HGRN2_CHUNKS_FROM = 48, 96
+_STATE_CHUNK = 16           # tokens a chunk of state_chunks.cu
+
+
+def _state_chunks(ctx, delta: bool, heads: int, dim: int, vd: int, device):
+    """(workspace, chunks, tokens from which a portion is long, whether portions remain for the walk) of a step's long portions;
+    None where all are short."""
+    least = DELTA_CHUNKS_FROM if delta else HGRN2_CHUNKS_FROM
+    long = [n for n in ctx.q_lens if n >= least] if dim <= 128 and ctx.max_q_len >= least else []
+    if not long:
+        return None
+    n_chunks = sum(-(-n // _STATE_CHUNK) for n in long)
+    floats = fn("state_chunks", "cellm_state_chunks_floats")(int(delta), dim, vd)
+    return torch.empty((n_chunks * heads * floats,), dtype=torch.float32, device=device), n_chunks, least, len(long) < ctx.B
+
+
 def hgrn2_scan(proj: torch.Tensor, col_q: int, col_f: int, col_v: int, f_bias: torch.Tensor, lower: torch.Tensor, state: torch.Tensor,
-               ctx, heads: int, dim: int, vd: int) -> torch.Tensor:
+               ctx, heads: int, dim: int, vd: int, chunked: bool = False) -> torch.Tensor:
     """The HGRN2 recurrence over every request's tokens of the step; state [slots, heads, dim, vd] float32 is moved on.
     Returns S^T q per token and head, float32 [T, heads * vd]. The q and f columns of `proj` are replaced by silu(q) and
-    by the forget gate."""
+    by the forget gate. `chunked`: portions of HGRN2_CHUNKS_FROM tokens and more run in chunks (heads of up to 128 rows), the
+    others token by token; without it all run token by token, and a state is then bit-identical however the sequence was cut."""
     _f32(proj, f_bias, lower, state)
     o = torch.empty((ctx.T, heads * vd), dtype=torch.float32, device=proj.device)
-    check(fn(_LIB, "cellm_hgrn2_scan")(ptr(o), ptr(state), state.stride(0), state.shape[0], ptr(proj), proj.stride(0), int(col_q), int(col_f),
-                                       int(col_v), ptr(f_bias), ptr(lower), ptr(ctx.cu_seqlens), ptr(ctx.slot_ids), ctx.B, ctx.T, heads, dim, vd,
-                                       ptr(ctx.err), stream_of(proj)), "hgrn2_scan")
+    chunks = _state_chunks(ctx, False, heads, dim, vd, proj.device) if chunked else None
+    if chunks is None:
+        check(fn(_LIB, "cellm_hgrn2_scan")(ptr(o), ptr(state), state.stride(0), state.shape[0], ptr(proj), proj.stride(0), int(col_q), int(col_f),
+                                           int(col_v), ptr(f_bias), ptr(lower), ptr(ctx.cu_seqlens), ptr(ctx.slot_ids), ctx.B, ctx.T, heads, dim, vd,
+                                           ptr(ctx.err), stream_of(proj)), "hgrn2_scan")
+        return o
+    ws, n_chunks, least, rest = chunks
+    check(fn(_LIB, "cellm_hgrn2_gates")(ptr(proj), proj.stride(0), int(col_q), int(col_f), ptr(f_bias), ptr(lower), ctx.T, heads, dim,
+                                        stream_of(proj)), "hgrn2_gates")
+    where = (ptr(o), ptr(state), state.stride(0), state.shape[0], ptr(proj), proj.stride(0), int(col_q), int(col_f), int(col_v),
+             ptr(ctx.cu_seqlens), ptr(ctx.slot_ids), ctx.B)
+    check(fn("state_chunks", "cellm_hgrn2_chunks")(*where, n_chunks, least, heads, dim, vd, ptr(ws), ptr(ctx.err), stream_of(proj)),
+          "hgrn2_chunks")
+    count_launch()
+    if rest:
+        check(fn(_LIB, "cellm_hgrn2_walk")(*where, heads, dim, vd, least - 1, ptr(ctx.err), stream_of(proj)), "hgrn2_walk")
     return o
 
 
@@ -227,14 +261,24 @@ def delta_prep(proj: torch.Tensor, col0: int, col_b: int, taps, n_taps: int, con
     return qk, v, beta, decay
 
 
-def delta_scan(qk, v, beta, decay, state: torch.Tensor, ctx, heads: int, kvh: int, dim: int, vd: int) -> torch.Tensor:
+def delta_scan(qk, v, beta, decay, state: torch.Tensor, ctx, heads: int, kvh: int, dim: int, vd: int, chunked: bool = False) -> torch.Tensor:
     """The gated delta rule over every request's tokens of the step; state [slots, heads, dim, vd] float32 is moved on.
-    Returns S^T q per token and head, float32 [T, heads * vd]."""
+    Returns S^T q per token and head, float32 [T, heads * vd]. `chunked` as in hgrn2_scan,
+    from DELTA_CHUNKS_FROM tokens on."""
     _f32(qk, v, beta, decay, state)
     o = torch.empty((ctx.T, heads * vd), dtype=torch.float32, device=qk.device)
-    check(fn(_LIB, "cellm_delta_scan")(ptr(o), ptr(state), state.stride(0), state.shape[0], ptr(qk), ptr(v), ptr(beta), ptr(decay),
-                                       ptr(ctx.cu_seqlens), ptr(ctx.slot_ids), ctx.B, heads, kvh, dim, vd, ptr(ctx.err), stream_of(qk)),
-          "delta_scan")
+    where = (ptr(o), ptr(state), state.stride(0), state.shape[0], ptr(qk), ptr(v), ptr(beta), ptr(decay), ptr(ctx.cu_seqlens),
+             ptr(ctx.slot_ids), ctx.B)
+    chunks = _state_chunks(ctx, True, heads, dim, vd, qk.device) if chunked else None
+    if chunks is None:
+        check(fn(_LIB, "cellm_delta_scan")(*where, heads, kvh, dim, vd, ptr(ctx.err), stream_of(qk)), "delta_scan")
+        return o
+    ws, n_chunks, least, rest = chunks
+    check(fn("state_chunks", "cellm_delta_chunks")(*where, n_chunks, least, heads, kvh, dim, vd, ptr(ws), ptr(ctx.err), stream_of(qk)),
+          "delta_chunks")
+    count_launch()
+    if rest:
+        check(fn(_LIB, "cellm_delta_walk")(*where, heads, kvh, dim, vd, least - 1, ptr(ctx.err), stream_of(qk)), "delta_walk")
     return o
 
 

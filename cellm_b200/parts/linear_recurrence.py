@@ -90,7 +90,8 @@ class Hgrn2Mixer(Mixer):
         state = bindings_of(cache, 1)[0].state
         hd = self.heads * self.dim
         proj = self.in_proj(x, out_dtype=torch.float32)
-        o = ops.hgrn2_scan(proj, 0, hd, 2 * hd, self.f_bias, self.lower, state, ctx, self.heads, self.dim, self.vd)
+        o = ops.hgrn2_scan(proj, 0, hd, 2 * hd, self.f_bias, self.lower, state, ctx, self.heads, self.dim, self.vd,
+                           chunked=self.dtype == torch.bfloat16)
         y = ops.head_norm_gate(o, self.norm_w, None, self.heads, self.vd, self.eps, self.dtype)
         return self.out_proj(y, out_dtype=torch.float32 if self.out32 else None)
 
@@ -164,7 +165,7 @@ class GatedDeltaMixer(Mixer):
                                             self.heads, self.qkh, self.dim, self.vd, self.unit_eps)
         if conv_state is not None:
             ops.conv_state_update(conv_state, proj, 0, None, self.taps, ctx)
-        o = ops.delta_scan(qk, v, beta, decay, state, ctx, self.heads, self.qkh, self.dim, self.vd)
+        o = ops.delta_scan(qk, v, beta, decay, state, ctx, self.heads, self.qkh, self.dim, self.vd, chunked=self.dtype == torch.bfloat16)
         y = ops.head_norm_gate(o, self.norm_w, gate, self.heads, self.vd, self.eps, self.dtype)
         return self.out_proj(y)
 

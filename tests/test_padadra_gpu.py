@@ -465,6 +465,80 @@ def test_delta_rule_alone(heads, kvh, dim, vd):
         assert torch.equal(outs["whole"][b], outs["portions"][b])
 
 
+def state_walk_in_64_bits(kind, d, S, heads, dim, vd):
+    """Read-outs [n, heads * vd] and the state behind the last token, from the state S."""
+    n, out = d["v"].shape[0], []
+    rows = lambda x: x.double().reshape(n, -1, dim).repeat_interleave(heads // (x.shape[1] // dim), dim=1)
+    q, g, v = rows(d["q"]), rows(d["g"]), d["v"].double().reshape(n, heads, vd)
+    for t in range(n):
+        S = g[t][:, :, None] * S
+        if kind == "delta":
+            k = rows(d["k"])[t]
+            S = S + k[:, :, None] * (d["beta"][t].double()[:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k)))[:, None, :]
+        else:
+            S = S + (1 - g[t])[:, :, None] * v[t][:, None, :]
+        out.append(torch.einsum("hdv,hd->hv", S, q[t]).reshape(-1))
+    return torch.stack(out), S
+
+
+@pytest.mark.parametrize("kind", ["delta", "hgrn2"])
+@pytest.mark.parametrize("heads,kvh,dim,vd,decays", [(2, 1, 128, 128, "mixed"), (2, 2, 64, 128, "strong"), (3, 1, 100, 17, "weak"), (4, 2, 5, 3, "mixed"),
+                                                     (1, 1, 65, 16, "strong"), (2, 1, 33, 40, "weak"), (2, 1, 136, 12, "mixed")])
+def test_recurrences_in_chunks(kind, heads, kvh, dim, vd, decays):
+    """Portions around the chunk's and the rule's edges (a chunk of one token, whole chunks, short portions beside them that
+    are walked token by token), from states that are not zero, in slots of any order; decays near 0, near 1 (keys that
+    repeat, so that T is far from the unit matrix) and mixed. Against 64 bits with the walk's bound, and no further off than
+    twice the walk. Heads of more than 128 rows are walked whatever is asked."""
+    from cellm_b200 import ops
+    from cellm_b200.ops.recurrent import DELTA_CHUNKS_FROM, HGRN2_CHUNKS_FROM
+    F = DELTA_CHUNKS_FROM if kind == "delta" else HGRN2_CHUNKS_FROM
+    g = torch.Generator().manual_seed(dim * 10 + vd)
+    lens, slots = [F, 7, F + 1, F + 15, 3 * F + 16, 1, F - 1], [5, 0, 3, 6, 1, 2, 7]
+    kvh = kvh if kind == "delta" else heads
+    unit = lambda n: torch.nn.functional.normalize(torch.randn(n, kvh, dim, generator=g), dim=-1).reshape(n, -1)
+    low, high = {"mixed": (0.0, 1.0), "strong": (0.0, 1e-3), "weak": (0.999, 1.0)}[decays]
+    data = [dict(q=unit(n), k=unit(n), v=torch.randn(n, heads * vd, generator=g), beta=torch.rand(n, heads, generator=g),
+                 g=low + (high - low) * torch.rand(n, heads * dim, generator=g)) for n in lens]
+    for d in data:
+        if decays == "weak":
+            d["k"][1::2] = d["k"][:1]           # the same key again and again
+    S0 = torch.randn(8, heads, dim, vd, generator=g)
+    want = [state_walk_in_64_bits(kind, d, S0[s].double(), heads, dim, vd) for d, s in zip(data, slots)]
+    ctx = step_ctx(lens, [0] * len(lens), slots)
+    whole = lambda key: torch.cat([d[key] for d in data]).to(DEV).contiguous()
+    errors = {}
+    for chunked in (False, True):
+        state = S0.to(DEV).clone()
+        if kind == "delta":
+            qk = torch.cat([whole("q"), whole("k")], dim=1).contiguous()
+            o = ops.delta_scan(qk, whole("v"), whole("beta"), whole("g"), state, ctx, heads, kvh, dim, vd, chunked=chunked)
+        else:
+            # the gates are formed from pre-activations: silu's and the sigmoid's inverses are not exact in 32 bits, so the
+            # oracle's inputs are what the gates' own kernel left
+            f = whole("g")
+            proj = torch.cat([whole("q") * 3, torch.logit(f.double().clamp(1e-6, 1 - 1e-6)).float(), whole("v")], dim=1).contiguous()
+            zero = torch.zeros(heads * dim, device=DEV)
+            o = ops.hgrn2_scan(proj, 0, heads * dim, 2 * heads * dim, zero, zero, state, ctx, heads, dim, vd, chunked=chunked)
+            at = 0
+            for i, (d, s) in enumerate(zip(data, slots)):
+                n = lens[i]
+                rows = proj[at:at + n].cpu()
+                at += n
+                d = dict(q=rows[:, :heads * dim], g=rows[:, heads * dim:2 * heads * dim], v=rows[:, 2 * heads * dim:])
+                want[i] = state_walk_in_64_bits(kind, d, S0[s].double(), heads, dim, vd)
+        assert int(ctx.err.item()) == 0
+        assert torch.equal(state[4].cpu(), S0[4])               # nobody's slot
+        at, off = 0, 0.0
+        for n, s, (out, S) in zip(lens, slots, want):
+            got, moved = o[at:at + n].cpu().double(), state[s].cpu().double()
+            torch.testing.assert_close(got, out, rtol=2e-5, atol=2e-5 * float(out.abs().max()))
+            torch.testing.assert_close(moved, S, rtol=2e-5, atol=2e-5 * float(S.abs().max()))
+            off = max(off, float((got - out).norm() / out.norm()), float((moved - S).norm() / S.norm()))
+            at += n
+        errors[chunked] = off
+    assert errors[True] <= 2 * errors[False] + 2.0 ** -23, errors
+
+
 def test_delta_rule_inputs_and_the_convolutions_state():
     """Convolution + silu, unit vectors, beta and decays from the projections, with the convolution's last inputs carried
     from portion to portion (a portion shorter than the taps included)."""
