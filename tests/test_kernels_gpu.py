@@ -419,6 +419,30 @@ def test_attention_plain(dtype, nh, nkv, hd, ps, window):
     close(out, attention_reference(c, nh, nkv, hd, hd ** -0.5, window), dtype)
 
 
+@pytest.mark.parametrize("nh,nkv,hd,ps", [(24, 8, 64, 16), (4, 4, 128, 8), (32, 1, 64, 4), (33, 1, 32, 16), (6, 2, 100, 16), (3, 1, 4, 1), (8, 2, 18, 8)])
+@pytest.mark.parametrize("window", [0, 70])
+def test_attention_in_32_bits_does_not_depend_on_the_cutting(nh, nkv, hd, ps, window):
+    """Portions that share a block with another request's, contexts that end inside a block of keys, single tokens; more
+    heads a group than a block has rows, and widths of no whole 16 bytes (both on the kernel of one block a row). Against
+    the oracle, and bit for bit against the same tokens one at a time; then with infinities in the keys and values behind
+    a token, which it must not feel."""
+    from cellm_b200 import ops
+    lens, ctxs = [37, 1, 70, 2], [0, 200, 61, 64]
+    c = paged_case(lens, ctxs, nh, nkv, hd, ps, torch.float32, seed=11)
+    e = err_word()
+    run = lambda q, pos, seq: ops.attention_plain(q, c["kp"], c["vp"], pos, seq, c["bt"], nh, hd ** -0.5, window, e)
+    out = run(c["q"], c["pos"], c["seq"])
+    close(out, attention_reference(c, nh, nkv, hd, hd ** -0.5, window), torch.float32)
+    for t in range(0, out.shape[0], 3):
+        assert torch.equal(run(c["q"][t:t + 1].contiguous(), c["pos"][t:t + 1], c["seq"][t:t + 1]), out[t:t + 1]), t
+    last = int(c["pos"][36])
+    for pool in (c["kp"], c["vp"]):
+        pool[int(c["bt"][0, last // ps]), :, last % ps] = float("inf")
+    again = run(c["q"], c["pos"], c["seq"])
+    assert torch.equal(again[:36], out[:36]) and not bool(torch.isfinite(again[36]).all()) and torch.equal(again[37:], out[37:])
+    assert e.item() == 0
+
+
 @pytest.mark.parametrize("kernel", ["plain32", "plain16", "flash", "decode", "tc"])
 def test_a_far_key_among_hundreds_is_found(kernel):
     """One early key is scaled so that its score towers over 600 others: the
@@ -603,6 +627,20 @@ def test_gemm_plain(dtype, out, M, N, K):
     close(ops.gemm_plain(a, w, out), a.double() @ w.double().T, out)
     big = torch.randn(M, K + 3, device=DEV).to(dtype)
     close(ops.gemm_plain(big[:, :K], w, out), big[:, :K].double() @ w.double().T, out, "strided rows")
+
+
+@pytest.mark.parametrize("M,N,K", [(213, 2560, 1536), (300, 33, 257), (65, 700, 2304), (40, 31, 8200), (17, 129, 256), (9, 96, 63)])
+def test_gemm_plain_in_32_bits_does_not_depend_on_the_tile(M, N, K):
+    """Sums of one run of products and of several, more runs than a block forms at once, runs and tiles that end early, rows
+    that start on no 16-byte border: a row alone, in another tile, is the same bit for bit."""
+    from cellm_b200 import ops
+    a, w = torch.randn(M, K + 1, device=DEV), torch.randn(N, K, device=DEV)
+    for rows in (a[:, :K], a[:, :K].contiguous()):
+        out = ops.gemm_plain(rows, w, torch.float32)
+        close(out, rows.double() @ w.double().T, torch.float32)
+        for m in (0, M // 2, M - 1):
+            assert torch.equal(ops.gemm_plain(rows[m:m + 1], w, torch.float32), out[m:m + 1])
+        assert torch.equal(ops.gemm_plain(rows[:min(M, 70)], w[:min(N, 40)], torch.float32), out[:min(M, 70), :min(N, 40)])
 
 
 @pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
