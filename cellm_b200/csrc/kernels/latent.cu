@@ -237,6 +237,7 @@ head_product_kernel(TA* __restrict__ out, long long ldo, long long out_hs, const
 // and add their sums by three shuffles. K (a multiple of 64) is summed in the same order for every token count up to
 // HP_SMALL_T.
 #define HP_SMALL_T 16
+#define HP_SMALL_AHEAD 8        // pieces of a row asked for ahead: all of K up to 512
 __global__ void __launch_bounds__(128)
 head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long long out_hs, const __nv_bfloat16* __restrict__ in,
                           long long ldi, long long in_hs, const __nv_bfloat16* __restrict__ w, int T, int N, int K, int vec_in) {
@@ -246,6 +247,11 @@ head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long l
     const int n = blockIdx.x * 16 + (threadIdx.x >> 3), kq = threadIdx.x & 7;
     const bool on = n < N;
     const __nv_bfloat16* wr = w + ((size_t)h * N + (on ? n : 0)) * K;
+    // the matrices are not the work of the kernel before this one: a row's first pieces are asked for before the wait on it
+    uint4 wq[HP_SMALL_AHEAD];
+#pragma unroll
+    for (int i = 0; i < HP_SMALL_AHEAD; ++i)
+        if (kq * 8 + i * 64 < K) wq[i] = *reinterpret_cast<const uint4*>(wr + kq * 8 + i * 64);
     pdl_wait();
     if (vec_in) {                        // the inputs' rows start on 16-byte borders: eight values a load
         const int K8 = K / 8;
@@ -263,10 +269,8 @@ head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long l
     float acc[HP_SMALL_T];
 #pragma unroll
     for (int t = 0; t < HP_SMALL_T; ++t) acc[t] = 0.f;
-#pragma unroll 2
-    for (int k0 = kq * 8; k0 < K; k0 += 64) {
-        const uint4 wq = *reinterpret_cast<const uint4*>(wr + k0);
-        const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wq);
+    auto piece = [&](const uint4& w8, int k0) {
+        const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&w8);
         float wv[8];
 #pragma unroll
         for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(wp[j]); wv[2 * j] = f.x; wv[2 * j + 1] = f.y; }
@@ -283,7 +287,11 @@ head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long l
                 }
             }
         }
-    }
+    };
+#pragma unroll
+    for (int i = 0; i < HP_SMALL_AHEAD; ++i)
+        if (kq * 8 + i * 64 < K) piece(wq[i], kq * 8 + i * 64);
+    for (int k0 = kq * 8 + HP_SMALL_AHEAD * 64; k0 < K; k0 += 64) piece(*reinterpret_cast<const uint4*>(wr + k0), k0);
 #pragma unroll
     for (int t = 0; t < HP_SMALL_T; ++t) {
         if (t < T) {

@@ -594,6 +594,41 @@ def test_latent_kernel_with_gates_and_sinks(nh, kw, dv, page, window):
     assert int(ctx.err.item()) == 0
 
 
+@pytest.mark.parametrize("nh,kw,dv", [(16, 576, 512), (12, 512, 512), (1, 144, 128), (17, 272, 256), (40, 400, 384), (3, 528, 512)])
+@pytest.mark.parametrize("window", [0, 1, 70])
+def test_latent_attention_of_single_tokens(nh, kw, dv, window):
+    """A token a request, in tiles of 16 heads (fewer, and more than one tile): contexts of nothing, around the edges of a block
+    of 64 rows, of more blocks than two stages; whole and in more pieces than there are blocks; a step in which one request has
+    two tokens and another none. Sinks and gates. Against 64-bit torch over the same rounded inputs, bounded as the other forms."""
+    from cellm_b200 import ops
+    page = 16
+    for q_lens, ctx_lens in (([1] * 6, [0, 62, 63, 64, 200, 500]), ([2, 0, 1], [63, 5, 130])):
+        g = torch.Generator().manual_seed(nh * kw + window)
+        T = sum(q_lens)
+        cache, table = paged([c + n for c, n in zip(ctx_lens, q_lens)], kw, page, torch.bfloat16, g)
+        pool = (torch.randn(cache.k.shape, generator=g) * 0.7).to(torch.bfloat16)
+        q = (torch.randn(T, nh * kw, generator=g) * 0.7).to(torch.bfloat16)
+        gate, sinks = torch.randn(T, nh, generator=g) * 3, torch.linspace(-3.0, 4.0, nh)
+        scale, want, t = 1.7 * kw ** -0.5, torch.zeros(T, nh, dv, dtype=torch.float64), 0
+        for b, n in enumerate(q_lens):
+            rows = torch.stack([pool[table[b, j // page], 0, j % page] for j in range(ctx_lens[b] + n)]).double()
+            for i in range(n):
+                hi = ctx_lens[b] + i + 1
+                lo = max(0, hi - window) if window else 0
+                s = (q[t].double().reshape(nh, kw) @ rows[lo:hi].T) * scale
+                top = torch.maximum(s.amax(-1), sinks.double())[:, None]
+                e = torch.exp(s - top)
+                want[t] = (e / (e.sum(-1, keepdim=True) + torch.exp(sinks.double()[:, None] - top))) @ rows[lo:hi, :dv]
+                t += 1
+        want = want * torch.sigmoid(gate.double())[:, :, None]
+        ctx = step_ctx(q_lens, ctx_lens)
+        for nsplit in (1, 3, 8):
+            out = ops.attention_latent(q.to(DEV), pool.to(DEV), ctx.cu_seqlens, ctx.ctx_lens, cache.block_table, q_lens, nh, dv, scale, nsplit,
+                                       ctx.err, window, sinks.to(DEV), gate.to(DEV))
+            torch.testing.assert_close(out.cpu().double().reshape(T, nh, dv), want, rtol=2e-2, atol=1e-2)
+        assert int(ctx.err.item()) == 0
+
+
 EXPANDED = [  # heads, dim, rot_dim, vdim, rank
     (4, 128, 64, 128, 512), (2, 64, 0, 64, 64), (3, 16, 16, 16, 24), (2, 48, 32, 80, 40), (1, 96, 64, 112, 128), (2, 192, 64, 128, 64), (5, 32, 0, 32, 96),
     (2, 128, 0, 48, 72), (1, 64, 96, 96, 16),
