@@ -501,3 +501,52 @@ def test_command_lines_take_the_design(models, tmp_path):
     got = traces.collect(steps, outs)
     for rid, toks in reqs.items():
         check_close(traces.as_matrix(got[rid], len(toks)), ref[rid], "float32", f"trace_run {rid}")
+
+
+@pytest.mark.parametrize("T,E,top,H", [(17, 64, 6, 264), (341, 3, 3, 64), (1025, 70, 5, 72), (2, 1, 1, 2056), (700, 40, 9, 66)])
+def test_sort_and_sum_of_the_experts_slots(T, E, top, H):
+    """Slots that are no multiple of a warp's stretch, experts without a slot and with every slot, choices that are none; sums of
+    one to nine rows, of widths that are taken eight columns a thread and two. The order of the sorted rows is the slots' own."""
+    import ctypes
+    from cellm_b200.csrc import build
+    lib, P = build.load("kernels_common"), ctypes.c_void_p
+    g = torch.Generator().manual_seed(T)
+    S = T * top
+    idx = torch.randint(0, E, (S,), generator=g, dtype=torch.int32)
+    idx[idx == 2] = 1                       # an expert that nobody chose
+    if T == 341:
+        idx[:] = 1
+    if T == 1025:
+        idx[7] = -1                         # no expert
+    rows = -(-(S + min(E, S) * 127) // 128) * 128
+    tiles = rows // 128
+    dev = lambda t: t.to(DEV).contiguous()
+    row_slot, slot_row, group = (torch.full((n,), -7, dtype=torch.int32, device=DEV) for n in (rows, S, tiles))
+    idx_d, stream = dev(idx), P(torch.cuda.current_stream().cuda_stream)
+    ptr = lambda t: P(t.data_ptr()) if t is not None else P(None)
+    assert lib.cellm_moe_sort(ptr(row_slot), ptr(slot_row), ptr(group), ptr(idx_d), S, E, tiles, stream) == 0
+    at, order, groups = 0, {}, []
+    for e in range(E):
+        mine = (idx == e).nonzero()[:, 0].tolist()
+        for i, slot in enumerate(mine):
+            order[at + i] = slot
+        n = -(-len(mine) // 128)
+        groups += [e] * n
+        at += n * 128
+    assert group.cpu().tolist() == groups + [-1] * (tiles - len(groups))
+    got = row_slot.cpu().tolist()
+    assert all(got[r] == order.get(r, -1) for r in range(at))
+    back = slot_row.cpu().tolist()
+    assert all(back[slot] == r for r, slot in order.items())
+    if T == 1025:
+        slot_row[7] = 0
+    Y, wts, shared, gate = (torch.randn(*s, generator=g) for s in ((rows, H), (T, top), (T, H), (T,)))
+    Y = Y.to(torch.bfloat16)
+    sums = (wts.double()[:, :, None] * Y.double()[slot_row.cpu().long()].reshape(T, top, H)).sum(1)
+    Yd, wd, sd, gd = dev(Y), dev(wts), dev(shared), dev(gate)
+    for sh, ga, want in ((None, None, sums), (sd, None, sums + shared.double()), (sd, gd, sums + gate.double()[:, None] * shared.double())):
+        for name, dtype, tol in (("cellm_moe_combine", torch.bfloat16, 2.0 ** -8), ("cellm_moe_combine32", torch.float32, 0.0)):
+            out = torch.empty(T, H, dtype=dtype, device=DEV)
+            assert getattr(lib, name)(ptr(out), ptr(Yd), ptr(slot_row), ptr(wd), ptr(sh), ptr(ga), T, H, top, stream) == 0
+            bound = tol * want.abs() + 1e-6 * (top + 1) * 4          # rounding of the result, and of top + 1 terms of a few units
+            assert bool(((out.cpu().double() - want).abs() <= bound).all())
