@@ -811,7 +811,10 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
 #pragma unroll
                             for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_xielu(__uint_as_float(r[i]), ap, aq));
                         }
-                    } else if (act >= 0) {
+                    } else if (act == 0) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_gelu_flat(__uint_as_float(r[i])));
+                    } else if (act > 0) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_activate(__uint_as_float(r[i]), act));
                     }

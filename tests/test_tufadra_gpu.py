@@ -550,3 +550,24 @@ def test_sort_and_sum_of_the_experts_slots(T, E, top, H):
             assert getattr(lib, name)(ptr(out), ptr(Yd), ptr(slot_row), ptr(wd), ptr(sh), ptr(ga), T, H, top, stream) == 0
             bound = tol * want.abs() + 1e-6 * (top + 1) * 4          # rounding of the result, and of top + 1 terms of a few units
             assert bool(((out.cpu().double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("rows,cols", [(17, 8), (128, 256), (300, 520)])
+def test_gelu_in_the_products_epilogue(rows, cols):
+    """The product with a diagonal matrix leaves the operand itself for the activation: both sides of the places where its two
+    forms meet (|z| = sqrt 2), far out, zeros, infinities and no number; within half a unit of the 16-bit result's last place
+    (8 significant bits: at most 2^-8 of the value) and the 32-bit form's 1e-6 (4.5e-7 over [-8, 8], where a result is not
+    the operand itself or nothing)."""
+    from cellm_b200 import ops
+    g = torch.Generator().manual_seed(rows)
+    k = -(-cols // 8) * 8
+    z = (torch.randn(rows, k, generator=g) * torch.logspace(-3, 1.2, k)[None]).to(torch.bfloat16)
+    z[0, :6] = torch.tensor([0.0, 1.4140625, -1.4140625, 1.421875, -1.421875, -30.0])
+    want = torch.nn.functional.gelu(z.double())[:, :cols]
+    for out_dtype, unit in ((torch.bfloat16, 2.0 ** -8), (torch.float32, 2.0 ** -23)):
+        got = ops.gemm_act(z.to(DEV), torch.eye(k, dtype=torch.bfloat16, device=DEV)[:cols].contiguous(), "gelu", out_dtype).cpu().double()
+        assert bool(((got - want).abs() <= unit * want.abs() + 1e-6).all())
+    for v in (float("inf"), float("nan")):          # 0 times either is no number, and stays none
+        a = torch.full((17, 8), v, dtype=torch.bfloat16, device=DEV)
+        got = ops.gemm_act(a, torch.zeros(8, 8, dtype=torch.bfloat16, device=DEV), "gelu", torch.float32)
+        assert tuple(got.shape) == (17, 8) and bool(torch.isnan(got).all())
