@@ -20,8 +20,8 @@ sink_attn_prep_kernel(TA* __restrict__ q_out, TA* __restrict__ k_pool, TA* __res
                       const int* __restrict__ positions, const int* __restrict__ seq_of_token,
                       const int* __restrict__ cu_seqlens, const int* __restrict__ slot_ids,
                       const int* __restrict__ block_table, int bt_stride, int num_pages, int page_size,
-                      int nh, int nkv, int hd, int vd, const float* __restrict__ q_mult, int* __restrict__ err) {
-    extern __shared__ float sm[];
+                      int nh, int nkv, int hd, int vd, const float* __restrict__ q_mult, int fours, int* __restrict__ err) {
+    extern __shared__ __align__(16) float sm[];
     const int Cq = nh * hd, Ck = nkv * hd, Cv = nkv * vd, C = Cq + Ck + Cv;
     float* buf = sm;                       // [C]
     float* cq = buf + C;                   // [rot/2] cos, then [rot/2] sin
@@ -44,7 +44,12 @@ sink_attn_prep_kernel(TA* __restrict__ q_out, TA* __restrict__ k_pool, TA* __res
     const bool page_ok = page >= 0 && page < num_pages;
     if (!page_ok && threadIdx.x == 0) atomicOr(err, CELLM_DEV_BAD_PAGE);
     pdl_wait();
-    for (int c = threadIdx.x; c < C; c += blockDim.x) buf[c] = conv_taps_at(cv, t, start, c);
+    // (four channels a thread where the rows lie on 16-byte borders: 2,560 channels of four taps are 27 loads a thread of 256
+    // instead of 90; two prompts of about 700 tokens through both mixers side by side went from 315 to 294 us with it)
+    if (fours)
+        for (int c = threadIdx.x * 4; c < C; c += blockDim.x * 4) *reinterpret_cast<float4*>(buf + c) = conv_taps_four(cv, t, start, c);
+    else
+        for (int c = threadIdx.x; c < C; c += blockDim.x) buf[c] = conv_taps_at(cv, t, start, c);
     __syncthreads();
     if (q_norm_w) {
         float s1 = 0.f, s2 = 0.f;
@@ -116,6 +121,7 @@ CELLM_API int cellm_sink_attn_prep(void* q_out, void* k_pool, void* v_pool, cons
     // few tokens: a thread about four channels, since a step of single tokens is too few blocks to hide a thread's chain
     // of loads behind other blocks (the sums of squares are then added in another order: a rounding apart)
     const int threads = T >= 512 ? 256 : cv.C >= 4096 ? 1024 : cv.C >= 2048 ? 512 : 256;
+    const int fours = conv_taps_in_fours(cv, state, slot_stride);
 #define PREP_RUN(TA)                                                                                                          \
     do {                                                                                                                      \
         if (smem > 48 * 1024) {                                                                                               \
@@ -124,7 +130,7 @@ CELLM_API int cellm_sink_attn_prep(void* q_out, void* k_pool, void* v_pool, cons
         }                                                                                                                     \
         CELLM_RUN(sink_attn_prep_kernel<TA>, T, threads, smem, stream, (TA*)q_out, (TA*)k_pool, (TA*)v_pool, cv, state, slot_stride, \
                   n_slots, q_norm_w, k_norm_w, eps, qk_freq, rot, v_freq, interleaved, positions, seq_of_token, cu_seqlens, \
-                  slot_ids, block_table, bt_stride, num_pages, page_size, nh, nkv, hd, vd, q_mult, err);                             \
+                  slot_ids, block_table, bt_stride, num_pages, page_size, nh, nkv, hd, vd, q_mult, fours, err);                             \
     } while (0)
     if (dtype == CELLM_F32) PREP_RUN(float);
     else if (dtype == CELLM_BF16) PREP_RUN(__nv_bfloat16);

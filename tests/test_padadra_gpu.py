@@ -572,6 +572,34 @@ def test_delta_rule_inputs_and_the_convolutions_state():
     assert float(state[0].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("taps,bias", [(4, True), (3, False), (0, True)])
+def test_attention_preparation_in_fours_and_one_by_one(taps, bias):
+    """Rows that start on no 16-byte border take the channels one by one: the same values bit for bit."""
+    from cellm_b200 import ops
+    from cellm_b200.parts import CacheBinding
+    from cellm_b200.parts.rope import split_inv_freq
+    nh, nkv, hd = 6, 2, 64
+    lens = [37, 1, 2, 20]
+    g = torch.Generator().manual_seed(taps)
+    T, C = sum(lens), (nh + 2 * nkv) * hd
+    rnd = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    proj = rnd(T, C + 3)
+    b, w, state = rnd(C) if bias else None, rnd(C, taps) if taps else None, rnd(len(lens), taps - 1, C) if taps > 1 else None
+    norms, freq = (rnd(nh * hd), rnd(nkv * hd)), split_inv_freq(1e4, hd).to(DEV)
+    ctx, got = step_ctx(lens, [0] * len(lens), list(range(len(lens)))), []
+    pages = -(-max(lens) // 8)
+    table = torch.arange(pages * len(lens), dtype=torch.int32, device=DEV).reshape(len(lens), pages)
+    for rows, col in ((proj[:, 1:], 0), (proj, 1), (torch.cat([proj[:, 1:C + 1], proj[:, :4]], 1).contiguous(), 0)):
+        pool = lambda: torch.zeros(pages * len(lens), nkv, 8, hd, dtype=torch.bfloat16, device=DEV)
+        cache = CacheBinding(k=pool(), v=pool(), block_table=table, page_size=8, num_pages=pages * len(lens))
+        q = ops.sink_attn_prep(rows, col, b, w, taps, state, *norms, 1e-5, freq, hd, freq, True, ctx, cache, nh, nkv, hd, hd, torch.bfloat16)
+        got.append((q, cache.k, cache.v))
+    for other in got[:2]:
+        for x, y in zip(other, got[2]):
+            assert torch.equal(x, y)
+    assert int(ctx.err.item()) == 0
+
+
 def test_pair_hash_embedding_and_the_first_token():
     from cellm_b200 import ops
     V, H, buckets, mp, mc = 50, 24, 13, 31, 5
