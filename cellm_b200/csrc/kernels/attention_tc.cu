@@ -79,7 +79,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const int* __restrict__ cu_seqlens, const int* __restrict__ ctx_lens,
                     const int* __restrict__ block_table, int bt_stride, int B, int num_pages, int page_size, int nh,
                     int nkv, float scale_log2e, int window, const float* __restrict__ sinks, const float* __restrict__ gate,
-                    long long gate_ld, int chunk, int* __restrict__ err) {
+                    long long gate_ld, int chunk, int nsplit, float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     TcSmem& sm = *reinterpret_cast<TcSmem*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -152,6 +152,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // tile 1 holds later tokens: its blocks start and end no earlier than tile 0's
         kb0 = tr[0].lo;
         nblk = (tr[1].has ? tr[1].hi : tr[0].hi) - kb0;
+        if (nsplit > 1) {           // this piece of the pair's key blocks; a tile may have none in it
+            const int per = (nblk + nsplit - 1) / nsplit;
+            kb0 += (int)blockIdx.z * per;
+            nblk = max(0, min(per, nblk - (int)blockIdx.z * per));
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                tr[t].lo = max(tr[t].lo, kb0);
+                tr[t].hi = max(tr[t].lo, min(tr[t].hi, kb0 + nblk));
+            }
+        }
     }
     const int* bt = block_table + (size_t)(live ? b : 0) * bt_stride;
     const int pages_per_block = TN / page_size;
@@ -344,6 +354,22 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             // a sink: one more term exp(sink_h) in the row's denominator, against the maximum the row's sums were formed
             // with; an output gate: the row times the sigmoid of one number per (token, head)
             const int head = kvh * G + r % G;
+            if (nsplit > 1) {       // the piece's maximum, sum and unnormalised output (none where it had no block)
+                const size_t row = ((size_t)blockIdx.z * cu_seqlens[B] + t_base + tok) * nh + head;
+                if (row_ok) *reinterpret_cast<float2*>(part_ml + row * 2) = make_float2(n_blocks > 0 ? m : -INFINITY, l);
+#pragma unroll 1
+                for (int c = 0; c < (n_blocks > 0 ? HD / 32 : 0); ++c) {
+                    uint32_t o[32];
+                    tmem_ld32(lane_base + o_col + (uint32_t)(c * 32), o);
+                    if (row_ok) {
+                        float4* dst = reinterpret_cast<float4*>(part_o + row * HD + c * 32);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            dst[i] = make_float4(__uint_as_float(o[4 * i]), __uint_as_float(o[4 * i + 1]), __uint_as_float(o[4 * i + 2]),
+                                                 __uint_as_float(o[4 * i + 3]));
+                    }
+                }
+            } else {
             if (sinks && row_ok) l += exp2f(sinks[head] * 1.4426950408889634f - (m == -INFINITY ? 0.f : m));
             float inv = l > 0.f ? 1.0f / l : 0.f;
             if (gate && row_ok) inv *= 1.f / (1.f + __expf(-gate[(size_t)(t_base + tok) * gate_ld + head]));
@@ -363,11 +389,36 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     }
                 }
             }
+            }
         }
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, TMEM_TN);
+}
+
+// The pieces of a row merged in their order: out = sum_s 2^(m_s - M) o_s / sum_s 2^(m_s - M) l_s. 16 threads a row.
+__global__ void __launch_bounds__(256)
+attention_tc_merge_kernel(__nv_bfloat16* __restrict__ out, const float* part_o, const float* part_ml, long long rows, int nsplit) {
+    pdl_trigger();
+    pdl_wait();
+    const long long r = (long long)blockIdx.x * 16 + (threadIdx.x >> 4);
+    const int c = (threadIdx.x & 15) * 4;
+    if (r >= rows) return;
+    float M = -INFINITY;
+    for (int s = 0; s < nsplit; ++s) M = fmaxf(M, part_ml[(s * rows + r) * 2]);
+    float L = 0.f;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < nsplit; ++s) {
+        const float2 ml = *reinterpret_cast<const float2*>(part_ml + (s * rows + r) * 2);
+        if (ml.x == -INFINITY) continue;            // (its output was never written)
+        const float w = fast_exp2(ml.x - M);
+        const float4 o = *reinterpret_cast<const float4*>(part_o + (s * rows + r) * HD + c);
+        L = fmaf(w, ml.y, L);
+        a.x = fmaf(w, o.x, a.x), a.y = fmaf(w, o.y, a.y), a.z = fmaf(w, o.z, a.z), a.w = fmaf(w, o.w, a.w);
+    }
+    const float inv = L > 0.f ? 1.f / L : 0.f;
+    *reinterpret_cast<uint2*>(out + r * HD + c) = make_uint2(pack_bf16(a.x * inv, a.y * inv), pack_bf16(a.z * inv, a.w * inv));
 }
 
 // ---------------------------------------------------------------- host side
@@ -408,7 +459,7 @@ static int attention_tc_impl(void* out, const void* q, const void* k_pool, const
                              const int* cu_seqlens, const int* ctx_lens, const int* block_table, int bt_stride,
                              int B, int T, int n_tiles, int num_pages, int page_size, int nh, int nkv, int hd,
                              float scale, int window, const float* sinks, const float* gate, long long gate_ld, int* err,
-                             cudaStream_t stream, int chunk = 0, int uneven = 0) {
+                             cudaStream_t stream, int chunk = 0, int uneven = 0, int nsplit = 1, float* part_o = nullptr, float* part_ml = nullptr) {
     if (T <= 0 || n_tiles <= 0) return CELLM_OK;
     if (!attention_tc_takes(hd, nh, nkv, page_size, uneven) || scale <= 0.f) return CELLM_ERR_SIZE;
     if (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out) & 15) return CELLM_ERR_ALIGN;
@@ -433,10 +484,16 @@ static int attention_tc_impl(void* out, const void* q, const void* k_pool, const
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    dim3 grid((unsigned)n_tiles, (unsigned)nkv);
+    if (nsplit > 1 && (!part_o || !part_ml || sinks || gate)) return CELLM_ERR_ARG;
+    if (nsplit < 1 || nsplit > 64) return CELLM_ERR_SIZE;
+    if (nsplit > 1 && ((((uintptr_t)part_o) & 15) || (((uintptr_t)part_ml) & 7))) return CELLM_ERR_ALIGN;
+    dim3 grid((unsigned)n_tiles, (unsigned)nkv, (unsigned)nsplit);
     CELLM_RUN(attention_tc_kernel, grid, THREADS, smem, stream, mq, mk, mv, (__nv_bfloat16*)out, cu_seqlens,
               ctx_lens, block_table, bt_stride, B, num_pages, page_size, nh, nkv, scale * 1.4426950408889634f, window, sinks,
-              gate, gate_ld, chunk, err);
+              gate, gate_ld, chunk, nsplit, part_o, part_ml, err);
+    if (nsplit > 1)
+        CELLM_RUN(attention_tc_merge_kernel, (unsigned)(((long long)T * nh + 15) / 16), 256, 0, stream, (__nv_bfloat16*)out, part_o, part_ml,
+                  (long long)T * nh, nsplit);
     return CELLM_OK;
 }
 
@@ -448,13 +505,17 @@ CELLM_API int cellm_attention_tc(void* out, const void* q, const void* k_pool, c
                              page_size, nh, nkv, hd, scale, window, nullptr, nullptr, 0, err, stream);
 }
 
-// The same for groups of heads that need not divide 128 (three quarters of a tile's rows must be in use).
-CELLM_API int cellm_attention_tc_uneven(void* out, const void* q, const void* k_pool, const void* v_pool,
-                                        const int* cu_seqlens, const int* ctx_lens, const int* block_table, int bt_stride,
-                                        int B, int T, int n_tiles, int num_pages, int page_size, int nh, int nkv, int hd,
-                                        float scale, int window, int* err, cudaStream_t stream) {
+// The same for groups of heads that need not divide 128 (three quarters of a tile's rows must be in use), and with the keys of
+// every pair of tiles in `nsplit` pieces (a CTA each) whose results meet in part_o [nsplit, T * nh, 64] and part_ml
+// [nsplit, T * nh, 2] and are merged by a second kernel: where the pairs fill the SMs' last round badly (200 CTAs of 72
+// blocks on 148 SMs are two rounds, 400 of 36 three of half the length: a layer of 24 heads over 8, 2,048 queries behind
+// 8,192 keys, 509 us whole and 442 in two pieces). The caller chooses.
+CELLM_API int cellm_attention_tc_split(void* out, float* part_o, float* part_ml, const void* q, const void* k_pool, const void* v_pool,
+                                       const int* cu_seqlens, const int* ctx_lens, const int* block_table, int bt_stride,
+                                       int B, int T, int n_tiles, int num_pages, int page_size, int nh, int nkv, int hd,
+                                       float scale, int window, int nsplit, int* err, cudaStream_t stream) {
     return attention_tc_impl(out, q, k_pool, v_pool, cu_seqlens, ctx_lens, block_table, bt_stride, B, T, n_tiles, num_pages,
-                             page_size, nh, nkv, hd, scale, window, nullptr, nullptr, 0, err, stream, 0, 1);
+                             page_size, nh, nkv, hd, scale, window, nullptr, nullptr, 0, err, stream, 0, 1, nsplit, part_o, part_ml);
 }
 
 // The same with a sink per head in every row's denominator (`sinks` [nh], 32-bit; null: none) and an output gate (`gate`

@@ -30,6 +30,8 @@ typedef int (*AttentionDecodeFn)(P out, P part_o, P part_ml, P counters, CP q, C
                                  int nsplit, P err, P stream);
 typedef int (*AttentionTcFn)(P out, CP q, CP kp, CP vp, CP cu, CP ctx, CP bt, int bt_stride, int B, int T, int n_tiles, int pages,
                              int page_size, int nh, int nkv, int hd, float scale, int window, P err, P stream);
+typedef int (*AttentionTcSplitFn)(P out, P part_o, P part_ml, CP q, CP kp, CP vp, CP cu, CP ctx, CP bt, int bt_stride, int B, int T, int n_tiles,
+                                  int pages, int page_size, int nh, int nkv, int hd, float scale, int window, int nsplit, P err, P stream);
 typedef int (*AttentionFlashFn)(P out, P part_o, P part_ml, CP q, CP kp, CP vp, CP cu, CP ctx, CP bt, int bt_stride, int B, int T,
                                 int n_tiles, int pages, int page_size, int nh, int nkv, int hd, float scale, int window, int wide,
                                 int nsplit, P err, P stream);
@@ -402,6 +404,7 @@ struct Run {
 
     void feed_forward(const SwiGLUParams& L, const void* x, void* out);
     void gated_mlp(const GatedMlpParams& L, const void* x, void* out);
+    i64 tc_pieces(i64 ctas, i64 nh, i64 window) const;
     void routed_mlp(const RoutedMlpParams& L, const void* x, void* out);
     void mingru(const MinGruParams& L, const ExecItem& it, const void* x, void* out);
     void latent_attention(const LatentAttentionParams& L, const ExecItem& it, const void* x, void* out);
@@ -646,10 +649,27 @@ void* Run::attend(const AttentionParams& L, const ExecItem& it, const void* q, v
             for (i64 b = 0; b < s.B; ++b) tc_tiles += ceil_div(s.q_lens[b], per_tile);
             const i64 min_ctas = p.tc_min_ctas < 0 ? p.sms / 8 : p.tc_min_ctas;
             if (tc_tiles * nkv >= min_ctas && (double)T >= p.tc_min_fill * (double)(tc_tiles * per_tile)) {
-                LAUNCH(fn<AttentionTcFn>(128 % G == 0 ? FN_ATTENTION_TC : FN_ATTENTION_TC_UNEVEN)(o, q, it.k, it.v, s.cu_seqlens, s.ctx_lens, it.block_table, (int)it.bt_stride,
-                                                      (int)s.B, (int)T, (int)tc_tiles, (int)it.num_pages, (int)ps, (int)nh, (int)nkv,
-                                                      (int)hd, scale, (int)L.window, s.err, s.stream),
-                   "attention_tc");
+                const i64 nsplit = tc_pieces(tc_tiles * nkv, nh, L.window);
+                if (nsplit == 1 && 128 % G == 0) {
+                    LAUNCH(fn<AttentionTcFn>(FN_ATTENTION_TC)(o, q, it.k, it.v, s.cu_seqlens, s.ctx_lens, it.block_table, (int)it.bt_stride,
+                                                          (int)s.B, (int)T, (int)tc_tiles, (int)it.num_pages, (int)ps, (int)nh, (int)nkv,
+                                                          (int)hd, scale, (int)L.window, s.err, s.stream),
+                           "attention_tc");
+                    return o;
+                }
+                void *part_o = nullptr, *part_ml = nullptr;
+                if (nsplit > 1) {
+                    const i64 rows = T * nh;
+                    need_attn_ws = std::max(need_attn_ws, nsplit * rows * (hd + 2));
+                    if (!dry && nsplit * rows * (hd + 2) > s.attn_ws_floats) throw std::runtime_error("executor: the attention workspace is too small");
+                    part_o = s.attn_ws;
+                    part_ml = (float*)s.attn_ws + nsplit * rows * hd;
+                }
+                LAUNCH(fn<AttentionTcSplitFn>(FN_ATTENTION_TC_SPLIT)(o, part_o, part_ml, q, it.k, it.v, s.cu_seqlens, s.ctx_lens, it.block_table,
+                                                                 (int)it.bt_stride, (int)s.B, (int)T, (int)tc_tiles, (int)it.num_pages, (int)ps,
+                                                                 (int)nh, (int)nkv, (int)hd, scale, (int)L.window, (int)nsplit, s.err, s.stream),
+                       "attention_tc_split");
+                if (nsplit > 1) ++launches;                    // the merge of the pieces
                 return o;
             }
         }
@@ -691,6 +711,28 @@ void* Run::attend(const AttentionParams& L, const ExecItem& it, const void* q, v
                                                 (int)L.window, (int)act, s.err, s.stream),
        "attention_plain");
     return o;
+}
+
+// Into how many pieces the tcgen05 prompt attention cuts every pair of tiles' keys: the rounds of CTAs over the SMs (one an SM)
+// times a CTA's length in blocks of 128 keys, plus two blocks' time to start and to end it, plus the pieces' way through memory
+// (about 3 us a block, 6 TB/s). Taken where that is a tenth shorter than whole; steps whose contexts the host does not
+// know stay whole.
+i64 Run::tc_pieces(i64 ctas, i64 nh, i64 window) const {
+    if (!s.host_ctx_lens) return 1;
+    double blocks = 0;          // of a CTA, on average over the tokens
+    for (i64 b = 0; b < s.B; ++b) {
+        const double keys = (double)s.host_ctx_lens[b] + 0.5 * (double)s.q_lens[b];
+        blocks += (double)s.q_lens[b] * (window > 0 ? std::min(keys, (double)window) : keys) / 128.0;
+    }
+    blocks = blocks / (double)s.T + 1.0;
+    i64 best = 1;
+    double least = 0;
+    for (i64 n = 1; n <= 8 && (double)n * 8.0 <= std::max(blocks, 8.0); ++n) {
+        const double rounds = (double)ceil_div(ctas * n, p.sms), merge = n > 1 ? (double)(2 * n * s.T * nh * 264) / 6e6 / 3.0 + 2.0 : 0.0;
+        const double cost = rounds * (blocks / (double)n + 2.0) + merge;
+        if (n == 1 || cost < (best == 1 ? 0.9 * least : least)) best = n, least = cost;
+    }
+    return best;
 }
 
 void Run::attention(const AttentionParams& L, const ExecItem& it, const void* x, void* out) {

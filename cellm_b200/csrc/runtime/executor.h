@@ -181,7 +181,7 @@ enum ExecFn {
     FN_MOE_SORT, FN_MOE_GATHER, FN_MOE_COMBINE, FN_GEMM_GROUPED, FN_ATTENTION_PLAIN_MASKED,
     FN_ROUTE_SOFTMAX, FN_EXPERTS_GATED_ROWWISE, FN_MOE_COMBINE32, FN_GEMM_GATED, FN_GEMM_GROUPED_GATED, FN_CLAMPED_GATE,
     FN_NORM_ADD_NORM, FN_SOFT_CAP, FN_ROUTE_SOFTMAX_ALL, FN_LATENT_ROWS, FN_ATTENTION_EXPANDED, FN_EXPANDED_SUPPORTS,
-    FN_ATTENTION_TC_UNEVEN, FN_COUNT
+    FN_ATTENTION_TC_SPLIT, FN_COUNT
 };
 
 struct ExecProgram {

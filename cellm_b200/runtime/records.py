@@ -135,7 +135,7 @@ ENTRY_POINTS = [("kernels_common", "cellm_embed"), ("kernels_common", "cellm_add
                 ("kernels_common", "cellm_clamped_gate_act"), ("kernels_common", "cellm_norm_add_norm"), ("kernels_common", "cellm_soft_cap"),
                 ("kernels_common", "cellm_route_softmax_all"), ("attention_expanded", "cellm_latent_rows"),
                 ("attention_expanded", "cellm_attention_expanded"), ("attention_expanded", "cellm_attention_expanded_supports"),
-                ("attention_tc", "cellm_attention_tc_uneven")]
+                ("attention_tc", "cellm_attention_tc_split")]
 # libraries a model whose activations are 32-bit never calls into (they need not be compiled for it)
 BF16_ONLY_LIBRARIES = ("attention_decode", "attention_tc", "attention_flash", "gemm_tcgen05", "attention_latent", "attention_expanded")
 # libraries that only records of these kinds reach (a program without such a record need not have them compiled)

@@ -547,7 +547,7 @@ def test_attention_takes_groups_that_do_not_divide_a_tile(monkeypatch, ps, nh, n
     c = paged_case(lens, ctxs, nh, nkv, hd, ps, torch.bfloat16, seed=6)
     e = err_word()
     ctx = portions_ctx(c, lens, ctxs, e)
-    name = "cellm_attention_tc" if 128 % (nh // nkv) == 0 else "cellm_attention_tc_uneven"
+    name = "cellm_attention_tc" if 128 % (nh // nkv) == 0 else "cellm_attention_tc_split"
     for scale in (hd ** -0.5, 1.0):
         before = program.CALLS[name]
         out = ops.attention(c["q"], c["kp"], c["vp"], ctx, c["bt"], nh, scale, window)
@@ -561,6 +561,29 @@ def test_attention_takes_groups_that_do_not_divide_a_tile(monkeypatch, ps, nh, n
     before = program.CALLS["cellm_attention_flash"]
     ops.attention(d["q"], d["kp"], d["vp"], portions_ctx(d, [40], [0], e), d["bt"], 43, 0.125, 0)
     assert program.CALLS["cellm_attention_flash"] == before + 1
+
+
+@pytest.mark.parametrize("ps,nh,nkv", [(16, 6, 2), (8, 8, 2), (64, 3, 3)])
+@pytest.mark.parametrize("window,chunk_of", [(0, 2), (0, 5), (300, 3), (33, 8)])
+def test_attention_tc_with_the_keys_in_pieces(ps, nh, nkv, window, chunk_of):
+    """Pieces of several blocks, of one, and more pieces than a pair of tiles has blocks (or than one of its tiles has): the
+    merged rows against the oracle. Contexts behind which nothing, a part of a block and several blocks lie."""
+    import ctypes
+    from cellm_b200.csrc import build
+    hd, lens, ctxs = 64, [170, 1, 33, 129], [0, 500, 59, 1640]
+    c = paged_case(lens, ctxs, nh, nkv, hd, ps, torch.bfloat16, seed=6)
+    e, P = err_word(), ctypes.c_void_p
+    T, rows = sum(lens), sum(lens) * nh
+    out, part_o, part_ml = torch.empty_like(c["q"]), torch.full((chunk_of * rows * hd,), float("nan"), device=DEV), torch.empty(chunk_of * rows * 2, device=DEV)
+    ptr = lambda t: P(t.data_ptr())
+    tiles = sum(-(-n // (2 * (128 // (nh // nkv)))) for n in lens)
+    status = build.load("attention_tc").cellm_attention_tc_split(
+        ptr(out), ptr(part_o), ptr(part_ml), ptr(c["q"]), ptr(c["kp"]), ptr(c["vp"]), ptr(c["cu"]), ptr(c["ctx"]), ptr(c["bt"]), c["bt"].stride(0),
+        len(lens), T, tiles, c["kp"].shape[0], ps, nh, nkv, hd, ctypes.c_float(hd ** -0.5), window, chunk_of, ptr(e),
+        P(torch.cuda.current_stream().cuda_stream))
+    assert status == 0
+    close(out, attention_reference(c, nh, nkv, hd, hd ** -0.5, window), torch.bfloat16)
+    assert e.item() == 0
 
 
 def test_attention_tc_refuses_what_it_does_not_take():
