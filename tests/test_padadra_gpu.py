@@ -572,6 +572,32 @@ def test_delta_rule_inputs_and_the_convolutions_state():
     assert float(state[0].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("dim,taps", [(64, 2), (64, 4), (128, 3), (128, 4)])
+@pytest.mark.parametrize("many", [1, 9])
+def test_delta_rule_inputs_of_many_tokens(dim, taps, many):
+    """Runs of tokens that hold several requests' ends and starts, requests shorter than the taps, states that are not zero,
+    channels of v that are no whole head: bit for bit what the form for few tokens leaves for each request alone."""
+    from cellm_b200 import ops
+    heads, kvh, vd = 4, 2, 40
+    lens = [40, 1, 2, 30, 63] * many
+    g = torch.Generator().manual_seed(dim + taps)
+    C, T = 2 * kvh * dim + heads * vd, sum(lens)
+    rnd = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    proj, w, a2, dt, A = rnd(T, C + heads), rnd(C, taps), rnd(T, heads * dim) * 3, rnd(heads * dim), rnd(heads)
+    state = rnd(len(lens) + 1, taps - 1, C)
+    slots = [len(lens) - i for i in range(len(lens))]
+    run = lambda rows, a, ctx: ops.delta_prep(rows, 0, C, w, taps, state, a, dt, A, ctx, heads, kvh, dim, vd, 1e-6)
+    ctx = step_ctx(lens, [0] * len(lens), slots)
+    whole = run(proj, a2, ctx)
+    at = 0
+    for n, slot in zip(lens, slots):
+        alone = run(proj[at:at + n].contiguous(), a2[at:at + n].contiguous(), step_ctx([n], [0], [slot]))
+        for a, b in zip(whole, alone):
+            assert torch.equal(a[at:at + n], b)
+        at += n
+    assert int(ctx.err.item()) == 0
+
+
 @pytest.mark.parametrize("taps,bias", [(4, True), (3, False), (0, True)])
 def test_attention_preparation_in_fours_and_one_by_one(taps, bias):
     """Rows that start on no 16-byte border take the channels one by one: the same values bit for bit."""
