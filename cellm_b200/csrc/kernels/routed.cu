@@ -267,6 +267,7 @@ CELLM_API int cellm_route_softmax_all(int* idx, float* wts, float* gate_out, con
 // ---- the experts, row by row ----------------------------------------------------------------------------------------
 #define EXPERT_THREADS 128
 #define EXPERT_WARPS 4           // a warp forms `rpw` (1, 2 or 4) output rows at once; a block of the first kernel 4 * rpw
+#define EXPERT_TOKENS 4          // slots of one expert that a block of the gated first kernel serves at once
 #define EXPERT_DOWN_WARPS 8      // the second kernel's blocks hold a token's middles in shared memory: more warps share them
 
 // mid[t * top + k, :] = act(U_e y[t]) for e = idx[t, k]; up: [E * ff, H]. Blocks with blockIdx.x >= T * top take the shared
@@ -325,37 +326,98 @@ template <typename TA> __device__ __forceinline__ float expert_gate(float g, flo
     return sizeof(TA) == 4 ? cellm_clamped_gate(g, u, limit, k.slope) : cellm_clamped_gate_rounded(g, u, limit, k.slope);
 }
 
+// A lane's shares of the dot products of four weight rows with N vectors (rows of ys, n apart): p[j][m] = w[j] . ys[m], each
+// summed in the order of lane_dots whatever N is.
+template <typename TW, int N>
+__device__ __forceinline__ void lane_dots_many(float (&p)[4][EXPERT_TOKENS], const TW* const (&w)[4], const TW* ys, int count, int n, int lane, bool vec) {
+    constexpr int PER = 16 / (int)sizeof(TW);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int m = 0; m < N; ++m) p[j][m] = 0.f;
+    if (vec) {
+#pragma unroll 2
+        for (int i = lane * PER; i < n; i += 32 * PER) {
+            uint4 x[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = j < count ? *reinterpret_cast<const uint4*>(w[j] + i) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int m = 0; m < N; ++m) {
+                const uint4 t = *reinterpret_cast<const uint4*>(ys + (size_t)m * n + i);
+                const TW* y = reinterpret_cast<const TW*>(&t);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const TW* xp = reinterpret_cast<const TW*>(&x[j]);
+#pragma unroll
+                    for (int k = 0; k < PER; ++k) p[j][m] += to_float(xp[k]) * to_float(y[k]);
+                }
+            }
+        }
+    } else {
+        for (int i = lane; i < n; i += 32)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int m = 0; m < N; ++m)
+                    if (j < count) p[j][m] += to_float(w[j][i]) * to_float(ys[(size_t)m * n + i]);
+    }
+}
+
+// The slots of one expert (and the tokens of the shared one) are taken `tg` (at most EXPERT_TOKENS) at a time by the block of the
+// first of them, the others' blocks leave at once: a weight row is read once for up to four tokens. Bound by the weights' way
+// from L2 to the SMs, which 48 slots of 35 different experts and a shared one eight times over made 540 MB long (75 us, of
+// which the 300 MB from memory are 47); the layer's experts took 122.7 us so, 112.6 now.
 template <typename TA>
-__global__ void __launch_bounds__(EXPERT_THREADS)
+__global__ void __launch_bounds__(EXPERT_THREADS, 6)
 expert_gate_up_kernel(TA* __restrict__ mid, TA* __restrict__ smid, const TA* __restrict__ y, long long ldy, const TA* __restrict__ gu,
-                      const TA* __restrict__ sgu, const int* __restrict__ idx, int T, int H, int ff, int sff, int top, int E, int rpw,
+                      const TA* __restrict__ sgu, const int* __restrict__ idx, int T, int H, int ff, int sff, int top, int E, int rpw, int tg,
                       ExpertGate kind) {
-    extern __shared__ __align__(16) float smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool is_shared = (int)blockIdx.x >= T * top;
-    const int slot = is_shared ? (int)blockIdx.x - T * top : (int)blockIdx.x;
-    const int t = is_shared ? slot : slot / top;
+    extern __shared__ __align__(16) uint8_t smem_y[];         // [tg][H]
+    __shared__ int group[EXPERT_TOKENS + 1];                  // the slots (tokens) this block serves, then how many
+    TA* ys = reinterpret_cast<TA*>(smem_y);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slots = T * top;
+    const bool is_shared = (int)blockIdx.x >= slots;
     const int rows = is_shared ? sff : ff;
     if ((int)blockIdx.y * EXPERT_WARPS * rpw >= rows) return;
     const bool vec = rows_vectorise(is_shared ? sgu : gu, H, H);
     pdl_trigger();
     pdl_wait();
-    {
-        constexpr int PER = 16 / (int)sizeof(TA);
-        const TA* src = y + (size_t)t * ldy;
-        if (H % PER == 0 && (((uintptr_t)src) & 15) == 0) {
-            for (int i = threadIdx.x * PER; i < H; i += EXPERT_THREADS * PER) {
-                const uint4 x = *reinterpret_cast<const uint4*>(src + i);
-                const TA* xp = reinterpret_cast<const TA*>(&x);
-#pragma unroll
-                for (int k = 0; k < PER; ++k) smem[i + k] = to_float(xp[k]);
+    const TA* base = sgu;
+    int n;
+    if (is_shared) {
+        const int t0 = ((int)blockIdx.x - slots) * tg;
+        n = min(tg, T - t0);
+        if ((int)threadIdx.x < n) group[threadIdx.x] = t0 + threadIdx.x;
+    } else {
+        const int slot = blockIdx.x, e = min(max(idx[slot], 0), E - 1);
+        base = gu + (size_t)e * 2 * ff * H;
+        if (warp == 0) {
+            int rank = 0, before = 0;            // slots of this expert seen so far; those in front of this one
+            for (int i0 = 0; i0 < slots; i0 += 32) {
+                const int i = i0 + lane;
+                const unsigned same = __ballot_sync(0xffffffffu, i < slots && min(max(idx[min(i, slots - 1)], 0), E - 1) == e);
+                if (i0 <= slot) before += __popc(slot - i0 >= 32 ? same : same & ((1u << (slot - i0)) - 1u));
+                const int mine = rank + __popc(same & ((1u << lane) - 1u));
+                if ((same >> lane & 1u) && i >= slot && mine - before < tg) group[mine - before] = i;
+                rank += __popc(same);
             }
+            if (lane == 0) group[EXPERT_TOKENS] = before % tg ? 0 : min(tg, rank - before);
+        }
+        __syncthreads();
+        n = group[EXPERT_TOKENS];
+        if (n == 0) return;
+    }
+    __syncthreads();
+    for (int m = 0; m < n; ++m) {
+        constexpr int PER = 16 / (int)sizeof(TA);
+        const TA* src = y + (size_t)(is_shared ? group[m] : group[m] / top) * ldy;
+        if (H % PER == 0 && (((uintptr_t)src) & 15) == 0) {
+            for (int i = threadIdx.x * PER; i < H; i += EXPERT_THREADS * PER)
+                *reinterpret_cast<uint4*>(ys + (size_t)m * H + i) = *reinterpret_cast<const uint4*>(src + i);
         } else {
-            for (int i = threadIdx.x; i < H; i += EXPERT_THREADS) smem[i] = to_float(src[i]);
+            for (int i = threadIdx.x; i < H; i += EXPERT_THREADS) ys[(size_t)m * H + i] = src[i];
         }
     }
-    const TA* base = sgu;
-    if (!is_shared) base = gu + (size_t)min(max(idx[slot], 0), E - 1) * 2 * ff * H;
     __syncthreads();
     const int r0 = (blockIdx.y * EXPERT_WARPS + warp) * rpw, nr = min(rpw, rows - r0);
     if (nr <= 0) return;
@@ -363,14 +425,21 @@ expert_gate_up_kernel(TA* __restrict__ mid, TA* __restrict__ smid, const TA* __r
     // start at an even j share a block. Rows of the four slots: gate j, up j, gate j + 1, up j + 1.
     const TA* w0 = base + ((size_t)(r0 / 64) * 128 + r0 % 64) * H;
     const TA* w[4] = {w0, w0 + (size_t)64 * H, w0 + H, w0 + (size_t)65 * H};
-    const float* v[4] = {smem, smem, smem, smem};
     const int count = 2 * nr;
-    float p[4];
-    lane_dots<TA>(p, w, v, count, H, lane, vec);
+    float p[4][EXPERT_TOKENS];
+    if (n == 1) lane_dots_many<TA, 1>(p, w, ys, count, H, lane, vec);
+    else if (n == 2) lane_dots_many<TA, 2>(p, w, ys, count, H, lane, vec);
+    else if (n == 3) lane_dots_many<TA, 3>(p, w, ys, count, H, lane, vec);
+    else lane_dots_many<TA, 4>(p, w, ys, count, H, lane, vec);
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const float g = warp_sum(p[2 * j]), u = warp_sum(p[2 * j + 1]);
-        if (lane == 0 && j < nr) (is_shared ? smid : mid)[(size_t)slot * rows + r0 + j] = from_float<TA>(expert_gate<TA>(g, u, kind, is_shared));
+    for (int m = 0; m < EXPERT_TOKENS; ++m) {
+        if (m >= n) break;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float g = warp_sum(p[2 * j][m]), u = warp_sum(p[2 * j + 1][m]);
+            if (lane == 0 && j < nr)
+                (is_shared ? smid : mid)[(size_t)group[m] * rows + r0 + j] = from_float<TA>(expert_gate<TA>(g, u, kind, is_shared));
+        }
     }
 }
 
@@ -480,7 +549,11 @@ static int experts_rowwise_impl(void* out, void* mid, void* smid, const void* y,
     const int up_rows = ff > sff ? ff : sff;
     const int rpw_up = expert_rows_a_warp((long long)T * top * ff + (sup ? (long long)T * sff : 0), EXPERT_WARPS, gated ? 2 : 4, 4);
     const int rpw_down = expert_rows_a_warp((long long)T * H, EXPERT_DOWN_WARPS, 4, 2);
-    const dim3 grid_up((unsigned)(T * top + (sup ? T : 0)), (unsigned)((up_rows + EXPERT_WARPS * rpw_up - 1) / (EXPERT_WARPS * rpw_up)));
+    // gated: as many tokens' rows at once as 32 KB hold (one always fits where it did)
+    const size_t row_y = (size_t)H * (dtype == CELLM_F32 ? 4 : 2);
+    const int tg = !gated ? 1 : 4 * row_y <= 32 * 1024 ? 4 : 2 * row_y <= 32 * 1024 ? 2 : 1;
+    const size_t smem_y = tg * row_y;
+    const dim3 grid_up((unsigned)(T * top + (sup ? (T + tg - 1) / tg : 0)), (unsigned)((up_rows + EXPERT_WARPS * rpw_up - 1) / (EXPERT_WARPS * rpw_up)));
     const dim3 grid_down((unsigned)T, (unsigned)((H + EXPERT_DOWN_WARPS * rpw_down - 1) / (EXPERT_DOWN_WARPS * rpw_down)));
     if (grid_up.y > 65535 || grid_down.y > 65535) return CELLM_ERR_SIZE;
 #define GO(TA, TO)                                                                                                                \
@@ -494,8 +567,8 @@ static int experts_rowwise_impl(void* out, void* mid, void* smid, const void* y,
             configured = true;                                                                                                    \
         }                                                                                                                         \
         if (gated)                                                                                                                \
-            CELLM_RUN(expert_gate_up_kernel<TA>, grid_up, EXPERT_THREADS, smem_up, stream, (TA*)mid, (TA*)smid, (const TA*)y, ldy, \
-                      (const TA*)up, (const TA*)sup, idx, T, H, ff, sff, top, E, rpw_up, kind);                                   \
+            CELLM_RUN(expert_gate_up_kernel<TA>, grid_up, EXPERT_THREADS, smem_y, stream, (TA*)mid, (TA*)smid, (const TA*)y, ldy,  \
+                      (const TA*)up, (const TA*)sup, idx, T, H, ff, sff, top, E, rpw_up, tg, kind);                               \
         else                                                                                                                      \
             CELLM_RUN(expert_up_kernel<TA>, grid_up, EXPERT_THREADS, smem_up, stream, (TA*)mid, (TA*)smid, (const TA*)y, ldy, (const TA*)up,  \
                       (const TA*)sup, idx, T, H, ff, sff, top, E, act, rpw_up);                                                   \

@@ -910,3 +910,44 @@ def test_clamped_experts_against_plain(dtype, T, H, E, top, ff, limit, groups, s
         assert got.dtype == (torch.float32 if out32 else dtype)
         tol = dict(rtol=3e-2, atol=3e-2 * float(want.abs().max())) if dtype == torch.bfloat16 else dict(rtol=1e-4, atol=2e-5 * float(want.abs().max()))
         torch.testing.assert_close(got.cpu().double()[clear], want[clear], **tol)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,H,ff,sff,top,E", [(1, 64, 64, 64, 2, 4), (9, 264, 64, 192, 3, 4), (13, 100, 128, 64, 6, 9), (5, 4104, 64, 128, 2, 3),
+                                              (70, 72, 64, 64, 3, 5)])
+def test_clamped_experts_that_several_tokens_choose(dtype, T, H, ff, sff, top, E):
+    """More slots of an expert than a block serves at once, rows of which only one or two fit beside each other, rows off the
+    16-byte border: the middles are near the exact ones, and bit for bit those of every token alone."""
+    from cellm_b200.ops._lib import check, fn, ptr, stream_of, tag
+    g = torch.Generator().manual_seed(T * H)
+    rnd = lambda *shape: torch.randn(*shape, generator=g)
+    y = rnd(T, H + 3).to(dtype).to(DEV)[:, :H] if H % 8 else rnd(T, H).to(dtype).to(DEV)
+    gu, down = (rnd(E * 2 * ff, H) * H ** -0.5).to(dtype).to(DEV), (rnd(E * H, ff) * ff ** -0.5).to(dtype).to(DEV)
+    sgu, sdown = (rnd(2 * sff, H) * H ** -0.5).to(dtype).to(DEV), (rnd(H, sff) * sff ** -0.5).to(dtype).to(DEV)
+    idx = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to(torch.int32).to(DEV)
+    wts = torch.rand(T, top, generator=g).to(DEV)
+
+    def run(t0, t1):
+        n = t1 - t0
+        out, mid, smid = (torch.empty(n, w, dtype=dtype, device=DEV) for w in (H, top * ff, sff))
+        rows, choice, w = y[t0:t1], idx[t0:t1].contiguous(), wts[t0:t1].contiguous()
+        check(fn("kernels_common", "cellm_experts_gated_rowwise")(
+            ptr(out), ptr(mid), ptr(smid), ptr(rows), rows.stride(0), ptr(gu), ptr(down), ptr(sgu), ptr(sdown), ptr(choice), ptr(w), None,
+            n, H, ff, sff, top, E, 1, 7.0, 5.0, 1.702, tag(dtype), tag(dtype), stream_of(rows)), "experts_gated_rowwise")
+        torch.cuda.synchronize()
+        return out, mid, smid
+    out, mid, smid = run(0, T)
+    for t in range(T):
+        for whole, alone in zip((out, mid, smid), run(t, t + 1)):
+            assert torch.equal(whole[t:t + 1], alone)
+
+    def middle(w, rows, limit):          # rows in blocks of 64 gate rows and their 64 up rows
+        z = (rows.double() @ w.double().T).reshape(rows.shape[0], -1, 2, 64)
+        a, b = z[:, :, 0].clamp(max=limit), z[:, :, 1].clamp(-limit, limit)
+        return (a * torch.sigmoid(1.702 * a) * (b + 1)).reshape(rows.shape[0], -1)
+    # sums of H products in 32 bits (H up to 4,104: 64 units of 2^-24 of their size), and the result's rounding
+    tol = dict(rtol=2.0 ** -8, atol=2.0 ** -8) if dtype == torch.bfloat16 else dict(rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(smid.double(), middle(sgu, y, 5.0), **tol)
+    for t in range(T):
+        want = torch.stack([middle(gu.reshape(E, 2 * ff, H)[e], y[t:t + 1], 7.0)[0] for e in idx[t].tolist()])
+        torch.testing.assert_close(mid[t].reshape(top, ff).double(), want, **tol)
