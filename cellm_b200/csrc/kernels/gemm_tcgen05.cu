@@ -662,6 +662,65 @@ template <> __device__ __forceinline__ void store_half_row<__nv_bfloat16>(__nv_b
     }
 }
 
+// One thread's row p of a tile whose first column is q0: its sums out of tensor memory (lane_addr), through the activation or
+// the joining of gate and up, to C. `release` says that the accumulator has been read.
+template <int EPI, typename TO, typename Release>
+__device__ __forceinline__ void drain_tile(TO* __restrict__ C, int M, int N, long long ldc, int p, int q0, int bn, uint32_t lane_addr, int act,
+                                           const float* __restrict__ act_numbers, const GateEpi& gate_epi, Release release) {
+    if constexpr (EPI == 0) {
+        const bool aligned = ((reinterpret_cast<uintptr_t>(C) | (uintptr_t)(ldc * sizeof(TO))) & 15) == 0 &&
+                             ((q0 * sizeof(TO)) & 15) == 0;
+        const int chunks = (bn + 31) / 32;
+#pragma unroll 1
+        for (int c = 0; c < chunks; ++c) {
+            uint32_t r[32];
+            const int cols = bn - c * 32 >= 32 ? 32 : 16;          // the last chunk of a width that is an odd multiple of 16
+            if (cols == 32) tmem_ld32(lane_addr + (uint32_t)(c * 32), r);
+            else tmem_ld16(lane_addr + (uint32_t)(c * 32), r);
+            if (c == chunks - 1) { tc_fence_before(); release(); }
+            if (act == 6) {
+                const float ap = cellm_softplus(act_numbers[0]), aq = 0.5f + cellm_softplus(act_numbers[1]);
+                if constexpr (sizeof(TO) == 2) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_xielu_rounded(__uint_as_float(r[i]), ap, aq));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_xielu(__uint_as_float(r[i]), ap, aq));
+                }
+            } else if (act == 0) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_gelu_flat(__uint_as_float(r[i])));
+            } else if (act > 0) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_activate(__uint_as_float(r[i]), act));
+            }
+            const int q = q0 + c * 32;
+            if (p < M && q < N) {
+                if (cols == 32) store_row<TO>(C + (size_t)p * ldc + q, r, N - q, aligned);
+                else store_half_row<TO>(C + (size_t)p * ldc + q, r, N - q, aligned);
+            }
+        }
+    } else {
+        const int o0 = q0 / 2;
+        const bool aligned = ((reinterpret_cast<uintptr_t>(C) | (uintptr_t)(ldc * sizeof(TO))) & 15) == 0 &&
+                             ((o0 * sizeof(TO)) & 15) == 0;
+#pragma unroll 1
+        for (int j = 0; j < bn / 128; ++j) {
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                uint32_t g[32], u[32];
+                tmem_ld32(lane_addr + (uint32_t)(j * 128 + h * 32), g);
+                tmem_ld32(lane_addr + (uint32_t)(j * 128 + 64 + h * 32), u);
+                if (j == bn / 128 - 1 && h == 1) { tc_fence_before(); release(); }
+#pragma unroll
+                for (int i = 0; i < 32; ++i) g[i] = __float_as_uint(gate_up(__uint_as_float(g[i]), __uint_as_float(u[i]), gate_epi));
+                const int o = o0 + j * 64 + h * 32;
+                if (p < M && o < N / 2) store_row<TO>(C + (size_t)p * ldc + o, g, N / 2 - o, aligned);
+            }
+        }
+    }
+}
+
 // Persistent form for large products (plain tiles, no K split): one CTA per SM walks
 // the tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... (row tiles of A fastest, so
 // CTAs that run side by side share a tile of W in L2). The accumulator is double
@@ -791,64 +850,197 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const 
             const int p0 = (tile_group ? tile / n_tiles : tile % m_tiles) * BM, q0 = (tile_group ? tile % n_tiles : tile / m_tiles) * bn;
             const int p = p0 + pl;
             const uint32_t lane_addr = tmem + ((uint32_t)(qtr * 32) << 16) + (uint32_t)(buf * BN);
-            if constexpr (EPI == 0) {
-                const bool aligned = ((reinterpret_cast<uintptr_t>(C) | (uintptr_t)(ldc * sizeof(TO))) & 15) == 0 &&
-                                     ((q0 * sizeof(TO)) & 15) == 0;
-                const int chunks = (bn + 31) / 32;
-#pragma unroll 1
-                for (int c = 0; c < chunks; ++c) {
-                    uint32_t r[32];
-                    const int cols = bn - c * 32 >= 32 ? 32 : 16;          // the last chunk of a width that is an odd multiple of 16
-                    if (cols == 32) tmem_ld32(lane_addr + (uint32_t)(c * 32), r);
-                    else tmem_ld16(lane_addr + (uint32_t)(c * 32), r);
-                    if (c == chunks - 1) { tc_fence_before(); mbar_arrive(&sm.acc_empty2[buf]); }
-                    if (act == 6) {
-                        const float ap = cellm_softplus(act_numbers[0]), aq = 0.5f + cellm_softplus(act_numbers[1]);
-                        if constexpr (sizeof(TO) == 2) {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_xielu_rounded(__uint_as_float(r[i]), ap, aq));
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_xielu(__uint_as_float(r[i]), ap, aq));
-                        }
-                    } else if (act == 0) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_gelu_flat(__uint_as_float(r[i])));
-                    } else if (act > 0) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_activate(__uint_as_float(r[i]), act));
-                    }
-                    const int q = q0 + c * 32;
-                    if (p < M && q < N) {
-                        if (cols == 32) store_row<TO>(C + (size_t)p * ldc + q, r, N - q, aligned);
-                        else store_half_row<TO>(C + (size_t)p * ldc + q, r, N - q, aligned);
-                    }
-                }
-            } else {
-                const int o0 = q0 / 2;
-                const bool aligned = ((reinterpret_cast<uintptr_t>(C) | (uintptr_t)(ldc * sizeof(TO))) & 15) == 0 &&
-                                     ((o0 * sizeof(TO)) & 15) == 0;
-#pragma unroll 1
-                for (int j = 0; j < bn / 128; ++j) {
-#pragma unroll 1
-                    for (int h = 0; h < 2; ++h) {
-                        uint32_t g[32], u[32];
-                        tmem_ld32(lane_addr + (uint32_t)(j * 128 + h * 32), g);
-                        tmem_ld32(lane_addr + (uint32_t)(j * 128 + 64 + h * 32), u);
-                        if (j == bn / 128 - 1 && h == 1) { tc_fence_before(); mbar_arrive(&sm.acc_empty2[buf]); }
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) g[i] = __float_as_uint(gate_up(__uint_as_float(g[i]), __uint_as_float(u[i]), gate_epi));
-                        const int o = o0 + j * 64 + h * 32;
-                        if (p < M && o < N / 2) store_row<TO>(C + (size_t)p * ldc + o, g, N / 2 - o, aligned);
-                    }
-                }
-            }
+            drain_tile<EPI, TO>(C, M, N, ldc, p, q0, bn, lane_addr, act, act_numbers, gate_epi, [&] { mbar_arrive(&sm.acc_empty2[buf]); });
             ++tcount;
         }
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, TMEM_COLS);
+}
+
+// ---------------------------------------------------------------- pairs of SMs
+// The two CTAs of a cluster work on one tile of 256 rows: CTA r holds rows r * 128 .. of A and half of the tile's columns
+// of W, and the leader (rank 0) issues products of 256 x bn x 16 (cta_group::2) that read both CTAs' shared memory and leave
+// each CTA the sums of its own 128 rows. So a K block costs a CTA 32 KB of loads instead of 48 and seven stages fit instead
+// of four.
+constexpr int PAIR_STAGES = 7;
+constexpr int PAIR_BN = 256;
+
+struct alignas(1024) PairSmem {
+    uint8_t a[PAIR_STAGES][BM * BK * 2];
+    uint8_t b[PAIR_STAGES][PAIR_BN / 2 * BK * 2];
+    uint64_t full[PAIR_STAGES];       // the leader's counts both CTAs' loads
+    uint64_t empty[PAIR_STAGES];
+    uint64_t acc_full[2];
+    uint64_t acc_empty[2];            // the leader's: one arrival per epilogue warp of both CTAs
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+__device__ __forceinline__ uint32_t in_cta(const void* local, uint32_t rank) {
+    uint32_t addr;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(local)), "r"(rank));
+    return addr;
+}
+// A box into this CTA's shared memory whose bytes are counted by a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Arrives on the barrier at this place of both CTAs when the products issued so far are done.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
+// The persistent kernel for pairs: the same roles, ring and double buffer, pair c walks the tiles c, c + pairs, ... The
+// leader's barriers run the products; a stage and an accumulator become free in both CTAs by one commit. No CTA leaves before
+// the other has finished (the barrier at the end): the products read the peer's shared memory and write its tensor memory.
+template <int EPI, typename TO>
+__global__ void __launch_bounds__(192)
+gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, TO* __restrict__ C, int M, int N,
+                         int K, long long ldc, int w_is_static, int* __restrict__ err, int bn, int act, const float* __restrict__ act_numbers,
+                         const GateEpi gate_epi) {
+    extern __shared__ uint8_t smem_raw[];
+    auto& sm = *reinterpret_cast<PairSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)cluster_rank(), first = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    const int m_tiles = (M + 2 * BM - 1) / (2 * BM), n_tiles = (N + bn - 1) / bn, num_tiles = m_tiles * n_tiles;
+    const int nkb = (K + BK - 1) / BK;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < PAIR_STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&sm.acc_full[b], 1); mbar_init(&sm.acc_empty[b], 8); }
+        sm.abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+    }
+    __syncwarp();
+    if (warp == 1) tmem_alloc_pair(&sm.tmem_base, 2 * PAIR_BN);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();             // the peer's barriers and tensor memory are there
+    tc_fence_after();
+    pdl_trigger();
+    const uint32_t tmem = sm.tmem_base;
+    volatile int* abort_flag = &sm.abort_flag;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint32_t bytes = (uint32_t)((2 * BM + bn) * BK * 2);          // of both CTAs
+            int it = 0;
+            bool waited = false;
+            if (!w_is_static) { pdl_wait(); waited = true; }
+            for (int tile = first; tile < num_tiles && !*abort_flag; tile += pairs) {
+                const int p0 = tile % m_tiles * 2 * BM + rank * BM, q0 = tile / m_tiles * bn + rank * (bn / 2);
+                int kb = 0;
+                if (!waited) {
+                    // static weights: the ring's first loads of W go out before the wait on the preceding kernel
+                    const int early = nkb < PAIR_STAGES ? nkb : PAIR_STAGES;
+                    for (int i = 0; i < early; ++i) {
+                        if (rank == 0) mbar_expect_tx(&sm.full[i], bytes);
+                        tma_load_2d_pair(sm.b[i], &map_w, i * BK, q0, in_cta(&sm.full[i], 0));
+                    }
+                    pdl_wait();
+                    waited = true;
+                    for (int i = 0; i < early; ++i) tma_load_2d_pair(sm.a[i], &map_a, i * BK, p0, in_cta(&sm.full[i], 0));
+                    kb = early;
+                    it = early;
+                }
+                for (; kb < nkb; ++kb, ++it) {
+                    const int s = it % PAIR_STAGES;
+                    const uint32_t phase = (uint32_t)(it / PAIR_STAGES) & 1u;
+                    if (!mbar_wait(&sm.empty[s], phase ^ 1u, abort_flag)) { *abort_flag = 1; atomicOr(err, CELLM_DEV_WAIT_TIMEOUT); break; }
+                    // the peer's bytes may be counted before the leader says how many there will be: the phase ends only
+                    // with the leader's arrival
+                    if (rank == 0) mbar_expect_tx(&sm.full[s], bytes);
+                    const uint32_t full = in_cta(&sm.full[s], 0);
+                    tma_load_2d_pair(sm.a[s], &map_a, kb * BK, p0, full);
+                    tma_load_2d_pair(sm.b[s], &map_w, kb * BK, q0, full);
+                }
+            }
+            // the last commits arrive here too: this CTA stays until they have
+            for (int i = it > PAIR_STAGES ? it - PAIR_STAGES : 0; i < it && !*abort_flag; ++i)
+                if (!mbar_wait(&sm.empty[i % PAIR_STAGES], (uint32_t)(i / PAIR_STAGES) & 1u, abort_flag)) { *abort_flag = 1; atomicOr(err, CELLM_DEV_WAIT_TIMEOUT); }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (rank == 0 && lane == 0) {
+            const uint32_t idesc = umma_idesc(2 * BM, bn);
+            int it = 0, tcount = 0;
+            for (int tile = first; tile < num_tiles && !*abort_flag; tile += pairs) {
+                const int buf = tcount & 1;
+                const uint32_t acc_phase = (uint32_t)(tcount >> 1) & 1u;
+                if (!mbar_wait(&sm.acc_empty[buf], acc_phase ^ 1u, abort_flag)) { *abort_flag = 1; atomicOr(err, CELLM_DEV_WAIT_TIMEOUT); break; }
+                tc_fence_after();
+                const uint32_t acc = tmem + (uint32_t)(buf * PAIR_BN);
+                bool ok = true;
+                for (int kb = 0; kb < nkb; ++kb, ++it) {
+                    const int s = it % PAIR_STAGES;
+                    const uint32_t phase = (uint32_t)(it / PAIR_STAGES) & 1u;
+                    if (!mbar_wait(&sm.full[s], phase, abort_flag)) { *abort_flag = 1; atomicOr(err, CELLM_DEV_WAIT_TIMEOUT); ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t da = umma_desc(smem_u32(sm.a[s])), db = umma_desc(smem_u32(sm.b[s]));
+#pragma unroll
+                    for (int k = 0; k < BK / UMMA_K; ++k)
+                        umma_bf16_pair(acc, da + (uint64_t)(k * UMMA_K * 2 / 16), db + (uint64_t)(k * UMMA_K * 2 / 16), idesc,
+                                       (kb | k) != 0 ? 1u : 0u);
+                    umma_commit_pair(&sm.empty[s]);
+                }
+                if (!ok) break;
+                umma_commit_pair(&sm.acc_full[buf]);
+                ++tcount;
+            }
+        }
+        __syncwarp();
+    } else {
+        const int qtr = warp & 3;
+        bool waited = false;
+        int tcount = 0;
+        for (int tile = first; tile < num_tiles; tile += pairs) {
+            const int buf = tcount & 1;
+            const uint32_t acc_phase = (uint32_t)(tcount >> 1) & 1u;
+            if (!mbar_wait(&sm.acc_full[buf], acc_phase, abort_flag)) {
+                if (lane == 0) { *abort_flag = 1; atomicOr(err, CELLM_DEV_WAIT_TIMEOUT); }
+                break;
+            }
+            tc_fence_after();
+            if (!waited) { pdl_wait(); waited = true; }    // stores must not pass the kernel before this one
+            const int p = tile % m_tiles * 2 * BM + rank * BM + qtr * 32 + lane, q0 = tile / m_tiles * bn;
+            const uint32_t lane_addr = tmem + ((uint32_t)(qtr * 32) << 16) + (uint32_t)(buf * PAIR_BN);
+            drain_tile<EPI, TO>(C, M, N, ldc, p, q0, bn, lane_addr, act, act_numbers, gate_epi, [&] {
+                __syncwarp();
+                if (lane == 0) mbar_arrive_at(in_cta(&sm.acc_empty[buf], 0));
+            });
+            ++tcount;
+        }
+        __syncwarp();
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc_pair(tmem, 2 * PAIR_BN);
 }
 
 // ---------------------------------------------------------------- host side
@@ -888,25 +1080,104 @@ int launch(const CUtensorMap& m_rows, const CUtensorMap& m_cols, TO* C, float* w
     return e == cudaSuccess ? CELLM_OK : (int)e;
 }
 
-template <int BN, int STAGES, int EPI, typename TO>
-int launch_persistent(const CUtensorMap& m_a, const CUtensorMap& m_w, TO* C, int M, int N, int K, long long ldc,
-                      int w_is_static, int* err, cudaStream_t stream, int bn, const int* tile_group = nullptr, int act = -1,
-                      const float* act_numbers = nullptr, const GateEpi& gate_epi = GateEpi()) {
-    const size_t smem = sizeof(GemmSmem<BN, STAGES>) + 1024;
+// The device's SMs (0: unknown).
+int sm_count() {
     static int sms = 0;
     if (sms == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
+    }
+    return sms;
+}
+
+// Whether an unsplit product with tiles of bn columns runs on pairs of SMs, whose width is bn rounded up to a multiple of 32.
+// A pair's launch and its two cluster barriers cost 1 to 2 us more than a single CTA's; its steady state is 5 to 7 % faster
+// (by 20 % where a long product runs under the power cap: N 65,536, K 2,048, M 2,048 377 us against 453). So it takes
+// products of which an SM has at least 90 K blocks of 256 columns to do (M 2,048: N 6,144, K 2,048, 96 blocks, 40.5 us against 42.5;
+// N 16,384 with SwiGLU, 224 blocks, 94.5 against 99.6; N 2,048, K 8,192, 128 blocks, 49.8 against 50.8; but N 3,072, K 2,048,
+// 64 blocks, 29.4 against 28.1, and N 2,048, K 2,048, 32 blocks, 18.6 against 16.6), unless rows beyond M or the wider
+// tiles take away more than that.
+bool in_pairs(int M, int N, int K, int bn) {
+    const int sms = sm_count();
+    if (sms < 2) return false;
+    const long long w = (bn + 31) & ~31, kblocks = (K + BK - 1) / BK;
+    const long long tiles_p = (long long)((N + w - 1) / w) * ((M + 2 * BM - 1) / (2 * BM)), tiles_s = (long long)((N + bn - 1) / bn) * ((M + BM - 1) / BM);
+    const long long waves_p = (tiles_p + sms / 2 - 1) / (sms / 2), waves_s = (tiles_s + sms - 1) / sms;
+    return waves_p * w * kblocks >= 90 * 256 && waves_p * w * 15 <= waves_s * bn * 16;
+}
+
+template <int EPI, typename TO>
+int launch_pairs(const CUtensorMap& m_a, const CUtensorMap& m_w, TO* C, int M, int N, int K, long long ldc, int w_is_static, int* err,
+                 cudaStream_t stream, int bn, int act, const float* act_numbers, const GateEpi& gate_epi) {
+    const size_t smem = sizeof(PairSmem) + 1024;
+    static bool configured = false;
+    auto kernel = gemm_tcgen05_pair_kernel<EPI, TO>;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int tiles = ((N + bn - 1) / bn) * ((M + 2 * BM - 1) / (2 * BM)), pairs = sm_count() / 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
+    cfg.blockDim = dim3(192);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, m_a, m_w, C, M, N, K, ldc, w_is_static, err, bn, act, act_numbers, gate_epi);
+    return e == cudaSuccess ? CELLM_OK : (int)e;
+}
+
+template <int BN, int STAGES, int EPI, typename TO>
+int launch_persistent(const CUtensorMap& m_a, const CUtensorMap& m_w, TO* C, int M, int N, int K, long long ldc,
+                      int w_is_static, int* err, cudaStream_t stream, int bn, const int* tile_group, int act,
+                      const float* act_numbers, const GateEpi& gate_epi) {
+    const size_t smem = sizeof(GemmSmem<BN, STAGES>) + 1024;
+    static bool configured = false;
+    if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_persistent_kernel<BN, STAGES, EPI, TO>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            return CELLM_ERR_ARG;
+        configured = true;
     }
-    const int tiles = ((N + bn - 1) / bn) * ((M + BM - 1) / BM);
+    const int tiles = ((N + bn - 1) / bn) * ((M + BM - 1) / BM), sms = sm_count();
+    if (sms == 0) return CELLM_ERR_ARG;
     dim3 grid((unsigned)(tiles < sms ? tiles : sms));
     cudaError_t e = cellm_launch(gemm_tcgen05_persistent_kernel<BN, STAGES, EPI, TO>, grid, dim3(192), smem, stream, m_a,
                                  m_w, C, M, N, K, ldc, w_is_static, err, bn, tile_group, act, act_numbers, gate_epi);
     return e == cudaSuccess ? CELLM_OK : (int)e;
+}
+
+// An unsplit product with tiles of bn columns (128, or up to 256), grouped or not (see the persistent kernel): the tensor
+// maps, and the kernel that serves these sizes.
+template <int EPI>
+int launch_unsplit(void* C, const void* A, const void* W, int M, int N, int K, int groups, long long lda, long long ldw, long long ldc,
+                   int out_dtype, int w_is_static, int* err, cudaStream_t stream, int bn, const int* tile_group, int act,
+                   const float* act_numbers, const GateEpi& gate_epi) {
+    const bool pairs = !tile_group && in_pairs(M, N, K, bn);
+    if (pairs) bn = (bn + 31) & ~31;             // a product of 256 rows takes columns in steps of 32
+    CUtensorMap map_a, map_w;
+    if (!tensor_map(&map_a, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, (uint32_t)BM)) return CELLM_ERR_ARG;
+    if (!tensor_map(&map_w, W, (uint64_t)groups * (uint64_t)N, (uint64_t)K, (uint64_t)ldw * 2, (uint32_t)(pairs ? bn / 2 : bn))) return CELLM_ERR_ARG;
+    const bool f32 = out_dtype == CELLM_F32;
+    float* cf = (float*)C;
+    __nv_bfloat16* cb = (__nv_bfloat16*)C;
+    if (pairs)
+        return f32 ? launch_pairs<EPI, float>(map_a, map_w, cf, M, N, K, ldc, w_is_static, err, stream, bn, act, act_numbers, gate_epi)
+                   : launch_pairs<EPI, __nv_bfloat16>(map_a, map_w, cb, M, N, K, ldc, w_is_static, err, stream, bn, act, act_numbers, gate_epi);
+    if (bn == 128)
+        return f32 ? launch_persistent<128, 6, EPI, float>(map_a, map_w, cf, M, N, K, ldc, w_is_static, err, stream, bn, tile_group, act, act_numbers, gate_epi)
+                   : launch_persistent<128, 6, EPI, __nv_bfloat16>(map_a, map_w, cb, M, N, K, ldc, w_is_static, err, stream, bn, tile_group, act, act_numbers, gate_epi);
+    return f32 ? launch_persistent<256, 4, EPI, float>(map_a, map_w, cf, M, N, K, ldc, w_is_static, err, stream, bn, tile_group, act, act_numbers, gate_epi)
+               : launch_persistent<256, 4, EPI, __nv_bfloat16>(map_a, map_w, cb, M, N, K, ldc, w_is_static, err, stream, bn, tile_group, act, act_numbers, gate_epi);
 }
 
 }  // namespace
@@ -976,24 +1247,18 @@ static int gemm_impl(void* C, const void* A, const void* W, int M, int N, int K,
                                      : (long long)((N + narrow - 1) / narrow) * ((M + BM - 1) / BM);
         if (tiles > GEMM_MAX_COUNTERS) return CELLM_ERR_SIZE;
     }
+    // Unsplit products with plain tiles of 128 to 256 columns run a persistent kernel.
+    if (!swap && split == 1 && narrow >= 128) {
+        if (epilogue == 0)
+            return launch_unsplit<0>(C, A, W, M, N, K, 1, lda, ldw, ldc, out_dtype, w_is_static, err, stream, narrow, nullptr, -1, nullptr, gate_epi);
+        return launch_unsplit<1>(C, A, W, M, N, K, 1, lda, ldw, ldc, out_dtype, w_is_static, err, stream, narrow, nullptr, -1, nullptr, gate_epi);
+    }
     CUtensorMap map_a, map_w;
     if (!tensor_map(&map_a, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, swap ? (uint32_t)narrow : (uint32_t)BM)) return CELLM_ERR_ARG;
     if (!tensor_map(&map_w, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw * 2, swap ? (uint32_t)BM : (uint32_t)narrow)) return CELLM_ERR_ARG;
     const CUtensorMap& m_rows = swap ? map_w : map_a;
     const CUtensorMap& m_cols = swap ? map_a : map_w;
     int rc = CELLM_ERR_SIZE;
-    // Large unsplit products with plain tiles of 128 or 256 columns run the persistent kernel.
-    if (!swap && split == 1 && narrow >= 128) {
-#define GOP(BN_, ST_, EP_)                                                                                          \
-    do {                                                                                                            \
-        if (out_dtype == CELLM_F32) rc = launch_persistent<BN_, ST_, EP_, float>(map_a, map_w, (float*)C, M, N, K, ldc, w_is_static, err, stream, narrow, nullptr, -1, nullptr, gate_epi); \
-        else rc = launch_persistent<BN_, ST_, EP_, __nv_bfloat16>(map_a, map_w, (__nv_bfloat16*)C, M, N, K, ldc, w_is_static, err, stream, narrow, nullptr, -1, nullptr, gate_epi); \
-    } while (0)
-        if (narrow == 128) { if (epilogue == 0) GOP(128, 6, 0); else GOP(128, 6, 1); }
-        else { if (epilogue == 0) GOP(256, 4, 0); else GOP(256, 4, 1); }       // 144 to 256 columns
-#undef GOP
-        return rc;
-    }
 #define GO3(BN_, ST_, SW_, EP_, CL_)                                                                                  \
     do {                                                                                                              \
         if (out_dtype == CELLM_F32) rc = launch<BN_, ST_, SW_, EP_, CL_, float>(m_rows, m_cols, (float*)C, workspace, counters, M, N, K, ldc, split, per, w_is_static, err, stream, conv, rope, gate_epi); \
@@ -1048,16 +1313,7 @@ CELLM_API int cellm_gemm_grouped_tcgen05(void* C, const void* A, const void* W, 
     if (((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((lda * 2) & 15) || ((ldw * 2) & 15)) return CELLM_ERR_ALIGN;
     if (out_dtype != CELLM_F32 && out_dtype != CELLM_BF16) return CELLM_ERR_DTYPE;
     if (act > 4) return CELLM_ERR_ARG;
-    const int bn = N > 128 ? 256 : 128;
-    CUtensorMap map_a, map_w;
-    if (!tensor_map(&map_a, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, (uint32_t)BM)) return CELLM_ERR_ARG;
-    if (!tensor_map(&map_w, W, (uint64_t)groups * (uint64_t)N, (uint64_t)K, (uint64_t)ldw * 2, (uint32_t)bn)) return CELLM_ERR_ARG;
-    if (bn == 128) {
-        if (out_dtype == CELLM_F32) return launch_persistent<128, 6, 0, float>(map_a, map_w, (float*)C, M, N, K, ldc, 0, err, stream, bn, tile_group, act);
-        return launch_persistent<128, 6, 0, __nv_bfloat16>(map_a, map_w, (__nv_bfloat16*)C, M, N, K, ldc, 0, err, stream, bn, tile_group, act);
-    }
-    if (out_dtype == CELLM_F32) return launch_persistent<256, 4, 0, float>(map_a, map_w, (float*)C, M, N, K, ldc, 0, err, stream, bn, tile_group, act);
-    return launch_persistent<256, 4, 0, __nv_bfloat16>(map_a, map_w, (__nv_bfloat16*)C, M, N, K, ldc, 0, err, stream, bn, tile_group, act);
+    return launch_unsplit<0>(C, A, W, M, N, K, groups, lda, ldw, ldc, out_dtype, 0, err, stream, N > 128 ? 256 : 128, tile_group, act, nullptr, GateEpi());
 }
 
 // The grouped product over gate and up (epilogue 1): W holds `groups` matrices of N rows (N a multiple of 128) in blocks of
@@ -1074,15 +1330,7 @@ CELLM_API int cellm_gemm_grouped_gated_tcgen05(void* C, const void* A, const voi
     GateEpi gate_epi;
     gate_epi.kind = gate_kind, gate_epi.limit = limit, gate_epi.slope = slope;
     const int bn = (N & 255) == 0 ? 256 : 128;      // a tile of 256 columns must not reach into the next matrix's rows
-    CUtensorMap map_a, map_w;
-    if (!tensor_map(&map_a, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, (uint32_t)BM)) return CELLM_ERR_ARG;
-    if (!tensor_map(&map_w, W, (uint64_t)groups * (uint64_t)N, (uint64_t)K, (uint64_t)ldw * 2, (uint32_t)bn)) return CELLM_ERR_ARG;
-    if (bn == 128) {
-        if (out_dtype == CELLM_F32) return launch_persistent<128, 6, 1, float>(map_a, map_w, (float*)C, M, N, K, ldc, 0, err, stream, bn, tile_group, -1, nullptr, gate_epi);
-        return launch_persistent<128, 6, 1, __nv_bfloat16>(map_a, map_w, (__nv_bfloat16*)C, M, N, K, ldc, 0, err, stream, bn, tile_group, -1, nullptr, gate_epi);
-    }
-    if (out_dtype == CELLM_F32) return launch_persistent<256, 4, 1, float>(map_a, map_w, (float*)C, M, N, K, ldc, 0, err, stream, bn, tile_group, -1, nullptr, gate_epi);
-    return launch_persistent<256, 4, 1, __nv_bfloat16>(map_a, map_w, (__nv_bfloat16*)C, M, N, K, ldc, 0, err, stream, bn, tile_group, -1, nullptr, gate_epi);
+    return launch_unsplit<1>(C, A, W, M, N, K, groups, lda, ldw, ldc, out_dtype, 0, err, stream, bn, tile_group, -1, nullptr, gate_epi);
 }
 
 // An ordinary product of any M with xIELU in its epilogue: C [M, N] = xielu(A [M, K] . W [N, K]^T) with the two learned
@@ -1094,16 +1342,7 @@ CELLM_API int cellm_gemm_xielu_tcgen05(void* C, const void* A, const void* W, in
     if (!act_numbers) return CELLM_ERR_ARG;
     if (((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((lda * 2) & 15) || ((ldw * 2) & 15)) return CELLM_ERR_ALIGN;
     if (out_dtype != CELLM_F32 && out_dtype != CELLM_BF16) return CELLM_ERR_DTYPE;
-    const int bn = N > 128 ? 256 : 128;
-    CUtensorMap map_a, map_w;
-    if (!tensor_map(&map_a, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, (uint32_t)BM)) return CELLM_ERR_ARG;
-    if (!tensor_map(&map_w, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw * 2, (uint32_t)bn)) return CELLM_ERR_ARG;
-    if (bn == 128) {
-        if (out_dtype == CELLM_F32) return launch_persistent<128, 6, 0, float>(map_a, map_w, (float*)C, M, N, K, ldc, 0, err, stream, bn, nullptr, 6, act_numbers);
-        return launch_persistent<128, 6, 0, __nv_bfloat16>(map_a, map_w, (__nv_bfloat16*)C, M, N, K, ldc, 0, err, stream, bn, nullptr, 6, act_numbers);
-    }
-    if (out_dtype == CELLM_F32) return launch_persistent<256, 4, 0, float>(map_a, map_w, (float*)C, M, N, K, ldc, 0, err, stream, bn, nullptr, 6, act_numbers);
-    return launch_persistent<256, 4, 0, __nv_bfloat16>(map_a, map_w, (__nv_bfloat16*)C, M, N, K, ldc, 0, err, stream, bn, nullptr, 6, act_numbers);
+    return launch_unsplit<0>(C, A, W, M, N, K, 1, lda, ldw, ldc, out_dtype, 0, err, stream, N > 128 ? 256 : 128, nullptr, 6, act_numbers, GateEpi());
 }
 
 // The product described above gemm_impl.

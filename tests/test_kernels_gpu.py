@@ -690,6 +690,36 @@ def test_gemm_tcgen05(out, M, N, K, bn, split):
     assert float((c.double() - ref).abs().max()) <= k * (1 + float(ref.abs().max()))
 
 
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K,bn,epilogue", [
+    (2048, 6144, 2048, 240, 0), (2001, 16392, 1032, 256, 0), (256, 264, 6008, 256, 0), (130, 150, 9800, 160, 0), (129, 128, 12000, 128, 0),
+    (2001, 16512, 1032, 256, 1), (300, 384, 12008, 128, 1)])
+def test_gemm_tcgen05_on_pairs_of_sms(out, M, N, K, bn, epilogue):
+    """Products long enough for pairs, with rows, columns and a piece of K that fill no tile (the second CTA's half of a tile may
+    lie wholly outside): near the exact sums, and bit for bit what short products of the same rows, which single CTAs do, give."""
+    from cellm_b200.ops.gemm_bf16 import error_word, gemm_tcgen05
+    a = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
+    w = (torch.randn(N, K, device=DEV) * 0.05).bfloat16()
+    c = gemm_tcgen05(a, w, out, bn, 1, epilogue=epilogue)
+    torch.cuda.synchronize()
+    assert error_word(a.device).item() == 0
+    ref = a.double() @ w.double().T
+    if epilogue == 0:
+        # each of the K / 16 steps may cut a unit of 32-bit rounding off the running sum (K = 12,000: 9e-5 of its size)
+        k = 2.0 ** -23 * K / 16 if out == torch.float32 else 6e-3
+        assert float((c.double() - ref).abs().max()) <= k * (1 + float(ref.abs().max()))
+    else:
+        g, u = ref.reshape(M, -1, 2, 64).unbind(2)
+        want = (torch.nn.functional.silu(g) * u).reshape(M, N // 2)
+        assert float((c.double() - want).abs().max()) <= 6e-3 * (1 + float(want.abs().max()))
+    # one row tile of a hundred rows and few columns: less work than a pair is given
+    n = min(N, 1024) // 128 * 128
+    if 256 * -(-K // 64) < 90 * 256:
+        for m0 in (0, M - 100):
+            few = gemm_tcgen05(a[m0:m0 + 100].contiguous(), w[:n], out, bn, 1, epilogue=epilogue)
+            assert torch.equal(few, c[m0:m0 + 100, :few.shape[1]])
+
+
 @pytest.mark.parametrize("M,ff,K,bn,split", [(8, 192, 64, -16, 1), (3, 128, 2048, -16, 4), (40, 320, 96, -64, 1), (64, 64, 512, -64, 2),
                                               (150, 256, 512, -64, 1), (100, 128, 1024, -64, 4), (400, 192, 2048, 128, 8),
                                               (130, 192, 64, 128, 1), (300, 256, 1024, 256, 1), (70, 128, 4096, 128, 4), (200, 384, 2048, 256, 2),
