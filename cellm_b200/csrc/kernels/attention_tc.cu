@@ -31,6 +31,8 @@
 // crates/cellm-cache/src/kvcache.rs:753-787, :1206-1227.
 //
 // Cache layout of one layer: [page][kv_head][slot in page][64].
+#include <climits>
+
 #include "tcgen05_attn.cuh"
 
 namespace {
@@ -261,11 +263,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int qt = warp & 3;                                      // quarter of the tile's rows = of tensor memory's lanes
         const int r = qt * 32 + lane;                                 // row of the tile = lane of tensor memory
         const int tok = tr[t].tok0 + r / G;                           // token within the portion
-        // where G is no divisor of 128 the rows behind the tile's last token are nobody's: their queries were never
-        // loaded, every score of theirs is masked and nothing of them is written
+        // where G is no divisor of 128 the rows behind the tile's last token are nobody's: their queries were never loaded and
+        // nothing of them is written. They count as seeing every key: masked row by row they sent their warp, and with it
+        // the tile, through the masking of 128 scores in every block: 442 us instead of 295 for a layer of 24 heads over 8,
+        // 2,048 queries behind 8,192 keys.
         const bool row_ok = r < tok_per_tile * G && tok < q_len;
-        const int pos = row_ok ? ctx + tok : -1;
-        const int lo = first_key(pos, window, chunk);
+        const int pos = row_ok ? ctx + tok : INT_MAX;
+        const int lo = row_ok ? first_key(pos, window, chunk) : INT_MIN;
         const uint32_t lane_base = tmem + ((uint32_t)(qt * 32) << 16);
         const uint32_t s_col = (uint32_t)(t * TN);
         const uint32_t o_col = (uint32_t)(O_COL + t * HD);
@@ -284,7 +288,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             tc_fence_before();
             mbar_arrive(&sm.s_empty[t]);                              // the scores are in registers now
             const int jbase = (tr[t].lo + it) * TN;
-            const bool open_block = row_ok && jbase + TN - 1 <= pos && jbase >= lo;
+            const bool open_block = jbase + TN - 1 <= pos && jbase >= lo;
             if (!open_block) {
 #pragma unroll
                 for (int i = 0; i < TN; ++i) {
@@ -443,7 +447,7 @@ CELLM_API int cellm_attention_tc_supports(int hd, int nh, int nkv, int page_size
 }
 
 // Groups that do not divide 128 leave a tile's last rows empty (2 of 128 for G = 3, 32 at most here). They are taken where at
-// least three quarters of the rows are in use: with 24 heads over 8, 2,048 queries behind 8,192 keys, the layer takes 509 us
+// least three quarters of the rows are in use: with 24 heads over 8, 2,048 queries behind 8,192 keys, the layer takes 295 us
 // here and 813 us on the mma.sync kernel, a ratio that a quarter of a tile does not use up. `uneven`: 0 for the entry points
 // that take divisors only.
 static bool attention_tc_takes(int hd, int nh, int nkv, int page_size, int uneven) {
@@ -509,7 +513,7 @@ CELLM_API int cellm_attention_tc(void* out, const void* q, const void* k_pool, c
 // every pair of tiles in `nsplit` pieces (a CTA each) whose results meet in part_o [nsplit, T * nh, 64] and part_ml
 // [nsplit, T * nh, 2] and are merged by a second kernel: where the pairs fill the SMs' last round badly (200 CTAs of 72
 // blocks on 148 SMs are two rounds, 400 of 36 three of half the length: a layer of 24 heads over 8, 2,048 queries behind
-// 8,192 keys, 509 us whole and 442 in two pieces). The caller chooses.
+// 8,192 keys, 509 us whole and 442 in two pieces, both before rows of no token were left unmasked). The caller chooses.
 CELLM_API int cellm_attention_tc_split(void* out, float* part_o, float* part_ml, const void* q, const void* k_pool, const void* v_pool,
                                        const int* cu_seqlens, const int* ctx_lens, const int* block_table, int bt_stride,
                                        int B, int T, int n_tiles, int num_pages, int page_size, int nh, int nkv, int hd,
