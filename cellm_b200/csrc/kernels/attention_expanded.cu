@@ -24,6 +24,8 @@
 // Sinks (one more term in a row's denominator) and the output gate (sigmoid of one number per token and head) enter in the
 // epilogue. Every wait on an mbarrier is bounded: a role that gives up sets CELLM_DEV_WAIT_TIMEOUT and an abort flag; the
 // CTA frees its tensor memory and returns.
+#include <climits>
+
 #include "tcgen05_attn.cuh"
 
 namespace {
@@ -266,8 +268,10 @@ attention_expanded_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         const int qt = warp & 3;                                      // quarter of the tile's rows = of tensor memory's lanes
         const int tok = (t ? tok0[1] : tok0[0]) + qt * 32 + lane;                     // token within the portion
         const bool row_ok = tok < q_len;
-        const int pos = row_ok ? ctx + tok : -1;
-        const int lo = window > 0 ? pos - window + 1 : 0;
+        // rows behind the portion's end count as seeing every key (nothing of them is written): masked row by row they sent
+        // their warp, and the tile that waits for it, through the masking of 128 scores in every block (a portion that ends one token into a tile: 0.4 us of a layer).
+        const int pos = row_ok ? ctx + tok : INT_MAX;
+        const int lo = row_ok && window > 0 ? pos - window + 1 : 0;
         const uint32_t lane_base = tmem + ((uint32_t)(qt * 32) << 16);
         const uint32_t s_col = (uint32_t)(t * TN), o_col = (uint32_t)(O_COL + t * TN);
         const int n_blocks = hi_t - lo_t;
@@ -284,14 +288,8 @@ attention_expanded_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
             for (int c = 0; c < TN / 32; ++c) tmem_ld32_nowait(lane_base + s_col + (uint32_t)(c * 32), s + c * 32);
             tmem_ld_wait();
             const int jbase = (lo_t + it) * TN;
-            const bool open_block = row_ok && jbase + TN - 1 <= pos && jbase >= lo;
-            if (!open_block) {
-#pragma unroll
-                for (int i = 0; i < TN; ++i) {
-                    const int key = jbase + i;
-                    if (!(key <= pos && key >= lo)) s[i] = 0xff800000u;            // -inf
-                }
-            }
+            const bool open_block = jbase + TN - 1 <= pos && jbase >= lo;
+            if (!open_block) mask_scores<TN>(s, lo - jbase, pos - jbase);
             float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
             for (int i = 0; i < TN; i += 4) {

@@ -269,7 +269,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // 2,048 queries behind 8,192 keys.
         const bool row_ok = r < tok_per_tile * G && tok < q_len;
         const int pos = row_ok ? ctx + tok : INT_MAX;
-        const int lo = row_ok ? first_key(pos, window, chunk) : INT_MIN;
+        const int lo = row_ok ? first_key(pos, window, chunk) : 0;
         const uint32_t lane_base = tmem + ((uint32_t)(qt * 32) << 16);
         const uint32_t s_col = (uint32_t)(t * TN);
         const uint32_t o_col = (uint32_t)(O_COL + t * HD);
@@ -289,13 +289,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             mbar_arrive(&sm.s_empty[t]);                              // the scores are in registers now
             const int jbase = (tr[t].lo + it) * TN;
             const bool open_block = jbase + TN - 1 <= pos && jbase >= lo;
-            if (!open_block) {
-#pragma unroll
-                for (int i = 0; i < TN; ++i) {
-                    const int key = jbase + i;
-                    if (!(key <= pos && key >= lo)) s[i] = 0xff800000u;            // -inf
-                }
-            }
+            if (!open_block) mask_scores<TN>(s, lo - jbase, pos - jbase);
             float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
             for (int i = 0; i < TN; i += 4) {
