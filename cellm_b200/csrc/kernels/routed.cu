@@ -391,7 +391,9 @@ expert_gate_up_kernel(TA* __restrict__ mid, TA* __restrict__ smid, const TA* __r
     } else {
         const int slot = blockIdx.x, e = min(max(idx[slot], 0), E - 1);
         base = gu + (size_t)e * 2 * ff * H;
-        if (warp == 0) {
+        if (tg == 1) {
+            if (threadIdx.x == 0) group[0] = slot, group[EXPERT_TOKENS] = 1;
+        } else if (warp == 0) {
             int rank = 0, before = 0;            // slots of this expert seen so far; those in front of this one
             for (int i0 = 0; i0 < slots; i0 += 32) {
                 const int i = i0 + lane;
@@ -549,9 +551,9 @@ static int experts_rowwise_impl(void* out, void* mid, void* smid, const void* y,
     const int up_rows = ff > sff ? ff : sff;
     const int rpw_up = expert_rows_a_warp((long long)T * top * ff + (sup ? (long long)T * sff : 0), EXPERT_WARPS, gated ? 2 : 4, 4);
     const int rpw_down = expert_rows_a_warp((long long)T * H, EXPERT_DOWN_WARPS, 4, 2);
-    // gated: as many tokens' rows at once as 32 KB hold (one always fits where it did)
+    // gated: as many tokens' rows at once as 32 KB hold (one always fits where it did); a token's own experts are different ones
     const size_t row_y = (size_t)H * (dtype == CELLM_F32 ? 4 : 2);
-    const int tg = !gated ? 1 : 4 * row_y <= 32 * 1024 ? 4 : 2 * row_y <= 32 * 1024 ? 2 : 1;
+    const int tg = !gated || T == 1 ? 1 : 4 * row_y <= 32 * 1024 ? 4 : 2 * row_y <= 32 * 1024 ? 2 : 1;
     const size_t smem_y = tg * row_y;
     const dim3 grid_up((unsigned)(T * top + (sup ? (T + tg - 1) / tg : 0)), (unsigned)((up_rows + EXPERT_WARPS * rpw_up - 1) / (EXPERT_WARPS * rpw_up)));
     const dim3 grid_down((unsigned)T, (unsigned)((H + EXPERT_DOWN_WARPS * rpw_down - 1) / (EXPERT_DOWN_WARPS * rpw_down)));
