@@ -480,8 +480,8 @@ delta_prep_kernel(float* __restrict__ qk, float* __restrict__ v_out, float* __re
 // Many tokens, heads of 32 K entries, NT taps: a warp takes a q or k head, 32 K channels of v or a head's decays through a run of
 // neighbouring tokens with its taps in registers (the taps' loads lie 4 NT bytes apart and cost more than the rows', which
 // the taps share through L1); all rows of a token travel together. The same sums in the same order as above, whatever the run.
-// 2,048 tokens of 4,096 channels: 104 us with a block a token; the layer's mixer went from 414 to 353 us. Fewer than 64 tokens are
-// too few warps this way and stay with the blocks.
+// 2,048 tokens of 4,096 channels: 104 us with a block a token; the layer's mixer went from 414 to 353 us. Below 512 tokens the
+// form above cuts a token into several blocks and is the better one (a mixer over 90 tokens 155 us, 167 with runs of two).
 template <int K, int NT>
 __global__ void __launch_bounds__(256)
 delta_prep_run_kernel(float* __restrict__ qk, float* __restrict__ v_out, float* __restrict__ beta, float* __restrict__ decay,
@@ -580,9 +580,9 @@ CELLM_API int cellm_delta_prep(float* qk, float* v_out, float* beta, float* deca
     cv.proj = proj; cv.ld = ld; cv.col0 = col0; cv.bias = nullptr; cv.taps = taps; cv.state = nullptr; cv.n_taps = n_taps;
     cv.C = 2 * kvh * dim + heads * vd;
     if (dim > RECURRENT_MAX_DIM) return CELLM_ERR_SIZE;
-    if (T >= 64 && (dim == 64 || dim == 128) && n_taps >= 2 && n_taps <= 4) {
+    if (T >= 512 && (dim == 64 || dim == 128) && n_taps >= 2 && n_taps <= 4) {
         // runs of eight tokens, shorter ones where they would leave SMs idle
-        const int run = T >= 1024 ? 8 : T >= 256 ? 4 : 2, units = 2 * kvh + (heads * vd + dim - 1) / dim + heads + 1;
+        const int run = T >= 1024 ? 8 : 4, units = 2 * kvh + (heads * vd + dim - 1) / dim + heads + 1;
 #define PREP_RUN(K, NT)                                                                                            \
     CELLM_RUN((delta_prep_run_kernel<K, NT>), dim3((T + run - 1) / run, (units + 7) / 8), 256, 0, stream, qk, v_out, beta, decay, cv, slot_stride, \
               n_slots, state, col_b, a2, ld_a2, dt_bias, A_log, seq_of_token, cu_seqlens, slot_ids, T, run, heads, kvh, dim, vd, l2_eps, err)
