@@ -164,7 +164,7 @@ class Program:
         self._keep += [a, b, per_layer, layer_arr, order_arr]
         self.program = p
         self._arena = self._gemm_ws = self._attn_ws = None
-        self._live = None               # (ctx, bindings, logit rows, logits, arena, tensors of Python parts) of the running step
+        self._live = None               # (ctx, bindings, logit rows, logits, buffers, tensors of Python parts) of the running step
         self._raised: Optional[BaseException] = None
         self.last_launches = 0
 
@@ -217,16 +217,19 @@ class Program:
         s.counters = counters(self.device).data_ptr()
         return s, (items, q_lens, ctx_lens)
 
-    def _buffers(self, s, need) -> torch.Tensor:
+    def _buffers(self, s, need) -> tuple:
+        """The step's arena and workspaces (None: not needed), their addresses in `s`. The caller holds them until its launches
+        are queued: under capture nobody else does, and the next tensor would be given the same memory."""
         arena = self._grow("_arena", need[0] + 256, torch.uint8)
         s.arena, s.arena_bytes = arena.data_ptr(), arena.numel()
+        gemm_ws = attn_ws = None
         if need[1]:
-            ws = self._grow("_gemm_ws", need[1], torch.float32)
-            s.gemm_ws, s.gemm_ws_floats = ws.data_ptr(), ws.numel()
+            gemm_ws = self._grow("_gemm_ws", need[1], torch.float32)
+            s.gemm_ws, s.gemm_ws_floats = gemm_ws.data_ptr(), gemm_ws.numel()
         if need[2]:
-            ws = self._grow("_attn_ws", need[2], torch.float32)
-            s.attn_ws, s.attn_ws_floats = ws.data_ptr(), ws.numel()
-        return arena
+            attn_ws = self._grow("_attn_ws", need[2], torch.float32)
+            s.attn_ws, s.attn_ws_floats = attn_ws.data_ptr(), attn_ws.numel()
+        return arena, gemm_ws, attn_ws
 
     def forward(self, ctx, bindings, logit_rows: Optional[torch.Tensor], max_layers: Optional[int] = None,
                 stream: Optional[int] = None) -> Optional[torch.Tensor]:
@@ -239,10 +242,10 @@ class Program:
         need = (R.I64 * 3)()
         if self._rt.cellm_exec_need(ctypes.byref(p), ctypes.byref(s), need) != 0:
             raise CacheError(last_error())
-        arena = self._buffers(s, need)
+        lent = self._buffers(s, need)
         logits = torch.empty((s.R, p.V), dtype=torch.float32, device=self.device) if s.R else None
         s.logits = logits.data_ptr() if s.R else None
-        self._live, self._raised = (ctx, bindings, logit_rows, logits, arena, {}), None
+        self._live, self._raised = (ctx, bindings, logit_rows, logits, lent, {}), None
         try:
             rc = self._rt.cellm_exec_forward(ctypes.byref(p), ctypes.byref(s))
         finally:
@@ -283,11 +286,12 @@ class Program:
         op = ctypes.byref(record.op)
         if self._rt.cellm_exec_part(ctypes.byref(p), ctypes.byref(s), op, x.data_ptr(), None, 1, need) != 0:
             raise ValueError(f"native executor: {last_error()}")
-        self._buffers(s, need)
+        lent = self._buffers(s, need)
         if out is None:
             out = torch.empty((s.T, p.H), dtype=self.dtype, device=x.device)
         if self._rt.cellm_exec_part(ctypes.byref(p), ctypes.byref(s), op, x.data_ptr(), out.data_ptr(), 0, need) != 0:
             raise _kernel_error(last_error())
+        del lent                # (not before the launches are queued)
         klib.count_launch(int(s.launches))
         _count_calls(s)
         return out
@@ -296,7 +300,7 @@ class Program:
     def _view(self, address: int, shape, dtype) -> torch.Tensor:
         """The tensor behind an address the executor names: a buffer of the step's arena, or what a Python part
         left earlier in this step."""
-        ctx, bindings, rows, logits, arena, mine = self._live
+        ctx, bindings, rows, logits, (arena, *_), mine = self._live
         t = mine.get(address)
         if t is not None:
             return t
@@ -329,7 +333,7 @@ class Program:
             from ..parts.base import Residual
             role, part = self.python_parts[token]
             regs = regs_ptr.contents
-            ctx, bindings, rows, logits, arena, mine = self._live
+            ctx, bindings, rows, logits, _, mine = self._live
             T, H = ctx.T, self.program.H
             x = self._view(regs.x, (T, H), torch.float32)
             pending = self._view(regs.pending, (T, H), self.dtype) if regs.pending else None

@@ -88,6 +88,36 @@ def test_a_parts_own_forward_launches_what_its_record_launches_in_the_program(mo
     assert [c for part in alone for c in sizes(part)] == in_program
 
 
+@pytest.mark.parametrize("tokens", [3, 200])
+def test_a_captured_steps_memory_is_held_until_its_launches_are_queued(monkeypatch, tokens):
+    """Under capture the arena and the workspaces are tensors of the call's own: were they dropped before the launches, the
+    result (made after them) would be given the same memory, and a product would write over what it still reads."""
+    import weakref
+    from cellm_b200.ops import _lib
+    from cellm_b200.runtime.program import Program
+    lent, gone = [], []
+    check = lambda *a: gone.extend(r for r in lent if r() is None)
+    Recorder(monkeypatch, hooks={name: check for sigs in _lib._SIGNATURES.values() for name in sigs})
+    cfg, plan, model = zero_model(dict(SMALL, intermediate_size=4096))
+    step = run_step(model, plan, [tokens], [0], prepare_only=True)
+    grow = Program._grow
+
+    def remembered(self, name, n, dtype):
+        t = grow(self, name, n, dtype)
+        lent.append(weakref.ref(t))
+        return t
+    monkeypatch.setattr(Program, "_grow", remembered)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    x = torch.zeros((tokens, 256), dtype=torch.bfloat16)
+    for call in (lambda: step.run(model.forward), lambda: model.blocks[0].mixer.forward(x, step.ctx, step.bindings[0]),
+                 lambda: model.blocks[1].mixer.forward(x, step.ctx, step.bindings[1]),
+                 lambda: model.blocks[2].feed_forward.forward(x, step.ctx)):
+        del lent[:]
+        call()
+        assert lent and not gone
+        assert all(r() is None for r in lent)           # and is given back then
+
+
 def test_a_part_without_a_record_is_called_back_between_native_parts(monkeypatch):
     """A norm and a mixer defined here, with forward() only: the executor runs the native records around them and
     calls the interpreter for these two, with the registers they are to work on."""
