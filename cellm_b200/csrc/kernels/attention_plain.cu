@@ -287,18 +287,20 @@ attention_rows_kernel(const RowsArgs a) {
                     }
                 }
             }
-            // whether every row of the block sees every key of this block
-            bool paged = true;
+            // which of the thread's keys have a page: read before the barrier, behind which a warp that is ahead may already put the
+            // pages of the block after the next in this place
+            unsigned paged = 0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) paged &= pages[c & 1][x + 16 * j] >= 0;
-            const bool open = __syncthreads_and(paged) && j0 + ROWS_KEYS - 1 <= first_pos && (a.window <= 0 || j0 > last_pos - a.window);
+            for (int j = 0; j < 4; ++j) paged |= (pages[c & 1][x + 16 * j] >= 0 ? 1u : 0u) << j;
+            // whether every row of the block sees every key of this block
+            const bool open = __syncthreads_and(paged == 15u) && j0 + ROWS_KEYS - 1 <= first_pos && (a.window <= 0 || j0 > last_pos - a.window);
 #pragma unroll
             for (int i = 0; i < RI; ++i) {
                 float s[4], top = -INFINITY;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int key = j0 + x + 16 * j;
-                    const bool sees = key <= pos[i] && key >= lo[i] && pages[c & 1][x + 16 * j] >= 0;
+                    const bool sees = key <= pos[i] && key >= lo[i] && (paged >> j & 1u);
                     s[j] = sees ? (s4[i][j].x + s4[i][j].y) + (s4[i][j].z + s4[i][j].w) : -INFINITY;
                     top = fmaxf(top, s[j]);
                 }

@@ -443,6 +443,22 @@ def test_attention_in_32_bits_does_not_depend_on_the_cutting(nh, nkv, hd, ps, wi
     assert e.item() == 0
 
 
+@pytest.mark.parametrize("window", [0, 260])
+def test_attention_in_32_bits_over_many_blocks_of_keys(window):
+    """Three and more blocks of 64 keys, the last with one key or a few: whether a key has a page must be known of the block at hand
+    in every warp, also in one that is behind while the next blocks' pages are looked up. The same bits over and over, near the oracle."""
+    from cellm_b200 import ops
+    nh, nkv, hd, ps = 24, 8, 64, 16
+    lens, ctxs = [150, 1, 40, 9], [171, 1024, 473, 248]
+    c = paged_case(lens, ctxs, nh, nkv, hd, ps, torch.float32, seed=12)
+    e = err_word()
+    run = lambda: ops.attention_plain(c["q"], c["kp"], c["vp"], c["pos"], c["seq"], c["bt"], nh, hd ** -0.5, window, e)
+    out = run()
+    close(out, attention_reference(c, nh, nkv, hd, hd ** -0.5, window), torch.float32)
+    assert all(torch.equal(run(), out) for _ in range(50))
+    assert e.item() == 0
+
+
 @pytest.mark.parametrize("kernel", ["plain32", "plain16", "flash", "decode", "tc"])
 def test_a_far_key_among_hundreds_is_found(kernel):
     """One early key is scaled so that its score towers over 600 others: the
