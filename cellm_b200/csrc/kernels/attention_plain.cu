@@ -201,10 +201,10 @@ attention_rows_kernel(const RowsArgs a) {
     pdl_wait();
     const int t_end = min(a.T, (int)(blockIdx.x + 1) * a.tokens);
     for (int t0 = blockIdx.x * a.tokens; t0 < t_end;) {
-        // the block's next tokens of one request: t0 .. t0 + n - 1
+        // the block's next tokens of one request, positions ascending (the first's and the last's bound the keys): t0 .. t0 + n - 1
         const int b = a.seq_of_token[t0];
         int n = 1;
-        while (t0 + n < t_end && a.seq_of_token[t0 + n] == b) ++n;
+        while (t0 + n < t_end && a.seq_of_token[t0 + n] == b && a.positions[t0 + n] >= a.positions[t0 + n - 1]) ++n;
         const int* bt = a.block_table + (size_t)b * a.bt_stride;
         const int first_pos = a.positions[t0], last_pos = a.positions[t0 + n - 1];
         const int lo_all = a.window > 0 ? max(0, first_pos - a.window + 1) : 0;

@@ -443,6 +443,26 @@ def test_attention_in_32_bits_does_not_depend_on_the_cutting(nh, nkv, hd, ps, wi
     assert e.item() == 0
 
 
+@pytest.mark.parametrize("window", [0, 20])
+def test_attention_in_32_bits_takes_tokens_in_any_order(window):
+    """Enough tokens that a block takes several of a request: in any order of the tokens every one gets the bits it gets in theirs."""
+    from cellm_b200 import ops
+    nh, nkv, hd, ps = 24, 8, 64, 16
+    c = paged_case([90, 70, 60], [3, 130, 0], nh, nkv, hd, ps, torch.float32, seed=13)
+    e = err_word()
+    run = lambda at: ops.attention_plain(c["q"][at].contiguous(), c["kp"], c["vp"], c["pos"][at].contiguous(), c["seq"][at].contiguous(), c["bt"],
+                                         nh, hd ** -0.5, window, e)
+    T = len(c["pos"])
+    whole = run(torch.arange(T, device=DEV))
+    close(whole, attention_reference(c, nh, nkv, hd, hd ** -0.5, window), torch.float32)
+    g = torch.Generator().manual_seed(2)
+    some = torch.randperm(T, generator=g)
+    within = torch.cat([90 + torch.randperm(70, generator=g), torch.arange(90).flip(0), torch.arange(160, T)])
+    for at in (torch.arange(T).flip(0), some, within):
+        assert torch.equal(run(at.to(DEV)), whole[at.to(DEV)])
+    assert e.item() == 0
+
+
 @pytest.mark.parametrize("window", [0, 260])
 def test_attention_in_32_bits_over_many_blocks_of_keys(window):
     """Three and more blocks of 64 keys, the last with one key or a few: whether a key has a page must be known of the block at hand
