@@ -23,7 +23,12 @@
 // While one tile's softmax runs, the tensor cores work on the other tile. The output
 // accumulators stay in tensor memory; one is rescaled (read, multiplied, written
 // back) only when a row's maximum has grown by more than 2^8 since the last rescale,
-// so most blocks skip that pass; the stale maximum only scales P.
+// so most blocks skip that pass; the stale maximum only scales P. Groups that do not
+// divide 128 rescale whenever a maximum grows: a row's largest weight is then 1 and
+// is not rounded (behind 8,192 random keys P's rounding costs the result 0.00161 of
+// its size so and 0.00168 with a stale maximum), as in the mma.sync kernel, which
+// took them before. 2,048 queries of 24 heads over 8 behind 8,192 keys: 246 us with
+// a stale maximum, 255 so.
 //
 // Every wait on an mbarrier is bounded, as in gemm_tcgen05.cu: a role that gives up
 // sets CELLM_DEV_WAIT_TIMEOUT and an abort flag; the CTA frees its tensor memory and
@@ -81,7 +86,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const int* __restrict__ cu_seqlens, const int* __restrict__ ctx_lens,
                     const int* __restrict__ block_table, int bt_stride, int B, int num_pages, int page_size, int nh,
                     int nkv, float scale_log2e, int window, const float* __restrict__ sinks, const float* __restrict__ gate,
-                    long long gate_ld, int chunk, int nsplit, float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ err) {
+                    long long gate_ld, int chunk, float step, int nsplit, float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     TcSmem& sm = *reinterpret_cast<TcSmem*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -297,9 +302,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 mx2 = fmaxf(mx2, __uint_as_float(s[i + 2])); mx3 = fmaxf(mx3, __uint_as_float(s[i + 3]));
             }
             const float m_new = fmaxf(m, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * scale_log2e);
-            // rescale O only when the maximum has grown much (or nothing has been accumulated with it yet);
+            // rescale O only when the maximum has grown by more than `step` (or nothing has been accumulated with it yet);
             // the accumulator (and below, P) is free once the last block's P.V is done
-            const bool want = m_new > m + RESCALE_STEP || (m == -INFINITY && m_new != -INFINITY);
+            const bool want = m_new > m + step || (m == -INFINITY && m_new != -INFINITY);
             bool pv_seen = it == 0;
             if (__any_sync(0xffffffffu, want)) {
                 if (it > 0) {
@@ -488,7 +493,7 @@ static int attention_tc_impl(void* out, const void* q, const void* k_pool, const
     dim3 grid((unsigned)n_tiles, (unsigned)nkv, (unsigned)nsplit);
     CELLM_RUN(attention_tc_kernel, grid, THREADS, smem, stream, mq, mk, mv, (__nv_bfloat16*)out, cu_seqlens,
               ctx_lens, block_table, bt_stride, B, num_pages, page_size, nh, nkv, scale * 1.4426950408889634f, window, sinks,
-              gate, gate_ld, chunk, nsplit, part_o, part_ml, err);
+              gate, gate_ld, chunk, 128 % G ? 0.f : RESCALE_STEP, nsplit, part_o, part_ml, err);
     if (nsplit > 1)
         CELLM_RUN(attention_tc_merge_kernel, (unsigned)(((long long)T * nh + 15) / 16), 256, 0, stream, (__nv_bfloat16*)out, part_o, part_ml,
                   (long long)T * nh, nsplit);
