@@ -404,7 +404,9 @@ struct Run {
 
     void feed_forward(const SwiGLUParams& L, const void* x, void* out);
     void gated_mlp(const GatedMlpParams& L, const void* x, void* out);
+    double tc_key_blocks(i64 window) const;
     i64 tc_pieces(i64 ctas, i64 nh, i64 window) const;
+    bool tc_uneven_pays(i64 ctas, i64 nsplit, i64 window) const;
     void routed_mlp(const RoutedMlpParams& L, const void* x, void* out);
     void mingru(const MinGruParams& L, const ExecItem& it, const void* x, void* out);
     void latent_attention(const LatentAttentionParams& L, const ExecItem& it, const void* x, void* out);
@@ -648,8 +650,9 @@ void* Run::attend(const AttentionParams& L, const ExecItem& it, const void* q, v
             i64 tc_tiles = 0;
             for (i64 b = 0; b < s.B; ++b) tc_tiles += ceil_div(s.q_lens[b], per_tile);
             const i64 min_ctas = p.tc_min_ctas < 0 ? p.sms / 8 : p.tc_min_ctas;
-            if (tc_tiles * nkv >= min_ctas && (double)T >= p.tc_min_fill * (double)(tc_tiles * per_tile)) {
-                const i64 nsplit = tc_pieces(tc_tiles * nkv, nh, L.window);
+            const i64 nsplit = tc_pieces(tc_tiles * nkv, nh, L.window);
+            if (tc_tiles * nkv >= min_ctas && (double)T >= p.tc_min_fill * (double)(tc_tiles * per_tile) &&
+                (128 % G == 0 || p.tc_min_ctas >= 0 || tc_uneven_pays(tc_tiles * nkv, nsplit, L.window))) {
                 if (nsplit == 1 && 128 % G == 0) {
                     LAUNCH(fn<AttentionTcFn>(FN_ATTENTION_TC)(o, q, it.k, it.v, s.cu_seqlens, s.ctx_lens, it.block_table, (int)it.bt_stride,
                                                           (int)s.B, (int)T, (int)tc_tiles, (int)it.num_pages, (int)ps, (int)nh, (int)nkv,
@@ -713,18 +716,34 @@ void* Run::attend(const AttentionParams& L, const ExecItem& it, const void* q, v
     return o;
 }
 
+// Blocks of 128 keys that a CTA of the tcgen05 prompt attention walks, on average over the tokens.
+double Run::tc_key_blocks(i64 window) const {
+    double blocks = 0;
+    for (i64 b = 0; b < s.B; ++b) {
+        const double keys = s.host_ctx_lens ? (double)s.host_ctx_lens[b] + 0.5 * (double)s.q_lens[b] : (double)s.max_total_len;
+        blocks += (double)s.q_lens[b] * (window > 0 ? std::min(keys, (double)window) : keys) / 128.0;
+    }
+    return blocks / (double)s.T + 1.0;
+}
+
+// Whether a group of heads that does not divide 128 goes to the tcgen05 kernel: where its CTAs fill a third of the SMs and see
+// more than 64 keys, or see more than 176 and are a fifth of them, short of work each (six blocks) or cut into pieces. What was
+// measured beside it is the mma.sync kernel of the same steps, 296 of them (groups of 3, 6, 7 and 21; 1 to 12 portions of 20
+// to 420 tokens behind 0 to 3,000): up to 2.7 times as long where the line says yes, at most 4 % shorter; where it says
+// no the tcgen05 kernel took up to 1.4 times as long (12 x 20 tokens of 21 heads over 1: 8.8 against 6.4 us; 300 tokens behind
+// 1,500 in one piece: 35 against 29 us), and was at most a quarter faster.
+bool Run::tc_uneven_pays(i64 ctas, i64 nsplit, i64 window) const {
+    const i64 keys = window > 0 ? std::min<i64>(s.max_total_len, window + s.max_q_len) : s.max_total_len;
+    return (keys > 64 && ctas >= p.sms * 5 / 16) || (keys > 176 && (ctas >= p.sms / 5 || nsplit > 1 || tc_key_blocks(window) <= 6.0));
+}
+
 // Into how many pieces the tcgen05 prompt attention cuts every pair of tiles' keys: the rounds of CTAs over the SMs (one an SM)
 // times a CTA's length in blocks of 128 keys, plus two blocks' time to start and to end it, plus the pieces' way through memory
 // (about 3 us a block, 6 TB/s). Taken where that is a tenth shorter than whole; steps whose contexts the host does not
 // know stay whole.
 i64 Run::tc_pieces(i64 ctas, i64 nh, i64 window) const {
     if (!s.host_ctx_lens) return 1;
-    double blocks = 0;          // of a CTA, on average over the tokens
-    for (i64 b = 0; b < s.B; ++b) {
-        const double keys = (double)s.host_ctx_lens[b] + 0.5 * (double)s.q_lens[b];
-        blocks += (double)s.q_lens[b] * (window > 0 ? std::min(keys, (double)window) : keys) / 128.0;
-    }
-    blocks = blocks / (double)s.T + 1.0;
+    const double blocks = tc_key_blocks(window);
     i64 best = 1;
     double least = 0;
     for (i64 n = 1; n <= 8 && (double)n * 8.0 <= std::max(blocks, 8.0); ++n) {

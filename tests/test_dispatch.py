@@ -12,6 +12,9 @@ WIDE = {"architectures": ["Lfm2ForCausalLM"], "model_type": "lfm2", "vocab_size"
         "block_multiple_of": 256, "rope_theta": 1e6, "conv_L_cache": 3, "norm_eps": 1e-5, "tie_embedding": True,
         "max_position_embeddings": 128000}
 H, FF, V = 2048, 8192, 65536
+# an attention layer alone, small around its heads
+SHORT = dict(WIDE, num_hidden_layers=1, layer_types=["full_attention"], hidden_size=256, intermediate_size=512, vocab_size=1000,
+             block_auto_adjust_ff_dim=False)
 # positions of the arguments in the entry points' signatures
 G_M, G_N, G_K, G_OUT, G_BN, G_SPLIT, G_EPI, G_WS = 3, 4, 5, 9, 10, 11, 12, 14
 
@@ -55,6 +58,21 @@ def test_decode_attention_pieces_by_batch_and_context(monkeypatch):
         dec = rec.of("cellm_attention_decode")[0]
         assert dec[20] == want, (lens, dec[20])
         assert (dec[1] is not None) == (want > 8)                  # a workspace only beyond one cluster
+
+
+@pytest.mark.parametrize("nh,nkv,lens,ctxs,on_tcgen05", [
+    (24, 8, [2048], [8192], True), (24, 8, [300], [0], True), (24, 8, [200], [0], True), (24, 8, [200], [1000], False),
+    (24, 8, [250], [4000], True), (24, 8, [64] * 8, [0] * 8, False), (24, 8, [64] * 8, [30] * 8, True), (21, 1, [20] * 12, [0] * 12, False),
+    (28, 4, [40] * 6, [0] * 6, False), (28, 4, [40] * 6, [300] * 6, True), (32, 8, [40] * 6, [0] * 6, True), (43, 1, [900], [0], False)])
+def test_groups_that_do_not_divide_a_tile_go_to_tcgen05_where_that_pays(monkeypatch, nh, nkv, lens, ctxs, on_tcgen05):
+    """By the measured times of both kernels: not a few short portions, nor long keys before few CTAs that stay whole. Groups that
+    divide a tile, and groups that leave more than a quarter of it empty, go where they always went."""
+    rec = Recorder(monkeypatch)
+    cfg, plan, model = zero_model(dict(SHORT, num_attention_heads=nh, num_key_value_heads=nkv))
+    run_step(model, plan, lens, ctxs)
+    names = rec.names()
+    assert names.count("cellm_attention_flash") == int(not on_tcgen05)
+    assert names.count("cellm_attention_tc") + names.count("cellm_attention_tc_split") == int(on_tcgen05)
 
 
 def test_decode_step_without_the_fused_decode_kernels(monkeypatch):
