@@ -258,10 +258,10 @@ latent_decode_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_o
     __nv_bfloat16* k_s = q_s + LD_BM * stride;                              // two stages
     float* half_s = reinterpret_cast<float*>(k_s + 2 * LD_BN * stride);     // [2][16][SP]: the scores' halves
     __nv_bfloat16* p_s = reinterpret_cast<__nv_bfloat16*>(half_s + 2 * LD_BM * SP);     // [16][PP]
-    float* corr_s = reinterpret_cast<float*>(p_s + LD_BM * PP);             // [16]: the rows' factors; then maxima [16] and sums [16]
-    float* m_s = corr_s + LD_BM;
+    float* corr_s = reinterpret_cast<float*>(p_s + LD_BM * PP);             // [16][2]: the rows' factors; then maxima [16] and sums [16]
+    float* m_s = corr_s + 2 * LD_BM;
     float* l_s = m_s + LD_BM;
-    long long* row_at = reinterpret_cast<long long*>(l_s + 2 * LD_BM);      // [2][LD_BN]
+    long long* row_at = reinterpret_cast<long long*>(l_s + LD_BM);      // [2][LD_BN]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, CH = kw / 8;
     pdl_trigger();
     int tile = blockIdx.x, b = 0, rows = 0;
@@ -348,7 +348,8 @@ latent_decode_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_o
             }
         }
         __syncthreads();
-        // weights: a warp two rows, a lane two keys
+        // weights: a warp two rows, a lane two keys. The maximum moves after 32 keys and after 64, as in the kernel above: a weight
+        // is rounded against its row's maximum up to its own run of 32 keys, so that the largest of them is 1 and exact
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int r = warp * 2 + i, j = kb * LD_BN + lane * 2;
@@ -358,24 +359,30 @@ latent_decode_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_o
             const float s1 = (j + 1 <= pos[i] && j + 1 >= lo[i]) ? a.y + c.y : -INFINITY;
             float top = fmaxf(s0, s1);
 #pragma unroll
-            for (int d = 16; d; d >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
-            const float m_new = fmaxf(m[i], top * scale_log2e), use = m_new == -INFINITY ? 0.f : m_new;
-            const float corr = fast_exp2(m[i] - use);
-            m[i] = m_new;
+            for (int d = 8; d; d >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
+            const float other = __shfl_xor_sync(0xffffffffu, top, 16);
+            const float m1 = fmaxf(m[i], (lane < 16 ? top : other) * scale_log2e), m2 = fmaxf(m1, (lane < 16 ? other : top) * scale_log2e);
+            const float use1 = m1 == -INFINITY ? 0.f : m1, use2 = m2 == -INFINITY ? 0.f : m2, use = lane < 16 ? use1 : use2;
+            const float corr1 = fast_exp2(m[i] - use1), corr2 = fast_exp2(m1 - use2);
+            m[i] = m2;
             const float p0 = fast_exp2(fmaf(s0, scale_log2e, -use)), p1 = fast_exp2(fmaf(s1, scale_log2e, -use));
-            l[i] = l[i] * corr + (p0 + p1);             // a lane's share: summed over the lanes at the end
+            // a lane's share: summed over the lanes at the end
+            l[i] = lane < 16 ? (l[i] * corr1 + (p0 + p1)) * corr2 : l[i] * corr1 * corr2 + (p0 + p1);
             *reinterpret_cast<uint32_t*>(p_s + r * PP + lane * 2) = pack_bf16(p0, p1);
-            if (lane == 0) corr_s[r] = corr;
+            if (lane == 0) *reinterpret_cast<float2*>(corr_s + 2 * r) = make_float2(corr1, corr2);
         }
         __syncthreads();
         {   // O += P V over this warp's value columns
-            const float corr_a = corr_s[lane >> 2], corr_b = corr_s[(lane >> 2) + 8];
-#pragma unroll
-            for (int n = 0; n < NT; ++n) { o[n][0] *= corr_a; o[n][1] *= corr_a; o[n][2] *= corr_b; o[n][3] *= corr_b; }
+            const float2 corr_a = *reinterpret_cast<const float2*>(corr_s + 2 * (lane >> 2)), corr_b = *reinterpret_cast<const float2*>(corr_s + 2 * (lane >> 2) + 16);
             const __nv_bfloat16* p_row = p_s + (lane & 15) * PP + (lane >> 4) * 8;
             const __nv_bfloat16* v_row = ks + ((lane & 7) + (((lane >> 3) & 1) << 3)) * stride + warp * (NT * 8) + (lane >> 4) * 8;
 #pragma unroll
             for (int kk = 0; kk < LD_BN / 16; ++kk) {
+                if (kk % 2 == 0) {
+                    const float ca = kk ? corr_a.y : corr_a.x, cb = kk ? corr_b.y : corr_b.x;
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) { o[n][0] *= ca; o[n][1] *= ca; o[n][2] *= cb; o[n][3] *= cb; }
+                }
                 uint32_t pf[4];
                 ldmatrix_x4(pf, p_row + kk * 16);
 #pragma unroll

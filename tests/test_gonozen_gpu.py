@@ -629,6 +629,30 @@ def test_latent_attention_of_single_tokens(nh, kw, dv, window):
         assert int(ctx.err.item()) == 0
 
 
+@pytest.mark.parametrize("nh,kw,dv,nsplit", [(16, 576, 512, 1), (16, 576, 512, 5), (12, 320, 256, 3)])
+def test_latent_attention_of_single_tokens_rounds_as_the_other_form(nh, kw, dv, nsplit):
+    """A step of single tokens gives what the kernel for several tokens gives: the weights are rounded against the same maxima, so
+    all but the few results differ not at all whose scores' two halves, added last, round the other way."""
+    from cellm_b200 import ops
+    B, page = 9, 16
+    g = torch.Generator().manual_seed(nh + kw)
+    ctx_lens = [0, 31, 64, 200, 500, 777, 1024, 1500, 2047, 3]
+    cache, table = paged([c + 2 for c in ctx_lens], kw, page, torch.bfloat16, g)
+    pool = torch.randn(cache.k.shape, generator=g).to(torch.bfloat16).to(DEV)
+    q = (torch.randn(B + 2, nh * kw, generator=g) * 0.5).to(torch.bfloat16).to(DEV)
+
+    def run(q_lens):
+        ctx = step_ctx(q_lens, ctx_lens[:len(q_lens)])
+        out = ops.attention_latent(q[:sum(q_lens)].contiguous(), pool, ctx.cu_seqlens, ctx.ctx_lens, cache.block_table, q_lens, nh, dv, kw ** -0.5,
+                                   nsplit, ctx.err)
+        assert int(ctx.err.item()) == 0
+        return out[:B]
+    alone, beside = run([1] * B), run([1] * B + [2])            # the last request's two tokens: the kernel for several
+    assert float((alone == beside).double().mean()) > 0.98
+    # a weight that rounds the other way moves a result by 2^-8 of one term
+    assert float((alone.double() - beside.double()).norm() / beside.double().norm()) < 2.0 ** -11
+
+
 EXPANDED = [  # heads, dim, rot_dim, vdim, rank
     (4, 128, 64, 128, 512), (2, 64, 0, 64, 64), (3, 16, 16, 16, 24), (2, 48, 32, 80, 40), (1, 96, 64, 112, 128), (2, 192, 64, 128, 64), (5, 32, 0, 32, 96),
     (2, 128, 0, 48, 72), (1, 64, 96, 96, 16),
