@@ -547,6 +547,15 @@ CELLM_API int cellm_attention_latent_supports(int kw, int dv) {
     return smem <= 227 * 1024 ? 1 : 0;
 }
 
+// 1 if a step runs in tiles of 16 (token, head) rows: a token a request, and up to 16 heads or few enough tiles. Every tile of a
+// token's heads reads its keys again, which the tiles of 64 rows read once for 64 heads; that is the faster way while the tiles'
+// pieces are two rounds of CTAs at most. Times of the 64-row form over this one's, 24 to 128 heads, 1 to 32 requests behind 500
+// to 8,192 rows, kw 576 and 320, pieces as the executor cuts them: within two rounds 0.98 to 2.0, beyond 0.67 to 1.1.
+CELLM_API int cellm_attention_latent_single(int B, int T, int nh, int kw, int dv, int nsplit) {
+    return T == B && dv % 128 == 0 && dv <= 512 && decode_smem(kw) <= 227 * 1024 &&
+           (nh <= LD_BM || (long long)B * ((nh + LD_BM - 1) / LD_BM) * nsplit <= 2 * 148);
+}
+
 // q: [T, nh, kw] (a head's query against the cached rows); out: [T, nh, dv]; pool: one layer's rows. part_o
 // [nsplit, T * nh, dv] and part_ml [nsplit, T * nh, 2] floats are needed when nsplit > 1. n_tiles: the sum over the
 // requests of ceil(tokens * nh / 64). window: 0, or how many of its last rows a token reads (itself included). sinks [nh]
@@ -571,8 +580,8 @@ CELLM_API int cellm_attention_latent(void* out, float* part_o, float* part_ml, c
                       part_o, part_ml, (size_t)T * nh, dv, nsplit, sinks, gate, nh);
         return CELLM_OK;
     };
-    // a token a request: tiles of 16 rows (a request's tiles are at most its tokens times the tiles of one token)
-    if (T == B && dv % 128 == 0 && dv <= 512 && decode_smem(kw) <= 227 * 1024) {
+    // (a request's tiles are at most its tokens times the tiles of one token)
+    if (cellm_attention_latent_single(B, T, nh, kw, dv, nsplit)) {
         const dim3 dgrid((unsigned)B * (unsigned)((nh + LD_BM - 1) / LD_BM), (unsigned)nsplit);
 #define DECODE(NT)                                                                                                       \
     do {                                                                                                                 \

@@ -125,6 +125,7 @@ _SIGNATURES = {
     "attention_latent": {
         "cellm_attention_latent": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, P, P, P, P],
         "cellm_attention_latent_supports": [I, I],
+        "cellm_attention_latent_single": [I, I, I, I, I, I],
         "cellm_head_product_mma": [P, L, L, P, L, L, P, I, I, I, I, P],
     },
     "gemm_tcgen05": {

@@ -219,3 +219,14 @@ def test_a_long_portion_expands_its_keys_once(monkeypatch):
         cfg, plan, model = zero_model(config())
         run_step(model, plan, q_lens, ctx_lens)
         assert len(rec.of("cellm_attention_expanded")) == (1 if ctx_lens == [40000] else 0), (q_lens, ctx_lens)      # the window leaves few rows
+
+
+@pytest.mark.parametrize("B,T,nh,kw,dv,nsplit,small", [
+    (8, 8, 16, 576, 512, 18, 1), (64, 64, 16, 576, 512, 2, 1), (300, 300, 12, 320, 256, 1, 1), (8, 9, 16, 576, 512, 18, 0),
+    (4, 4, 32, 576, 512, 37, 1), (8, 8, 64, 576, 512, 18, 0), (32, 32, 48, 576, 512, 4, 0), (1, 1, 128, 576, 512, 16, 1), (1, 1, 128, 320, 256, 64, 0),
+    (8, 8, 16, 208, 192, 4, 0)])
+def test_which_steps_of_single_tokens_run_in_tiles_of_16_rows(B, T, nh, kw, dv, nsplit, small):
+    """A token's heads in one tile always; in several, each of which reads the keys again, while the tiles' pieces are two rounds of
+    CTAs over 148 SMs at most."""
+    from cellm_b200.ops._lib import fn
+    assert fn("attention_latent", "cellm_attention_latent_single")(B, T, nh, kw, dv, nsplit) == small

@@ -598,8 +598,8 @@ def test_latent_kernel_with_gates_and_sinks(nh, kw, dv, page, window):
 @pytest.mark.parametrize("window", [0, 1, 70])
 def test_latent_attention_of_single_tokens(nh, kw, dv, window):
     """A token a request, in tiles of 16 heads (fewer, and more than one tile): contexts of nothing, around the edges of a block
-    of 64 rows, of more blocks than two stages; whole and in more pieces than there are blocks; a step in which one request has
-    two tokens and another none. Sinks and gates. Against 64-bit torch over the same rounded inputs, bounded as the other forms."""
+    of 64 rows, of more blocks than two stages; whole and in more pieces than there are blocks (for 17 and 40 heads 30 of them go to
+    the tiles of 64 rows); a step in which one request has two tokens and another none. Sinks and gates. Against 64-bit torch over the same rounded inputs, bounded as the other forms."""
     from cellm_b200 import ops
     page = 16
     for q_lens, ctx_lens in (([1] * 6, [0, 62, 63, 64, 200, 500]), ([2, 0, 1], [63, 5, 130])):
@@ -622,7 +622,7 @@ def test_latent_attention_of_single_tokens(nh, kw, dv, window):
                 t += 1
         want = want * torch.sigmoid(gate.double())[:, :, None]
         ctx = step_ctx(q_lens, ctx_lens)
-        for nsplit in (1, 3, 8):
+        for nsplit in (1, 3, 8, 30):
             out = ops.attention_latent(q.to(DEV), pool.to(DEV), ctx.cu_seqlens, ctx.ctx_lens, cache.block_table, q_lens, nh, dv, scale, nsplit,
                                        ctx.err, window, sinks.to(DEV), gate.to(DEV))
             torch.testing.assert_close(out.cpu().double().reshape(T, nh, dv), want, rtol=2e-2, atol=1e-2)
