@@ -41,8 +41,9 @@ struct ChunkArgs {
     int per;                                // heads that share a row of q and k
     const int *cu_seqlens, *slot_ids;
     int B, min_len, heads, dim, vd;
-    float* ws;                              // a chunk's and head's numbers at (chunk * heads + head) * stride floats
+    float* ws;                              // a chunk's and head's numbers at ((chunk - chunk0) * heads + head) * stride floats
     long long stride;
+    int chunk0, chunks;                     // the step's chunks that are in the workspace
 };
 
 // A (chunk, head) in the workspace: [NV][DIM] the rows of -W and Q (HGRN2: Q alone), [CT][DIM] k E(., end), [DIM] E(., end), then
@@ -83,9 +84,9 @@ chunk_vectors_kernel(const ChunkArgs a) {
     __shared__ float beta[CT];
     pdl_trigger();
     pdl_wait();
-    const int chunk = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int t0 = 0, len = 0;
-    for (int b = 0, c = chunk; b < a.B; ++b) {
+    for (int b = 0, c = a.chunk0 + blockIdx.x; b < a.B; ++b) {
         const int start = a.cu_seqlens[b], n = a.cu_seqlens[b + 1] - start;
         if (n < a.min_len) continue;
         const int nc = (n + CT - 1) / CT;
@@ -93,7 +94,7 @@ chunk_vectors_kernel(const ChunkArgs a) {
         c -= nc;
     }
     if (len == 0) return;
-    float* ws = a.ws + ((size_t)chunk * a.heads + h) * a.stride;
+    float* ws = a.ws + ((size_t)blockIdx.x * a.heads + h) * a.stride;
     const bool mine = tid < a.dim;
     const float* qp = a.q + (size_t)t0 * a.ld_q + (h / a.per) * a.dim + tid;
     const float* gp = a.g + (size_t)t0 * a.ld_g + h * a.dim + tid;
@@ -259,7 +260,7 @@ __device__ __forceinline__ void copy_bulk(float* dst, const float* src, int floa
 }
 __device__ __forceinline__ void set_barrier(int set) { asm volatile("bar.sync %0, 128;" ::"r"(set + 1) : "memory"); }
 
-// A block carries CB columns of one (request, head)'s S through the request's chunks; 16 columns make 128 blocks of a prompt
+// A block carries CB columns of one (request, head)'s S through the request's chunks that are in the workspace; 16 columns make 128 blocks of a prompt
 // over 16 heads of 128 columns, which is nearly the GPU. Two sets of four warps carry eight columns each, on their own barriers,
 // so that one set's first product runs beside the other's second; a ninth warp copies the chunks ahead of them. S lies twice: a
 // thread's own entries in registers, which the second product moves on, and all of it by columns in shared memory, which the
@@ -282,7 +283,7 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     __shared__ uint64_t full[STAGES], empty[STAGES];
     __shared__ int abort_flag_;
     volatile int* abort_flag = &abort_flag_;
-    const int blk = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int b = blockIdx.x, h = blockIdx.y, blk = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         for (int i = 0; i < STAGES; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], WALK_THREADS / 32);
         abort_flag_ = 0;
@@ -294,16 +295,17 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     if (slot < 0 || slot >= n_slots) { if (tid == 0) atomicOr(err, CELLM_DEV_BAD_SLOT); return; }
     const int start = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - start;
     if (len < a.min_len) return;
+    int before = 0;                              // chunks of the requests before this one
+    for (int i = 0; i < b; ++i) {
+        const int n = a.cu_seqlens[i + 1] - a.cu_seqlens[i];
+        if (n >= a.min_len) before += (n + CT - 1) / CT;
+    }
+    const int c0 = max(0, a.chunk0 - before), n_chunks = min((len + CT - 1) / CT, a.chunk0 + a.chunks - before) - c0;
+    if (n_chunks <= 0) return;
     __syncthreads();
-    const int n_chunks = (len + CT - 1) / CT;
     if (warp == WALK_THREADS / 32) {
         if (lane != 0) return;
-        int first = 0;
-        for (int i = 0; i < b; ++i) {
-            const int n = a.cu_seqlens[i + 1] - a.cu_seqlens[i];
-            if (n >= a.min_len) first += (n + CT - 1) / CT;
-        }
-        const float* ws = a.ws + ((size_t)first * a.heads + h) * a.stride;
+        const float* ws = a.ws + ((size_t)(before + c0 - a.chunk0) * a.heads + h) * a.stride;
         int issued = 0;
         for (; issued < n_chunks; ++issued, ws += (size_t)a.heads * a.stride) {
             const int st = issued % STAGES;
@@ -344,7 +346,8 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     publish();
     const int ks = lane & 15, cols1 = set * (CB / 2) + (lane >> 4) * 4;
     float* uset = ush + set * CT * (CB / 2);
-    float* o_row = o_out + (size_t)start * a.heads * a.vd + (size_t)h * a.vd + col0;
+    const int left = len - c0 * CT;              // tokens from the first of these chunks on
+    float* o_row = o_out + (size_t)(start + c0 * CT) * a.heads * a.vd + (size_t)h * a.vd + col0;
     bool ok = true;
     for (int c = 0; c < n_chunks; ++c) {
         const float* stage = sm + (c % STAGES) * L::STAGE;
@@ -386,7 +389,7 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
                 uset[v * (CB / 2) + j % (CB / 2)] = acc[i] + uo[v * CB + j];
             } else {
                 const int t = v - (L::NV - CT);
-                if (ok && c * CT + t < len && col0 + j < a.vd) o_row[(size_t)(c * CT + t) * a.heads * a.vd + j] = acc[i] + uo[(CT + t) * CB + j];
+                if (ok && c * CT + t < left && col0 + j < a.vd) o_row[(size_t)(c * CT + t) * a.heads * a.vd + j] = acc[i] + uo[(CT + t) * CB + j];
             }
         }
         set_barrier(set);        // u is whole, and the set's columns of S have been read
@@ -427,20 +430,23 @@ template <int DIM, bool DELTA> int floats_a_chunk(int vd) {
 }
 
 template <int DIM, bool DELTA>
-int run(float* o_out, float* state, long long slot_stride, int n_slots, ChunkArgs a, int n_chunks, int* err, cudaStream_t stream) {
+int run(float* o_out, float* state, long long slot_stride, int n_slots, ChunkArgs a, int n_chunks, int ws_chunks, int* err, cudaStream_t stream) {
     using L = Layout<DIM, DELTA>;
     a.stride = floats_a_chunk<DIM, DELTA>(a.vd);
     const size_t smem = (size_t)(STAGES * L::STAGE + CB * (DIM + 4) + CT * CB) * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(chunk_walk_kernel<DIM, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    CELLM_RUN((chunk_vectors_kernel<DIM, DELTA>), dim3(n_chunks, a.heads), DIM, 0, stream, a);
-    CELLM_RUN((chunk_walk_kernel<DIM, DELTA>), dim3((a.vd + CB - 1) / CB, a.heads, a.B), WALK_THREADS + 32, smem, stream, o_out, state,
-              slot_stride, n_slots, a, err);
+    for (a.chunk0 = 0; a.chunk0 < n_chunks; a.chunk0 += ws_chunks) {
+        a.chunks = std::min(ws_chunks, n_chunks - a.chunk0);
+        CELLM_RUN((chunk_vectors_kernel<DIM, DELTA>), dim3(a.chunks, a.heads), DIM, 0, stream, a);
+        CELLM_RUN((chunk_walk_kernel<DIM, DELTA>), dim3(a.B, a.heads, (a.vd + CB - 1) / CB), WALK_THREADS + 32, smem, stream, o_out, state,
+                  slot_stride, n_slots, a, err);
+    }
     return CELLM_OK;
 }
 
-bool fits(int B, int heads, int per, int dim, int vd, int n_chunks, const void* ws) {
-    return B > 0 && heads > 0 && per > 0 && heads % per == 0 && dim > 0 && dim <= 128 && vd > 0 && n_chunks > 0 &&
+bool fits(int B, int heads, int per, int dim, int vd, int n_chunks, int ws_chunks, const void* ws) {
+    return B > 0 && heads > 0 && per > 0 && heads % per == 0 && dim > 0 && dim <= 128 && vd > 0 && n_chunks > 0 && ws_chunks > 0 &&
            (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
 }
 
@@ -454,25 +460,26 @@ CELLM_API int cellm_state_chunks_floats(int delta, int dim, int vd) {
 }
 
 // The gated delta rule over the portions of at least min_len tokens (n_chunks: the sum of their lengths / 16, each rounded up);
-// the others are left alone. Arguments as cellm_delta_scan; ws: n_chunks * heads * cellm_state_chunks_floats(1, ..) floats,
-// 16-byte aligned.
+// the others are left alone. Arguments as cellm_delta_scan; ws: ws_chunks * heads * cellm_state_chunks_floats(1, ..) floats,
+// 16-byte aligned: where it holds fewer chunks than there are, they go through it in runs (two launches each), the state
+// through memory between them; the result is the same.
 CELLM_API int cellm_delta_chunks(float* o_out, float* state, long long slot_stride, int n_slots, const float* qk, const float* v,
                                  const float* beta, const float* decay, const int* cu_seqlens, const int* slot_ids, int B, int n_chunks,
-                                 int min_len, int heads, int kvh, int dim, int vd, float* ws, int* err, cudaStream_t stream) {
-    if (kvh <= 0 || heads % kvh || !fits(B, heads, heads / kvh, dim, vd, n_chunks, ws) || min_len < 1) return CELLM_ERR_SIZE;
+                                 int ws_chunks, int min_len, int heads, int kvh, int dim, int vd, float* ws, int* err, cudaStream_t stream) {
+    if (kvh <= 0 || heads % kvh || !fits(B, heads, heads / kvh, dim, vd, n_chunks, ws_chunks, ws) || min_len < 1) return CELLM_ERR_SIZE;
     const long long ld = 2LL * kvh * dim;
     ChunkArgs a{qk, qk + (size_t)kvh * dim, decay, v, beta, ld, ld, (long long)heads * dim, (long long)heads * vd, heads / kvh,
-                cu_seqlens, slot_ids, B, min_len, heads, dim, vd, ws, 0};
-    return dim <= 64 ? run<64, true>(o_out, state, slot_stride, n_slots, a, n_chunks, err, stream)
-                     : run<128, true>(o_out, state, slot_stride, n_slots, a, n_chunks, err, stream);
+                cu_seqlens, slot_ids, B, min_len, heads, dim, vd, ws, 0, 0, 0};
+    return dim <= 64 ? run<64, true>(o_out, state, slot_stride, n_slots, a, n_chunks, ws_chunks, err, stream)
+                     : run<128, true>(o_out, state, slot_stride, n_slots, a, n_chunks, ws_chunks, err, stream);
 }
 
 // HGRN2 likewise; q and f (already silu and forget gate, as cellm_hgrn2_gates leaves them) and v are columns of proj [T, ld].
 CELLM_API int cellm_hgrn2_chunks(float* o_out, float* state, long long slot_stride, int n_slots, const float* proj, long long ld, int col_q,
-                                 int col_f, int col_v, const int* cu_seqlens, const int* slot_ids, int B, int n_chunks, int min_len,
-                                 int heads, int dim, int vd, float* ws, int* err, cudaStream_t stream) {
-    if (!fits(B, heads, 1, dim, vd, n_chunks, ws) || min_len < 1) return CELLM_ERR_SIZE;
-    ChunkArgs a{proj + col_q, nullptr, proj + col_f, proj + col_v, nullptr, ld, 0, ld, ld, 1, cu_seqlens, slot_ids, B, min_len, heads, dim, vd, ws, 0};
-    return dim <= 64 ? run<64, false>(o_out, state, slot_stride, n_slots, a, n_chunks, err, stream)
-                     : run<128, false>(o_out, state, slot_stride, n_slots, a, n_chunks, err, stream);
+                                 int col_f, int col_v, const int* cu_seqlens, const int* slot_ids, int B, int n_chunks, int ws_chunks,
+                                 int min_len, int heads, int dim, int vd, float* ws, int* err, cudaStream_t stream) {
+    if (!fits(B, heads, 1, dim, vd, n_chunks, ws_chunks, ws) || min_len < 1) return CELLM_ERR_SIZE;
+    ChunkArgs a{proj + col_q, nullptr, proj + col_f, proj + col_v, nullptr, ld, 0, ld, ld, 1, cu_seqlens, slot_ids, B, min_len, heads, dim, vd, ws, 0, 0, 0};
+    return dim <= 64 ? run<64, false>(o_out, state, slot_stride, n_slots, a, n_chunks, ws_chunks, err, stream)
+                     : run<128, false>(o_out, state, slot_stride, n_slots, a, n_chunks, ws_chunks, err, stream);
 }

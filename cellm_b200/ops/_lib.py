@@ -110,8 +110,8 @@ _SIGNATURES = {
     },
     "state_chunks": {
         "cellm_state_chunks_floats": [I, I, I],
-        "cellm_delta_chunks": [P, P, L, I, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P, P],
-        "cellm_hgrn2_chunks": [P, P, L, I, P, L, I, I, I, P, P, I, I, I, I, I, I, P, P, P],
+        "cellm_delta_chunks": [P, P, L, I, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P, P],
+        "cellm_hgrn2_chunks": [P, P, L, I, P, L, I, I, I, P, P, I, I, I, I, I, I, I, P, P, P],
     },
     "decay_chunks": {
         "cellm_decay_chunks": [P, P, L, I, P, L, P, L, P, L, P, L, P, L, P, P, I, I, I, I, I, I, I, P, P, P, P],

@@ -200,18 +200,22 @@ def attention_flash_masked(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: i
 # 64 x 128 15 against 27 us at 64 tokens, 45 against 27 at 128; 627 against 177 at 2,048.
 DELTA_CHUNKS_FROM, HGRN2_CHUNKS_FROM = 48, 96
 _STATE_CHUNK = 16           # tokens a chunk of state_chunks.cu
+# The chunks' workspace is at most this large (or one chunk): longer portions go through it in runs. The delta rule with 16 heads of
+# 128 x 128 takes 664 KB a chunk, so a run is 3,232 tokens.
+STATE_CHUNKS_BYTES = 128 << 20
 
 
 def _state_chunks(ctx, delta: bool, heads: int, dim: int, vd: int, device):
-    """(workspace, chunks, tokens from which a portion is long, whether portions remain for the walk) of a step's long portions;
-    None where all are short."""
+    """(workspace, chunks, chunks it holds, tokens from which a portion is long, whether portions remain for the walk) of a step's
+    long portions; None where all are short."""
     least = DELTA_CHUNKS_FROM if delta else HGRN2_CHUNKS_FROM
     long = [n for n in ctx.q_lens if n >= least] if dim <= 128 and ctx.max_q_len >= least else []
     if not long:
         return None
     n_chunks = sum(-(-n // _STATE_CHUNK) for n in long)
     floats = fn("state_chunks", "cellm_state_chunks_floats")(int(delta), dim, vd)
-    return torch.empty((n_chunks * heads * floats,), dtype=torch.float32, device=device), n_chunks, least, len(long) < ctx.B
+    held = min(n_chunks, max(1, STATE_CHUNKS_BYTES // (heads * floats * 4)))
+    return torch.empty((held * heads * floats,), dtype=torch.float32, device=device), n_chunks, held, least, len(long) < ctx.B
 
 
 def hgrn2_scan(proj: torch.Tensor, col_q: int, col_f: int, col_v: int, f_bias: torch.Tensor, lower: torch.Tensor, state: torch.Tensor,
@@ -228,14 +232,14 @@ def hgrn2_scan(proj: torch.Tensor, col_q: int, col_f: int, col_v: int, f_bias: t
                                            int(col_v), ptr(f_bias), ptr(lower), ptr(ctx.cu_seqlens), ptr(ctx.slot_ids), ctx.B, ctx.T, heads, dim, vd,
                                            ptr(ctx.err), stream_of(proj)), "hgrn2_scan")
         return o
-    ws, n_chunks, least, rest = chunks
+    ws, n_chunks, held, least, rest = chunks
     check(fn(_LIB, "cellm_hgrn2_gates")(ptr(proj), proj.stride(0), int(col_q), int(col_f), ptr(f_bias), ptr(lower), ctx.T, heads, dim,
                                         stream_of(proj)), "hgrn2_gates")
     where = (ptr(o), ptr(state), state.stride(0), state.shape[0], ptr(proj), proj.stride(0), int(col_q), int(col_f), int(col_v),
              ptr(ctx.cu_seqlens), ptr(ctx.slot_ids), ctx.B)
-    check(fn("state_chunks", "cellm_hgrn2_chunks")(*where, n_chunks, least, heads, dim, vd, ptr(ws), ptr(ctx.err), stream_of(proj)),
+    check(fn("state_chunks", "cellm_hgrn2_chunks")(*where, n_chunks, held, least, heads, dim, vd, ptr(ws), ptr(ctx.err), stream_of(proj)),
           "hgrn2_chunks")
-    count_launch()
+    count_launch(2 * -(-n_chunks // held) - 1)
     if rest:
         check(fn(_LIB, "cellm_hgrn2_walk")(*where, heads, dim, vd, least - 1, ptr(ctx.err), stream_of(proj)), "hgrn2_walk")
     return o
@@ -273,10 +277,10 @@ def delta_scan(qk, v, beta, decay, state: torch.Tensor, ctx, heads: int, kvh: in
     if chunks is None:
         check(fn(_LIB, "cellm_delta_scan")(*where, heads, kvh, dim, vd, ptr(ctx.err), stream_of(qk)), "delta_scan")
         return o
-    ws, n_chunks, least, rest = chunks
-    check(fn("state_chunks", "cellm_delta_chunks")(*where, n_chunks, least, heads, kvh, dim, vd, ptr(ws), ptr(ctx.err), stream_of(qk)),
+    ws, n_chunks, held, least, rest = chunks
+    check(fn("state_chunks", "cellm_delta_chunks")(*where, n_chunks, held, least, heads, kvh, dim, vd, ptr(ws), ptr(ctx.err), stream_of(qk)),
           "delta_chunks")
-    count_launch()
+    count_launch(2 * -(-n_chunks // held) - 1)
     if rest:
         check(fn(_LIB, "cellm_delta_walk")(*where, heads, kvh, dim, vd, least - 1, ptr(ctx.err), stream_of(qk)), "delta_walk")
     return o

@@ -180,3 +180,16 @@ def test_step_runner_builds_the_step_and_runs_it(monkeypatch):
     with pytest.raises(OutOfPages):
         runner.run([StepEntry(9, list(range(200)), [])])            # 8 pages of 16 tokens do not hold it
     assert cache.tokens(9) == 1                                     # and nothing was committed
+
+
+@pytest.mark.parametrize("delta,heads,dim,vd", [(True, 16, 128, 128), (False, 12, 64, 128), (True, 64, 128, 512)])
+def test_the_chunks_of_a_recurrence_go_through_a_bounded_workspace(delta, heads, dim, vd):
+    """However long a portion is, its chunks take 128 MB at most; those of a portion of 2,048 tokens of 16 heads are all held at once."""
+    from types import SimpleNamespace
+    from cellm_b200.ops import recurrent
+    for n in (96, 2048, 32768, 120000):
+        ctx = SimpleNamespace(q_lens=[n, 3], B=2, max_q_len=n)
+        ws, chunks, held, least, rest = recurrent._state_chunks(ctx, delta, heads, dim, vd, "cpu")
+        assert chunks == -(-n // 16) and rest and 1 <= held <= chunks
+        assert ws.numel() % held == 0 and ws.numel() * 4 <= 128 << 20
+        assert held == chunks or n > 2048 or heads > 16

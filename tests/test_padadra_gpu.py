@@ -539,6 +539,34 @@ def test_recurrences_in_chunks(kind, heads, kvh, dim, vd, decays):
     assert errors[True] <= 2 * errors[False] + 2.0 ** -23, errors
 
 
+@pytest.mark.parametrize("kind", ["delta", "hgrn2"])
+@pytest.mark.parametrize("held", [1, 4, 7, 100])
+def test_chunks_go_through_a_small_workspace_in_runs(monkeypatch, kind, held):
+    """Runs that end inside a request, at its end and behind several, of one chunk and of all: the same bits, states and read-outs."""
+    from cellm_b200 import ops
+    from cellm_b200.ops import recurrent
+    heads, kvh, dim, vd = (4, 2, 64, 40) if kind == "delta" else (4, 4, 64, 40)
+    g = torch.Generator().manual_seed(held)
+    lens, slots = [100, 9, 96, 1, 250, 112], [5, 0, 3, 6, 1, 2]
+    T = sum(lens)
+    unit = lambda: torch.nn.functional.normalize(torch.randn(T, kvh, dim, generator=g), dim=-1).reshape(T, -1)
+    qk, v = torch.cat([unit(), unit()], 1).to(DEV).contiguous(), torch.randn(T, heads * vd, generator=g).to(DEV)
+    beta, decay = torch.rand(T, heads, generator=g).to(DEV), torch.rand(T, heads * dim, generator=g).to(DEV)
+    proj, zero = torch.randn(T, heads * (2 * dim + vd), generator=g).to(DEV), torch.zeros(heads * dim, device=DEV)
+    S0, ctx, got = torch.randn(7, heads, dim, vd, generator=g), step_ctx(lens, [0] * len(lens), slots), []
+    floats = ops._lib.fn("state_chunks", "cellm_state_chunks_floats")(int(kind == "delta"), dim, vd)
+    for limit in (held * heads * floats * 4, recurrent.STATE_CHUNKS_BYTES):
+        monkeypatch.setattr(recurrent, "STATE_CHUNKS_BYTES", limit)
+        state = S0.to(DEV).clone()
+        if kind == "delta":
+            o = ops.delta_scan(qk, v, beta, decay, state, ctx, heads, kvh, dim, vd, chunked=True)
+        else:
+            o = ops.hgrn2_scan(proj.clone(), 0, heads * dim, 2 * heads * dim, zero, zero, state, ctx, heads, dim, vd, chunked=True)
+        got.append((o, state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert int(ctx.err.item()) == 0
+
+
 def test_delta_rule_inputs_and_the_convolutions_state():
     """Convolution + silu, unit vectors, beta and decays from the projections, with the convolution's last inputs carried
     from portion to portion (a portion shorter than the taps included)."""
