@@ -64,12 +64,13 @@ __device__ __forceinline__ float cellm_activate(float z, int act) {
     }
 }
 
-// gelu, exact form, without branches: for epilogues that form 32 of them a thread in a row. erf(x) is x times a polynomial in
-// x^2 for |x| < 1, else 1 - 2^q(|x|), q a polynomial for log2 erfc on [1, 4] (behind 4 erf is 1 in 32 bits); both were fitted in
-// 64 bits (least squares, reweighted towards the largest error: 3e-11). Over [-8, 8] the largest error of z (1 + erf) / 2 is
-// 4.5e-7, as with an erf that is rounded once. (erff's branches, taken for one value after the other, made the epilogue of a
-// product of 2,048 x 2,048 over K = 2,048 40 us long.)
-__device__ __forceinline__ float cellm_gelu_flat(float z) {
+// gelu, exact form, without branches: for epilogues that form 32 of them a thread in a row and round them to bfloat16 at once.
+// erf(x) is x times a polynomial in x^2 for |x| < 1, else 1 - 2^q(|x|), q a polynomial for log2 erfc on [1, 4] (behind 4 erf is
+// 1 in 32 bits); both were fitted in 64 bits (least squares, reweighted towards the largest error: 3e-11). With the fast
+// exponential the value is off by up to 8e-8 on [-2, -1], where the form with erff is off by 5e-8 (4e-8 and 3e-8 on [-1, 0], 1.0e-7
+// and 0.7e-7 on [0, 1]; elsewhere no more than that form), so 32-bit results take erff; rounded to bfloat16 the two are equally far off everywhere. (erff's branches, taken
+// for one value after the other, made the epilogue of a product of 2,048 x 2,048 over K = 2,048 40 us long.)
+__device__ __forceinline__ float cellm_gelu_rounded(float z) {
     const float x = z * 0.70710678118654752f, a = fminf(fabsf(x), 4.f), s = x * x;
     float p = -9.680135917733423e-06f;
     p = fmaf(p, s, 0.00011270544200669974f);

@@ -687,10 +687,10 @@ __device__ __forceinline__ void drain_tile(TO* __restrict__ C, int M, int N, lon
 #pragma unroll
                     for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_xielu(__uint_as_float(r[i]), ap, aq));
                 }
-            } else if (act == 0) {
+            } else if (sizeof(TO) == 2 && act == 0) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_gelu_flat(__uint_as_float(r[i])));
-            } else if (act > 0) {
+                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_gelu_rounded(__uint_as_float(r[i])));
+            } else if (act >= 0) {
 #pragma unroll
                 for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(cellm_activate(__uint_as_float(r[i]), act));
             }

@@ -554,10 +554,10 @@ def test_sort_and_sum_of_the_experts_slots(T, E, top, H):
 
 @pytest.mark.parametrize("rows,cols", [(17, 8), (128, 256), (300, 520)])
 def test_gelu_in_the_products_epilogue(rows, cols):
-    """The product with a diagonal matrix leaves the operand itself for the activation: both sides of the places where its two
-    forms meet (|z| = sqrt 2), far out, zeros, infinities and no number; within half a unit of the 16-bit result's last place
-    (8 significant bits: at most 2^-8 of the value) and the 32-bit form's 1e-6 (4.5e-7 over [-8, 8], where a result is not
-    the operand itself or nothing)."""
+    """The product with a diagonal matrix leaves the operand itself for the activation: both sides of the places where the 16-bit
+    result's two forms meet (|z| = sqrt 2), far out, zeros, infinities and no number; within half a unit of the 16-bit result's
+    last place (8 significant bits: at most 2^-8 of the value) and 1e-6 (4.5e-7 in 32 bits over [-8, 8], where a result is
+    not the operand itself or nothing)."""
     from cellm_b200 import ops
     g = torch.Generator().manual_seed(rows)
     k = -(-cols // 8) * 8
@@ -571,3 +571,24 @@ def test_gelu_in_the_products_epilogue(rows, cols):
         a = torch.full((17, 8), v, dtype=torch.bfloat16, device=DEV)
         got = ops.gemm_act(a, torch.zeros(8, 8, dtype=torch.bfloat16, device=DEV), "gelu", torch.float32)
         assert tuple(got.shape) == (17, 8) and bool(torch.isnan(got).all())
+
+
+def test_gelu_of_32_bit_results_is_as_near_as_with_erf_itself():
+    """All 16-bit values and as many 32-bit ones between them (a sum of two operands is the product): a 32-bit result lies no further
+    from 64 bits than the formula with torch's erf in 32 bits, range by range (by the root mean square, a tenth for contractions)."""
+    from cellm_b200 import ops
+    bits = torch.arange(1 << 16, dtype=torch.int32, device=DEV).to(torch.int16).view(torch.bfloat16).float()
+    high = bits[torch.isfinite(bits) & (bits.abs() <= 8) & (bits.abs() > 1e-4)]
+    g = torch.Generator(device=DEV).manual_seed(4)
+    a = torch.zeros(high.numel(), 64, dtype=torch.bfloat16, device=DEV)
+    a[:, 0], a[:, 1] = high, high * (torch.rand(high.numel(), generator=g, device=DEV) - 0.5) * 2.0 ** -7
+    w = torch.zeros(128, 64, dtype=torch.bfloat16, device=DEV)
+    w[:, :2] = 1
+    z = a[:, 0].float() + a[:, 1].float()
+    exact = 0.5 * z.double() * torch.special.erfc(-z.double() * 0.5 ** 0.5)
+    got = ops.gemm_act(a, w, "gelu", torch.float32)[:, 3]
+    plain_form = 0.5 * z * (1 + torch.erf(z * 0.70710678118654752))
+    for lo, hi in ((-8, -4), (-4, -2), (-2, -1), (-1, 0), (0, 1), (1, 2), (2, 4), (4, 8)):
+        at = (z >= lo) & (z < hi)
+        off = lambda y: float((y[at].double() - exact[at]).square().mean().sqrt())
+        assert off(got) <= 1.1 * off(plain_form), (lo, off(got), off(plain_form))
