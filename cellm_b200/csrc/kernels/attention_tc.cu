@@ -86,7 +86,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const int* __restrict__ cu_seqlens, const int* __restrict__ ctx_lens,
                     const int* __restrict__ block_table, int bt_stride, int B, int num_pages, int page_size, int nh,
                     int nkv, float scale_log2e, int window, const float* __restrict__ sinks, const float* __restrict__ gate,
-                    long long gate_ld, int chunk, float step, int nsplit, float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ err) {
+                    long long gate_ld, int chunk, float step, int nsplit, int T, float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     TcSmem& sm = *reinterpret_cast<TcSmem*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -358,7 +358,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             // with; an output gate: the row times the sigmoid of one number per (token, head)
             const int head = kvh * G + r % G;
             if (nsplit > 1) {       // the piece's maximum, sum and unnormalised output (none where it had no block)
-                const size_t row = ((size_t)blockIdx.z * cu_seqlens[B] + t_base + tok) * nh + head;
+                const size_t row = ((size_t)blockIdx.z * T + t_base + tok) * nh + head;
                 if (row_ok) *reinterpret_cast<float2*>(part_ml + row * 2) = make_float2(n_blocks > 0 ? m : -INFINITY, l);
 #pragma unroll 1
                 for (int c = 0; c < (n_blocks > 0 ? HD / 32 : 0); ++c) {
@@ -493,7 +493,7 @@ static int attention_tc_impl(void* out, const void* q, const void* k_pool, const
     dim3 grid((unsigned)n_tiles, (unsigned)nkv, (unsigned)nsplit);
     CELLM_RUN(attention_tc_kernel, grid, THREADS, smem, stream, mq, mk, mv, (__nv_bfloat16*)out, cu_seqlens,
               ctx_lens, block_table, bt_stride, B, num_pages, page_size, nh, nkv, scale * 1.4426950408889634f, window, sinks,
-              gate, gate_ld, chunk, 128 % G ? 0.f : RESCALE_STEP, nsplit, part_o, part_ml, err);
+              gate, gate_ld, chunk, 128 % G ? 0.f : RESCALE_STEP, nsplit, T, part_o, part_ml, err);
     if (nsplit > 1)
         CELLM_RUN(attention_tc_merge_kernel, (unsigned)(((long long)T * nh + 15) / 16), 256, 0, stream, (__nv_bfloat16*)out, part_o, part_ml,
                   (long long)T * nh, nsplit);

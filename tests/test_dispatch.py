@@ -182,6 +182,27 @@ def test_step_runner_builds_the_step_and_runs_it(monkeypatch):
     assert cache.tokens(9) == 1                                     # and nothing was committed
 
 
+@pytest.mark.parametrize("nh,nkv,lens,ctxs,pieces", [(24, 8, [2048], [8192], 2), (32, 8, [256], [2048], 2), (16, 8, [64] * 4, [9000] * 4, 4),
+                                                     (32, 8, [2048], [8192], 1), (24, 8, [2048], [0], 1)])
+def test_prompt_attention_in_pieces_gets_a_workspace_that_holds_them(monkeypatch, nh, nkv, lens, ctxs, pieces):
+    """Where whole keys fill the SMs' last round badly, the executor asks for pieces, and lends unnormalised outputs and (maximum,
+    sum) pairs for every piece of every row, side by side in the attention workspace."""
+    rec = Recorder(monkeypatch)
+    cfg, plan, model = zero_model(dict(SHORT, num_attention_heads=nh, num_key_value_heads=nkv))
+    run_step(model, plan, lens, ctxs)
+    calls = rec.of("cellm_attention_tc_split")
+    if pieces == 1:
+        assert all(c[20] == 1 and c[1] is None and c[2] is None for c in calls)
+        return
+    (call,) = calls
+    T = sum(lens)
+    assert (call[11], call[20]) == (T, pieces)
+    ws = model.program._attn_ws
+    rows = pieces * T * nh
+    assert call[1] == ws.data_ptr() and call[2] == ws.data_ptr() + rows * 64 * 4
+    assert ws.numel() >= rows * 66
+
+
 @pytest.mark.parametrize("delta,heads,dim,vd", [(True, 16, 128, 128), (False, 12, 64, 128), (True, 64, 128, 512)])
 def test_the_chunks_of_a_recurrence_go_through_a_bounded_workspace(delta, heads, dim, vd):
     """However long a portion is, its chunks take 128 MB at most; those of a portion of 2,048 tokens of 16 heads are all held at once."""

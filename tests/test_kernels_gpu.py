@@ -599,6 +599,45 @@ def test_attention_takes_groups_that_do_not_divide_a_tile(monkeypatch, ps, nh, n
     assert program.CALLS["cellm_attention_flash"] == before + 1
 
 
+@pytest.mark.parametrize("nh,nkv,lens,ctxs,window", [(32, 8, [256], [2100], 0), (24, 8, [230, 40, 1], [3000, 4100, 77], 0), (16, 8, [260], [5000], 3000)])
+def test_the_executor_cuts_keys_into_pieces(nh, nkv, lens, ctxs, window):
+    """Few CTAs before long keys, through the executor's own choice and workspace: it runs the kernel with pieces and the merge
+    (a launch more), against the oracle."""
+    from cellm_b200 import ops
+    from cellm_b200.ops import _lib
+    from cellm_b200.runtime import program
+    hd = 64
+    c = paged_case(lens, ctxs, nh, nkv, hd, 16, torch.bfloat16, seed=9)
+    e = err_word()
+    before, launches = program.CALLS["cellm_attention_tc_split"], _lib.LAUNCHES[0]
+    out = ops.attention(c["q"], c["kp"], c["vp"], portions_ctx(c, lens, ctxs, e), c["bt"], nh, hd ** -0.5, window)
+    assert program.CALLS["cellm_attention_tc_split"] == before + 1 and _lib.LAUNCHES[0] == launches + 2
+    close(out, attention_reference(c, nh, nkv, hd, hd ** -0.5, window), torch.bfloat16)
+    assert e.item() == 0
+
+
+@pytest.mark.parametrize("spare", [0, 5])
+def test_pieces_lie_the_callers_number_of_tokens_apart(spare):
+    """The merge reads the pieces T rows of heads apart, whatever the lengths on the device add up to."""
+    import ctypes
+    from cellm_b200.csrc import build
+    nh, nkv, hd, ps, nsplit, lens, ctxs = 8, 2, 64, 16, 3, [100, 40], [900, 400]
+    c = paged_case(lens, ctxs, nh, nkv, hd, ps, torch.bfloat16, seed=6)
+    e, P = err_word(), ctypes.c_void_p
+    n, T = sum(lens), sum(lens) + spare
+    q = torch.cat([c["q"], c["q"][:spare]])
+    out = torch.empty_like(q)
+    part_o, part_ml = torch.zeros(nsplit * T * nh * hd, device=DEV), torch.zeros(nsplit * T * nh * 2, device=DEV)
+    ptr = lambda t: P(t.data_ptr())
+    tiles = sum(-(-k // (2 * (128 // (nh // nkv)))) for k in lens)
+    assert build.load("attention_tc").cellm_attention_tc_split(
+        ptr(out), ptr(part_o), ptr(part_ml), ptr(q), ptr(c["kp"]), ptr(c["vp"]), ptr(c["cu"]), ptr(c["ctx"]), ptr(c["bt"]), c["bt"].stride(0),
+        len(lens), T, tiles, c["kp"].shape[0], ps, nh, nkv, hd, ctypes.c_float(hd ** -0.5), 0, nsplit, ptr(e),
+        P(torch.cuda.current_stream().cuda_stream)) == 0
+    close(out[:n], attention_reference(c, nh, nkv, hd, hd ** -0.5, 0), torch.bfloat16)
+    assert e.item() == 0
+
+
 @pytest.mark.parametrize("nh,nkv,lens,ctxs", [(24, 8, [300], [2100]), (14, 2, [180, 130], [3000, 900])])
 def test_groups_that_do_not_divide_a_tile_lose_no_precision(monkeypatch, nh, nkv, lens, ctxs):
     """The tcgen05 kernel's distance from the result in 64 bits is that of the mma.sync kernel that took these groups before. Both
