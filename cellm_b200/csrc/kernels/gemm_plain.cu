@@ -213,6 +213,7 @@ CELLM_API int cellm_gemm_plain(void* C, const void* A, const void* W, int M, int
         int best = 0;
         double least = 0;
         for (int i = 0; i < 4; ++i) {
+            if (i > 0 && (M + tile[i].bm - 1) / tile[i].bm > 65535) break;      // as many rows as 64 x 64 tiles take, whatever their number
             const long long tiles = (long long)((M + tile[i].bm - 1) / tile[i].bm) * ((N + tile[i].bn - 1) / tile[i].bn), waves = (tiles + 147) / 148;
             const double cost = waves == 1 ? tile[i].alone : (double)waves * tile[i].wave;
             if (i == 0 || cost < least) best = i, least = cost;

@@ -771,6 +771,17 @@ def test_gemm_plain_in_32_bits_does_not_depend_on_the_tile(M, N, K):
         assert torch.equal(ops.gemm_plain(rows[:min(M, 70)], w[:min(N, 40)], torch.float32), out[:min(M, 70), :min(N, 40)])
 
 
+@pytest.mark.parametrize("N", [8, 40])
+def test_gemm_plain_in_32_bits_of_a_million_rows(N):
+    """More rows than a grid of tiles of 16 (or 32) of them holds, and so few columns that those would be chosen."""
+    from cellm_b200 import ops
+    M = 65536 * 32 + 5
+    a, w = torch.randn(M, 4, device=DEV), torch.randn(N, 4, device=DEV)
+    out = ops.gemm_plain(a, w, torch.float32)
+    for part in (slice(0, 100), slice(M // 2, M // 2 + 100), slice(M - 100, M)):
+        close(out[part], a[part].double() @ w.double().T, torch.float32)
+
+
 @pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M,N,K,bn,split", [
     (128, 128, 64, 128, 1), (200, 1000, 96, 128, 1), (300, 520, 1024, 256, 1), (100, 72, 2048, 64, 1),
