@@ -1182,6 +1182,9 @@ int launch_unsplit(void* C, const void* A, const void* W, int M, int N, int K, i
 
 }  // namespace
 
+// 1 if an unsplit product in plain tiles of bn columns runs on pairs of SMs (tests ask).
+CELLM_API int cellm_gemm_runs_in_pairs(int M, int N, int K, int bn) { return in_pairs(M, N, K, bn) ? 1 : 0; }
+
 // Most tiles a product may have when K is split (one counter each).
 #define GEMM_MAX_COUNTERS 65536
 

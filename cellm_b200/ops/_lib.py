@@ -130,6 +130,7 @@ _SIGNATURES = {
     },
     "gemm_tcgen05": {
         "cellm_gemm_tcgen05": [P, P, P, I, I, I, L, L, L, I, I, I, I, I, P, P, P, P],
+        "cellm_gemm_runs_in_pairs": [I, I, I, I],
         "cellm_gemm_grouped_tcgen05": [P, P, P, I, I, I, I, L, L, L, I, P, I, P, P],
         "cellm_gemm_gated_tcgen05": [P, P, P, I, I, I, L, L, L, I, I, I, I, F, F, I, P, P, P, P],
         "cellm_gemm_grouped_gated_tcgen05": [P, P, P, I, I, I, I, L, L, L, I, P, I, F, F, P, P],

@@ -812,8 +812,10 @@ def test_gemm_tcgen05(out, M, N, K, bn, split):
     (2001, 16512, 1032, 256, 1), (300, 384, 12008, 128, 1)])
 def test_gemm_tcgen05_on_pairs_of_sms(out, M, N, K, bn, epilogue):
     """Products long enough for pairs, with rows, columns and a piece of K that fill no tile (the second CTA's half of a tile may
-    lie wholly outside): near the exact sums, and bit for bit what short products of the same rows, which single CTAs do, give."""
+    lie wholly outside): near the exact sums, and bit for bit what single CTAs make of some of the rows and columns."""
+    from cellm_b200.ops._lib import fn
     from cellm_b200.ops.gemm_bf16 import error_word, gemm_tcgen05
+    assert fn("gemm_tcgen05", "cellm_gemm_runs_in_pairs")(M, N, K, bn) == 1
     a = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
     w = (torch.randn(N, K, device=DEV) * 0.05).bfloat16()
     c = gemm_tcgen05(a, w, out, bn, 1, epilogue=epilogue)
@@ -828,12 +830,11 @@ def test_gemm_tcgen05_on_pairs_of_sms(out, M, N, K, bn, epilogue):
         g, u = ref.reshape(M, -1, 2, 64).unbind(2)
         want = (torch.nn.functional.silu(g) * u).reshape(M, N // 2)
         assert float((c.double() - want).abs().max()) <= 6e-3 * (1 + float(want.abs().max()))
-    # one row tile of a hundred rows and few columns: less work than a pair is given
+    # tiles of 64 columns, or of 64 rows of A where gate and up are joined: neither is ever given to a pair
     n = min(N, 1024) // 128 * 128
-    if 256 * -(-K // 64) < 90 * 256:
-        for m0 in (0, M - 100):
-            few = gemm_tcgen05(a[m0:m0 + 100].contiguous(), w[:n], out, bn, 1, epilogue=epilogue)
-            assert torch.equal(few, c[m0:m0 + 100, :few.shape[1]])
+    for m0 in (0, M - 100):
+        few = gemm_tcgen05(a[m0:m0 + 100].contiguous(), w[:n], out, -64 if epilogue else 64, 1, epilogue=epilogue)
+        assert torch.equal(few, c[m0:m0 + 100, :few.shape[1]])
 
 
 @pytest.mark.parametrize("M,ff,K,bn,split", [(8, 192, 64, -16, 1), (3, 128, 2048, -16, 4), (40, 320, 96, -64, 1), (64, 64, 512, -64, 2),

@@ -601,10 +601,11 @@ def test_delta_rule_inputs_and_the_convolutions_state():
 
 
 @pytest.mark.parametrize("dim,taps", [(64, 2), (64, 4), (128, 3), (128, 4)])
-@pytest.mark.parametrize("many", [1, 9])
+@pytest.mark.parametrize("many", [1, 4, 9])
 def test_delta_rule_inputs_of_many_tokens(dim, taps, many):
-    """Runs of tokens that hold several requests' ends and starts, requests shorter than the taps, states that are not zero,
-    channels of v that are no whole head: bit for bit what the form for few tokens leaves for each request alone."""
+    """136 tokens in blocks, 544 in runs of four and 1,224 in runs of eight, which hold several requests' ends and starts; requests
+    shorter than the taps, states that are not zero, channels of v that are no whole head: bit for bit what the form for few
+    tokens leaves for each request alone."""
     from cellm_b200 import ops
     heads, kvh, vd = 4, 2, 40
     lens = [40, 1, 2, 30, 63] * many
