@@ -567,6 +567,25 @@ def test_chunks_go_through_a_small_workspace_in_runs(monkeypatch, kind, held):
     assert int(ctx.err.item()) == 0
 
 
+def test_chunks_behind_more_requests_than_a_grids_second_dimension():
+    """70,000 requests of one token and a long portion behind them: the portion in chunks, the others token by token."""
+    from cellm_b200 import ops
+    n, heads, dim, vd = 70000, 1, 4, 4
+    lens = [1] * n + [100]
+    T = sum(lens)
+    g = torch.Generator().manual_seed(1)
+    qk, v = torch.randn(T, 2 * dim, generator=g).to(DEV) * 0.3, torch.randn(T, vd, generator=g).to(DEV)
+    beta, decay = torch.rand(T, heads, generator=g).to(DEV), torch.rand(T, dim, generator=g).to(DEV)
+    ctx, got = step_ctx(lens, [0] * len(lens), list(range(n + 1))), []
+    for chunked in (False, True):
+        state = torch.ones(n + 1, heads, dim, vd, device=DEV)
+        got.append((ops.delta_scan(qk, v, beta, decay, state, ctx, heads, 1, dim, vd, chunked=chunked), state))
+    assert torch.equal(got[0][0][:n], got[1][0][:n]) and torch.equal(got[0][1][:n], got[1][1][:n])
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, rtol=2e-5, atol=2e-5 * float(b.abs().max()))
+    assert int(ctx.err.item()) == 0
+
+
 def test_delta_rule_inputs_and_the_convolutions_state():
     """Convolution + silu, unit vectors, beta and decays from the projections, with the convolution's last inputs carried
     from portion to portion (a portion shorter than the taps included)."""
