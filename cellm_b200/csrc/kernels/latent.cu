@@ -239,7 +239,7 @@ head_product_kernel(TA* __restrict__ out, long long ldo, long long out_hs, const
 #define HP_SMALL_T 16
 #define HP_SMALL_AHEAD 8        // pieces of a row asked for ahead: all of K up to 512
 __global__ void __launch_bounds__(128)
-head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long long out_hs, const __nv_bfloat16* __restrict__ in,
+head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long long out_hs, const __nv_bfloat16* in,
                           long long ldi, long long in_hs, const __nv_bfloat16* __restrict__ w, int T, int N, int K, int vec_in) {
     extern __shared__ __align__(16) __nv_bfloat16 xin[];       // [T][K]
     pdl_trigger();
@@ -247,7 +247,8 @@ head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long l
     const int n = blockIdx.x * 16 + (threadIdx.x >> 3), kq = threadIdx.x & 7;
     const bool on = n < N;
     const __nv_bfloat16* wr = w + ((size_t)h * N + (on ? n : 0)) * K;
-    // the matrices are not the work of the kernel before this one: a row's first pieces are asked for before the wait on it
+    // the matrices are not the work of the kernel before this one: a row's first pieces are asked for before the wait on it (`in`
+    // is, and is not declared __restrict__: its loads may not move up to these)
     uint4 wq[HP_SMALL_AHEAD];
 #pragma unroll
     for (int i = 0; i < HP_SMALL_AHEAD; ++i)

@@ -730,9 +730,10 @@ CELLM_API int cellm_moe_gather(void* xs, const void* y, long long ldy, const int
 __device__ __forceinline__ void store_pair(__nv_bfloat16* p, float a, float b) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b); }
 __device__ __forceinline__ void store_pair(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
 
+// (`gate` is read right behind the wait and is not declared __restrict__, so that the load cannot move in front of it.)
 template <typename TO>
 __global__ void moe_combine_kernel(TO* __restrict__ out, const __nv_bfloat16* __restrict__ Y, const int* __restrict__ slot_row,
-                                   const float* __restrict__ wts, const float* __restrict__ shared, const float* __restrict__ gate, int H,
+                                   const float* __restrict__ wts, const float* __restrict__ shared, const float* gate, int H,
                                    int top) {
     pdl_trigger();
     pdl_wait();
@@ -765,7 +766,7 @@ __device__ __forceinline__ void store_four(float* p, const float* a) { *reinterp
 template <typename TO>
 __global__ void __launch_bounds__(256)
 moe_combine8_kernel(TO* __restrict__ out, const __nv_bfloat16* __restrict__ Y, const int* __restrict__ slot_row, const float* __restrict__ wts,
-                    const float* __restrict__ shared, const float* __restrict__ gate, int H, int top) {
+                    const float* __restrict__ shared, const float* gate, int H, int top) {
     pdl_trigger();
     pdl_wait();
     const size_t t = blockIdx.x;
