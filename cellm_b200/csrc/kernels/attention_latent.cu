@@ -237,8 +237,9 @@ latent_flash_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_o,
 // keys is worked on by all warps, twice over: for the scores a warp takes 16 keys and half of their entries, for the sums a
 // warp takes an eighth of the value columns and all 64 keys; the scores' halves, the weights and the rows' factors pass
 // through shared memory. The two halves of a score are added in one order, so a score is the same sum for every warp that
-// needs it. Two blocks are under way from the start (a piece is two blocks or more), looked up before the wait on the kernel
-// before. 8 requests behind 2,048 rows, 16 heads, kw 576: 25 -> 14.6 us from flushed caches.
+// needs it. Two blocks are under way from the start (a piece is two blocks or more where the executor counts blocks of 64
+// keys, one or more where the other form's are 32: 128 and 384 value columns), looked up before the wait on the kernel before.
+// 8 requests behind 2,048 rows, 16 heads, kw 576: 25 -> 14.7 us from flushed caches.
 constexpr int LD_BM = 16, LD_BN = 64;
 
 constexpr size_t decode_smem(int kw) {

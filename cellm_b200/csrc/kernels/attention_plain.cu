@@ -1,12 +1,14 @@
-// Plain attention over the paged cache: one block per (token, head), every
-// earlier key of the request (or the last `window` of them) read through the
-// block table. It serves the 32-bit path and is the reference for the faster
-// attention kernels.
+// Plain attention over the paged cache, every earlier key of the request (or the
+// last `window` of them) read through the block table: one block per (token, head),
+// which takes every form (sinks, gates, values turned back, kept first keys, any
+// width, bfloat16) and is the reference for the faster attention kernels; and for
+// the usual form in 32 bits a block per rows of several tokens and heads
+// (attention_rows_kernel).
 //
 // For head h the key/value head is h / (nh / nkv); scores are q.k * scale;
 // softmax takes the maximum off first; all of it in 32-bit
 // (crates/cellm-cache/src/kvcache.rs:753-787, :1206-1227). Keys are walked in
-// chunks that start at multiples of the chunk size counted from key 0, so the
+// chunks (128 keys, 64 by rows) that start at multiples of their size counted from key 0, so the
 // order of every sum depends only on the token's position, never on how the
 // sequence was cut into steps or what else is in the batch.
 //
@@ -151,13 +153,14 @@ attention_plain_kernel(TA* __restrict__ out, const TA* __restrict__ q, const TA*
 // ------------------------------------------------------------------------------------------------ the usual form in 32 bits
 // Queries, keys and values of one width hd (a multiple of 4, up to 128), no sink, no gate, nothing turned back: a block takes
 // RI * 8 rows, the heads of one key/value head for as many neighbouring tokens as fit, and brings every key and value of
-// theirs into shared memory once, in blocks of 64 keys that start at multiples of 64 and arrive two ahead by asynchronous
-// copies. (One block a (token, head) read them again for each: a layer of 24 heads of 64, three portions of 213 tokens in all
-// behind 100 keys on average, its two products included, went from 998 to 237 us; 66 of them are this kernel.) 16 neighbouring threads share a row; a thread holds RI rows by 4 keys of the scores and RI rows by 4
-// values of each 64 of the output. Every sum's order depends on the row's own position alone: a score is four sums over
-// every fourth entry, added in pairs; a block's weights are summed four a thread and over the 16 threads; the output runs over
-// the keys in order. Keys that a row does not see are passed over, not multiplied by zero, so what later tokens hold (infinities
-// among it) reaches no earlier one.
+// theirs into shared memory once, in blocks of 64 keys that start at multiples of 64 and arrive by asynchronous copies while the
+// block before is worked on. (One block a (token, head) read them again for each: a layer of 24 heads of 64, three portions of
+// 213 tokens in all behind 100 keys on average, its two products included, went from 998 to 231 us, 66 of them this kernel.
+// Steps of single tokens gain as well, 1 to 256 requests behind 100 to 8,192 keys: 2.2 to 28 times the speed.) 16 neighbouring
+// threads share a row; a thread holds RI rows by 4 keys of the scores and RI rows by 4 values of each 64 of the output. Every
+// sum's order depends on the row's own position alone: a score is four sums over every fourth entry, added in pairs; a block's
+// weights are summed four a thread and over the 16 threads; the output runs over the keys in order. Keys that a row does not see
+// are passed over, not multiplied by zero, so what later tokens hold (infinities among it) reaches no earlier one.
 #define ROWS_KEYS 64
 #define ROWS_THREADS 128
 

@@ -113,8 +113,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
     }
-    // V stages start as zeros: rows that are never loaded must not carry NaN bits into P.V (0 * NaN);
-    // what K rows hold there does not matter, their scores are masked
+    // V stages start as zeros: rows that are never loaded must not carry NaN bits into P.V (0 * NaN) of a tile's tokens. What
+    // K's and Q's rows hold there does not matter: a key's scores are masked for every token that does not see it, and rows of
+    // no token, which are not masked, keep whatever comes of them to themselves (products and softmax go row by row) and
+    // are never written
     for (int i = threadIdx.x; i < (int)sizeof(sm.v) / 16; i += blockDim.x)
         reinterpret_cast<uint4*>(sm.v)[i] = make_uint4(0, 0, 0, 0);
     proxy_fence();
@@ -446,7 +448,7 @@ CELLM_API int cellm_attention_tc_supports(int hd, int nh, int nkv, int page_size
 }
 
 // Groups that do not divide 128 leave a tile's last rows empty (2 of 128 for G = 3, 32 at most here). They are taken where at
-// least three quarters of the rows are in use: with 24 heads over 8, 2,048 queries behind 8,192 keys, the layer takes 295 us
+// least three quarters of the rows are in use: with 24 heads over 8, 2,048 queries behind 8,192 keys, the layer takes 304 us
 // here and 813 us on the mma.sync kernel, a ratio that a quarter of a tile does not use up. `uneven`: 0 for the entry points
 // that take divisors only.
 static bool attention_tc_takes(int hd, int nh, int nkv, int page_size, int uneven) {
@@ -511,8 +513,9 @@ CELLM_API int cellm_attention_tc(void* out, const void* q, const void* k_pool, c
 // The same for groups of heads that need not divide 128 (three quarters of a tile's rows must be in use), and with the keys of
 // every pair of tiles in `nsplit` pieces (a CTA each) whose results meet in part_o [nsplit, T * nh, 64] and part_ml
 // [nsplit, T * nh, 2] and are merged by a second kernel: where the pairs fill the SMs' last round badly (200 CTAs of 72
-// blocks on 148 SMs are two rounds, 400 of 36 three of half the length: a layer of 24 heads over 8, 2,048 queries behind
-// 8,192 keys, 509 us whole and 442 in two pieces, both before rows of no token were left unmasked). The caller chooses.
+// blocks on 148 SMs are two rounds, 400 of 36 three of half the length: 24 heads over 8, 2,048 queries behind 8,192 keys,
+// 306 us whole and 254 in two pieces with their merge) or do not fill one (512 queries of 32 heads over 8 there: 137 and 77).
+// The caller chooses.
 CELLM_API int cellm_attention_tc_split(void* out, float* part_o, float* part_ml, const void* q, const void* k_pool, const void* v_pool,
                                        const int* cu_seqlens, const int* ctx_lens, const int* block_table, int bt_stride,
                                        int B, int T, int n_tiles, int num_pages, int page_size, int nh, int nkv, int hd,

@@ -23,7 +23,7 @@
 //   chunk_walk      a block carries 16 columns of one (request, head)'s S through the chunks: two small products a chunk
 //
 // Everything is 32-bit fused multiply-adds, as token by token (relative error of the read-outs against 64 bits over 2,048 tokens
-// 8.9e-8, token by token 8.7e-8). One prompt of 2,048 tokens, 16 heads of 128 x 128: 915 -> 217 us (49 of them chunk_vectors).
+// 8.9e-8, token by token 8.7e-8). One prompt of 2,048 tokens, 16 heads of 128 x 128: 938 -> 215 us (49 of them chunk_vectors).
 #include <algorithm>
 #include <climits>
 
@@ -271,7 +271,7 @@ __device__ __forceinline__ void set_barrier(int set) { asm volatile("bar.sync %0
 //                   are added: u goes to shared memory, o to memory.
 //   second product  S <- diag(E) S + (k E)^T u, a thread two or four rows by two columns.
 // Bound by shared memory's bandwidth (every warp reads its share of the chunk's rows and the set's columns). With all eight warps
-// on one barrier and every thread copying, the phases added up: 290 us a prompt of 2,048 tokens where this form takes 130.
+// on one barrier and every thread copying, the phases added up: 290 us a prompt of 2,048 tokens where this form takes 166.
 template <int DIM, bool DELTA>
 __global__ void __launch_bounds__(WALK_THREADS + 32)
 chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long long slot_stride, int n_slots, const ChunkArgs a,
