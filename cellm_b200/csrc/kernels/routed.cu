@@ -631,14 +631,16 @@ CELLM_API int cellm_activation(void* h, const float* u, long long ld, int T, int
 // For the grouped tensor-core product every expert's slots form one run of rows, padded to whole tiles of 128 rows, in
 // the order of the slots themselves (so a row's place depends on the step's tokens alone, never on timing).
 #define MOE_TILE 128
-#define MOE_SORT_THREADS 1024
+#define MOE_SORT_FEW 1024           // slots that 256 threads a block sort; more: 1,024 threads
 
 // One block an expert: it counts the slots of every expert (a histogram in shared memory), finds where its own run
 // begins, names its tiles, and places its slots in their order. row_slot[row] = slot or -1 (padding); slot_row[slot] = row;
 // tile_group[tile] = expert or -1 (behind the last run). Bound by latency: a warp takes one stretch of the slots in both passes
 // (counting, then placing behind the stretches before it), so the block meets twice whatever the number of slots
-// (48 rounds of 256 threads that met twice each took 17 us for 12,288 slots, this takes 7.6).
-__global__ void __launch_bounds__(MOE_SORT_THREADS)
+// (48 rounds of 256 threads that met twice each took 17 us for 12,288 slots, this takes 7.6). Few slots are less than a block of
+// 1,024 threads costs to start and to meet (102 slots of 64 experts: 2.5 us in rounds of 256 threads, 3.2 with 1,024).
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
 moe_sort_kernel(int* __restrict__ row_slot, int* __restrict__ slot_row, int* __restrict__ tile_group, const int* __restrict__ idx, int S,
                 int E, int max_tiles) {
     extern __shared__ int sh[];
@@ -648,9 +650,9 @@ moe_sort_kernel(int* __restrict__ row_slot, int* __restrict__ slot_row, int* __r
     const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_trigger();
     pdl_wait();
-    for (int i = tid; i < E; i += MOE_SORT_THREADS) hist[i] = 0;
+    for (int i = tid; i < E; i += THREADS) hist[i] = 0;
     __syncthreads();
-    const int stretch = (S + MOE_SORT_THREADS - 1) / MOE_SORT_THREADS * 32, from = min(S, warp * stretch), to = min(S, from + stretch);
+    const int stretch = (S + THREADS - 1) / THREADS * 32, from = min(S, warp * stretch), to = min(S, from + stretch);
     int n = 0;
 #pragma unroll 4
     for (int i = from + lane; i < to; i += 32) {
@@ -663,7 +665,7 @@ moe_sort_kernel(int* __restrict__ row_slot, int* __restrict__ slot_row, int* __r
     if (lane == 0) found[warp] = n;
     __syncthreads();
     int start = 0;
-    for (int f = tid; f < e; f += MOE_SORT_THREADS) start += (hist[f] + MOE_TILE - 1) / MOE_TILE * MOE_TILE;
+    for (int f = tid; f < e; f += THREADS) start += (hist[f] + MOE_TILE - 1) / MOE_TILE * MOE_TILE;
 #pragma unroll
     for (int d = 16; d; d >>= 1) start += __shfl_xor_sync(0xffffffffu, start, d);
     if (lane == 0) parts[warp] = start;
@@ -671,15 +673,15 @@ moe_sort_kernel(int* __restrict__ row_slot, int* __restrict__ slot_row, int* __r
     start = 0;
     int at = 0;
 #pragma unroll
-    for (int w = 0; w < 32; ++w) {
+    for (int w = 0; w < THREADS / 32; ++w) {
         start += parts[w];
         at += w < warp ? found[w] : 0;
     }
     const int count = hist[e], padded = (count + MOE_TILE - 1) / MOE_TILE * MOE_TILE;
-    for (int i = tid; i < padded / MOE_TILE; i += MOE_SORT_THREADS) tile_group[start / MOE_TILE + i] = e;
+    for (int i = tid; i < padded / MOE_TILE; i += THREADS) tile_group[start / MOE_TILE + i] = e;
     if (e == E - 1)
-        for (int i = (start + padded) / MOE_TILE + tid; i < max_tiles; i += MOE_SORT_THREADS) tile_group[i] = -1;
-    for (int i = count + tid; i < padded; i += MOE_SORT_THREADS) row_slot[start + i] = -1;
+        for (int i = (start + padded) / MOE_TILE + tid; i < max_tiles; i += THREADS) tile_group[i] = -1;
+    for (int i = count + tid; i < padded; i += THREADS) row_slot[start + i] = -1;
     at += start;
     for (int i0 = from; i0 < to; i0 += 32) {
         const int i = i0 + lane;
@@ -697,7 +699,11 @@ moe_sort_kernel(int* __restrict__ row_slot, int* __restrict__ slot_row, int* __r
 CELLM_API int cellm_moe_sort(int* row_slot, int* slot_row, int* tile_group, const int* idx, int S, int E, int max_tiles, cudaStream_t stream) {
     if (S <= 0) return CELLM_OK;
     if (E < 1 || max_tiles < 1 || E > 8192) return CELLM_ERR_SIZE;
-    CELLM_RUN(moe_sort_kernel, E, MOE_SORT_THREADS, (size_t)(E + 64) * sizeof(int), stream, row_slot, slot_row, tile_group, idx, S, E, max_tiles);
+    const size_t smem = (size_t)(E + 64) * sizeof(int);
+    if (S <= MOE_SORT_FEW)
+        CELLM_RUN(moe_sort_kernel<256>, E, 256, smem, stream, row_slot, slot_row, tile_group, idx, S, E, max_tiles);
+    else
+        CELLM_RUN(moe_sort_kernel<1024>, E, 1024, smem, stream, row_slot, slot_row, tile_group, idx, S, E, max_tiles);
     return CELLM_OK;
 }
 

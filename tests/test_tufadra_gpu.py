@@ -503,7 +503,7 @@ def test_command_lines_take_the_design(models, tmp_path):
         check_close(traces.as_matrix(got[rid], len(toks)), ref[rid], "float32", f"trace_run {rid}")
 
 
-@pytest.mark.parametrize("T,E,top,H", [(17, 64, 6, 264), (341, 3, 3, 64), (1025, 70, 5, 72), (2, 1, 1, 2056), (700, 40, 9, 66)])
+@pytest.mark.parametrize("T,E,top,H", [(17, 64, 6, 264), (341, 3, 3, 64), (128, 33, 8, 72), (1025, 70, 5, 72), (2, 1, 1, 2056), (700, 40, 9, 66)])
 def test_sort_and_sum_of_the_experts_slots(T, E, top, H):
     """Slots that are no multiple of a warp's stretch, experts without a slot and with every slot, choices that are none; sums of
     one to nine rows, of widths that are taken eight columns a thread and two. The order of the sorted rows is the slots' own."""
