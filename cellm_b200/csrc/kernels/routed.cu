@@ -551,9 +551,11 @@ static int experts_rowwise_impl(void* out, void* mid, void* smid, const void* y,
     const int up_rows = ff > sff ? ff : sff;
     const int rpw_up = expert_rows_a_warp((long long)T * top * ff + (sup ? (long long)T * sff : 0), EXPERT_WARPS, gated ? 2 : 4, 4);
     const int rpw_down = expert_rows_a_warp((long long)T * H, EXPERT_DOWN_WARPS, 4, 2);
-    // gated: as many tokens' rows at once as 32 KB hold (one always fits where it did); a token's own experts are different ones
+    // gated: as many tokens' rows at once as 32 KB hold (one always fits where it did). A token's own experts are different ones, and
+    // two tokens share half a slot on average (6 of 64, 4 of 32 chosen): not worth the look for it, a wait on memory more (two
+    // tokens, 4 of 32 experts of 512: 12.8 us without, 13.9 with it)
     const size_t row_y = (size_t)H * (dtype == CELLM_F32 ? 4 : 2);
-    const int tg = !gated || T == 1 ? 1 : 4 * row_y <= 32 * 1024 ? 4 : 2 * row_y <= 32 * 1024 ? 2 : 1;
+    const int tg = !gated || T <= 2 ? 1 : 4 * row_y <= 32 * 1024 ? 4 : 2 * row_y <= 32 * 1024 ? 2 : 1;
     const size_t smem_y = tg * row_y;
     const dim3 grid_up((unsigned)(T * top + (sup ? (T + tg - 1) / tg : 0)), (unsigned)((up_rows + EXPERT_WARPS * rpw_up - 1) / (EXPERT_WARPS * rpw_up)));
     const dim3 grid_down((unsigned)T, (unsigned)((H + EXPERT_DOWN_WARPS * rpw_down - 1) / (EXPERT_DOWN_WARPS * rpw_down)));

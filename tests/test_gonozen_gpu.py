@@ -937,7 +937,7 @@ def test_clamped_experts_against_plain(dtype, T, H, E, top, ff, limit, groups, s
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("T,H,ff,sff,top,E", [(1, 64, 64, 64, 2, 4), (9, 264, 64, 192, 3, 4), (13, 100, 128, 64, 6, 9), (5, 4104, 64, 128, 2, 3),
+@pytest.mark.parametrize("T,H,ff,sff,top,E", [(1, 64, 64, 64, 2, 4), (2, 72, 64, 128, 3, 4), (9, 264, 64, 192, 3, 4), (13, 100, 128, 64, 6, 9), (5, 4104, 64, 128, 2, 3),
                                               (70, 72, 64, 64, 3, 5)])
 def test_clamped_experts_that_several_tokens_choose(dtype, T, H, ff, sff, top, E):
     """More slots of an expert than a block serves at once, rows of which only one or two fit beside each other, rows off the
