@@ -9,8 +9,9 @@
 // core kernels (the reference's own linear is a scalar loop over k,
 // crates/cellm-model/src/lfm.rs:970-978).
 //
-// 32-bit operands: the runs of a tile are summed by different groups of threads at once (gemm_runs_kernel); bfloat16 operands
-// (products the tensor-core kernels do not take) by one group, run after run. Both give the same sums.
+// 32-bit operands: the runs of a tile are summed by different groups of threads at once (gemm_runs_kernel); short products of
+// many tiles, rows off the 16-byte border and bfloat16 operands (products the tensor-core kernels do not take) by one group, run
+// after run. Both give the same sums.
 #include "common.cuh"
 
 #define GP_BM 64
@@ -137,7 +138,7 @@ static int run_tiles(float* C, const float* A, const float* W, int M, int N, int
     return CELLM_OK;
 }
 
-// ------------------------------------------------------------------------------------------------ bfloat16 operands
+// ------------------------------------------------------------------------------------------------ run after run
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256)
 gemm_plain_kernel(TO* __restrict__ C, const TI* __restrict__ A, const TI* __restrict__ W, int M, int N,
@@ -203,9 +204,16 @@ CELLM_API int cellm_gemm_plain(void* C, const void* A, const void* W, int M, int
                                cudaStream_t stream) {
     if (M <= 0 || N <= 0) return CELLM_OK;
     if (K <= 0) return CELLM_ERR_SIZE;
-    if (in_dtype == CELLM_F32 && out_dtype == CELLM_F32) {
+    // 32-bit operands go to the groups of threads from two runs of products on, and below where the 64 x 64 tiles are few; rows off
+    // the 16-byte border (copied value by value) only where those are very few. Elsewhere the tile's 256 threads of the other kernel
+    // hide more. Its time over the groups', products of 1 to 2,048 rows by 512 to 8,192 columns: K 512 to 1,536 0.97 to 5.2; K 32 to
+    // 300 0.98 to 2.5 where the line says groups, 0.46 to 1.02 where it does not (2,048 x 2,048 x 64: 27 against 40 us); K 513 1.65
+    // to 1.8 and 0.56 to 1.0. The sums are the same bits either way.
+    const int vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    const long long tiles64 = (long long)((M + GP_BM - 1) / GP_BM) * ((N + GP_BN - 1) / GP_BN);
+    const long long few = M <= 16 ? 32 : vec ? (K / 4 < 32 ? K / 4 : 32) : 8;
+    if (in_dtype == CELLM_F32 && out_dtype == CELLM_F32 && ((vec && K >= 2 * GP_RUN) || tiles64 <= few)) {
         const int n_runs = (K + GP_RUN - 1) / GP_RUN, rounds = (n_runs + 7) / 8, groups = (n_runs + rounds - 1) / rounds;
-        const int vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
         // The tile whose waves over the SMs take least. Microseconds of K = 1,536 measured for one tile an SM and for each
         // wave of several (the smaller tiles share an SM then): with 213 x 2,560 sums 64 x 64 takes 125 us, 32 x 64 68, 32 x 32
         // 87, 16 x 32 96; with 16 x 1,536 they take 63, 34, 22 and 18; with 2,048 x 2,048 (K 2,048) 545, 577, 723 and 836.
@@ -229,7 +237,8 @@ CELLM_API int cellm_gemm_plain(void* C, const void* A, const void* W, int M, int
     if (grid.y > 65535) return CELLM_ERR_SIZE;
 #define LAUNCH(TI, TO) \
     CELLM_RUN((gemm_plain_kernel<TI, TO>), grid, 256, 0, stream, (TO*)C, (const TI*)A, (const TI*)W, M, N, K, lda, ldw, ldc)
-    if (in_dtype == CELLM_BF16 && out_dtype == CELLM_BF16) LAUNCH(__nv_bfloat16, __nv_bfloat16);
+    if (in_dtype == CELLM_F32 && out_dtype == CELLM_F32) LAUNCH(float, float);
+    else if (in_dtype == CELLM_BF16 && out_dtype == CELLM_BF16) LAUNCH(__nv_bfloat16, __nv_bfloat16);
     else if (in_dtype == CELLM_BF16 && out_dtype == CELLM_F32) LAUNCH(__nv_bfloat16, float);
     else return CELLM_ERR_DTYPE;
 #undef LAUNCH

@@ -771,12 +771,23 @@ def test_gemm_plain_in_32_bits_does_not_depend_on_the_tile(M, N, K):
         assert torch.equal(ops.gemm_plain(rows[:min(M, 70)], w[:min(N, 40)], torch.float32), out[:min(M, 70), :min(N, 40)])
 
 
-@pytest.mark.parametrize("N", [8, 40])
-def test_gemm_plain_in_32_bits_of_a_million_rows(N):
+@pytest.mark.parametrize("K", [16, 64, 300, 508, 512, 513])
+def test_gemm_plain_in_32_bits_either_way(K):
+    """Products of many tiles and short or misaligned rows go run after run, those of few tiles to groups of threads: rows and
+    columns of the large one, multiplied alone, are the same bits."""
+    from cellm_b200 import ops
+    a, w = torch.randn(700, K, device=DEV), torch.randn(1000, K, device=DEV)
+    out = ops.gemm_plain(a, w, torch.float32)
+    close(out, a.double() @ w.double().T, torch.float32)
+    for rows, cols in ((slice(0, 16), slice(0, 64)), (slice(640, 700), slice(900, 1000)), (slice(5, 6), slice(0, 1000))):
+        assert torch.equal(ops.gemm_plain(a[rows].contiguous(), w[cols].contiguous(), torch.float32), out[rows, cols])
+
+
+@pytest.mark.parametrize("M,N,K", [(65536 * 16 + 5, 8, 512), (65536 * 32 + 5, 40, 4)])
+def test_gemm_plain_in_32_bits_of_a_million_rows(M, N, K):
     """More rows than a grid of tiles of 16 (or 32) of them holds, and so few columns that those would be chosen."""
     from cellm_b200 import ops
-    M = 65536 * 32 + 5
-    a, w = torch.randn(M, 4, device=DEV), torch.randn(N, 4, device=DEV)
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
     out = ops.gemm_plain(a, w, torch.float32)
     for part in (slice(0, 100), slice(M // 2, M // 2 + 100), slice(M - 100, M)):
         close(out[part], a[part].double() @ w.double().T, torch.float32)
