@@ -22,19 +22,24 @@
 //   chunk_vectors   W, Q, k E(., end), E(., end), U0 and O0 of every chunk and head, all of them at once
 //   chunk_walk      a block carries 16 columns of one (request, head)'s S through the chunks: two small products a chunk
 //
-// Everything is 32-bit fused multiply-adds, as token by token (relative error of the read-outs against 64 bits over 2,048 tokens
-// 8.9e-8, token by token 8.7e-8). One prompt of 2,048 tokens, 16 heads of 128 x 128: 938 -> 215 us (49 of them chunk_vectors).
+// chunk_vectors is 32-bit fused multiply-adds, as token by token; chunk_walk takes its products of 32-bit numbers on the tensor cores,
+// in three bfloat16 parts a factor. Against 64 bits over 2,048 tokens, in brackets with fused multiply-adds in the walk too (4 heads
+// of 128 x 128, decays uniform in 0.8 .. 1): read-outs 1.11e-7 (1.16e-7), the state behind them 7.2e-8 (8.9e-8); decays in
+// 0.999 .. 1 and repeating keys 3.3e-7 (5.0e-7) and 3.3e-7 (5.3e-7); uniform in 0 .. 1 9.2e-8 (9.3e-8) and 5.9e-8 (5.1e-8). HGRN2
+// 8.2e-8 (8.5e-8), 5.9e-8 (7.9e-8); 5.1e-7 (8.2e-7), 8.7e-7 (1.4e-6); 7.3e-8 (7.3e-8), 4.9e-8 (3.9e-8).
+// One prompt of 2,048 tokens, 16 heads of 128 x 128: token by token 938 us, in chunks with multiply-adds 214, now 163 (58 of them
+// chunk_vectors, which forms the parts).
 #include <algorithm>
 #include <climits>
 
+#include "mma_tiles.cuh"
 #include "tcgen05.cuh"
 
 namespace {
 
 constexpr int CT = 16;          // tokens a chunk
 constexpr int CB = 16;          // columns of S a block of the walk holds
-constexpr int WALK_THREADS = 256;
-constexpr int STAGES = 3;
+constexpr int MIN_STAGES = 3, MAX_STAGES = 4;
 
 struct ChunkArgs {
     const float *q, *k, *g, *v, *beta;      // k, beta: null for HGRN2
@@ -45,16 +50,60 @@ struct ChunkArgs {
     float* ws;                              // a chunk's and head's numbers at ((chunk - chunk0) * heads + head) * stride floats
     long long stride;
     int chunk0, chunks;                     // the step's chunks that are in the workspace
+    int stages;                             // of the walk's shared memory
 };
 
-// A (chunk, head) in the workspace: [NV][DIM] the rows of -W and Q (HGRN2: Q alone), [CT][DIM] k E(., end), [DIM] E(., end), then
-// per block of CB columns [CT][CB] of U0 and [CT][CB] of O0.
+// A (chunk, head) in the workspace, as the walk's products take it (operands of mma.sync m16n8k16 in three bfloat16 parts, a lane's
+// registers side by side): for every 16 channels -W (delta rule), Q and k E(., end) as right operands; E(., end) [DIM]; then
+// per block of CB columns U0 [CB][CT] (HGRN2: as a left operand) and O0 [CB][CT].
 template <int DIM, bool DELTA> struct Layout {
-    static constexpr int NV = DELTA ? 2 * CT : CT;
-    static constexpr int ROWS = (NV + CT + 1) * DIM;
-    static constexpr int COLS = 2 * CT * CB;
+    static constexpr int KINDS = DELTA ? 3 : 2, OPERAND = 3 * 32 * 4;
+    static constexpr int DECAY = DIM / 16 * KINDS * OPERAND, ROWS = DECAY + DIM;
+    static constexpr int O0 = DELTA ? CT * CB : OPERAND, COLS = O0 + CT * CB;
     static constexpr int STAGE = ROWS + COLS;
 };
+
+// A pair of 32-bit numbers as three pairs of bfloat16 numbers whose sums they are (8 bits each; what is left of 24 is below 2^-26).
+__device__ __forceinline__ uint64_t minus_parts(uint64_t x, uint32_t part) {
+    const uint64_t y = (uint64_t)(part & 0xffff0000u) << 32 | (part << 16);
+    uint64_t d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+    return d;
+}
+__device__ __forceinline__ uint32_t pack_pair(uint64_t x) { return pack_bf16(__uint_as_float((uint32_t)x), __uint_as_float((uint32_t)(x >> 32))); }
+__device__ __forceinline__ void split3(uint32_t& hi, uint32_t& mid, uint32_t& low, float x, float y) {
+    uint64_t pair = (uint64_t)__float_as_uint(y) << 32 | __float_as_uint(x);
+    hi = pack_pair(pair);
+    pair = minus_parts(pair, hi);
+    mid = pack_pair(pair);
+    low = pack_pair(minus_parts(pair, mid));
+}
+// Chunks of portion b, 0 where it is short; where a warp looks through the portions, a lane takes one of 32 (one after the other they
+// cost a block 0.3 us each).
+__device__ __forceinline__ int chunks_of(const ChunkArgs& a, int b) {
+    const int n = a.cu_seqlens[b + 1] - a.cu_seqlens[b];
+    return n < a.min_len ? 0 : (n + CT - 1) / CT;
+}
+// The portion that chunk c of the step lies in (c: which of its chunks), or -1.
+__device__ __forceinline__ int portion_of(const ChunkArgs& a, int& c, int lane) {
+    for (int b0 = 0; b0 < a.B; b0 += 32) {
+        int sum = b0 + lane < a.B ? chunks_of(a, b0 + lane) : 0;
+        const int own = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, sum, d);
+            if (lane >= d) sum += up;
+        }
+        const unsigned behind = __ballot_sync(0xffffffffu, sum > c);
+        if (behind) {
+            const int l = __ffs(behind) - 1;
+            c -= __shfl_sync(0xffffffffu, sum - own, l);
+            return b0 + l;
+        }
+        c -= __shfl_sync(0xffffffffu, sum, 31);
+    }
+    return -1;
+}
 
 // N values a lane, summed over 2 * TOP neighbouring lanes; a lane is left with N / (2 * TOP) of the sums, those from the
 // returned index on.
@@ -74,8 +123,9 @@ template <int N, int TOP> __device__ __forceinline__ int scatter_sums(float (&x)
     return first;
 }
 
-// A block a (chunk, head), a thread a channel. Bound by latency and by what it writes (41 KB a block of the delta rule with
-// 128 x 128).
+// A block a (chunk, head), a thread a channel. Bound by the instructions of the sums over channels and by what it writes (54 KB a
+// block of the delta rule with 128 x 128). The walk's operands leave here in parts, once for all of a head's blocks of columns: 47 ->
+// 58 us for 2,048 tokens and 16 heads, where splitting them in every block cost the walk 20.
 template <int DIM, bool DELTA>
 __global__ void __launch_bounds__(DIM)
 chunk_vectors_kernel(const ChunkArgs a) {
@@ -86,16 +136,12 @@ chunk_vectors_kernel(const ChunkArgs a) {
     pdl_trigger();
     pdl_wait();
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int t0 = 0, len = 0;
-    for (int b = 0, c = a.chunk0 + blockIdx.x; b < a.B; ++b) {
-        const int start = a.cu_seqlens[b], n = a.cu_seqlens[b + 1] - start;
-        if (n < a.min_len) continue;
-        const int nc = (n + CT - 1) / CT;
-        if (c < nc) { t0 = start + c * CT; len = min(CT, n - c * CT); break; }
-        c -= nc;
-    }
-    if (len == 0) return;
+    int c = a.chunk0 + blockIdx.x;
+    const int b = portion_of(a, c, lane);
+    if (b < 0) return;
+    const int t0 = a.cu_seqlens[b] + c * CT, len = min(CT, a.cu_seqlens[b + 1] - t0);
     float* ws = a.ws + ((size_t)blockIdx.x * a.heads + h) * a.stride;
+    uint32_t* operand = reinterpret_cast<uint32_t*>(ws) + (tid >> 4) * (L::KINDS * L::OPERAND);        // those of the thread's 16 channels
     const bool mine = tid < a.dim;
     const float* qp = a.q + (size_t)t0 * a.ld_q + (h / a.per) * a.dim + tid;
     const float* gp = a.g + (size_t)t0 * a.ld_g + h * a.dim + tid;
@@ -111,13 +157,22 @@ chunk_vectors_kernel(const ChunkArgs a) {
     }
     if (DELTA && tid < CT) beta[tid] = tid < len ? a.beta[(size_t)(t0 + tid) * a.heads + h] : 0.f;
     {
-        float e = 1.f;
+        // tokens 4 t .. 4 t + 3 of a channel are two registers of lane t of its row
+        uint32_t* out = operand + (L::KINDS - 1) * L::OPERAND + (((tid >> 2) & 3) * 2 + (tid & 1)) * 16 + (tid & 2);
+        float e = 1.f, ke[4];
 #pragma unroll
         for (int t = CT - 1; t >= 0; --t) {
-            ws[(L::NV + t) * DIM + tid] = k[t] * e;
+            ke[t & 3] = k[t] * e;
+            if ((t & 3) == 0) {
+                uint32_t x[3], y[3];
+                split3(x[0], x[1], x[2], ke[0], ke[1]);
+                split3(y[0], y[1], y[2], ke[2], ke[3]);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(out + p * 128 + t) = make_uint2(x[p], y[p]);
+            }
             e *= g[t];
         }
-        ws[(L::NV + CT) * DIM + tid] = e;
+        ws[L::DECAY + tid] = e;
     }
     // A and B: for every s the sums over the channels of (k_t | q_t) E(s, t) k_s, t = s .. CT - 1
     if constexpr (DELTA) {
@@ -187,32 +242,46 @@ chunk_vectors_kernel(const ChunkArgs a) {
         __syncthreads();
     }
     {
-        float e = 1.f, w[CT];
+        float e = 1.f;
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
             e *= g[t];
             q[t] *= e;
             k[t] *= e;
         }
+        // rows t and t + 8 of 16 channels as a pair of right operands: channels 4 i .. 4 i + 3 of a row are two registers of lane i of it;
+        // of two neighbouring channels the even one's thread takes row t of both, the odd one's row t + 8
+        auto rows_out = [&](uint32_t* out, const float (&x)[CT]) {
+            const bool odd = tid & 1;
+            out += ((tid >> 2) & 3) * 4 + 2 * odd + ((tid >> 1) & 1);
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                const float other = __shfl_xor_sync(0xffffffffu, odd ? x[t] : x[t + 8], 1);
+                uint32_t part[3];
+                split3(part[0], part[1], part[2], odd ? other : x[t], odd ? x[t + 8] : other);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) out[p * 128 + t * 16] = part[p];
+            }
+        };
         if constexpr (DELTA) {
+            float w[CT];
 #pragma unroll
             for (int t = 0; t < CT; ++t) {
                 float sum = 0.f;
 #pragma unroll
                 for (int s = 0; s <= t; ++s) sum = fmaf(Ts[t][s], k[s], sum);
                 w[t] = -sum;
-                ws[t * DIM + tid] = -sum;
             }
-        }
+            rows_out(operand, w);
 #pragma unroll
-        for (int t = 0; t < CT; ++t) {
-            float sum = q[t];
-            if constexpr (DELTA) {
+            for (int t = 0; t < CT; ++t) {
+                float sum = q[t];
 #pragma unroll
                 for (int s = 0; s <= t; ++s) sum = fmaf(Bs[t][s], w[s], sum);
+                q[t] = sum;
             }
-            ws[(L::NV - CT + t) * DIM + tid] = sum;
         }
+        rows_out(operand + (L::KINDS - 2) * L::OPERAND, q);
     }
     const int blocks = (a.vd + CB - 1) / CB;
 #pragma unroll 1
@@ -221,7 +290,7 @@ chunk_vectors_kernel(const ChunkArgs a) {
         float v[CT], u[CT];
 #pragma unroll
         for (int t = 0; t < CT; ++t) v[t] = (j < a.vd && t < len) ? a.v[(size_t)(t0 + t) * a.ld_v + h * a.vd + j] : 0.f;
-        float* out = ws + L::ROWS + (size_t)(j / CB) * L::COLS + j % CB;
+        float* out = ws + L::ROWS + (size_t)(j / CB) * L::COLS;
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
             if constexpr (DELTA) {
@@ -229,67 +298,112 @@ chunk_vectors_kernel(const ChunkArgs a) {
 #pragma unroll
                 for (int s = 0; s <= t; ++s) sum = fmaf(Ts[t][s], v[s], sum);
                 u[t] = sum;
+                if ((t & 3) == 3) *reinterpret_cast<float4*>(out + (j % CB) * CT + t - 3) = make_float4(u[t - 3], u[t - 2], u[t - 1], u[t]);
             } else {
+                // tokens 4 i .. 4 i + 3 of a column are two registers of lane i of it
                 u[t] = v[t];
+                if (t & 1) {
+                    uint32_t* to = reinterpret_cast<uint32_t*>(out) + ((j & 7) * 4 + (t >> 2)) * 4 + ((j >> 3) & 1) + (t & 2);
+                    split3(to[0], to[128], to[256], v[t - 1], v[t]);
+                }
             }
-            out[t * CB] = u[t];
         }
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
             float sum = 0.f;
 #pragma unroll
             for (int s = 0; s <= t; ++s) sum = fmaf(Bs[t][s], u[s], sum);
-            out[(CT + t) * CB] = sum;
+            v[t] = sum;
+            if ((t & 3) == 3) *reinterpret_cast<float4*>(out + L::O0 + (j % CB) * CT + t - 3) = make_float4(v[t - 3], v[t - 2], v[t - 1], v[t]);
         }
     }
 }
-
-// Two 32-bit multiply-adds in one instruction (each rounded as fmaf).
-__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
-    return (unsigned long long)__float_as_uint(hi) << 32 | __float_as_uint(lo);
-}
-__device__ __forceinline__ float low_of(unsigned long long x) { return __uint_as_float((unsigned)x); }
-__device__ __forceinline__ float high_of(unsigned long long x) { return __uint_as_float((unsigned)(x >> 32)); }
 
 // Contiguous floats (16-byte aligned, a multiple of four) into shared memory; the barrier counts the bytes.
 __device__ __forceinline__ void copy_bulk(float* dst, const float* src, int floats, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(dst)), "l"(src), "r"(floats * 4), "r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void set_barrier(int set) { asm volatile("bar.sync %0, 128;" ::"r"(set + 1) : "memory"); }
 
-// A block carries CB columns of one (request, head)'s S through the request's chunks that are in the workspace; 16 columns make 128 blocks of a prompt
-// over 16 heads of 128 columns, which is nearly the GPU. Two sets of four warps carry eight columns each, on their own barriers,
-// so that one set's first product runs beside the other's second; a ninth warp copies the chunks ahead of them. S lies twice: a
-// thread's own entries in registers, which the second product moves on, and all of it by columns in shared memory, which the
-// first one reads.
-//   first product   [-W ; Q] S: a warp takes a quarter of the rows, 16 lanes split the channels, a lane forms NV / 4 x 4 sums
-//                   over its share; the lanes' shares are added so that every lane ends with its own of the sums. U0 and O0
-//                   are added: u goes to shared memory, o to memory.
-//   second product  S <- diag(E) S + (k E)^T u, a thread two or four rows by two columns.
-// Bound by shared memory's bandwidth (every warp reads its share of the chunk's rows and the set's columns). With all eight warps
-// on one barrier and every thread copying, the phases added up: 290 us a prompt of 2,048 tokens where this form takes 166.
+// The operands of mma.sync m16n8k16 in three parts each, [part][register].
+struct Rows3 { uint32_t r[3][4]; };
+struct Cols3 { uint32_t r[3][2][2]; };       // two right operands side by side
+// A times each of the two of B (16 x 16 by 16 x 8) of 32-bit numbers: the products of the parts down to 2^-16 of the largest, as three
+// sums each (a chain of products waits 21 cycles for every one of two chains, 12 for one of eight). The tensor cores cut
+// their sums instead of rounding them, so the largest parts' products stand alone, in `most`, and the others, whose cut lies far below
+// a 32-bit sum's last place, in `rest`. CUT: what the cut took from `most` is formed too (the same products on top of minus their
+// sum: the tensor cores carry a few bits beyond 32-bit sums) and added to `rest`.
+template <bool CUT>
+__device__ __forceinline__ void product3(float (&most)[2][4], float (&rest)[2][4], const Rows3& a, const Cols3& b) {
+    float x[2][3][4], cut[2][4];
+#pragma unroll
+    for (int i = 0; i < 12; ++i) (&x[0][0][0])[i] = (&x[1][0][0])[i] = 0.f;
+    constexpr int PA[6] = {0, 2, 0, 1, 0, 1}, PB[6] = {0, 0, 2, 1, 1, 0}, TO[6] = {2, 0, 1, 0, 1, 0};
+#pragma unroll
+    for (int p = 0; p < 6; ++p)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) mma_bf16(x[j][TO[p]], a.r[PA[p]], b.r[PB[p]][j][0], b.r[PB[p]][j][1]);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        if constexpr (CUT) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) cut[j][i] = -x[j][2][i];
+            mma_bf16(cut[j], a.r[0], b.r[0][j][0], b.r[0][j][1]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            rest[j][i] = x[j][0][i] + x[j][1][i];
+            if constexpr (CUT) rest[j][i] += cut[j][i];
+            most[j][i] = x[j][2][i];
+        }
+}
+
+template <int DIM, bool DELTA> struct Walk {
+    static constexpr int WARPS = DIM / 16, READ = DELTA ? WARPS : 0, SUMS = 4, MEET = (WARPS + READ + SUMS) * 32, THREADS = MEET + 32;
+    static constexpr int PART = WARPS * CT * CB;        // a product's sums over every warp's channels
+    static constexpr int SMEM_FLOATS = DELTA ? 3 * PART + (2 * WARPS + 1) * 3 * 32 * 4 : 2 * PART;
+};
+
+// A block carries CB columns of one (request, head)'s S through the request's chunks that are in the workspace; 16 columns make 128
+// blocks of a prompt over 16 heads of 128 columns, which is nearly the GPU. Its warps by their work:
+//   WARPS   hold 16 channels by 16 columns of S^T each, as the accumulators of mma.sync m16n8k16, which are its left operand as well:
+//           S^T [-W]^T over their channels, for u; then S^T <- S^T diag(E) + u^T (k E) over the chunk's 16 tokens (HGRN2: u is given)
+//   READ    take the read-outs S^T Q^T over as many channels each, from copies of that left operand, beside the chain (HGRN2, whose chain
+//           is short: the state's warps do, and two blocks fit an SM, which many requests need)
+//   SUMS    add the warps' sums, in a fixed order, with U0 or O0 on top: u goes back as a left operand, o to memory
+//   1       copies the chunks ahead of them all
+// All numbers stay 32-bit: an operand enters as three bfloat16 numbers, a product as the six products of parts above 2^-24 of it
+// (product3); sums over more than 16 terms are 32-bit additions. An infinite entry of S or u makes its column's later results NaN.
+// Bound by the chain of a chunk, 0.8 us: products (24 of mma.sync a scheduler, 9 cycles each, twice), the meeting of the warps, u's sums, u
+// back to all of them. With multiply-adds on S in shared memory the walk took 166 us for 2,048 tokens and 16 heads of 128 x 128, bound
+// by shared memory's bandwidth; this form 105. What that took: no mbarrier on the chain, loads beside products, read-outs and
+// sums on warps of their own (with the sums on the state's warps and an mbarrier a hand-over 125). HGRN2 with heads of 64 x 64,
+// which has no u to wait for: 88 -> 45 us for 128 chunks. Where blocks are many (32 portions of 100 tokens, 16 heads of 128 x 128) HGRN2's
+// walk is bound by the products: 304 us with chunk_vectors, with multiply-adds 281; heads of 64 rows 170 (172).
 template <int DIM, bool DELTA>
-__global__ void __launch_bounds__(WALK_THREADS + 32)
+__global__ void __launch_bounds__(Walk<DIM, DELTA>::THREADS, DIM == 128 && DELTA ? 1 : 2)
 chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long long slot_stride, int n_slots, const ChunkArgs a,
                   int* __restrict__ err) {
     using L = Layout<DIM, DELTA>;
-    constexpr int MT = L::NV / 4, SP = DIM + 4, RPT = DIM / 32;
+    using W = Walk<DIM, DELTA>;
+    constexpr int WARPS = W::WARPS, SUMS = W::SUMS;
     extern __shared__ __align__(16) float sm[];
-    float* Ssh = sm + STAGES * L::STAGE;         // [CB][SP]: column by column
-    float* ush = Ssh + CB * SP;                  // [2 sets][CT][CB / 2]
-    __shared__ uint64_t full[STAGES], empty[STAGES];
+    float* part = sm + a.stages * L::STAGE;      // [3][WARPS][CT * CB]: read-outs of even and of odd chunks, u
+    float* u_part = part + 2 * W::PART;
+    uint32_t* frags = reinterpret_cast<uint32_t*>(part + 3 * W::PART);        // [2][WARPS] S before even and before odd chunks; u
+    uint32_t* ufrag = frags + 2 * WARPS * L::OPERAND;
+    __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES];
     __shared__ int abort_flag_;
     volatile int* abort_flag = &abort_flag_;
     // the column blocks of a head, its request's heads, the requests: neighbours run through the same chunks at the same time (with
     // the requests' blocks in turn, two prompts of unequal lengths took 326 us through both mixers instead of 295)
     const int blocks = (a.vd + CB - 1) / CB, blk = blockIdx.x % blocks, h = blockIdx.x / blocks % a.heads, b = blockIdx.x / blocks / a.heads;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
     if (tid == 0) {
-        for (int i = 0; i < STAGES; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], WALK_THREADS / 32);
+        for (int i = 0; i < a.stages; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
         abort_flag_ = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -300,133 +414,220 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     const int start = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - start;
     if (len < a.min_len) return;
     int before = 0;                              // chunks of the requests before this one
-    for (int i = 0; i < b; ++i) {
-        const int n = a.cu_seqlens[i + 1] - a.cu_seqlens[i];
-        if (n >= a.min_len) before += (n + CT - 1) / CT;
-    }
+    for (int i = lane; i < b; i += 32) before += chunks_of(a, i);
+    before = __reduce_add_sync(0xffffffffu, before);
     const int c0 = max(0, a.chunk0 - before), n_chunks = min((len + CT - 1) / CT, a.chunk0 + a.chunks - before) - c0;
     if (n_chunks <= 0) return;
     __syncthreads();
-    if (warp == WALK_THREADS / 32) {
+    const int warp = (tid >> 5) % WARPS;
+    const int g = lane >> 2, t4 = lane & 3, col0 = blk * CB;
+    int at = 0;                                  // the chunk's stage
+    uint32_t lap = 0;
+    auto next = [&]() { if (++at == a.stages) at = 0, ++lap; };
+    // the products' right operands over the warp's channels: -W (delta rule), Q, k E
+    auto right_operands = [&](Cols3& x, int kind) {
+        const float* from = sm + at * L::STAGE + (size_t)(warp * L::KINDS + kind) * L::OPERAND + lane * 4;
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            const uint4 y = *reinterpret_cast<const uint4*>(from + p * 128);
+            x.r[p][0][0] = y.x, x.r[p][0][1] = y.y, x.r[p][1][0] = y.z, x.r[p][1][1] = y.w;
+        }
+    };
+    auto left_operand = [&](Rows3& x, const uint32_t* from) {
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            const uint4 y = *reinterpret_cast<const uint4*>(from + (p * 32 + lane) * 4);
+            x.r[p][0] = y.x, x.r[p][1] = y.y, x.r[p][2] = y.z, x.r[p][3] = y.w;
+        }
+    };
+    float most[2][4], rest[2][4];
+    // a warp's product into its place among the warps'
+    auto put = [&](float* p) {
+        p += warp * (CT * CB) + lane * 4;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            *reinterpret_cast<float4*>(p + 128 * j) = make_float4(rest[j][0] + most[j][0], rest[j][1] + most[j][1], rest[j][2] + most[j][2], rest[j][3] + most[j][3]);
+    };
+    // Once a chunk all but the copying warp meet: from then on the next chunk is there, S before this one and every warp's share of -W S
+    // can be read, and so can the shares of read-outs (of the last chunk; HGRN2: of this one); the last chunk's stage is free. The state's warps of the delta rule only
+    // say so and wait where u is whole. (An mbarrier costs a wait 60 cycles even where it has been passed: only the sums' warps look at
+    // the copies' and tell the others.)
+    auto meet = []() { asm volatile("bar.sync 1, %0;" ::"n"(W::MEET) : "memory"); };
+    auto meet_later = []() { asm volatile("bar.arrive 1, %0;" ::"n"(W::MEET) : "memory"); };
+    auto u_whole = []() { asm volatile("bar.arrive 2, %0;" ::"n"((WARPS + SUMS) * 32) : "memory"); };
+    auto wait_u = []() { asm volatile("bar.sync 2, %0;" ::"n"((WARPS + SUMS) * 32) : "memory"); };
+    if (tid >= W::MEET) {        // ------------------------------------------------ copies
         if (lane != 0) return;
         const float* ws = a.ws + ((size_t)(before + c0 - a.chunk0) * a.heads + h) * a.stride;
         int issued = 0;
         for (; issued < n_chunks; ++issued, ws += (size_t)a.heads * a.stride) {
-            const int st = issued % STAGES;
-            if (issued >= STAGES && !mbar_wait(&empty[st], (uint32_t)(issued / STAGES - 1) & 1u, abort_flag)) break;
-            mbar_expect_tx(&full[st], L::STAGE * 4);
-            copy_bulk(sm + st * L::STAGE, ws, L::ROWS, &full[st]);
-            copy_bulk(sm + st * L::STAGE + L::ROWS, ws + L::ROWS + (size_t)blk * L::COLS, L::COLS, &full[st]);
+            if (lap && !mbar_wait(&empty[at], (lap - 1) & 1u, abort_flag)) break;
+            mbar_expect_tx(&full[at], L::STAGE * 4);
+            copy_bulk(sm + at * L::STAGE, ws, L::ROWS, &full[at]);
+            copy_bulk(sm + at * L::STAGE + L::ROWS, ws + L::ROWS + (size_t)blk * L::COLS, L::COLS, &full[at]);
+            next();
         }
         if (issued < n_chunks) {        // given up: the copies under way still land in this block's memory
             *abort_flag = 1;
             atomicOr(err, CELLM_DEV_WAIT_TIMEOUT);
         }
         int none = 0;
-        for (int c = max(0, issued - STAGES); c < issued; ++c) mbar_wait(&full[c % STAGES], (uint32_t)(c / STAGES) & 1u, &none);
+        for (int c = max(0, issued - a.stages); c < issued; ++c) mbar_wait(&full[c % a.stages], (uint32_t)(c / a.stages) & 1u, &none);
         return;
     }
-    const int set = warp >> 2, vg = warp & 3, col0 = blk * CB;
-    // the thread's entries of S: rows row .. row + RPT - 1, columns col, col + 1 of the block's
-    const int row = vg * (DIM / 4) + (lane >> 2) * RPT, col = set * (CB / 2) + (lane & 3) * 2;
-    float* st = state + (size_t)slot * slot_stride + (size_t)h * a.dim * a.vd;
-    unsigned long long S[RPT / 2][2];            // [pair of rows][column]
-    auto entry = [&](int r, int c) -> float* {
-        return (row + r < a.dim && col0 + col + c < a.vd) ? st + (size_t)(row + r) * a.vd + col0 + col + c : nullptr;
-    };
-    auto publish = [&]() {
+    if (tid >= (WARPS + W::READ) * 32) {                             // ------------------------------------------------ sums over the warps
+        // a thread: one column of two neighbouring tokens, registers 2 half and 2 half + 1 of lane l's accumulator j
+        const int r = tid - (WARPS + W::READ) * 32, l = (r >> 1) & 31, half = r & 1, j = r >> 6;
+        const int col = (l >> 2) + 8 * half, token = 8 * j + 2 * (l & 3);
+        auto add_up = [&](const float* p, float2 x) {
+            float2 y[WARPS];
 #pragma unroll
-        for (int r = 0; r < RPT / 2; ++r)
+            for (int w = 0; w < WARPS; ++w) y[w] = *reinterpret_cast<const float2*>(p + w * (CT * CB) + 2 * r);
 #pragma unroll
-            for (int c = 0; c < 2; ++c) *reinterpret_cast<unsigned long long*>(Ssh + (col + c) * SP + row + 2 * r) = S[r][c];
-    };
+            for (int n = WARPS / 2; n >= 1; n >>= 1)
 #pragma unroll
-    for (int r = 0; r < RPT / 2; ++r)
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const float *lo = entry(2 * r, c), *hi = entry(2 * r + 1, c);
-            S[r][c] = pair_of(lo ? *lo : 0.f, hi ? *hi : 0.f);
-        }
-    publish();
-    const int ks = lane & 15, cols1 = set * (CB / 2) + (lane >> 4) * 4;
-    float* uset = ush + set * CT * (CB / 2);
-    const int left = len - c0 * CT;              // tokens from the first of these chunks on
-    float* o_row = o_out + (size_t)(start + c0 * CT) * a.heads * a.vd + (size_t)h * a.vd + col0;
-    bool ok = true;
-    for (int c = 0; c < n_chunks; ++c) {
-        const float* stage = sm + (c % STAGES) * L::STAGE;
-        const float* uo = stage + L::ROWS;
-        if (!mbar_wait(&full[c % STAGES], (uint32_t)(c / STAGES) & 1u, abort_flag)) {
-            ok = false;
+                for (int w = 0; w < n; ++w) y[w].x += y[w + n].x, y[w].y += y[w + n].y;
+            return make_float2(x.x + y[0].x, x.y + y[0].y);
+        };
+        bool ok = true;
+        auto there = [&]() {
+            if (mbar_wait(&full[at], lap & 1u, abort_flag)) return;
+            ok = false;                          // bounded: every warp still runs through its chunks, and nothing is written
             *abort_flag = 1;
             atomicOr(err, CELLM_DEV_WAIT_TIMEOUT);
-        }
-        set_barrier(set);        // the set's columns of S are whole
-        // sums over the even and over the odd channels of the lane's share, side by side
-        unsigned long long sums[MT * 4];
-#pragma unroll
-        for (int i = 0; i < MT * 4; ++i) sums[i] = 0;
-#pragma unroll
-        for (int kk = 0; kk < DIM / 64; ++kk) {
-            const int at = kk * 64 + ks * 4;
-            ulonglong2 s[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s[j] = *reinterpret_cast<const ulonglong2*>(Ssh + (cols1 + j) * SP + at);
-#pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(stage + (vg * MT + m) * DIM + at);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    fma2(sums[m * 4 + j], w.x, s[j].x);
-                    fma2(sums[m * 4 + j], w.y, s[j].y);
-                }
+        };
+        const size_t o_ld = (size_t)a.heads * a.vd;
+        float* o = o_out + (size_t)(start + c0 * CT + token) * o_ld + (size_t)h * a.vd + col0 + col;
+        int left = col0 + col < a.vd ? len - c0 * CT - token : 0;        // tokens from the thread's first on
+        auto read_out = [&](int c, float2 x) {
+            x = add_up(part + (c & 1) * W::PART, x);
+            if (ok && left > 0) *o = x.x;
+            if (ok && left > 1) o[o_ld] = x.y;
+            o += CT * o_ld, left -= CT;
+        };
+        // u's pair among the left operand's registers: tokens 4 t .. 4 t + 3 of a column are lane t's registers half and half + 2
+        uint32_t* to = ufrag + ((l & 28) + 2 * j + ((l & 3) >> 1)) * 4 + half + 2 * (l & 1);
+        float2 u0 = make_float2(0.f, 0.f), o0 = u0;
+        there();
+        meet();
+        for (int c = 0; c < n_chunks; ++c) {
+            const float* uo = sm + at * L::STAGE + L::ROWS + col * CT + token;
+            const float2 o1 = *reinterpret_cast<const float2*>(uo + L::O0);
+            if constexpr (DELTA) u0 = *reinterpret_cast<const float2*>(uo);
+            const int last = at == 0 ? a.stages - 1 : at - 1;
+            next();
+            if (c + 1 < n_chunks) there();
+            meet();
+            if constexpr (DELTA) {
+                const float2 x = add_up(u_part, u0);
+                split3(to[0], to[128], to[256], x.x, x.y);
+                u_whole();
             }
+            if (c > 0 && r == 0) mbar_arrive(&empty[last]);
+            // the delta rule's read-outs are formed while u's sums are: they are there a chunk later
+            if constexpr (!DELTA) read_out(c, o1);
+            else if (c > 0) read_out(c - 1, o0);
+            o0 = o1;
         }
-        float acc[MT * 4];
-#pragma unroll
-        for (int i = 0; i < MT * 4; ++i) acc[i] = low_of(sums[i]) + high_of(sums[i]);
-        const int idx = scatter_sums<MT * 4, 8>(acc, ks);
-#pragma unroll
-        for (int i = 0; i < MT / 4; ++i) {
-            const int v = vg * MT + (idx + i) / 4, j = cols1 + (idx + i) % 4;
-            if (DELTA && v < CT) {
-                uset[v * (CB / 2) + j % (CB / 2)] = acc[i] + uo[v * CB + j];
-            } else {
-                const int t = v - (L::NV - CT);
-                if (ok && c * CT + t < left && col0 + j < a.vd) o_row[(size_t)(c * CT + t) * a.heads * a.vd + j] = acc[i] + uo[(CT + t) * CB + j];
-            }
-        }
-        set_barrier(set);        // u is whole, and the set's columns of S have been read
-        const float* ke = stage + L::NV * DIM + row;
-#pragma unroll
-        for (int r = 0; r < RPT / 2; ++r) {
-            const unsigned long long e = *reinterpret_cast<const unsigned long long*>(ke + CT * DIM + 2 * r);
-#pragma unroll
-            for (int j = 0; j < 2; ++j) S[r][j] = pair_of(low_of(S[r][j]) * low_of(e), high_of(S[r][j]) * high_of(e));
-        }
-#pragma unroll
-        for (int t = 0; t < CT; ++t) {
-            const float2 u = *reinterpret_cast<const float2*>(DELTA ? uset + t * (CB / 2) + (lane & 3) * 2 : uo + t * CB + col);
-            const unsigned long long u0 = pair_of(u.x, u.x), u1 = pair_of(u.y, u.y);
-            if constexpr (RPT == 4) {
-                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(ke + t * DIM);
-                fma2(S[0][0], k.x, u0), fma2(S[0][1], k.x, u1);
-                fma2(S[RPT / 2 - 1][0], k.y, u0), fma2(S[RPT / 2 - 1][1], k.y, u1);
-            } else {
-                const unsigned long long k = *reinterpret_cast<const unsigned long long*>(ke + t * DIM);
-                fma2(S[0][0], k, u0), fma2(S[0][1], k, u1);
-            }
-        }
-        publish();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[c % STAGES]);
+        meet();
+        if constexpr (DELTA) read_out(n_chunks - 1, o0);
+        return;
     }
-    if (!ok) return;             // the copies gave up: the state stays as it was
+    Cols3 w;
+    if (DELTA && tid >= WARPS * 32) {                             // ------------------------------------------------ read-outs
+        meet();
+        right_operands(w, L::KINDS - 2);
+        for (int c = 0; c < n_chunks; ++c) {
+            meet();
+            Rows3 s;
+            left_operand(s, frags + ((c & 1) * WARPS + warp) * L::OPERAND);
+            product3<false>(most, rest, s, w);
+            next();
+            if (c + 1 < n_chunks) right_operands(w, L::KINDS - 2);
+            put(part + (c & 1) * W::PART);
+        }
+        meet();
+        return;
+    }
+    // -------------------------------------------------------------------------------------------- the state
+    // the lane's entries of S: accumulator j's register 2 c + e is channel row + 2 j + e, column g + 8 c of the block
+    const int row = warp * 16 + t4 * 4;
+    float* st = state + (size_t)slot * slot_stride + (size_t)h * a.dim * a.vd;
+    auto entry = [&](int j, int i) -> float* {
+        const int r = row + 2 * j + (i & 1), c = col0 + g + 8 * (i >> 1);
+        return (r < a.dim && c < a.vd) ? st + (size_t)r * a.vd + c : nullptr;
+    };
+    float S[2][4];
+    Rows3 s;                                     // S as a left operand
 #pragma unroll
-    for (int r = 0; r < RPT; ++r)
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
-            if (float* p = entry(r, c)) *p = r & 1 ? high_of(S[r / 2][c]) : low_of(S[r / 2][c]);
+        for (int i = 0; i < 4; ++i) {
+            const float* p = entry(j, i);
+            S[j][i] = p ? *p : 0.f;
+        }
+    auto split_state = [&]() {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) split3(s.r[0][2 * j + c], s.r[1][2 * j + c], s.r[2][2 * j + c], S[j][2 * c], S[j][2 * c + 1]);
+    };
+    split_state();
+    Cols3 k;
+    Rows3 u;
+    float4 e;
+    // u^T (k E), with S's own decays
+    auto chunk_operands = [&]() {
+        right_operands(k, L::KINDS - 1);
+        e = *reinterpret_cast<const float4*>(sm + at * L::STAGE + L::DECAY + row);
+        if constexpr (!DELTA) left_operand(u, reinterpret_cast<const uint32_t*>(sm + at * L::STAGE + L::ROWS));
+    };
+    meet();
+    right_operands(w, 0);
+    if constexpr (!DELTA) chunk_operands();
+    for (int c = 0; c < n_chunks; ++c) {
+        // (loads stand where they run beside products, not beside the sums' loads, which everything waits for)
+        if constexpr (DELTA) chunk_operands();
+        product3<false>(most, rest, s, w);
+        if constexpr (DELTA) {
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+                *reinterpret_cast<uint4*>(frags + ((c & 1) * WARPS + warp) * L::OPERAND + (p * 32 + lane) * 4) =
+                    make_uint4(s.r[p][0], s.r[p][1], s.r[p][2], s.r[p][3]);
+            put(u_part);
+            meet_later();
+            wait_u();
+            left_operand(u, ufrag);
+        } else {
+            put(part + (c & 1) * W::PART);
+        }
+        product3<true>(most, rest, u, k);
+        const float4 f = e;
+        next();
+        if constexpr (DELTA) {
+            if (c + 1 < n_chunks) right_operands(w, 0);
+        } else {
+            meet();
+            if (c + 1 < n_chunks) {
+                right_operands(w, 0);
+                chunk_operands();
+            }
+        }
+        // one rounding where the chunk's tokens prevail, two where the state does
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            S[0][i] = fmaf(i & 1 ? f.y : f.x, S[0][i], rest[0][i]) + most[0][i];
+            S[1][i] = fmaf(i & 1 ? f.w : f.z, S[1][i], rest[1][i]) + most[1][i];
+        }
+        split_state();
+    }
+    meet();
+    if (*abort_flag) return;     // the copies gave up: the state stays as it was
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (float* p = entry(j, i)) *p = S[j][i];
 }
 
 template <int DIM, bool DELTA> int floats_a_chunk(int vd) {
@@ -437,15 +638,22 @@ template <int DIM, bool DELTA>
 int run(float* o_out, float* state, long long slot_stride, int n_slots, ChunkArgs a, int n_chunks, int ws_chunks, int* err, cudaStream_t stream) {
     using L = Layout<DIM, DELTA>;
     a.stride = floats_a_chunk<DIM, DELTA>(a.vd);
-    const size_t smem = (size_t)(STAGES * L::STAGE + CB * (DIM + 4) + CT * CB) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(chunk_walk_kernel<DIM, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
     const long long walk_blocks = (long long)a.B * a.heads * ((a.vd + CB - 1) / CB);
     if (walk_blocks > INT_MAX) return CELLM_ERR_SIZE;
+    // The walk's blocks become resident while chunk_vectors still runs, wherever it leaves room first: without a bound two of them met
+    // on one SM beside idle ones (delta rule, 128 blocks: 233 us for both kernels instead of 170). So a block asks for as
+    // much shared memory as lets an SM hold no more of them than an even spread needs, and makes stages of it (more than four bring
+    // nothing and keep the next kernel's blocks out: two prompts through both mixers 283 us with up to eight, 270 with four).
+    const int an_sm = (int)std::min<long long>((walk_blocks + 147) / 148, 8);
+    constexpr int fixed = Walk<DIM, DELTA>::SMEM_FLOATS * 4, stage = L::STAGE * 4;
+    a.stages = std::max(MIN_STAGES, std::min(MAX_STAGES, (224 * 1024 / an_sm - 2048 - fixed) / stage));
+    const size_t smem = std::max(a.stages * stage + fixed, 228 / (an_sm + 1) * 1024);
+    cudaError_t e = cudaFuncSetAttribute(chunk_walk_kernel<DIM, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+    if (e != cudaSuccess) return (int)e;
     for (a.chunk0 = 0; a.chunk0 < n_chunks; a.chunk0 += ws_chunks) {
         a.chunks = std::min(ws_chunks, n_chunks - a.chunk0);
         CELLM_RUN((chunk_vectors_kernel<DIM, DELTA>), dim3(a.chunks, a.heads), DIM, 0, stream, a);
-        CELLM_RUN((chunk_walk_kernel<DIM, DELTA>), (unsigned)walk_blocks, WALK_THREADS + 32, smem, stream, o_out, state,
+        CELLM_RUN((chunk_walk_kernel<DIM, DELTA>), (unsigned)walk_blocks, (Walk<DIM, DELTA>::THREADS), smem, stream, o_out, state,
                   slot_stride, n_slots, a, err);
     }
     return CELLM_OK;
@@ -475,7 +683,7 @@ CELLM_API int cellm_delta_chunks(float* o_out, float* state, long long slot_stri
     if (kvh <= 0 || heads % kvh || !fits(B, heads, heads / kvh, dim, vd, n_chunks, ws_chunks, ws) || min_len < 1) return CELLM_ERR_SIZE;
     const long long ld = 2LL * kvh * dim;
     ChunkArgs a{qk, qk + (size_t)kvh * dim, decay, v, beta, ld, ld, (long long)heads * dim, (long long)heads * vd, heads / kvh,
-                cu_seqlens, slot_ids, B, min_len, heads, dim, vd, ws, 0, 0, 0};
+                cu_seqlens, slot_ids, B, min_len, heads, dim, vd, ws, 0, 0, 0, 0};
     return dim <= 64 ? run<64, true>(o_out, state, slot_stride, n_slots, a, n_chunks, ws_chunks, err, stream)
                      : run<128, true>(o_out, state, slot_stride, n_slots, a, n_chunks, ws_chunks, err, stream);
 }
@@ -485,7 +693,7 @@ CELLM_API int cellm_hgrn2_chunks(float* o_out, float* state, long long slot_stri
                                  int col_f, int col_v, const int* cu_seqlens, const int* slot_ids, int B, int n_chunks, int ws_chunks,
                                  int min_len, int heads, int dim, int vd, float* ws, int* err, cudaStream_t stream) {
     if (!fits(B, heads, 1, dim, vd, n_chunks, ws_chunks, ws) || min_len < 1) return CELLM_ERR_SIZE;
-    ChunkArgs a{proj + col_q, nullptr, proj + col_f, proj + col_v, nullptr, ld, 0, ld, ld, 1, cu_seqlens, slot_ids, B, min_len, heads, dim, vd, ws, 0, 0, 0};
+    ChunkArgs a{proj + col_q, nullptr, proj + col_f, proj + col_v, nullptr, ld, 0, ld, ld, 1, cu_seqlens, slot_ids, B, min_len, heads, dim, vd, ws, 0, 0, 0, 0};
     return dim <= 64 ? run<64, false>(o_out, state, slot_stride, n_slots, a, n_chunks, ws_chunks, err, stream)
                      : run<128, false>(o_out, state, slot_stride, n_slots, a, n_chunks, ws_chunks, err, stream);
 }

@@ -567,6 +567,30 @@ def test_chunks_go_through_a_small_workspace_in_runs(monkeypatch, kind, held):
     assert int(ctx.err.item()) == 0
 
 
+@pytest.mark.parametrize("kind", ["delta", "hgrn2"])
+@pytest.mark.parametrize("requests,dim,vd", [(3, 128, 128), (9, 128, 128), (40, 64, 128)])
+def test_chunks_with_several_blocks_an_sm(kind, requests, dim, vd):
+    """1, 2 and 8 blocks of the walk an SM, with the stages that are left each: the walk's results, for every request (the bound is
+    that of the recurrences against 64 bits)."""
+    from cellm_b200 import ops
+    heads, g = 4, torch.Generator().manual_seed(requests)
+    lens = [96 + 7 * (i % 5) for i in range(requests)]
+    T, ctx, got = sum(lens), step_ctx(lens, [0] * requests, list(range(requests))), []
+    unit = lambda: torch.nn.functional.normalize(torch.randn(T, heads, dim, generator=g), dim=-1).reshape(T, -1)
+    qk, v = torch.cat([unit(), unit()], 1).to(DEV).contiguous(), torch.randn(T, heads * vd, generator=g).to(DEV)
+    beta, decay = torch.rand(T, heads, generator=g).to(DEV), (0.5 + 0.5 * torch.rand(T, heads * dim, generator=g)).to(DEV)
+    proj, zero, S0 = torch.randn(T, heads * (2 * dim + vd), generator=g).to(DEV), torch.zeros(heads * dim, device=DEV), torch.randn(requests, heads, dim, vd, generator=g)
+    for chunked in (False, True):
+        state = S0.to(DEV).clone()
+        if kind == "delta":
+            got.append((ops.delta_scan(qk, v, beta, decay, state, ctx, heads, heads, dim, vd, chunked=chunked), state))
+        else:
+            got.append((ops.hgrn2_scan(proj.clone(), 0, heads * dim, 2 * heads * dim, zero, zero, state, ctx, heads, dim, vd, chunked=chunked), state))
+    assert int(ctx.err.item()) == 0
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, rtol=2e-5, atol=2e-5 * float(b.abs().max()))
+
+
 def test_chunks_behind_more_requests_than_a_grids_second_dimension():
     """70,000 requests of one token and a long portion behind them: the portion in chunks, the others token by token."""
     from cellm_b200 import ops
