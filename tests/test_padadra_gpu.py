@@ -698,6 +698,45 @@ def test_attention_preparation_in_fours_and_one_by_one(taps, bias):
     assert int(ctx.err.item()) == 0
 
 
+@pytest.mark.parametrize("taps,bias,norms,interleaved,rot,dtype", [(4, True, True, True, 64, "bfloat16"), (3, False, False, False, 32, "float32"),
+                                                                   (2, True, True, False, 64, "float32"), (4, False, False, True, 16, "bfloat16")])
+def test_attention_preparation_of_many_tokens(taps, bias, norms, interleaved, rot, dtype):
+    """512 tokens and more go in runs of four, which end inside portions, at their ends and behind several; fewer a block a token. The
+    same values: bit for bit without norms; with them the squares are summed in another order (two orders of at most 384 terms
+    differ by less than 384 * 2^-24 of a sum, its root by half that), which may move a bfloat16 by its last place."""
+    from cellm_b200 import ops
+    from cellm_b200.parts import CacheBinding
+    from cellm_b200.parts.rope import split_inv_freq
+    nh, nkv, hd, dt = 6, 2, 64, getattr(torch, dtype)
+    lens = [37, 1, 2, 20, 400, 3, 130, 1, 1, 6]
+    g = torch.Generator().manual_seed(taps)
+    T, C = sum(lens), (nh + 2 * nkv) * hd
+    rnd = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    proj, b, w, state = rnd(T, C + 4), rnd(C) if bias else None, rnd(C, taps), rnd(len(lens), taps - 1, C)
+    nw = (rnd(nh * hd), rnd(nkv * hd)) if norms else (None, None)
+    mult, freq, vfreq = rnd(nh), split_inv_freq(1e4, rot).to(DEV), split_inv_freq(1e3, hd).to(DEV) if bias else None
+    pages = -(-max(lens) // 8)
+    table = torch.arange(pages * len(lens), dtype=torch.int32, device=DEV).reshape(len(lens), pages)
+    pool = lambda: torch.zeros(pages * len(lens), nkv, 8, hd, dtype=dt, device=DEV)
+    def run(rows, ctx, cache):
+        q = ops.sink_attn_prep(rows, 4, b, w, taps, state, *nw, 1e-5, freq, rot, vfreq, interleaved, ctx, cache, nh, nkv, hd, hd, dt, mult)
+        assert int(ctx.err.item()) == 0
+        return q
+    whole = CacheBinding(k=pool(), v=pool(), block_table=table, page_size=8, num_pages=pages * len(lens))
+    q = run(proj, step_ctx(lens, [0] * len(lens), list(range(len(lens)))), whole)
+    alone, got, at = CacheBinding(k=pool(), v=pool(), block_table=table, page_size=8, num_pages=pages * len(lens)), [], 0
+    for i, n in enumerate(lens):
+        alone.block_table = table[i:i + 1]
+        got.append(run(proj[at:at + n], step_ctx([n], [0], [i]), alone))
+        at += n
+    rel = (2.0 ** -7 if dtype == "bfloat16" else 2.0 ** -14) if norms else 0.0
+    for x, y in ((q, torch.cat(got)), (whole.k, alone.k), (whole.v, alone.v)):
+        if norms:
+            torch.testing.assert_close(x, y, rtol=rel, atol=rel)
+        else:
+            assert torch.equal(x, y)
+
+
 def test_pair_hash_embedding_and_the_first_token():
     from cellm_b200 import ops
     V, H, buckets, mp, mc = 50, 24, 13, 31, 5
