@@ -737,6 +737,44 @@ def test_attention_preparation_of_many_tokens(taps, bias, norms, interleaved, ro
             assert torch.equal(x, y)
 
 
+@pytest.mark.parametrize("T,heads,vd,lead,act", [(5, 3, 64, 0, "bfloat16"), (1, 1, 128, 0, "float32"), (9, 2, 128, 4, "bfloat16"), (3, 5, 64, 3, "float32"),
+                                                 (4, 3, 40, 0, "bfloat16")])
+def test_head_norms_by_fours_and_one_by_one(T, heads, vd, lead, act):
+    """Rows of 64 and 128 values on 16-byte borders, the last block part filled, gates whose rows lie apart; others value by value: 64
+    bits rounded once, and for 32-bit results the sum of squares' and the exponential's roundings."""
+    from cellm_b200 import ops
+    g = torch.Generator().manual_seed(T + vd)
+    o, gate, w = torch.randn(T, heads * vd, generator=g), torch.randn(T, heads * vd + 2 * lead, generator=g), torch.randn(heads * vd, generator=g)
+    dt = getattr(torch, act)
+    tol = dict(rtol=2.0 ** -8, atol=1e-6) if act == "bfloat16" else dict(rtol=1e-5, atol=1e-6)
+    x = o.double().view(T, heads, vd)
+    unit = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5)
+    z = gate[:, lead:lead + heads * vd].double().view(T, heads, vd)
+    at = gate.to(DEV)[:, lead:lead + heads * vd]
+    for weight in (w, w[:vd]):
+        want = unit * weight.double().view(-1, vd)
+        got = ops.head_norm_gate(o.to(DEV), weight.to(DEV).contiguous(), at, heads, vd, 1e-5, dt)
+        torch.testing.assert_close(got.cpu().double().view(T, heads, vd), want * torch.sigmoid(z), **tol)
+        got = ops.head_norm_gate(o.to(DEV), weight.to(DEV).contiguous(), None, heads, vd, 1e-5, dt)
+        torch.testing.assert_close(got.cpu().double().view(T, heads, vd), want, **tol)
+
+
+@pytest.mark.parametrize("T,heads,dim", [(1, 1, 4), (3, 5, 100), (7, 12, 64)])
+def test_hgrn2_gates_by_fours_and_one_by_one(T, heads, dim):
+    from cellm_b200.ops._lib import check, fn, ptr, stream_of
+    n, g = heads * dim, torch.Generator().manual_seed(T * dim)
+    x, b, low = torch.randn(T, 2 * n, generator=g).to(DEV), torch.randn(n, generator=g).to(DEV), torch.rand(n, generator=g).to(DEV)
+    got = []
+    for pad in (0, 1):
+        proj = torch.cat([torch.zeros(T, pad, device=DEV), x, torch.zeros(T, 4 - pad, device=DEV)], 1).contiguous()
+        check(fn("kernels_common", "cellm_hgrn2_gates")(ptr(proj), proj.stride(0), pad, pad + n, ptr(b), ptr(low), T, heads, dim, stream_of(proj)), "gates")
+        got.append(proj[:, pad:pad + 2 * n])
+    assert torch.equal(*got)
+    q, f = x[:, :n].double(), x[:, n:].double()
+    torch.testing.assert_close(got[0].double(), torch.cat([q * torch.sigmoid(q), low.double() + (1 - low.double()) * torch.sigmoid(f + b.double())], 1),
+                               rtol=1e-6, atol=1e-7)
+
+
 def test_pair_hash_embedding_and_the_first_token():
     from cellm_b200 import ops
     V, H, buckets, mp, mc = 50, 24, 13, 31, 5
