@@ -12,6 +12,9 @@
 // 32-bit operands: the runs of a tile are summed by different groups of threads at once (gemm_runs_kernel); short products of
 // many tiles, rows off the 16-byte border and bfloat16 operands (products the tensor-core kernels do not take) by one group, run
 // after run. Both give the same sums.
+#include <algorithm>
+#include <cmath>
+
 #include "common.cuh"
 
 #define GP_BM 64
@@ -20,13 +23,14 @@
 #define GP_RUN 256    // products summed in order before their sum joins the total; a multiple of GP_BK
 
 // ------------------------------------------------------------------------------------------------ 32-bit operands
-// A tile of 8 TM x 8 TN sums by groups of 64 threads (8 x 8, a thread TM x TN sums): every group forms whole runs of GP_RUN
+// A tile of LY TM x 8 TN sums by groups of 8 LY threads (64, or a warp; a thread TM x TN sums): every group forms whole runs of GP_RUN
 // products, as many runs at once as there are groups, and their sums are added in the runs' order from shared memory. What runs
 // of one tile share is only that addition, so a block is 2 to 16 warps of independent work on a tile whatever K is, and the
 // order of the sums is the one above. Operands go to shared memory as they lie (rows of GP_BK values, by asynchronous
 // copies, two stages a group) and are read four values of k at a time: (TM + TN) 16-byte reads for 4 TM TN multiply-adds, so
 // 64 x 64 is bound by the multiply-adds and the smaller tiles by shared memory; those are for products whose 64 x 64 tiles
-// leave SMs idle. 2,048 x 2,048 x 2,048: 31 TFLOP/s; 213 x 2,560 x 1,536: 25 (64 x 64 tiles of 256 threads, run after run: about 7).
+// leave SMs idle. Single warps have no barrier and a quarter of a 64-thread tile's rows: blocks of few registers that share an SM and
+// fill it evenly. 2,048 x 2,048 x 2,048: 37 TFLOP/s; 261 x 2,560 x 1,536: 27 (in tiles of 32 x 64 by 64 threads 20).
 #define GP_PITCH (GP_BK + 4)
 
 __device__ __forceinline__ void gp_copy(float* dst, const float* src, int bytes, bool in) {
@@ -36,31 +40,50 @@ __device__ __forceinline__ void gp_copy(float* dst, const float* src, int bytes,
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
 
-template <int TM, int TN> struct RunTile {
-    static constexpr int BM = 8 * TM, BN = 8 * TN, STAGE = (BM + BN) * GP_PITCH;      // floats a stage
+template <int TM, int TN, int LY> struct RunTile {
+    static constexpr int BM = LY * TM, BN = 8 * TN, STAGE = (BM + BN) * GP_PITCH;      // floats a stage
     static constexpr size_t smem(int groups) { return (size_t)(groups * 2 * STAGE + BM * BN) * sizeof(float); }
 };
 
-template <int TM, int TN>
-__global__ void __launch_bounds__(512)
+template <int TM, int TN, int LY>
+__global__ void __launch_bounds__(LY * 64)
 gemm_runs_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K,
                  long long lda, long long ldw, long long ldc, int vec) {
-    using T = RunTile<TM, TN>;
-    constexpr int BM = T::BM, BN = T::BN;
+    using T = RunTile<TM, TN, LY>;
+    constexpr int BM = T::BM, BN = T::BN, GT = 8 * LY;
     static_assert(BM * BN <= 2 * T::STAGE, "a group's sums take the place of its stages");
     extern __shared__ __align__(16) float gp_smem[];
-    const int groups = blockDim.x / 64, g = threadIdx.x / 64, tid = threadIdx.x & 63, tx = tid & 7, ty = tid >> 3;
+    const int groups = blockDim.x / GT, g = threadIdx.x / GT, tid = threadIdx.x % GT;
+    // a 16-byte read of shared memory costs half where neighbouring lanes read the same: one operand's in either form
+    const int tx = LY == 4 ? (tid >> 1) & 7 : tid & 7, ty = LY == 4 ? (tid & 1) | (tid >> 4) << 1 : tid >> 3;
     float* mine = gp_smem + g * 2 * T::STAGE;
     float* total = gp_smem + groups * 2 * T::STAGE;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN, n_runs = (K + GP_RUN - 1) / GP_RUN;
     pdl_trigger();
     pdl_wait();
     for (int i = threadIdx.x; i < BM * BN; i += blockDim.x) total[i] = 0.f;
-    auto group_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory"); };
+    auto group_sync = [&]() { if constexpr (GT == 32) __syncwarp(); else asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(GT) : "memory"); };
     auto issue = [&](int stage, int k0) {
         float* dst = mine + stage * T::STAGE;
-        const int shift = vec ? 2 : 4, width = vec ? 4 : 1;          // copies of a row: 4 of four values, or 16 of one
-        for (int i = tid; i < (BM + BN) << shift; i += 64) {
+        if (vec) {          // a thread's copies: the same four values of k in rows GT / 4 apart
+            const int kk = (tid & 3) * 4, r0 = tid >> 2, gk = k0 + kk;
+            const float *a = A + (size_t)(m0 + r0) * lda + gk, *w = W + (size_t)(n0 + r0) * ldw + gk;
+            float* to = dst + r0 * GP_PITCH + kk;
+#pragma unroll
+            for (int i = 0; i < BM; i += GT / 4) {
+                if (GT / 4 > BM && r0 >= BM) break;
+                const bool in = m0 + r0 + i < M && gk < K;
+                gp_copy(to + i * GP_PITCH, in ? a + (size_t)i * lda : A, 16, in);
+            }
+#pragma unroll
+            for (int i = 0; i < BN; i += GT / 4) {
+                const bool in = n0 + r0 + i < N && gk < K;
+                gp_copy(to + (BM + i) * GP_PITCH, in ? w + (size_t)i * ldw : W, 16, in);
+            }
+            return;
+        }
+        constexpr int shift = 4, width = 1;          // a row's copies: 16 of one value
+        for (int i = tid; i < (BM + BN) << shift; i += GT) {
             const int r = i >> shift, kk = (i & ((1 << shift) - 1)) * width, gk = k0 + kk;
             const bool w_row = r >= BM;
             const int row = w_row ? n0 + r - BM : m0 + r;
@@ -94,7 +117,7 @@ gemm_runs_kernel(float* __restrict__ C, const float* __restrict__ A, const float
                     for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const float4*>(ws + j * 8 * GP_PITCH + kk);
 #pragma unroll
                     for (int i = 0; i < TM; ++i) {
-                        const float4 a = *reinterpret_cast<const float4*>(as + i * 8 * GP_PITCH + kk);
+                        const float4 a = *reinterpret_cast<const float4*>(as + i * LY * GP_PITCH + kk);
 #pragma unroll
                         for (int j = 0; j < TN; ++j) {
                             acc[i][j] = fmaf(a.x, w[j].x, acc[i][j]);
@@ -110,7 +133,7 @@ gemm_runs_kernel(float* __restrict__ C, const float* __restrict__ A, const float
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) mine[(ty + 8 * i) * BN + tx + 8 * j] = acc[i][j];
+                for (int j = 0; j < TN; ++j) mine[(ty + LY * i) * BN + tx + 8 * j] = acc[i][j];
         }
         __syncthreads();
         for (int i = threadIdx.x; i < BM * BN; i += blockDim.x) {
@@ -126,15 +149,15 @@ gemm_runs_kernel(float* __restrict__ C, const float* __restrict__ A, const float
     }
 }
 
-template <int TM, int TN>
+template <int TM, int TN, int LY>
 static int run_tiles(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldw, long long ldc,
                      int groups, int vec, cudaStream_t stream) {
-    using T = RunTile<TM, TN>;
+    using T = RunTile<TM, TN, LY>;
     const dim3 grid((unsigned)((N + T::BN - 1) / T::BN), (unsigned)((M + T::BM - 1) / T::BM));
     if (grid.y > 65535) return CELLM_ERR_SIZE;
-    cudaError_t e = cudaFuncSetAttribute(gemm_runs_kernel<TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem(8));
+    cudaError_t e = cudaFuncSetAttribute(gemm_runs_kernel<TM, TN, LY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem(8));
     if (e != cudaSuccess) return (int)e;
-    CELLM_RUN((gemm_runs_kernel<TM, TN>), grid, groups * 64, T::smem(groups), stream, C, A, W, M, N, K, lda, ldw, ldc, vec);
+    CELLM_RUN((gemm_runs_kernel<TM, TN, LY>), grid, groups * 8 * LY, T::smem(groups), stream, C, A, W, M, N, K, lda, ldw, ldc, vec);
     return CELLM_OK;
 }
 
@@ -215,22 +238,34 @@ CELLM_API int cellm_gemm_plain(void* C, const void* A, const void* W, int M, int
     if (in_dtype == CELLM_F32 && out_dtype == CELLM_F32 && ((vec && K >= 2 * GP_RUN) || tiles64 <= few)) {
         const int n_runs = (K + GP_RUN - 1) / GP_RUN, rounds = (n_runs + 7) / 8, groups = (n_runs + rounds - 1) / rounds;
         // The tile whose waves over the SMs take least. Microseconds of K = 1,536 measured for one tile an SM and for each
-        // wave of several (the smaller tiles share an SM then): with 213 x 2,560 sums 64 x 64 takes 125 us, 32 x 64 68, 32 x 32
-        // 87, 16 x 32 96; with 16 x 1,536 they take 63, 34, 22 and 18; with 2,048 x 2,048 (K 2,048) 545, 577, 723 and 836.
-        static const struct { int bm, bn; double alone, wave; } tile[4] = {{64, 64, 62.8, 60.}, {32, 64, 34.4, 33.}, {32, 32, 22.4, 21.}, {16, 32, 18., 12.}};
+        // wave of several: whole waves where a block fills an SM; the groups of one warp share it, so that their waves melt together (from
+        // four groups on, below which they are too few warps). 213 x 2,560 sums take 108 us in tiles of 64 x 64, 63 of 32 x 64, 77 of
+        // 32 x 32, 85 of 16 x 32, 64 and 63 of those by single warps; 261 x 2,560 111, 91, 95, 105, 92, 77; 16 x 1,536 55, 31, 20, 14,
+        // 21, 16; 2,048 x 2,048 (K 2,048) 468, 540, 657, 859, 519, 560.
+        struct Tile { int bm, bn; double alone, wave, first; };
+        static const Tile long_k[6] = {
+            {64, 64, 58., 52., 0.}, {32, 64, 32., 30., 0.}, {32, 32, 20.5, 19.3, 0.}, {16, 32, 14.3, 11.5, 0.}, {32, 32, 25., 14.3, 10.},
+            {16, 32, 16.5, 7.65, 5.}};
+        // (fewer groups: their own measured costs)
+        static const Tile short_k[4] = {{64, 64, 62.8, 60., 0.}, {32, 64, 34.4, 33., 0.}, {32, 32, 22.4, 21., 0.}, {16, 32, 18., 12., 0.}};
         int best = 0;
         double least = 0;
-        for (int i = 0; i < 4; ++i) {
-            if (i > 0 && (M + tile[i].bm - 1) / tile[i].bm > 65535) break;      // as many rows as 64 x 64 tiles take, whatever their number
-            const long long tiles = (long long)((M + tile[i].bm - 1) / tile[i].bm) * ((N + tile[i].bn - 1) / tile[i].bn), waves = (tiles + 147) / 148;
-            const double cost = waves == 1 ? tile[i].alone : (double)waves * tile[i].wave;
+        const bool many = groups >= 4 && vec;
+        for (int i = 0; i < (many ? 6 : 4); ++i) {
+            const Tile t = many ? long_k[i] : short_k[i];
+            if (i > 0 && (M + t.bm - 1) / t.bm > 65535) continue;      // as many rows as 64 x 64 tiles take, whatever their number
+            const double waves = (double)((long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn)) / 148.;
+            double cost = waves <= 1. ? t.alone : i >= 4 ? std::max(33., t.first + waves * t.wave) : ceil(waves) * t.wave;
+            if (many && i == 3 && waves <= 1. && waves * 148. > 64.) cost = 19.6;           // (more than 64 of these wait for memory together)
             if (i == 0 || cost < least) best = i, least = cost;
         }
-#define RUNS(TM, TN) return run_tiles<TM, TN>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, groups, vec, stream)
-        if (best == 0) RUNS(8, 8);
-        if (best == 1) RUNS(4, 8);
-        if (best == 2) RUNS(4, 4);
-        RUNS(2, 4);
+#define RUNS(TM, TN, LY) return run_tiles<TM, TN, LY>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, groups, vec, stream)
+        if (best == 0) RUNS(8, 8, 8);
+        if (best == 1) RUNS(4, 8, 8);
+        if (best == 2) RUNS(4, 4, 8);
+        if (best == 3) RUNS(2, 4, 8);
+        if (best == 4) RUNS(8, 4, 4);
+        RUNS(4, 4, 4);
 #undef RUNS
     }
     const dim3 grid((unsigned)((N + GP_BN - 1) / GP_BN), (unsigned)((M + GP_BM - 1) / GP_BM));

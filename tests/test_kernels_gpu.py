@@ -783,6 +783,18 @@ def test_gemm_plain_in_32_bits_either_way(K):
         assert torch.equal(ops.gemm_plain(a[rows].contiguous(), w[cols].contiguous(), torch.float32), out[rows, cols])
 
 
+@pytest.mark.parametrize("M,N,K", [(261, 1500, 1100), (130, 2570, 1536), (410, 6100, 1028)])
+def test_gemm_plain_in_32_bits_by_single_warps(M, N, K):
+    """Sizes that tiles of 16 x 32 and of 32 x 32 by single warps take, with part-filled last tiles and runs: a corner of the product,
+    which other tiles take, is the same bits."""
+    from cellm_b200 import ops
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    out = ops.gemm_plain(a, w, torch.float32)
+    close(out, a.double() @ w.double().T, torch.float32)
+    for rows, cols in ((slice(M - 3, M), slice(N - 40, N)), (slice(0, 16), slice(0, 64)), (slice(M // 2, M // 2 + 70), slice(N // 2, N // 2 + 70))):
+        assert torch.equal(ops.gemm_plain(a[rows].contiguous(), w[cols].contiguous(), torch.float32), out[rows, cols])
+
+
 @pytest.mark.parametrize("M,N,K", [(65536 * 16 + 5, 8, 512), (65536 * 32 + 5, 40, 4)])
 def test_gemm_plain_in_32_bits_of_a_million_rows(M, N, K):
     """More rows than a grid of tiles of 16 (or 32) of them holds, and so few columns that those would be chosen."""
