@@ -16,6 +16,7 @@
 #include "common.cuh"
 
 #define SHORT_CONV_MAX_TAPS 16
+#define SHORT_CONV_RUN 4
 
 template <typename TA, typename TW>
 __global__ void short_conv_fwd_kernel(TA* __restrict__ y, const TA* __restrict__ bcx,
@@ -116,9 +117,11 @@ __global__ void short_conv_fwd_vec8_kernel(__nv_bfloat16* __restrict__ y, const 
 }
 
 // The same again for long portions (TAPS = 2, 3 or 4): a thread takes eight neighbouring channels
-// of a run of RUN tokens and keeps the last TAPS - 1 products B.x in registers as it walks the run, so
-// every row of bcx is read once. A run may cross from one request into the next: at a request's first
-// token the window is taken from that request's state.
+// of a run of RUN tokens and keeps the products B.x in registers, so every row of bcx is read once a run. The rows of a whole run
+// of one request are all under way before the first is needed; a run may also cross from one request into the next: it is walked, and
+// at a request's first token the window is taken from that request's state. Bound by latency up to some 1,000 tokens, then by
+// the rows: with the state's update 351 tokens of 2,048 channels take 4.9 us, 2,048 tokens 7.7 (walked in runs of eight, the
+// taps read one by one: 7.0 and 9.5).
 template <typename TW, int TAPS, int RUN>
 __global__ void short_conv_fwd_run_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ bcx,
                                           const TW* __restrict__ w, const TW* __restrict__ bias,
@@ -127,28 +130,105 @@ __global__ void short_conv_fwd_run_kernel(__nv_bfloat16* __restrict__ y, const _
                                           const int* __restrict__ cu_seqlens, int T, int H, int n_slots,
                                           int* __restrict__ err) {
     pdl_trigger();
-    pdl_wait();
     const int t0 = blockIdx.x * RUN;
     const int c0 = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
     if (c0 >= H || t0 >= T) return;
-    auto load8 = [](const __nv_bfloat16* p, float* out) {
-        const uint4 v = *reinterpret_cast<const uint4*>(p);
+    auto floats = [](uint4 v, float* out) {
         const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
         for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(h[j]); out[2 * j] = f.x; out[2 * j + 1] = f.y; }
     };
+    auto raw8 = [](const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); };
+    auto load8 = [&](const __nv_bfloat16* p, float* out) { floats(raw8(p), out); };
+    // weights and the step's index arrays are the work of no kernel of this step
     float wt[TAPS][8], bs[8];
+    if constexpr (sizeof(TW) == 2) {
+        if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {          // eight channels' taps: 16 TAPS bytes in a row
+            float all[8 * TAPS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+            for (int k = 0; k < TAPS; ++k) load8(reinterpret_cast<const __nv_bfloat16*>(w) + (size_t)c0 * TAPS + 8 * k, all + 8 * k);
 #pragma unroll
-        for (int k = 0; k < TAPS; ++k) wt[k][j] = to_float(w[(size_t)(c0 + j) * TAPS + k]);
-        bs[j] = bias ? to_float(bias[c0 + j]) : 0.f;
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int k = 0; k < TAPS; ++k) wt[k][j] = all[j * TAPS + k];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int k = 0; k < TAPS; ++k) wt[k][j] = to_float(w[(size_t)(c0 + j) * TAPS + k]);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int k = 0; k < TAPS; ++k) wt[k][j] = to_float(w[(size_t)(c0 + j) * TAPS + k]);
     }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) bs[j] = bias ? to_float(bias[c0 + j]) : 0.f;
+    auto finish = [&](int t, const float (&x)[8]) {
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const __nv_bfloat162 pk = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
+            o[j] = *reinterpret_cast<const uint32_t*>(&pk);
+        }
+        *reinterpret_cast<uint4*>(y + (size_t)t * H + c0) = make_uint4(o[0], o[1], o[2], o[3]);
+    };
+    const int first = seq_of_token[t0], last = t0 + RUN <= T ? seq_of_token[t0 + RUN - 1] : -1;
+    const int first_start = cu_seqlens[first], first_slot = slot_ids[first];
+    if (first == last && first_slot >= 0 && first_slot < n_slots) {         // a whole run of one request: all its rows are under way at once
+        const float* hist = state + (long long)first_slot * slot_stride;
+        float v[TAPS - 1 + RUN][8];          // B.x
+        uint4 rb[TAPS - 1 + RUN], rx[TAPS - 1 + RUN], rc[RUN];
+        pdl_wait();
+#pragma unroll
+        for (int k = 0; k < TAPS - 1 + RUN; ++k) {
+            const int t = t0 - (TAPS - 1) + k;
+            if (k < TAPS - 1 && t < first_start) {          // a row of the state: 32-bit values, as they lie
+                rb[k] = *reinterpret_cast<const uint4*>(hist + (size_t)(TAPS - 1 + t - first_start) * H + c0);
+                rx[k] = *reinterpret_cast<const uint4*>(hist + (size_t)(TAPS - 1 + t - first_start) * H + c0 + 4);
+            } else {
+                rb[k] = raw8(bcx + (size_t)t * 3 * H + c0);
+                rx[k] = raw8(bcx + (size_t)t * 3 * H + 2 * H + c0);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < RUN; ++i) rc[i] = raw8(bcx + (size_t)(t0 + i) * 3 * H + H + c0);
+#pragma unroll
+        for (int k = 0; k < TAPS - 1 + RUN; ++k) {
+            if (k < TAPS - 1 && t0 - (TAPS - 1) + k < first_start) {
+                const float4 a = *reinterpret_cast<const float4*>(&rb[k]), d = *reinterpret_cast<const float4*>(&rx[k]);
+                v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
+                v[k][4] = d.x; v[k][5] = d.y; v[k][6] = d.z; v[k][7] = d.w;
+            } else {
+                float bb[8], xx[8];
+                floats(rb[k], bb);
+                floats(rx[k], xx);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[k][j] = bb[j] * xx[j];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < RUN; ++i) {
+            float cc[8];
+            floats(rc[i], cc);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                float acc = 0.f;
+#pragma unroll
+                for (int k = 0; k < TAPS; ++k) acc += v[i + k][j] * wt[k][j];      // oldest tap first, as the other kernels add
+                cc[j] = cc[j] * (acc + bs[j]);
+            }
+            finish(t0 + i, cc);
+        }
+        return;
+    }
+    pdl_wait();
     float win[TAPS - 1][8];          // B.x of the TAPS - 1 tokens before the current one, oldest first
     int b = -1, b_start = 0;
     const float* st = nullptr;
     bool bad = false;
-#pragma unroll 4
+#pragma unroll 1
     for (int t = t0; t < min(T, t0 + RUN); ++t) {
         const int bt = seq_of_token[t];
         if (bt != b) {                // the run's first token, or the first token of the next request
@@ -185,7 +265,6 @@ __global__ void short_conv_fwd_run_kernel(__nv_bfloat16* __restrict__ y, const _
         load8(row + c0, bb);
         load8(row + H + c0, cc);
         load8(row + 2 * H + c0, xx);
-        uint32_t o[4];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             cur[j] = bb[j] * xx[j];
@@ -195,12 +274,7 @@ __global__ void short_conv_fwd_run_kernel(__nv_bfloat16* __restrict__ y, const _
             acc += cur[j] * wt[TAPS - 1][j];
             cc[j] = cc[j] * (acc + bs[j]);
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            __nv_bfloat162 pk = __floats2bfloat162_rn(cc[2 * j], cc[2 * j + 1]);
-            o[j] = *reinterpret_cast<uint32_t*>(&pk);
-        }
-        if (!bad) *reinterpret_cast<uint4*>(y + (size_t)t * H + c0) = make_uint4(o[0], o[1], o[2], o[3]);
+        if (!bad) finish(t, cc);
 #pragma unroll
         for (int k = 0; k + 1 < TAPS - 1; ++k)
 #pragma unroll
@@ -304,11 +378,12 @@ CELLM_API int cellm_short_conv(void* y, const void* bcx, const void* w, const vo
             break;                                                                                  \
         }                                                                                           \
         if (vec8 && T >= 256 && taps >= 2 && taps <= 4) {                                          \
-            /* long portions: runs of eight tokens per thread, each row of bcx read once */        \
-            dim3 grid_r((unsigned)((T + 7) / 8), (unsigned)((H / 8 + threads - 1) / threads));      \
-            if (taps == 2) CELLM_RUN((short_conv_fwd_run_kernel<TW, 2, 8>), grid_r, threads, 0, stream, (__nv_bfloat16*)y, (const __nv_bfloat16*)bcx, (const TW*)w, (const TW*)bias, (const float*)state, slot_stride, slot_ids, seq_of_token, cu_seqlens, T, H, n_slots, err); \
-            else if (taps == 3) CELLM_RUN((short_conv_fwd_run_kernel<TW, 3, 8>), grid_r, threads, 0, stream, (__nv_bfloat16*)y, (const __nv_bfloat16*)bcx, (const TW*)w, (const TW*)bias, (const float*)state, slot_stride, slot_ids, seq_of_token, cu_seqlens, T, H, n_slots, err); \
-            else CELLM_RUN((short_conv_fwd_run_kernel<TW, 4, 8>), grid_r, threads, 0, stream, (__nv_bfloat16*)y, (const __nv_bfloat16*)bcx, (const TW*)w, (const TW*)bias, (const float*)state, slot_stride, slot_ids, seq_of_token, cu_seqlens, T, H, n_slots, err); \
+            /* long portions: runs of four tokens per thread, each row of bcx read once in a run */              \
+            const int rt = H / 8 >= 512 ? 128 : 64;                                                 \
+            dim3 grid_r((unsigned)((T + SHORT_CONV_RUN - 1) / SHORT_CONV_RUN), (unsigned)((H / 8 + rt - 1) / rt)); \
+            if (taps == 2) CELLM_RUN((short_conv_fwd_run_kernel<TW, 2, SHORT_CONV_RUN>), grid_r, rt, 0, stream, (__nv_bfloat16*)y, (const __nv_bfloat16*)bcx, (const TW*)w, (const TW*)bias, (const float*)state, slot_stride, slot_ids, seq_of_token, cu_seqlens, T, H, n_slots, err); \
+            else if (taps == 3) CELLM_RUN((short_conv_fwd_run_kernel<TW, 3, SHORT_CONV_RUN>), grid_r, rt, 0, stream, (__nv_bfloat16*)y, (const __nv_bfloat16*)bcx, (const TW*)w, (const TW*)bias, (const float*)state, slot_stride, slot_ids, seq_of_token, cu_seqlens, T, H, n_slots, err); \
+            else CELLM_RUN((short_conv_fwd_run_kernel<TW, 4, SHORT_CONV_RUN>), grid_r, rt, 0, stream, (__nv_bfloat16*)y, (const __nv_bfloat16*)bcx, (const TW*)w, (const TW*)bias, (const float*)state, slot_stride, slot_ids, seq_of_token, cu_seqlens, T, H, n_slots, err); \
         } else if (vec8) {                                                                          \
             CELLM_RUN(short_conv_fwd_vec8_kernel<TW>, grid_v, threads, 0, stream, (__nv_bfloat16*)y,     \
                       (const __nv_bfloat16*)bcx, (const TW*)w, (const TW*)bias, (const float*)state, slot_stride, \

@@ -122,7 +122,7 @@ def test_short_conv_portions_carry_the_state(dtype, taps, bias, walk):
 
 @pytest.mark.parametrize("taps,bias", [(2, False), (3, True), (4, False), (5, True)])
 def test_short_conv_long_portions_of_several_requests(taps, bias):
-    """Portions of hundreds of bfloat16 tokens (the kernel that walks runs of eight
+    """Portions of hundreds of bfloat16 tokens (the kernel that takes runs of four
     tokens per thread): three requests whose portions start and end off the runs'
     edges, one of them continuing from a state, and a second step that continues all."""
     from cellm_b200 import ops
