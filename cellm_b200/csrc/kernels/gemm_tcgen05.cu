@@ -594,40 +594,65 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
 }
 
 // Sum of the K-split pieces of a product with plain tiles, ws[split][M][N], in the order of the splits; one
-// thread for four neighbouring outputs. EPI as in the product's kernel (1: gate and up blocks of 64 columns).
+// thread for four neighbouring outputs. EPI as in the product's kernel (1: gate and up blocks of 64 columns). Bound by the latency of
+// its loads: all pieces of an output are under way at once and four outputs are stored together.
 template <int EPI, typename TO>
 __global__ void splitk_sum_kernel(const float* __restrict__ ws, TO* __restrict__ C, int M, int N, long long ldc, int splits,
                                   const GateEpi gate_epi) {
     pdl_trigger();
     pdl_wait();
     const int NO = EPI == 1 ? N / 2 : N;                       // output columns
-    const long long groups = (long long)M * ((NO + 3) / 4);
-    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= groups) return;
-    const int m = (int)(g / ((NO + 3) / 4)), o0 = (int)(g % ((NO + 3) / 4)) * 4;
+    const unsigned per_row = (unsigned)(NO + 3) / 4;
+    const unsigned long long g = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= (unsigned long long)M * per_row) return;
+    const int m = (g >> 32) == 0 ? (int)((unsigned)g / per_row) : (int)(g / per_row), o0 = (int)(g - (unsigned long long)m * per_row) * 4;
     const size_t slice = (size_t)M * (size_t)N;
     float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
     // input column of output column o: itself, or the gate of block o / 64 (its up lies 64 further on)
     const int c0 = EPI == 1 ? (o0 / 64) * 128 + (o0 % 64) : o0;
     const bool vec = (N & 3) == 0 && o0 + 3 < NO;              // four columns never straddle a block of 64
-    for (int sp = 0; sp < splits; ++sp) {
-        const float* src = ws + (size_t)sp * slice + (size_t)m * N + c0;
-        if (vec) {
-            const float4 v = *reinterpret_cast<const float4*>(src);
-            a[0] += v.x; a[1] += v.y; a[2] += v.z; a[3] += v.w;
-            if (EPI == 1) {
-                const float4 u = *reinterpret_cast<const float4*>(src + 64);
-                b[0] += u.x; b[1] += u.y; b[2] += u.z; b[3] += u.w;
+    if (vec) {
+        constexpr int AHEAD = EPI == 1 ? 4 : 8;                // pieces under way at once
+        const float* src = ws + (size_t)m * N + c0;
+        for (int sp = 0; sp < splits; sp += AHEAD) {
+            float4 v[AHEAD], u[AHEAD];
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) {
+                if (sp + i >= splits) break;
+                v[i] = *reinterpret_cast<const float4*>(src + (size_t)(sp + i) * slice);
+                if (EPI == 1) u[i] = *reinterpret_cast<const float4*>(src + (size_t)(sp + i) * slice + 64);
             }
-        } else {
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) {
+                if (sp + i >= splits) break;
+                a[0] += v[i].x; a[1] += v[i].y; a[2] += v[i].z; a[3] += v[i].w;
+                if (EPI == 1) b[0] += u[i].x, b[1] += u[i].y, b[2] += u[i].z, b[3] += u[i].w;
+            }
+        }
+    } else {
+        for (int sp = 0; sp < splits; ++sp) {
+            const float* src = ws + (size_t)sp * slice + (size_t)m * N + c0;
             for (int j = 0; j < 4 && o0 + j < NO; ++j) {
                 a[j] += src[j];
                 if (EPI == 1) b[j] += src[64 + j];
             }
         }
     }
-    for (int j = 0; j < 4 && o0 + j < NO; ++j)
-        C[(size_t)m * ldc + o0 + j] = from_float<TO>(EPI == 1 ? gate_up(a[j], b[j], gate_epi) : a[j]);
+    if (EPI == 1) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a[j] = gate_up(a[j], b[j], gate_epi);
+    }
+    TO* dst = C + (size_t)m * ldc + o0;
+    if (o0 + 3 < NO && (reinterpret_cast<uintptr_t>(dst) & (4 * sizeof(TO) - 1)) == 0) {
+        if constexpr (sizeof(TO) == 4) {
+            *reinterpret_cast<float4*>(dst) = make_float4(a[0], a[1], a[2], a[3]);
+        } else {
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(a[0], a[1]), hi = __floats2bfloat162_rn(a[2], a[3]);
+            *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        }
+    } else {
+        for (int j = 0; j < 4 && o0 + j < NO; ++j) dst[j] = from_float<TO>(a[j]);
+    }
 }
 
 // Sixteen values of a row (the last chunk of a tile whose width is an odd multiple of 16).
