@@ -434,6 +434,46 @@ latent_decode_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_o
     }
 }
 
+// The same for at most 16 pieces and a thread for two neighbouring values: the pieces' values are under way before their maxima are looked
+// at, every warp forms the weights for itself, a lane a piece, and no block waits for a barrier. The same sums in the same order.
+// (A layer of latent attention decoding 8 requests behind 2,048 keys, 16 pieces of 128 rows of 512: 57.4 -> 52.3 us.)
+constexpr int MERGE_PIECES = 16;
+__global__ void __launch_bounds__(256)
+latent_merge_few_kernel(__nv_bfloat16* out, const float* part_o, const float* part_ml, size_t n_rows, int dv, int nsplit,
+                        const float* __restrict__ sinks, const float* gate, int nh) {
+    __shared__ float2 ml[8][MERGE_PIECES];        // a warp's: weight and sum of each piece
+    pdl_trigger();
+    pdl_wait();
+    const size_t r = blockIdx.x;
+    const int d = threadIdx.x * 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2 o[MERGE_PIECES];
+#pragma unroll
+    for (int s = 0; s < MERGE_PIECES; ++s)
+        o[s] = s < nsplit && d < dv ? *reinterpret_cast<const float2*>(part_o + ((size_t)s * n_rows + r) * dv + d) : make_float2(0.f, 0.f);
+    const float2 v = lane < nsplit ? *reinterpret_cast<const float2*>(part_ml + ((size_t)lane * n_rows + r) * 2) : make_float2(-INFINITY, 0.f);
+    const float M = warp_max(v.x);
+    if (lane < MERGE_PIECES) ml[warp][lane] = make_float2(v.x == -INFINITY ? 0.f : fast_exp2(v.x - M), v.y);
+    __syncwarp();
+    float L = 0.f, w[MERGE_PIECES];
+#pragma unroll
+    for (int s = 0; s < MERGE_PIECES; ++s) {
+        const float2 p = ml[warp][s];
+        w[s] = p.x;
+        if (s < nsplit && p.x != 0.f) L = fmaf(p.x, p.y, L);          // in the pieces' order
+    }
+    if (sinks) L += exp2f(sinks[r % nh] * 1.4426950408889634f - (M == -INFINITY ? 0.f : M));          // the sink counts once
+    const float inv = (L > 0.f ? 1.0f / L : 0.f) * (gate ? 1.0f / (1.0f + __expf(-gate[r])) : 1.0f);
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int s = 0; s < MERGE_PIECES; ++s) {
+        if (s >= nsplit) break;
+        const float wgt = w[s] * inv;
+        acc.x = fmaf(wgt, o[s].x, acc.x);
+        acc.y = fmaf(wgt, o[s].y, acc.y);
+    }
+    if (d < dv) *reinterpret_cast<__nv_bfloat162*>(out + r * dv + d) = __floats2bfloat162_rn(acc.x, acc.y);
+}
+
 // The pieces of a row merged in their order: out = sum_s 2^(m_s - M) o_s / sum_s 2^(m_s - M) l_s.
 __global__ void latent_merge_kernel(__nv_bfloat16* __restrict__ out, const float* part_o, const float* part_ml, size_t n_rows, int dv, int nsplit,
                                     const float* __restrict__ sinks, const float* gate, int nh) {
@@ -576,7 +616,10 @@ CELLM_API int cellm_attention_latent(void* out, float* part_o, float* part_ml, c
     const float scale_log2e = scale * 1.4426950408889634f;
     const dim3 grid((unsigned)n_tiles, (unsigned)nsplit);
     auto merge = [&]() -> int {
-        if (nsplit > 1)
+        if (nsplit > 1 && nsplit <= MERGE_PIECES && dv % 2 == 0 && dv <= 512 && (((uintptr_t)out) & 3) == 0 && (((uintptr_t)part_o | (uintptr_t)part_ml) & 7) == 0)
+            CELLM_RUN(latent_merge_few_kernel, (unsigned)((size_t)T * nh), (dv / 2 + 31) / 32 * 32, 0, stream, (__nv_bfloat16*)out, part_o, part_ml,
+                      (size_t)T * nh, dv, nsplit, sinks, gate, nh);
+        else if (nsplit > 1)
             CELLM_RUN(latent_merge_kernel, (unsigned)((size_t)T * nh), dv >= 256 ? 256 : (dv >= 128 ? 128 : 64), (size_t)nsplit * 2 * sizeof(float), stream, (__nv_bfloat16*)out,
                       part_o, part_ml, (size_t)T * nh, dv, nsplit, sinks, gate, nh);
         return CELLM_OK;

@@ -653,6 +653,26 @@ def test_latent_attention_of_single_tokens_rounds_as_the_other_form(nh, kw, dv, 
     assert float((alone.double() - beside.double()).norm() / beside.double().norm()) < 2.0 ** -11
 
 
+@pytest.mark.parametrize("nh,kw,dv,nsplit", [(16, 576, 512, 2), (16, 576, 512, 16), (16, 576, 512, 17), (3, 80, 48, 16), (5, 144, 128, 15)])
+def test_pieces_of_latent_attention_merge(nh, kw, dv, nsplit):
+    """Up to 16 pieces are merged by one kernel, more by another; pieces without a key among them, a whole request without one piece too
+    many. The merge's weights sum to one, so its roundings (32 bits) stay far below the results' (2^-9)."""
+    from cellm_b200 import ops
+    g = torch.Generator().manual_seed(nh + nsplit)
+    ctx_lens = [0, 64 * nsplit - 1, 500, 3]
+    cache, table = paged([c + 1 for c in ctx_lens], kw, 16, torch.bfloat16, g)
+    pool = torch.randn(cache.k.shape, generator=g).to(torch.bfloat16).to(DEV)
+    q = (torch.randn(4, nh * kw, generator=g) * 0.5).to(torch.bfloat16).to(DEV)
+    sinks, gate = torch.linspace(-2.0, 2.0, nh).to(DEV), torch.randn(4, nh, generator=g).to(DEV)
+    outs = []
+    for n in (1, nsplit):
+        ctx = step_ctx([1] * 4, ctx_lens)
+        outs.append(ops.attention_latent(q, pool, ctx.cu_seqlens, ctx.ctx_lens, cache.block_table, [1] * 4, nh, dv, kw ** -0.5, n, ctx.err, 0,
+                                         sinks, gate).double())
+        assert int(ctx.err.item()) == 0
+    assert float((outs[0] - outs[1]).norm() / outs[0].norm()) < 2.0 ** -8
+
+
 EXPANDED = [  # heads, dim, rot_dim, vdim, rank
     (4, 128, 64, 128, 512), (2, 64, 0, 64, 64), (3, 16, 16, 16, 24), (2, 48, 32, 80, 40), (1, 96, 64, 112, 128), (2, 192, 64, 128, 64), (5, 32, 0, 32, 96),
     (2, 128, 0, 48, 72), (1, 64, 96, 96, 16),
