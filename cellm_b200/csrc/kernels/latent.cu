@@ -71,6 +71,44 @@ latent_prep_kernel(TA* __restrict__ q_plain, TA* __restrict__ q_turned, long lon
         }
         return v;
     };
+    // A row divided by its root mean square, times its weight: a thread's first four values and their weights travel together, the
+    // weights (not the work of the kernel before this one) ahead of the wait, so that nothing but the sum's barrier lies between the
+    // row's arrival and its way out. put(i, value); `more` runs while the row's loads are under way.
+    auto normed = [&](const TP* src, const TW* w, int n, auto&& more, auto&& put) {
+        constexpr int NV = 4;
+        float wv[NV], v[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const int i = threadIdx.x + k * blockDim.x;
+            wv[k] = i < n ? to_float(w[i]) : 0.f;
+        }
+        pdl_wait();
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const int i = threadIdx.x + k * blockDim.x;
+            v[k] = i < n ? to_float(src[i]) : 0.f;
+        }
+        more();
+        float ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) ss += v[k] * v[k];
+        for (int i = threadIdx.x + NV * blockDim.x; i < n; i += blockDim.x) {
+            const float x = to_float(src[i]);
+            ss += x * x;
+        }
+        ss = warp_sum(ss);
+        const int lane = threadIdx.x & 31;
+        if (lane == 0) scratch[threadIdx.x >> 5] = ss;
+        __syncthreads();
+        ss = warp_sum(lane < (int)(blockDim.x >> 5) ? scratch[lane] : 0.f);
+        const float inv = 1.0f / sqrtf(ss / (float)n + eps);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const int i = threadIdx.x + k * blockDim.x;
+            if (i < n) put(i, v[k] * inv * wv[k]);
+        }
+        for (int i = threadIdx.x + NV * blockDim.x; i < n; i += blockDim.x) put(i, to_float(src[i]) * inv * to_float(w[i]));
+    };
     int role = blockIdx.y;
     if (roles & LP_LATENT) {
         if (role == 0) {
@@ -86,19 +124,13 @@ latent_prep_kernel(TA* __restrict__ q_plain, TA* __restrict__ q_turned, long lon
                 }
             }
             __syncthreads();
-            pdl_wait();
             const TP* down = down_rows + (size_t)t * ld;
-            float ss = 0.f;
-            for (int i = threadIdx.x; i < rank; i += blockDim.x) {
-                const float v = to_float(down[i]);
-                ss += v * v;
-            }
-            ss = block_sum(ss, scratch);
-            const float inv = 1.0f / sqrtf(ss / (float)rank + eps);
+            float key = 0.f;
+            normed(down, c_norm_w, rank, [&]() { if ((int)threadIdx.x < rot_dim) key = turned(down + rank, threadIdx.x); },
+                   [&](int i, float v) { if (cache_row) cache_row[i] = from_float<TA>(v); });
             if (cache_row) {
-                for (int i = threadIdx.x; i < rank; i += blockDim.x)
-                    cache_row[i] = from_float<TA>(to_float(down[i]) * inv * to_float(c_norm_w[i]));
-                for (int d = threadIdx.x; d < rot_dim; d += blockDim.x) cache_row[rank + d] = from_float<TA>(turned(down + rank, d));
+                if ((int)threadIdx.x < rot_dim) cache_row[rank + threadIdx.x] = from_float<TA>(key);
+                for (int d = threadIdx.x + blockDim.x; d < rot_dim; d += blockDim.x) cache_row[rank + d] = from_float<TA>(turned(down + rank, d));
             }
             return;
         }
@@ -107,19 +139,13 @@ latent_prep_kernel(TA* __restrict__ q_plain, TA* __restrict__ q_turned, long lon
     if (roles & LP_QUERY_NORM) {
         if (role == 0) {
             // the queries' latent: divided by its root mean square, times its weight; the heads' gates as 32-bit numbers
-            pdl_wait();
-            const TP* row = cq_rows + (size_t)t * ld;
-            float ss = 0.f;
-            for (int i = threadIdx.x; i < q_rank; i += blockDim.x) {
-                const float v = to_float(row[i]);
-                ss += v * v;
-            }
-            ss = block_sum(ss, scratch);
-            const float inv = 1.0f / sqrtf(ss / (float)q_rank + eps);
-            for (int i = threadIdx.x; i < q_rank; i += blockDim.x)
-                cq[(size_t)t * q_rank + i] = from_float<TA>(to_float(row[i]) * inv * to_float(cq_norm_w[i]));
+            float first_gate = 0.f;
+            const bool has_gate = gate_out && (int)threadIdx.x < heads;
+            normed(cq_rows + (size_t)t * ld, cq_norm_w, q_rank, [&]() { if (has_gate) first_gate = to_float(gate_rows[(size_t)t * ld + threadIdx.x]); },
+                   [&](int i, float v) { cq[(size_t)t * q_rank + i] = from_float<TA>(v); });
+            if (has_gate) gate_out[(size_t)t * heads + threadIdx.x] = first_gate;
             if (gate_out)
-                for (int h = threadIdx.x; h < heads; h += blockDim.x) gate_out[(size_t)t * heads + h] = to_float(gate_rows[(size_t)t * ld + h]);
+                for (int h = threadIdx.x + blockDim.x; h < heads; h += blockDim.x) gate_out[(size_t)t * heads + h] = to_float(gate_rows[(size_t)t * ld + h]);
             return;
         }
         --role;
@@ -132,14 +158,27 @@ latent_prep_kernel(TA* __restrict__ q_plain, TA* __restrict__ q_turned, long lon
     const int runs = (int)gridDim.y - ((roles & LP_LATENT) ? 1 : 0) - ((roles & LP_QUERY_NORM) ? 1 : 0);
     const int per = (heads + runs - 1) / runs;
     const int h_lo = min(heads, role * per), h_hi = min(heads, h_lo + per);
-    if (q_plain)
-        for (int i = h_lo * dim + threadIdx.x; i < h_hi * dim; i += blockDim.x) {
-            const int h = i / dim, d = i - h * dim;
-            q_plain[(size_t)t * heads * dim + i] = from_float<TA>(to_float(row[h * qw + d]));
+    // loads first, then what is made of them: a few values a thread of each kind at a time
+    constexpr int NQ = 4;
+    const int n_plain = q_plain ? (h_hi - h_lo) * dim : 0, n_turned = (h_hi - h_lo) * rot_dim;
+    for (int i0 = threadIdx.x; i0 < max(n_plain, n_turned); i0 += NQ * blockDim.x) {
+        float plain[NQ], turn[NQ];
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+            const int i = i0 + k * blockDim.x;
+            if (i < n_plain) { const int h = i / dim; plain[k] = to_float(row[(h_lo + h) * qw + i - h * dim]); }
         }
-    for (int i = h_lo * rot_dim + threadIdx.x; i < h_hi * rot_dim; i += blockDim.x) {
-        const int h = i / rot_dim, d = i - h * rot_dim;
-        q_turned[((size_t)t * heads + h) * turned_hs + d] = from_float<TA>(turned(row + h * qw + dim, d));
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+            const int i = i0 + k * blockDim.x;
+            if (i < n_turned) { const int h = i / rot_dim; turn[k] = turned(row + (h_lo + h) * qw + dim, i - h * rot_dim); }
+        }
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+            const int i = i0 + k * blockDim.x;
+            if (i < n_plain) q_plain[((size_t)t * heads + h_lo) * dim + i] = from_float<TA>(plain[k]);
+            if (i < n_turned) { const int h = i / rot_dim; q_turned[((size_t)t * heads + h_lo + h) * turned_hs + i - h * rot_dim] = from_float<TA>(turn[k]); }
+        }
     }
     if (gate_out && !(roles & LP_QUERY_NORM))
         for (int h = h_lo + threadIdx.x; h < h_hi; h += blockDim.x) gate_out[(size_t)t * heads + h] = to_float(gate_rows[(size_t)t * ld + h]);
@@ -234,25 +273,29 @@ head_product_kernel(TA* __restrict__ out, long long ldo, long long out_hs, const
 // A few tokens (decoding, bfloat16): the matrices are what has to be read, once. A block takes 16 output rows of one
 // head; the tokens' inputs wait in shared memory; eight neighbouring threads share a row and take neighbouring 16-byte
 // pieces of it by turns (so a row's loads are whole 128-byte lines and the inputs' reads fall into different banks),
-// and add their sums by three shuffles. K (a multiple of 64) is summed in the same order for every token count up to
+// and add their sums by shuffles. K (a multiple of 64) is summed in the same order for every token count up to
 // HP_SMALL_T.
 #define HP_SMALL_T 16
 #define HP_SMALL_AHEAD 8        // pieces of a row asked for ahead: all of K up to 512
+// LANES threads share a row: 8, or 16 from K = 256 on, where a thread's products are what takes time (with the preparation's loads
+// ahead of its barrier and of its stores a layer that decodes 8 requests went from 52.3 to 48.2 us).
+template <int LANES>
 __global__ void __launch_bounds__(128)
 head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long long out_hs, const __nv_bfloat16* in,
                           long long ldi, long long in_hs, const __nv_bfloat16* __restrict__ w, int T, int N, int K, int vec_in) {
     extern __shared__ __align__(16) __nv_bfloat16 xin[];       // [T][K]
     pdl_trigger();
     const int h = blockIdx.y;
-    const int n = blockIdx.x * 16 + (threadIdx.x >> 3), kq = threadIdx.x & 7;
+    constexpr int STEP = LANES * 8, AHEAD = HP_SMALL_AHEAD * 8 / LANES;
+    const int n = blockIdx.x * (128 / LANES) + threadIdx.x / LANES, kq = threadIdx.x % LANES;
     const bool on = n < N;
     const __nv_bfloat16* wr = w + ((size_t)h * N + (on ? n : 0)) * K;
     // the matrices are not the work of the kernel before this one: a row's first pieces are asked for before the wait on it (`in`
     // is, and is not declared __restrict__: its loads may not move up to these)
-    uint4 wq[HP_SMALL_AHEAD];
+    uint4 wq[AHEAD];
 #pragma unroll
-    for (int i = 0; i < HP_SMALL_AHEAD; ++i)
-        if (kq * 8 + i * 64 < K) wq[i] = *reinterpret_cast<const uint4*>(wr + kq * 8 + i * 64);
+    for (int i = 0; i < AHEAD; ++i)
+        if (kq * 8 + i * STEP < K) wq[i] = *reinterpret_cast<const uint4*>(wr + kq * 8 + i * STEP);
     pdl_wait();
     if (vec_in) {                        // the inputs' rows start on 16-byte borders: eight values a load
         const int K8 = K / 8;
@@ -290,9 +333,9 @@ head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long l
         }
     };
 #pragma unroll
-    for (int i = 0; i < HP_SMALL_AHEAD; ++i)
-        if (kq * 8 + i * 64 < K) piece(wq[i], kq * 8 + i * 64);
-    for (int k0 = kq * 8 + HP_SMALL_AHEAD * 64; k0 < K; k0 += 64) piece(*reinterpret_cast<const uint4*>(wr + k0), k0);
+    for (int i = 0; i < AHEAD; ++i)
+        if (kq * 8 + i * STEP < K) piece(wq[i], kq * 8 + i * STEP);
+    for (int k0 = kq * 8 + AHEAD * STEP; k0 < K; k0 += STEP) piece(*reinterpret_cast<const uint4*>(wr + k0), k0);
 #pragma unroll
     for (int t = 0; t < HP_SMALL_T; ++t) {
         if (t < T) {
@@ -300,6 +343,7 @@ head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long l
             v += __shfl_xor_sync(0xffffffffu, v, 1);
             v += __shfl_xor_sync(0xffffffffu, v, 2);
             v += __shfl_xor_sync(0xffffffffu, v, 4);
+            if (LANES == 16) v += __shfl_xor_sync(0xffffffffu, v, 8);
             if (kq == 0 && on) out[(size_t)t * ldo + h * out_hs + n] = __float2bfloat16_rn(v);
         }
     }
@@ -313,11 +357,14 @@ CELLM_API int cellm_head_product(void* out, long long ldo, long long out_hs, con
     // (32-bit activations always take the tiles below: one order of the sums whatever the number of tokens)
     if (dtype == CELLM_BF16 && T <= HP_SMALL_T && (size_t)T * K * 2 <= 48 * 1024 && (K & 63) == 0 &&
         ((uintptr_t)w & 15) == 0) {
-        const dim3 sgrid((unsigned)((N + 15) / 16), (unsigned)heads);
         const size_t smem = (size_t)T * K * 2;
-        CELLM_RUN(head_product_small_kernel, sgrid, 128, smem, stream, (__nv_bfloat16*)out, ldo, out_hs,
-                  (const __nv_bfloat16*)in, ldi, in_hs, (const __nv_bfloat16*)w, T, N, K,
-                  (int)((((uintptr_t)in & 15) == 0) && (ldi & 7) == 0 && (in_hs & 7) == 0));
+#define SMALL(LANES)                                                                                                       \
+    CELLM_RUN(head_product_small_kernel<LANES>, dim3((unsigned)((N + 128 / LANES - 1) / (128 / LANES)), (unsigned)heads), 128, smem, stream, \
+              (__nv_bfloat16*)out, ldo, out_hs, (const __nv_bfloat16*)in, ldi, in_hs, (const __nv_bfloat16*)w, T, N, K,         \
+              (int)((((uintptr_t)in & 15) == 0) && (ldi & 7) == 0 && (in_hs & 7) == 0))
+        if (K >= 256) SMALL(16);
+        else SMALL(8);
+#undef SMALL
         return CELLM_OK;
     }
     const dim3 grid((unsigned)((N + HP_TILE - 1) / HP_TILE), (unsigned)((T + HP_TILE - 1) / HP_TILE), (unsigned)heads);
