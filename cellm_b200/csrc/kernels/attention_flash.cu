@@ -327,6 +327,65 @@ attention_flash_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part
     }
 }
 
+// The same as below for at most 32 pieces: the pieces' values are under way together and before their maxima are looked at (one piece's
+// after the other's weight they cost a wait on L2 each); every warp forms the weights for itself, a lane a piece. The same sums in
+// the same order; values of a piece without weight (never written) are not used.
+__global__ void __launch_bounds__(64)
+attention_merge_few_kernel(__nv_bfloat16* out, const float* part_o, const float* part_ml, size_t n_rows, int hd, int nsplit,
+                           const float* __restrict__ sinks, const float* __restrict__ unrot, int interleaved,
+                           const int* __restrict__ positions, int nh, const FlashExtras ex) {
+    constexpr int MOST = 32;
+    __shared__ float2 ml[2][MOST];            // a warp's: weight and sum of each piece
+    pdl_trigger();
+    pdl_wait();
+    const size_t row = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float2 mine = lane < nsplit ? *reinterpret_cast<const float2*>(part_ml + ((size_t)lane * n_rows + row) * 2) : make_float2(-INFINITY, 0.f);
+    const int width = unrot ? hd / 2 : hd;    // a thread an entry, or a pair that is turned back by the row's position
+    float inv = 0.f;
+    for (int d = threadIdx.x; d - (int)threadIdx.x < width; d += blockDim.x) {
+        const bool on = d < width;
+        const int d0 = !unrot || !interleaved ? d : 2 * d, d1 = interleaved ? 2 * d + 1 : d + hd / 2;
+        float a[MOST], b[MOST];
+#pragma unroll
+        for (int s = 0; s < MOST; ++s) {
+            if (s >= nsplit) break;
+            a[s] = on ? part_o[((size_t)s * n_rows + row) * hd + d0] : 0.f;
+            if (unrot) b[s] = on ? part_o[((size_t)s * n_rows + row) * hd + d1] : 0.f;
+        }
+        if (d == (int)threadIdx.x) {
+            const float m = warp_max(mine.x), use = m == -INFINITY ? 0.f : m;
+            ml[warp][lane] = make_float2(exp2f(mine.x - use), mine.y);
+            __syncwarp();
+            float l = 0.f;
+            for (int s = 0; s < nsplit; ++s) l = fmaf(ml[warp][s].x, ml[warp][s].y, l);
+            if (sinks) l += exp2f(sinks[row % nh] * 1.4426950408889634f - use);
+            inv = (l > 0.f ? 1.0f / l : 0.f) * gate_factor(ex, (int)(row / nh), (int)(row % nh));
+        }
+        float u = 0.f, v = 0.f;
+#pragma unroll
+        for (int s = 0; s < MOST; ++s) {
+            if (s >= nsplit) break;
+            const float w = ml[warp][s].x;
+            if (w != 0.f) {
+                u = fmaf(w, a[s], u);
+                if (unrot) v = fmaf(w, b[s], v);
+            }
+        }
+        if (!on) continue;
+        u *= inv;
+        if (unrot) {
+            v *= inv;
+            float c, sn;
+            split_sincos((float)positions[row / nh], unrot[2 * d], unrot[2 * d + 1], &c, &sn);
+            out[row * hd + d0] = __float2bfloat16_rn(u * c + v * sn);
+            out[row * hd + d1] = __float2bfloat16_rn(v * c - u * sn);
+        } else {
+            out[row * hd + d0] = __float2bfloat16_rn(u);
+        }
+    }
+}
+
 // out[row] = sum_s 2^(m_s - m) O_s / sum_s 2^(m_s - m) l_s, pieces in order.
 __global__ void attention_merge_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ part_o,
                                        const float* __restrict__ part_ml, size_t n_rows, int hd, int nsplit,
@@ -432,7 +491,11 @@ static int attention_flash_impl(void* out, float* part_o, float* part_ml, const 
     else return CELLM_ERR_SIZE;
 #undef GO
     if (rc != CELLM_OK) return rc;
-    if (nsplit > 1) {
+    if (nsplit > 1 && nsplit <= 32 && ((uintptr_t)part_ml & 7) == 0) {
+        CELLM_RUN(attention_merge_few_kernel, (unsigned)((size_t)T * nh), hd >= 64 ? 64 : 32, 0, stream,
+                  (__nv_bfloat16*)out, (const float*)part_o, (const float*)part_ml, (size_t)T * nh, hd, nsplit, sinks, unrot,
+                  interleaved, positions, nh, ex);
+    } else if (nsplit > 1) {
         CELLM_RUN(attention_merge_kernel, (unsigned)((size_t)T * nh), hd >= 64 ? 64 : 32, 0, stream,
                   (__nv_bfloat16*)out, (const float*)part_o, (const float*)part_ml, (size_t)T * nh, hd, nsplit, sinks, unrot,
                   interleaved, positions, nh, ex);

@@ -654,8 +654,10 @@ CELLM_API int cellm_delta_prep(float* qk, float* v_out, float* beta, float* deca
 #undef PREP_RUN_OF
         return CELLM_OK;
     }
-    // few tokens: a token's channels over as many blocks as leave a thread about four of them (no sum crosses blocks)
-    const int widest = std::max(cv.C, heads * dim), parts = T >= 512 ? 1 : std::max(1, std::min((widest + 1023) / 1024, 64));
+    // few tokens: a token's channels over as many blocks as leave a thread about four of them (no sum crosses blocks), or one where
+    // the tokens are so few that such blocks find an SM of their own
+    const int widest = std::max(cv.C, heads * dim), four = (widest + 1023) / 1024, one = (widest + 255) / 256;
+    const int parts = T >= 512 ? 1 : std::max(1, std::min(std::max(four, std::min(one, 296 / T)), 64));
     CELLM_RUN(delta_prep_kernel, dim3(T, parts), 256, (size_t)8 * dim * sizeof(float), stream, qk, v_out, beta, decay, cv, slot_stride,
               n_slots, state, col_b, a2, ld_a2, dt_bias, A_log, seq_of_token, cu_seqlens, slot_ids, heads, kvh, dim, vd, l2_eps, err);
     return CELLM_OK;

@@ -136,6 +136,22 @@ def attention_plain_masked(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: i
     return out
 
 
+# Pieces of keys of the tensor-core attention below, of at least two blocks of 64 keys. Tiles of 64 rows (four warps) are cut only
+# where a step's tiles are few. Those of 16 rows are single warps that walk their keys alone, six of which an SM holds: what counts
+# is the blocks of keys a warp walks, and one more to begin with, times the rounds of 888 such warps, and the merge (8 kv heads, window
+# 1,024, both mixers of a layer: 8 requests 72 us in 4 pieces, 61 in 9; 16 95 in 2, 68 in 6, 76 in 9; 32 153 whole, 102 in 3; 64
+# 177 whole, 160 in 3).
+PIECES_FILL, PIECES_FILL_NARROW = 296, 888
+
+
+def _pieces(span: int, tiles: int, wide: bool) -> int:
+    tiles, most = max(1, tiles), min(-(-span // 128), 32)
+    if wide:
+        return max(1, min(most, PIECES_FILL // tiles))
+    cost = lambda n: -(-tiles * n // PIECES_FILL_NARROW) * (-(-span // (64 * n)) + 1) + (1.5 if n > 1 else 0)
+    return min((max(1, min(most, rounds * PIECES_FILL_NARROW // tiles)) for rounds in (0, 1, 2)), key=cost)
+
+
 def attention_flash_sink(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: int, scale: float, window: int,
                          sinks: Optional[torch.Tensor], unrot: Optional[torch.Tensor], interleaved: bool) -> torch.Tensor:
     """The same attention on the tensor cores (bfloat16; keys and values of one width hd of 32, 64 or 128): tiles of
@@ -149,10 +165,9 @@ def attention_flash_sink(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: int
     wide = ctx.max_q_len * G > 16
     rows = 64 if wide else 16
     n_tiles = sum(-(-n * G // rows) for n in ctx.q_lens)
-    # pieces of keys: only where a step's tiles are few; a piece is at least two blocks of 64 keys
     longest = ctx.max_total_len          # a captured step's bound: the width of its block tables
     span = min(longest, window + ctx.max_q_len) if window > 0 else longest
-    nsplit = max(1, min(-(-span // 128), 296 // max(1, n_tiles * nkv), 32))
+    nsplit = _pieces(span, n_tiles * nkv, wide)
     out = torch.empty((T, nh * hd), dtype=q.dtype, device=q.device)
     part_o = part_ml = None
     if nsplit > 1:
@@ -181,7 +196,7 @@ def attention_flash_masked(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: i
     n_tiles = sum(-(-n * G // rows) for n in ctx.q_lens)
     longest = ctx.max_total_len
     span = min(longest, window + keep_first + ctx.max_q_len) if window > 0 else longest
-    nsplit = max(1, min(-(-span // 128), 296 // max(1, n_tiles * nkv), 32))
+    nsplit = _pieces(span, n_tiles * nkv, wide)
     out = torch.empty((T, nh * hd), dtype=q.dtype, device=q.device)
     part_o = part_ml = None
     if nsplit > 1:
@@ -381,7 +396,7 @@ def attention_flash_chunked(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: 
     n_tiles = sum(-(-n * G // rows) for n in ctx.q_lens)
     longest = ctx.max_total_len
     span = min(longest, chunk + ctx.max_q_len) if chunk > 0 else longest
-    nsplit = max(1, min(-(-span // 128), 296 // max(1, n_tiles * nkv), 32))
+    nsplit = _pieces(span, n_tiles * nkv, wide)
     out = torch.empty((T, nh * hd), dtype=q.dtype, device=q.device)
     part_o = part_ml = None
     if nsplit > 1:

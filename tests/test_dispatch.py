@@ -214,3 +214,12 @@ def test_the_chunks_of_a_recurrence_go_through_a_bounded_workspace(delta, heads,
         assert chunks == -(-n // 16) and rest and 1 <= held <= chunks
         assert ws.numel() % held == 0 and ws.numel() * 4 <= 128 << 20
         assert held == chunks or n > 2048 or heads > 16
+
+
+@pytest.mark.parametrize("span,tiles,wide,pieces", [(1025, 64, False, 9), (1025, 128, False, 6), (1025, 256, False, 3), (1025, 512, False, 3),
+                                                    (1025, 800, False, 1), (1025, 5000, False, 1), (100, 8, False, 1), (129, 1, False, 1), (301, 8, False, 3),
+                                                    (70000, 8, False, 32), (1, 0, False, 1), (3000, 100, True, 2), (3000, 400, True, 1)])
+def test_pieces_of_keys_where_an_attention_walks_them_alone(span, tiles, wide, pieces):
+    """Never more pieces than pairs of blocks of 64 keys, nor than 32; whole where the tiles fill the GPU anyway."""
+    from cellm_b200.ops import recurrent
+    assert recurrent._pieces(span, tiles, wide) == pieces

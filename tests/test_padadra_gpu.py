@@ -737,6 +737,32 @@ def test_attention_preparation_of_many_tokens(taps, bias, norms, interleaved, ro
             assert torch.equal(x, y)
 
 
+@pytest.mark.parametrize("hd,window", [(64, 300), (32, 0), (128, 70)])
+def test_pieces_of_attention_with_sinks_merge(monkeypatch, hd, window):
+    """Single tokens in 2 pieces, in 31 and in 32 (most of them without a key), turned back and not: what one piece gives (the merge's weights
+    sum to one, so its 32-bit roundings stay far below the results' 2^-9)."""
+    from cellm_b200 import ops
+    from cellm_b200.ops import recurrent
+    from cellm_b200.parts import CacheBinding
+    from cellm_b200.parts.rope import split_inv_freq
+    nh, nkv, ctx_lens, g = 6, 2, [0, 700, 63, 200], torch.Generator().manual_seed(hd)
+    pages = -(-701 // 16)
+    table = torch.arange(pages * 4, dtype=torch.int32, device=DEV).reshape(4, pages)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).to(DEV)
+    cache = CacheBinding(k=rnd(pages * 4, nkv, 16, hd), v=rnd(pages * 4, nkv, 16, hd), block_table=table, page_size=16, num_pages=pages * 4)
+    q, sinks, freq = rnd(4, nh * hd), torch.linspace(-2.0, 2.0, nh).to(DEV), split_inv_freq(1e4, hd).to(DEV)
+    for unrot in (None, freq):
+        for interleaved in (True, False):
+            outs = []
+            for n in (1, 2, 31, 32):
+                monkeypatch.setattr(recurrent, "_pieces", lambda *_, n=n: n)
+                ctx = step_ctx([1] * 4, ctx_lens, list(range(4)))
+                outs.append(ops.attention_flash_sink(q, cache, ctx, nh, nkv, hd, hd ** -0.5, window, sinks, unrot, interleaved).double())
+                assert int(ctx.err.item()) == 0
+            for o in outs[1:]:
+                assert float((o - outs[0]).norm() / outs[0].norm()) < 2.0 ** -8
+
+
 @pytest.mark.parametrize("T,heads,vd,lead,act", [(5, 3, 64, 0, "bfloat16"), (1, 1, 128, 0, "float32"), (9, 2, 128, 4, "bfloat16"), (3, 5, 64, 3, "float32"),
                                                  (4, 3, 40, 0, "bfloat16")])
 def test_head_norms_by_fours_and_one_by_one(T, heads, vd, lead, act):
