@@ -286,8 +286,10 @@ CELLM_API int cellm_sink_attn_prep(void* q_out, void* k_pool, void* v_pool, cons
     const int fours = conv_taps_in_fours(cv, state, slot_stride);
     // (512 tokens: below, the blocks of a token each are what fills the SMs)
     const size_t run_smem = (size_t)(PREP_RUN * (cv.C + rot + vd)) * sizeof(float);
-    const bool outs = ((reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool)) & 15) == 0;
-    if (T >= 512 && n_taps >= 2 && n_taps <= 4 && fours && outs && hd % 8 == 0 && vd % 8 == 0 && rot % 8 == 0 && run_smem <= 100 * 1024) {
+    // (the norms' weights are read four at a time there, value by value in the form of a block a token)
+    const bool borders = ((reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool) |
+                           reinterpret_cast<uintptr_t>(q_norm_w) | reinterpret_cast<uintptr_t>(k_norm_w)) & 15) == 0;
+    if (T >= 512 && n_taps >= 2 && n_taps <= 4 && fours && borders && hd % 8 == 0 && vd % 8 == 0 && rot % 8 == 0 && run_smem <= 100 * 1024) {
         const int run_threads = std::min(512, std::max(128, (cv.C / 8 + 31) / 32 * 32));        // two pieces of four channels a thread
 #define RUN_OF(TA, NT)                                                                                                        \
     do {                                                                                                                      \

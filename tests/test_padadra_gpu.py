@@ -737,6 +737,43 @@ def test_attention_preparation_of_many_tokens(taps, bias, norms, interleaved, ro
             assert torch.equal(x, y)
 
 
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("hd,vd,rot,interleaved,turned_values,dtype", [(48, 80, 48, True, True, "float32"), (40, 64, 32, False, True, "bfloat16"), (128, 32, 64, False, False, "float32"),
+                                                                       (24, 56, 8, True, False, "float32"), (72, 40, 72, False, True, "float32")])
+def test_attention_preparation_of_many_tokens_of_any_width(hd, vd, rot, interleaved, turned_values, dtype, shift):
+    """Keys and values of different widths and of no power of two, channels that leave the threads unequal shares, and weights of the
+    norms off the 16-byte border (`shift`: those steps take the form of a block a token): what portions of fewer tokens give. Two
+    orders of at most 6 * 128 squares differ by less than 768 * 2^-24 of their sum, the root by half that."""
+    from cellm_b200 import ops
+    from cellm_b200.parts import CacheBinding
+    from cellm_b200.parts.rope import split_inv_freq
+    nh, nkv, taps, dt, lens = 6, 3, 4, getattr(torch, dtype), [201, 1, 5, 306]
+    g = torch.Generator().manual_seed(hd + vd)
+    T, C = sum(lens), (nh + nkv) * hd + nkv * vd
+    rnd = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    proj, b, w, state = rnd(T, C), rnd(C), rnd(C, taps), rnd(len(lens), taps - 1, C)
+    nw = [rnd(n * hd + shift)[shift:] for n in (nh, nkv)]
+    mult, freq, vfreq = rnd(nh), split_inv_freq(1e4, rot).to(DEV), split_inv_freq(1e3, vd).to(DEV) if turned_values else None
+    pages = -(-max(lens) // 8)
+    table = torch.arange(pages * len(lens), dtype=torch.int32, device=DEV).reshape(len(lens), pages)
+    pool = lambda d: torch.zeros(pages * len(lens), nkv, 8, d, dtype=dt, device=DEV)
+    def run(rows, ctx, cache):
+        q = ops.sink_attn_prep(rows, 0, b, w, taps, state, *nw, 1e-5, freq, rot, vfreq, interleaved, ctx, cache, nh, nkv, hd, vd, dt, mult)
+        assert int(ctx.err.item()) == 0
+        return q
+    whole = CacheBinding(k=pool(hd), v=pool(vd), block_table=table, page_size=8, num_pages=pages * len(lens))
+    q = run(proj, step_ctx(lens, [0] * len(lens), list(range(len(lens)))), whole)
+    alone, got, at = CacheBinding(k=pool(hd), v=pool(vd), block_table=table, page_size=8, num_pages=pages * len(lens)), [], 0
+    for i, n in enumerate(lens):
+        alone.block_table = table[i:i + 1]
+        got.append(run(proj[at:at + n], step_ctx([n], [0], [i]), alone))
+        at += n
+    assert torch.equal(whole.v, alone.v)
+    rel = 2.0 ** -7 if dtype == "bfloat16" else 2.0 ** -14
+    for x, y in ((q, torch.cat(got)), (whole.k, alone.k)):
+        torch.testing.assert_close(x, y, rtol=rel, atol=rel)
+
+
 @pytest.mark.parametrize("hd,window", [(64, 300), (32, 0), (128, 70)])
 def test_pieces_of_attention_with_sinks_merge(monkeypatch, hd, window):
     """Single tokens in 2 pieces, in 31 and in 32 (most of them without a key), turned back and not: what one piece gives (the merge's weights
