@@ -55,11 +55,11 @@ struct ChunkArgs {
 
 // A (chunk, head) in the workspace, as the walk's products take it (operands of mma.sync m16n8k16 in three bfloat16 parts, a lane's
 // registers side by side): for every 16 channels -W (delta rule), Q and k E(., end) as right operands; E(., end) [DIM]; then
-// per block of CB columns U0 [CB][CT] (HGRN2: as a left operand) and O0 [CB][CT].
+// per block of CB columns U0 [CB][CT] (delta rule; HGRN2's are the values themselves) and O0 [CB][CT].
 template <int DIM, bool DELTA> struct Layout {
     static constexpr int KINDS = DELTA ? 3 : 2, OPERAND = 3 * 32 * 4;
     static constexpr int DECAY = DIM / 16 * KINDS * OPERAND, ROWS = DECAY + DIM;
-    static constexpr int O0 = DELTA ? CT * CB : OPERAND, COLS = O0 + CT * CB;
+    static constexpr int O0 = DELTA ? CT * CB : 0, COLS = O0 + CT * CB;
     static constexpr int STAGE = ROWS + COLS;
 };
 
@@ -300,12 +300,7 @@ chunk_vectors_kernel(const ChunkArgs a) {
                 u[t] = sum;
                 if ((t & 3) == 3) *reinterpret_cast<float4*>(out + (j % CB) * CT + t - 3) = make_float4(u[t - 3], u[t - 2], u[t - 1], u[t]);
             } else {
-                // tokens 4 i .. 4 i + 3 of a column are two registers of lane i of it
                 u[t] = v[t];
-                if (t & 1) {
-                    uint32_t* to = reinterpret_cast<uint32_t*>(out) + ((j & 7) * 4 + (t >> 2)) * 4 + ((j >> 3) & 1) + (t & 2);
-                    split3(to[0], to[128], to[256], v[t - 1], v[t]);
-                }
             }
         }
 #pragma unroll
@@ -364,7 +359,7 @@ __device__ __forceinline__ void product3(float (&most)[2][4], float (&rest)[2][4
 template <int DIM, bool DELTA> struct Walk {
     static constexpr int WARPS = DIM / 16, READ = DELTA ? WARPS : 0, SUMS = 4, MEET = (WARPS + READ + SUMS) * 32, THREADS = MEET + 32;
     static constexpr int PART = WARPS * CT * CB;        // a product's sums over every warp's channels
-    static constexpr int SMEM_FLOATS = DELTA ? 3 * PART + (2 * WARPS + 1) * 3 * 32 * 4 : 2 * PART;
+    static constexpr int SMEM_FLOATS = DELTA ? 3 * PART + (2 * WARPS + 1) * 3 * 32 * 4 : 2 * PART + 2 * 3 * 32 * 4;
 };
 
 // A block carries CB columns of one (request, head)'s S through the request's chunks that are in the workspace; 16 columns make 128
@@ -381,8 +376,10 @@ template <int DIM, bool DELTA> struct Walk {
 // back to all of them. With multiply-adds on S in shared memory the walk took 166 us for 2,048 tokens and 16 heads of 128 x 128, bound
 // by shared memory's bandwidth; this form 105. What that took: no mbarrier on the chain, loads beside products, read-outs and
 // sums on warps of their own (with the sums on the state's warps and an mbarrier a hand-over 125). HGRN2 with heads of 64 x 64,
-// which has no u to wait for: 88 -> 45 us for 128 chunks. Where blocks are many (32 portions of 100 tokens, 16 heads of 128 x 128) HGRN2's
-// walk is bound by the products: 304 us with chunk_vectors, with multiply-adds 281; heads of 64 rows 170 (172).
+// which has no u to wait for: 88 -> 45 us for 128 chunks. Where blocks are many the workspace's bytes count: every block of columns reads its
+// head's operands. HGRN2's u is split here, out of the values, by the warps of the sums, two chunks ahead; with its parts in the
+// workspace 32 portions of 100 tokens over 16 heads of 128 x 128 took 260 us with chunk_vectors (multiply-adds 239), now 197; 16 portions of
+// 1,000 tokens 1,119 (1,026), now 810, with heads of 64 rows 666 (640), now 609.
 template <int DIM, bool DELTA>
 __global__ void __launch_bounds__(Walk<DIM, DELTA>::THREADS, DIM == 128 && DELTA ? 1 : 2)
 chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long long slot_stride, int n_slots, const ChunkArgs a,
@@ -393,8 +390,9 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     extern __shared__ __align__(16) float sm[];
     float* part = sm + a.stages * L::STAGE;      // [3][WARPS][CT * CB]: read-outs of even and of odd chunks, u
     float* u_part = part + 2 * W::PART;
-    uint32_t* frags = reinterpret_cast<uint32_t*>(part + 3 * W::PART);        // [2][WARPS] S before even and before odd chunks; u
-    uint32_t* ufrag = frags + 2 * WARPS * L::OPERAND;
+    uint32_t* frags = reinterpret_cast<uint32_t*>(part + 3 * W::PART);        // [2][WARPS] S before even and before odd chunks
+    // u as a left operand (HGRN2: of even and of odd chunks)
+    uint32_t* ufrag = DELTA ? frags + 2 * WARPS * L::OPERAND : reinterpret_cast<uint32_t*>(part + 2 * W::PART);
     __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES];
     __shared__ int abort_flag_;
     volatile int* abort_flag = &abort_flag_;
@@ -508,19 +506,37 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
         // u's pair among the left operand's registers: tokens 4 t .. 4 t + 3 of a column are lane t's registers half and half + 2
         uint32_t* to = ufrag + ((l & 28) + 2 * j + ((l & 3) >> 1)) * 4 + half + 2 * (l & 1);
         float2 u0 = make_float2(0.f, 0.f), o0 = u0;
+        // HGRN2: u is the values, which are fetched two chunks ahead
+        const float* v = a.v + (size_t)(start + c0 * CT + token) * a.ld_v + (size_t)h * a.vd + col0 + col;
+        auto values = [&](int ahead) {
+            const float* p = v + (size_t)ahead * CT * a.ld_v;
+            const int n = left - ahead * CT;
+            return make_float2(n > 0 ? p[0] : 0.f, n > 1 ? p[a.ld_v] : 0.f);
+        };
+        auto place = [&](int c, float2 x) {
+            uint32_t* dst = to + (DELTA ? 0 : (c & 1) * L::OPERAND);
+            split3(dst[0], dst[128], dst[256], x.x, x.y);
+        };
+        float2 v1 = u0, v2 = u0;
+        if constexpr (!DELTA) {
+            const float2 v0 = values(0);
+            v1 = values(1);
+            place(0, v0);
+        }
         there();
         meet();
         for (int c = 0; c < n_chunks; ++c) {
+            if constexpr (!DELTA) v2 = values(2), v += (size_t)CT * a.ld_v;
             const float* uo = sm + at * L::STAGE + L::ROWS + col * CT + token;
             const float2 o1 = *reinterpret_cast<const float2*>(uo + L::O0);
             if constexpr (DELTA) u0 = *reinterpret_cast<const float2*>(uo);
             const int last = at == 0 ? a.stages - 1 : at - 1;
             next();
+            if constexpr (!DELTA) place(c + 1, v1), v1 = v2;
             if (c + 1 < n_chunks) there();
             meet();
             if constexpr (DELTA) {
-                const float2 x = add_up(u_part, u0);
-                split3(to[0], to[128], to[256], x.x, x.y);
+                place(c, add_up(u_part, u0));
                 u_whole();
             }
             if (c > 0 && r == 0) mbar_arrive(&empty[last]);
@@ -580,7 +596,6 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     auto chunk_operands = [&]() {
         right_operands(k, L::KINDS - 1);
         e = *reinterpret_cast<const float4*>(sm + at * L::STAGE + L::DECAY + row);
-        if constexpr (!DELTA) left_operand(u, reinterpret_cast<const uint32_t*>(sm + at * L::STAGE + L::ROWS));
     };
     meet();
     right_operands(w, 0);
@@ -599,6 +614,7 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
             wait_u();
             left_operand(u, ufrag);
         } else {
+            left_operand(u, ufrag + (c & 1) * L::OPERAND);
             put(part + (c & 1) * W::PART);
         }
         product3<true>(most, rest, u, k);

@@ -216,6 +216,17 @@ def test_the_chunks_of_a_recurrence_go_through_a_bounded_workspace(delta, heads,
         assert held == chunks or n > 2048 or heads > 16
 
 
+def test_hgrn2_chunks_of_many_portions_are_one_run():
+    """Its chunks take no more workspace than operands of 32 bits and the read-outs' first terms would, so 32 portions of 100 tokens over 16
+    heads of 128 x 128 stay one run."""
+    import types
+
+    from cellm_b200.ops import recurrent
+    ctx = types.SimpleNamespace(q_lens=[100] * 32, max_q_len=100, B=32)
+    ws, chunks, held, _, _ = recurrent._state_chunks(ctx, False, 16, 128, 128, torch.device("meta"))
+    assert held == chunks == 32 * 7 and ws.numel() <= chunks * 16 * (33 * 128 + 8 * 2 * 16 * 16)
+
+
 @pytest.mark.parametrize("span,tiles,wide,pieces", [(1025, 64, False, 9), (1025, 128, False, 6), (1025, 256, False, 3), (1025, 512, False, 3),
                                                     (1025, 800, False, 1), (1025, 5000, False, 1), (100, 8, False, 1), (129, 1, False, 1), (301, 8, False, 3),
                                                     (70000, 8, False, 32), (1, 0, False, 1), (3000, 100, True, 2), (3000, 400, True, 1)])
