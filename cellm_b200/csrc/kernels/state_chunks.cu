@@ -22,12 +22,14 @@
 //   chunk_vectors   W, Q, k E(., end), E(., end), U0 and O0 of every chunk and head, all of them at once
 //   chunk_walk      a block carries 16 columns of one (request, head)'s S through the chunks: two small products a chunk
 //
-// chunk_vectors is 32-bit fused multiply-adds, as token by token; chunk_walk takes its products of 32-bit numbers on the tensor cores,
-// in three bfloat16 parts a factor. Against 64 bits over 2,048 tokens, in brackets with fused multiply-adds in the walk too (4 heads
-// of 128 x 128, decays uniform in 0.8 .. 1): read-outs 1.11e-7 (1.16e-7), the state behind them 7.2e-8 (8.9e-8); decays in
-// 0.999 .. 1 and repeating keys 3.3e-7 (5.0e-7) and 3.3e-7 (5.3e-7); uniform in 0 .. 1 9.2e-8 (9.3e-8) and 5.9e-8 (5.1e-8). HGRN2
-// 8.2e-8 (8.5e-8), 5.9e-8 (7.9e-8); 5.1e-7 (8.2e-7), 8.7e-7 (1.4e-6); 7.3e-8 (7.3e-8), 4.9e-8 (3.9e-8).
-// One prompt of 2,048 tokens, 16 heads of 128 x 128: token by token 938 us, in chunks with multiply-adds 214, now 163 (58 of them
+// chunk_vectors is 32-bit fused multiply-adds, as token by token; chunk_walk takes its products with S on the tensor cores, in three
+// bfloat16 parts a factor, and moves S on by 32-bit multiply-adds. Against 64 bits over 1,025 tokens, in brackets with multiply-adds
+// in all of the walk (8 heads of 128 x 128, decays uniform in 0.8 .. 1): read-outs 1.13e-7 (1.16e-7), the state behind them 8.6e-8
+// (8.6e-8); decays in 0.999 .. 1 and repeating keys 4.7e-7 (4.7e-7) and 5.5e-7 (5.5e-7); uniform in 0 .. 1 9.1e-8 (9.2e-8) and 5.0e-8
+// (5.0e-8). HGRN2 1.06e-7 (1.09e-7), 7.8e-8 (7.8e-8); 6.4e-7 (6.4e-7), 1.0e-6 (1.0e-6); 9.1e-8 (9.1e-8), 4.3e-8 (4.3e-8). (With S moved
+// by products in parts as well its error was smaller where decays are near 1 and up to 15 % larger where a chunk's last tokens prevail:
+// the tensor cores cut the small terms of a sum.)
+// One prompt of 2,048 tokens, 16 heads of 128 x 128: token by token 938 us, in chunks with multiply-adds 214, now 176 (55 of them
 // chunk_vectors, which forms the parts).
 #include <algorithm>
 #include <climits>
@@ -54,11 +56,11 @@ struct ChunkArgs {
 };
 
 // A (chunk, head) in the workspace, as the walk's products take it (operands of mma.sync m16n8k16 in three bfloat16 parts, a lane's
-// registers side by side): for every 16 channels -W (delta rule), Q and k E(., end) as right operands; E(., end) [DIM]; then
+// registers side by side): for every 16 channels -W (delta rule) and Q as right operands; k E(., end) [CT][DIM]; E(., end) [DIM]; then
 // per block of CB columns U0 [CB][CT] (delta rule; HGRN2's are the values themselves) and O0 [CB][CT].
 template <int DIM, bool DELTA> struct Layout {
-    static constexpr int KINDS = DELTA ? 3 : 2, OPERAND = 3 * 32 * 4;
-    static constexpr int DECAY = DIM / 16 * KINDS * OPERAND, ROWS = DECAY + DIM;
+    static constexpr int KINDS = DELTA ? 2 : 1, OPERAND = 3 * 32 * 4;
+    static constexpr int KE = DIM / 16 * KINDS * OPERAND, DECAY = KE + CT * DIM, ROWS = DECAY + DIM;
     static constexpr int O0 = DELTA ? CT * CB : 0, COLS = O0 + CT * CB;
     static constexpr int STAGE = ROWS + COLS;
 };
@@ -123,7 +125,7 @@ template <int N, int TOP> __device__ __forceinline__ int scatter_sums(float (&x)
     return first;
 }
 
-// A block a (chunk, head), a thread a channel. Bound by the instructions of the sums over channels and by what it writes (54 KB a
+// A block a (chunk, head), a thread a channel. Bound by the instructions of the sums over channels and by what it writes (50 KB a
 // block of the delta rule with 128 x 128). The walk's operands leave here in parts, once for all of a head's blocks of columns: 47 ->
 // 58 us for 2,048 tokens and 16 heads, where splitting them in every block cost the walk 20.
 template <int DIM, bool DELTA>
@@ -157,19 +159,10 @@ chunk_vectors_kernel(const ChunkArgs a) {
     }
     if (DELTA && tid < CT) beta[tid] = tid < len ? a.beta[(size_t)(t0 + tid) * a.heads + h] : 0.f;
     {
-        // tokens 4 t .. 4 t + 3 of a channel are two registers of lane t of its row
-        uint32_t* out = operand + (L::KINDS - 1) * L::OPERAND + (((tid >> 2) & 3) * 2 + (tid & 1)) * 16 + (tid & 2);
-        float e = 1.f, ke[4];
+        float e = 1.f;
 #pragma unroll
         for (int t = CT - 1; t >= 0; --t) {
-            ke[t & 3] = k[t] * e;
-            if ((t & 3) == 0) {
-                uint32_t x[3], y[3];
-                split3(x[0], x[1], x[2], ke[0], ke[1]);
-                split3(y[0], y[1], y[2], ke[2], ke[3]);
-#pragma unroll
-                for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(out + p * 128 + t) = make_uint2(x[p], y[p]);
-            }
+            ws[L::KE + t * DIM + tid] = k[t] * e;
             e *= g[t];
         }
         ws[L::DECAY + tid] = e;
@@ -281,7 +274,7 @@ chunk_vectors_kernel(const ChunkArgs a) {
                 q[t] = sum;
             }
         }
-        rows_out(operand + (L::KINDS - 2) * L::OPERAND, q);
+        rows_out(operand + (L::KINDS - 1) * L::OPERAND, q);
     }
     const int blocks = (a.vd + CB - 1) / CB;
 #pragma unroll 1
@@ -320,17 +313,20 @@ __device__ __forceinline__ void copy_bulk(float* dst, const float* src, int floa
                  ::"r"(smem_u32(dst)), "l"(src), "r"(floats * 4), "r"(smem_u32(bar)) : "memory");
 }
 
+// Two 32-bit multiply-adds in one instruction (each rounded as fmaf).
+__device__ __forceinline__ void fma2(float& x, float& y, float a, float b, float u) {
+    asm("{ .reg .b64 p, q, r; mov.b64 p, {%0, %1}; mov.b64 q, {%2, %3}; mov.b64 r, {%4, %4}; fma.rn.f32x2 p, q, r, p; mov.b64 {%0, %1}, p; }"
+        : "+f"(x), "+f"(y) : "f"(a), "f"(b), "f"(u));
+}
+
 // The operands of mma.sync m16n8k16 in three parts each, [part][register].
 struct Rows3 { uint32_t r[3][4]; };
 struct Cols3 { uint32_t r[3][2][2]; };       // two right operands side by side
 // A times each of the two of B (16 x 16 by 16 x 8) of 32-bit numbers: the products of the parts down to 2^-16 of the largest, as three
 // sums each (a chain of products waits 21 cycles for every one of two chains, 12 for one of eight). The tensor cores cut
-// their sums instead of rounding them, so the largest parts' products stand alone, in `most`, and the others, whose cut lies far below
-// a 32-bit sum's last place, in `rest`. CUT: what the cut took from `most` is formed too (the same products on top of minus their
-// sum: the tensor cores carry a few bits beyond 32-bit sums) and added to `rest`.
-template <bool CUT>
-__device__ __forceinline__ void product3(float (&most)[2][4], float (&rest)[2][4], const Rows3& a, const Cols3& b) {
-    float x[2][3][4], cut[2][4];
+// their sums instead of rounding them, so the largest parts' products stand alone.
+__device__ __forceinline__ void product3(float (&out)[2][4], const Rows3& a, const Cols3& b) {
+    float x[2][3][4];
 #pragma unroll
     for (int i = 0; i < 12; ++i) (&x[0][0][0])[i] = (&x[1][0][0])[i] = 0.f;
     constexpr int PA[6] = {0, 2, 0, 1, 0, 1}, PB[6] = {0, 0, 2, 1, 1, 0}, TO[6] = {2, 0, 1, 0, 1, 0};
@@ -339,47 +335,36 @@ __device__ __forceinline__ void product3(float (&most)[2][4], float (&rest)[2][4
 #pragma unroll
         for (int j = 0; j < 2; ++j) mma_bf16(x[j][TO[p]], a.r[PA[p]], b.r[PB[p]][j][0], b.r[PB[p]][j][1]);
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        if constexpr (CUT) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) cut[j][i] = -x[j][2][i];
-            mma_bf16(cut[j], a.r[0], b.r[0][j][0], b.r[0][j][1]);
-        }
-    }
-#pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            rest[j][i] = x[j][0][i] + x[j][1][i];
-            if constexpr (CUT) rest[j][i] += cut[j][i];
-            most[j][i] = x[j][2][i];
-        }
+        for (int i = 0; i < 4; ++i) out[j][i] = (x[j][0][i] + x[j][1][i]) + x[j][2][i];
 }
 
 template <int DIM, bool DELTA> struct Walk {
     static constexpr int WARPS = DIM / 16, READ = DELTA ? WARPS : 0, SUMS = 4, MEET = (WARPS + READ + SUMS) * 32, THREADS = MEET + 32;
     static constexpr int PART = WARPS * CT * CB;        // a product's sums over every warp's channels
-    static constexpr int SMEM_FLOATS = DELTA ? 3 * PART + (2 * WARPS + 1) * 3 * 32 * 4 : 2 * PART + 2 * 3 * 32 * 4;
+    static constexpr int UP = CT + 4, US = DELTA ? 1 : 3;           // u by columns, UP floats apart (a phase's reads and stores meet few banks twice)
+    static constexpr int SMEM_FLOATS = (DELTA ? 3 * PART + 2 * WARPS * 3 * 32 * 4 : 2 * PART) + US * CB * UP;
 };
 
 // A block carries CB columns of one (request, head)'s S through the request's chunks that are in the workspace; 16 columns make 128
 // blocks of a prompt over 16 heads of 128 columns, which is nearly the GPU. Its warps by their work:
-//   WARPS   hold 16 channels by 16 columns of S^T each, as the accumulators of mma.sync m16n8k16, which are its left operand as well:
-//           S^T [-W]^T over their channels, for u; then S^T <- S^T diag(E) + u^T (k E) over the chunk's 16 tokens (HGRN2: u is given)
+//   WARPS   hold 16 channels by 16 columns of S^T each, in the places of a left operand of mma.sync m16n8k16: S^T [-W]^T over their
+//           channels, for u; then S^T <- S^T diag(E) + u^T (k E), token after token (HGRN2: u is the values)
 //   READ    take the read-outs S^T Q^T over as many channels each, from copies of that left operand, beside the chain (HGRN2, whose chain
 //           is short: the state's warps do, and two blocks fit an SM, which many requests need)
-//   SUMS    add the warps' sums, in a fixed order, with U0 or O0 on top: u goes back as a left operand, o to memory
+//   SUMS    add the warps' sums, in a fixed order, with U0 or O0 on top: u goes back by columns, o to memory
 //   1       copies the chunks ahead of them all
-// All numbers stay 32-bit: an operand enters as three bfloat16 numbers, a product as the six products of parts above 2^-24 of it
-// (product3); sums over more than 16 terms are 32-bit additions. An infinite entry of S or u makes its column's later results NaN.
-// Bound by the chain of a chunk, 0.8 us: products (24 of mma.sync a scheduler, 9 cycles each, twice), the meeting of the warps, u's sums, u
-// back to all of them. With multiply-adds on S in shared memory the walk took 166 us for 2,048 tokens and 16 heads of 128 x 128, bound
-// by shared memory's bandwidth; this form 105. What that took: no mbarrier on the chain, loads beside products, read-outs and
-// sums on warps of their own (with the sums on the state's warps and an mbarrier a hand-over 125). HGRN2 with heads of 64 x 64,
-// which has no u to wait for: 88 -> 45 us for 128 chunks. Where blocks are many the workspace's bytes count: every block of columns reads its
-// head's operands. HGRN2's u is split here, out of the values, by the warps of the sums, two chunks ahead; with its parts in the
-// workspace 32 portions of 100 tokens over 16 heads of 128 x 128 took 260 us with chunk_vectors (multiply-adds 239), now 197; 16 portions of
-// 1,000 tokens 1,119 (1,026), now 810, with heads of 64 rows 666 (640), now 609.
+// All numbers stay 32-bit: a product's operand enters as three bfloat16 numbers, the product as the six products of parts above 2^-24 of
+// it (product3); sums over more than 16 terms are 32-bit additions. An infinite entry of S makes its column's later results NaN.
+// Bound by the chain of a chunk, 0.95 us: products (24 of mma.sync a scheduler, 9 cycles each), the meeting of the warps, u's sums, u
+// back to all of them, 64 multiply-adds of pairs a thread with their loads. With multiply-adds on S in shared memory for both products
+// the walk took 166 us for 2,048 tokens and 16 heads of 128 x 128, bound by shared memory's bandwidth; this form 121 (105 with both on
+// the tensor cores, see the errors above). What that took: no mbarrier on the chain, loads ahead of the waits, read-outs and
+// sums on warps of their own. HGRN2 with heads of 64 x 64, which has no u to wait for: 88 -> 49 us for 128 chunks. Where blocks are many
+// the workspace's bytes count: every block of columns reads its head's operands. HGRN2's values are fetched here, by the warps of the
+// sums, two chunks ahead. Vectors and walk of 32 portions of 100 tokens over 16 heads of 128 x 128: delta rule 387 us (multiply-adds 463),
+// HGRN2 202 (239); 16 portions of 1,000 tokens 1,479 (1,698) and 888 (1,026); heads of 64 x 64, 6 portions of 351 tokens, 77 (81) and 51 (53).
 template <int DIM, bool DELTA>
 __global__ void __launch_bounds__(Walk<DIM, DELTA>::THREADS, DIM == 128 && DELTA ? 1 : 2)
 chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long long slot_stride, int n_slots, const ChunkArgs a,
@@ -391,8 +376,7 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     float* part = sm + a.stages * L::STAGE;      // [3][WARPS][CT * CB]: read-outs of even and of odd chunks, u
     float* u_part = part + 2 * W::PART;
     uint32_t* frags = reinterpret_cast<uint32_t*>(part + 3 * W::PART);        // [2][WARPS] S before even and before odd chunks
-    // u as a left operand (HGRN2: of even and of odd chunks)
-    uint32_t* ufrag = DELTA ? frags + 2 * WARPS * L::OPERAND : reinterpret_cast<uint32_t*>(part + 2 * W::PART);
+    float* u_cols = DELTA ? reinterpret_cast<float*>(frags + 2 * WARPS * L::OPERAND) : part + 2 * W::PART;        // [US][CB][UP]
     __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES];
     __shared__ int abort_flag_;
     volatile int* abort_flag = &abort_flag_;
@@ -422,7 +406,7 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     int at = 0;                                  // the chunk's stage
     uint32_t lap = 0;
     auto next = [&]() { if (++at == a.stages) at = 0, ++lap; };
-    // the products' right operands over the warp's channels: -W (delta rule), Q, k E
+    // the products' right operands over the warp's channels: -W (delta rule), Q
     auto right_operands = [&](Cols3& x, int kind) {
         const float* from = sm + at * L::STAGE + (size_t)(warp * L::KINDS + kind) * L::OPERAND + lane * 4;
 #pragma unroll
@@ -438,13 +422,13 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
             x.r[p][0] = y.x, x.r[p][1] = y.y, x.r[p][2] = y.z, x.r[p][3] = y.w;
         }
     };
-    float most[2][4], rest[2][4];
+    float y[2][4];
     // a warp's product into its place among the warps'
     auto put = [&](float* p) {
         p += warp * (CT * CB) + lane * 4;
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-            *reinterpret_cast<float4*>(p + 128 * j) = make_float4(rest[j][0] + most[j][0], rest[j][1] + most[j][1], rest[j][2] + most[j][2], rest[j][3] + most[j][3]);
+            *reinterpret_cast<float4*>(p + 128 * j) = make_float4(y[j][0], y[j][1], y[j][2], y[j][3]);
     };
     // Once a chunk all but the copying warp meet: from then on the next chunk is there, S before this one and every warp's share of -W S
     // can be read, and so can the shares of read-outs (of the last chunk; HGRN2: of this one); the last chunk's stage is free. The state's warps of the delta rule only
@@ -503,8 +487,6 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
             if (ok && left > 1) o[o_ld] = x.y;
             o += CT * o_ld, left -= CT;
         };
-        // u's pair among the left operand's registers: tokens 4 t .. 4 t + 3 of a column are lane t's registers half and half + 2
-        uint32_t* to = ufrag + ((l & 28) + 2 * j + ((l & 3) >> 1)) * 4 + half + 2 * (l & 1);
         float2 u0 = make_float2(0.f, 0.f), o0 = u0;
         // HGRN2: u is the values, which are fetched two chunks ahead
         const float* v = a.v + (size_t)(start + c0 * CT + token) * a.ld_v + (size_t)h * a.vd + col0 + col;
@@ -513,10 +495,7 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
             const int n = left - ahead * CT;
             return make_float2(n > 0 ? p[0] : 0.f, n > 1 ? p[a.ld_v] : 0.f);
         };
-        auto place = [&](int c, float2 x) {
-            uint32_t* dst = to + (DELTA ? 0 : (c & 1) * L::OPERAND);
-            split3(dst[0], dst[128], dst[256], x.x, x.y);
-        };
+        auto place = [&](int c, float2 x) { *reinterpret_cast<float2*>(u_cols + (c % W::US * CB + col) * W::UP + token) = x; };
         float2 v1 = u0, v2 = u0;
         if constexpr (!DELTA) {
             const float2 v0 = values(0);
@@ -552,14 +531,14 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     Cols3 w;
     if (DELTA && tid >= WARPS * 32) {                             // ------------------------------------------------ read-outs
         meet();
-        right_operands(w, L::KINDS - 2);
+        right_operands(w, L::KINDS - 1);
         for (int c = 0; c < n_chunks; ++c) {
             meet();
             Rows3 s;
             left_operand(s, frags + ((c & 1) * WARPS + warp) * L::OPERAND);
-            product3<false>(most, rest, s, w);
+            product3(y, s, w);
             next();
-            if (c + 1 < n_chunks) right_operands(w, L::KINDS - 2);
+            if (c + 1 < n_chunks) right_operands(w, L::KINDS - 1);
             put(part + (c & 1) * W::PART);
         }
         meet();
@@ -589,21 +568,13 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
             for (int c = 0; c < 2; ++c) split3(s.r[0][2 * j + c], s.r[1][2 * j + c], s.r[2][2 * j + c], S[j][2 * c], S[j][2 * c + 1]);
     };
     split_state();
-    Cols3 k;
-    Rows3 u;
-    float4 e;
-    // u^T (k E), with S's own decays
-    auto chunk_operands = [&]() {
-        right_operands(k, L::KINDS - 1);
-        e = *reinterpret_cast<const float4*>(sm + at * L::STAGE + L::DECAY + row);
-    };
     meet();
     right_operands(w, 0);
-    if constexpr (!DELTA) chunk_operands();
     for (int c = 0; c < n_chunks; ++c) {
-        // (loads stand where they run beside products, not beside the sums' loads, which everything waits for)
-        if constexpr (DELTA) chunk_operands();
-        product3<false>(most, rest, s, w);
+        product3(y, s, w);
+        const float* stage = sm + at * L::STAGE;
+        next();
+        const float4 e = *reinterpret_cast<const float4*>(stage + L::DECAY + row);
         if constexpr (DELTA) {
 #pragma unroll
             for (int p = 0; p < 3; ++p)
@@ -611,29 +582,28 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
                     make_uint4(s.r[p][0], s.r[p][1], s.r[p][2], s.r[p][3]);
             put(u_part);
             meet_later();
-            wait_u();
-            left_operand(u, ufrag);
         } else {
-            left_operand(u, ufrag + (c & 1) * L::OPERAND);
             put(part + (c & 1) * W::PART);
         }
-        product3<true>(most, rest, u, k);
-        const float4 f = e;
-        next();
-        if constexpr (DELTA) {
-            if (c + 1 < n_chunks) right_operands(w, 0);
-        } else {
-            meet();
-            if (c + 1 < n_chunks) {
-                right_operands(w, 0);
-                chunk_operands();
-            }
-        }
-        // one rounding where the chunk's tokens prevail, two where the state does
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            S[0][i] = fmaf(i & 1 ? f.y : f.x, S[0][i], rest[0][i]) + most[0][i];
-            S[1][i] = fmaf(i & 1 ? f.w : f.z, S[1][i], rest[1][i]) + most[1][i];
+        for (int i = 0; i < 4; ++i) S[0][i] *= i & 1 ? e.y : e.x, S[1][i] *= i & 1 ? e.w : e.z;
+        float4 first[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) first[t] = *reinterpret_cast<const float4*>(stage + L::KE + t * DIM + row);
+        if constexpr (DELTA) wait_u(); else meet();
+        // S <- diag(E) S + (k E)^T u, token after token in 32 bits
+        const float* us = u_cols + (c % W::US * CB + g) * W::UP;
+        if (c + 1 < n_chunks) right_operands(w, 0);          // (beside the multiply-adds)
+#pragma unroll
+        for (int t = 0; t < CT; t += 4) {
+            const float4 ua = *reinterpret_cast<const float4*>(us + t), ub = *reinterpret_cast<const float4*>(us + 8 * W::UP + t);
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+                const float4 k = t == 0 ? first[d] : *reinterpret_cast<const float4*>(stage + L::KE + (t + d) * DIM + row);
+                const float a0 = d == 0 ? ua.x : d == 1 ? ua.y : d == 2 ? ua.z : ua.w, a1 = d == 0 ? ub.x : d == 1 ? ub.y : d == 2 ? ub.z : ub.w;
+                fma2(S[0][0], S[0][1], k.x, k.y, a0), fma2(S[0][2], S[0][3], k.x, k.y, a1);
+                fma2(S[1][0], S[1][1], k.z, k.w, a0), fma2(S[1][2], S[1][3], k.z, k.w, a1);
+            }
         }
         split_state();
     }

@@ -539,6 +539,40 @@ def test_recurrences_in_chunks(kind, heads, kvh, dim, vd, decays):
     assert errors[True] <= 2 * errors[False] + 2.0 ** -23, errors
 
 
+@pytest.mark.parametrize("dim", [64, 100, 128])
+@pytest.mark.parametrize("low,high", [(0.0, 0.1), (0.2, 0.6), (0.0, 1.0), (0.95, 1.0)])
+def test_chunks_move_the_state_as_exactly_as_multiply_adds(dim, low, high):
+    """HGRN2's state against 64 bits: no further off than the same sums by 32-bit multiply-adds, token after token in chunks of 16 (each
+    formed in 64 bits and rounded once, which is a fused multiply-add but for its rarest ties: 1 %), whichever tokens prevail."""
+    from cellm_b200 import ops
+    heads, vd, lens = 4, 48, [16 * 6 + 5, 16 * 7, 97]
+    g = torch.Generator().manual_seed(dim + int(100 * low))
+    T, zero = sum(lens), torch.zeros(heads * dim, device=DEV)
+    f = low + (high - low) * torch.rand(T, heads * dim, generator=g, dtype=torch.float64)
+    proj = torch.cat([torch.randn(T, heads * dim, generator=g), torch.logit(f.clamp(1e-6, 1 - 1e-6)).float(), torch.randn(T, heads * vd, generator=g)], 1).to(DEV)
+    state = torch.randn(len(lens), heads, dim, vd, generator=g).to(DEV)
+    exact, steps = state.double(), state.double()
+    ctx = step_ctx(lens, [0] * len(lens), list(range(len(lens))))
+    ops.hgrn2_scan(proj, 0, heads * dim, 2 * heads * dim, zero, zero, state, ctx, heads, dim, vd, chunked=True)
+    assert int(ctx.err.item()) == 0
+    at = 0
+    for b, n in enumerate(lens):
+        f = proj[at:at + n, heads * dim:2 * heads * dim].reshape(n, heads, dim)         # as the gates' kernel left them
+        v = proj[at:at + n, 2 * heads * dim:].double().reshape(n, heads, 1, vd)
+        at += n
+        for t in range(n):
+            exact[b] = exact[b] * f[t].double()[..., None] + (1 - f[t].double())[..., None] * v[t]
+        for c in range(0, n, 16):
+            e, ke = torch.ones_like(f[0]), []
+            for t in reversed(range(c, min(c + 16, n))):
+                ke.insert(0, (1 - f[t]) * e)
+                e = e * f[t]
+            steps[b] = (steps[b] * e.double()[..., None]).float().double()
+            for t, k in enumerate(ke):
+                steps[b] = (steps[b] + k.double()[..., None] * v[c + t]).float().double()
+    assert float((state.double() - exact).norm()) <= 1.01 * float((steps - exact).norm())
+
+
 @pytest.mark.parametrize("kind", ["delta", "hgrn2"])
 @pytest.mark.parametrize("held", [1, 4, 7, 100])
 def test_chunks_go_through_a_small_workspace_in_runs(monkeypatch, kind, held):
