@@ -29,7 +29,7 @@
 // (5.0e-8). HGRN2 1.06e-7 (1.09e-7), 7.8e-8 (7.8e-8); 6.4e-7 (6.4e-7), 1.0e-6 (1.0e-6); 9.1e-8 (9.1e-8), 4.3e-8 (4.3e-8). (With S moved
 // by products in parts as well its error was smaller where decays are near 1 and up to 15 % larger where a chunk's last tokens prevail:
 // the tensor cores cut the small terms of a sum.)
-// One prompt of 2,048 tokens, 16 heads of 128 x 128: token by token 938 us, in chunks with multiply-adds 214, now 176 (55 of them
+// One prompt of 2,048 tokens, 16 heads of 128 x 128: token by token 938 us, in chunks with multiply-adds 214, now 178 (55 of them
 // chunk_vectors, which forms the parts).
 #include <algorithm>
 #include <climits>
@@ -65,20 +65,34 @@ template <int DIM, bool DELTA> struct Layout {
     static constexpr int STAGE = ROWS + COLS;
 };
 
-// A pair of 32-bit numbers as three pairs of bfloat16 numbers whose sums they are (8 bits each; what is left of 24 is below 2^-26).
+// A pair of 32-bit numbers as three pairs of bfloat16 numbers whose sums they are (8 bits each, all 24; of numbers below 2^-109 the parts'
+// smallest step takes the last). No product of an infinite number's parts is finite, nor of those of a number that bfloat16 rounds to
+// infinity. FINITE: the first part stays finite, so that whole_of finds such numbers again (infinity is (the largest, infinity, NaN)); that
+// takes more instructions, which the walk's chain has no room for.
 __device__ __forceinline__ uint64_t minus_parts(uint64_t x, uint32_t part) {
     const uint64_t y = (uint64_t)(part & 0xffff0000u) << 32 | (part << 16);
     uint64_t d;
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
     return d;
 }
+__device__ __forceinline__ uint32_t pack_pair_finite(uint64_t x) {
+    uint32_t y;
+    asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(y) : "f"(__uint_as_float((uint32_t)(x >> 32))), "f"(__uint_as_float((uint32_t)x)));
+    return y;
+}
 __device__ __forceinline__ uint32_t pack_pair(uint64_t x) { return pack_bf16(__uint_as_float((uint32_t)x), __uint_as_float((uint32_t)(x >> 32))); }
-__device__ __forceinline__ void split3(uint32_t& hi, uint32_t& mid, uint32_t& low, float x, float y) {
+template <bool FINITE> __device__ __forceinline__ void split3(uint32_t& hi, uint32_t& mid, uint32_t& low, float x, float y) {
     uint64_t pair = (uint64_t)__float_as_uint(y) << 32 | __float_as_uint(x);
-    hi = pack_pair(pair);
+    hi = FINITE ? pack_pair_finite(pair) : pack_pair(pair);
     pair = minus_parts(pair, hi);
     mid = pack_pair(pair);
     low = pack_pair(minus_parts(pair, mid));
+}
+// The number again, of the pair's first (which = 0) or second.
+__device__ __forceinline__ float whole_of(uint32_t hi, uint32_t mid, uint32_t low, int which) {
+    auto part = [&](uint32_t x) { return __uint_as_float(which ? x & 0xffff0000u : x << 16); };
+    const float m = part(mid), sum = part(hi) + m;
+    return fabsf(m) < INFINITY ? sum + part(low) : sum;
 }
 // Chunks of portion b, 0 where it is short; where a warp looks through the portions, a lane takes one of 32 (one after the other they
 // cost a block 0.3 us each).
@@ -251,7 +265,7 @@ chunk_vectors_kernel(const ChunkArgs a) {
             for (int t = 0; t < 8; ++t) {
                 const float other = __shfl_xor_sync(0xffffffffu, odd ? x[t] : x[t + 8], 1);
                 uint32_t part[3];
-                split3(part[0], part[1], part[2], odd ? other : x[t], odd ? x[t + 8] : other);
+                split3<true>(part[0], part[1], part[2], odd ? other : x[t], odd ? x[t + 8] : other);
 #pragma unroll
                 for (int p = 0; p < 3; ++p) out[p * 128 + t * 16] = part[p];
             }
@@ -347,6 +361,55 @@ template <int DIM, bool DELTA> struct Walk {
     static constexpr int SMEM_FLOATS = (DELTA ? 3 * PART + 2 * WARPS * 3 * 32 * 4 : 2 * PART) + US * CB * UP;
 };
 
+// What a block of the walk below does, by multiply-adds from the numbers the workspace's parts stand for: for blocks where a product of
+// parts is not finite (an infinite operand's parts leave none, nor do those of the largest finite ones), once they have found that. The
+// warps that meet take part; sm: DIM (CB + 1) + CT CB floats of shared memory; ws, o, v: of the first chunk; left: the portion's tokens
+// from there on.
+template <int DIM, bool DELTA>
+__device__ __forceinline__ void walk_whole(float* sm, const float* ws, long long chunk_stride, int blk, float* st, int dim, int vd, float* o,
+                                        long long o_ld, const float* v, long long ld_v, int left, int n_chunks) {
+    using L = Layout<DIM, DELTA>;
+    using W = Walk<DIM, DELTA>;
+    auto meet = []() { asm volatile("bar.sync 1, %0;" ::"n"(W::MEET) : "memory"); };
+    float *S = sm, *u = sm + DIM * (CB + 1);     // [DIM][CB + 1], [CT][CB]
+    const int tid = threadIdx.x, col0 = blk * CB;
+    for (int i = tid; i < DIM * CB; i += W::MEET) {
+        const int r = i / CB, c = i % CB;
+        S[r * (CB + 1) + c] = r < dim && col0 + c < vd ? st[(size_t)r * vd + col0 + c] : 0.f;
+    }
+    for (int n = 0; n < n_chunks; ++n, ws += chunk_stride, o += CT * o_ld, v += CT * ld_v, left -= CT) {
+        meet();
+        const float* uo = ws + L::ROWS + (size_t)blk * L::COLS;
+        for (int i = tid; i < CT * CB; i += W::MEET) {
+            const int t = i / CB, c = i % CB;
+            const bool on = t < left && col0 + c < vd;
+            auto times_S = [&](int kind) {       // row t of the right operands of this kind
+                float sum = 0.f;
+                for (int r = 0; r < DIM; ++r) {
+                    const uint32_t* x = reinterpret_cast<const uint32_t*>(ws) + ((r >> 4) * L::KINDS + kind) * L::OPERAND +
+                                        ((t & 7) * 4 + ((r >> 2) & 3)) * 4 + (t >> 3) * 2 + ((r >> 1) & 1);
+                    sum = fmaf(whole_of(x[0], x[128], x[256], r & 1), S[r * (CB + 1) + c], sum);
+                }
+                return sum;
+            };
+            u[i] = DELTA ? uo[c * CT + t] + times_S(0) : on ? v[(long long)t * ld_v + c] : 0.f;
+            const float y = uo[L::O0 + c * CT + t] + times_S(L::KINDS - 1);
+            if (on) o[(long long)t * o_ld + c] = y;
+        }
+        meet();
+        for (int i = tid; i < DIM * CB; i += W::MEET) {
+            const int r = i / CB, c = i % CB;
+            float x = S[r * (CB + 1) + c] * ws[L::DECAY + r];
+            for (int t = 0; t < CT; ++t) x = fmaf(ws[L::KE + t * DIM + r], u[t * CB + c], x);
+            S[r * (CB + 1) + c] = x;
+        }
+    }
+    for (int i = tid; i < DIM * CB; i += W::MEET) {          // (the thread's own)
+        const int r = i / CB, c = i % CB;
+        if (r < dim && col0 + c < vd) st[(size_t)r * vd + col0 + c] = S[r * (CB + 1) + c];
+    }
+}
+
 // A block carries CB columns of one (request, head)'s S through the request's chunks that are in the workspace; 16 columns make 128
 // blocks of a prompt over 16 heads of 128 columns, which is nearly the GPU. Its warps by their work:
 //   WARPS   hold 16 channels by 16 columns of S^T each, in the places of a left operand of mma.sync m16n8k16: S^T [-W]^T over their
@@ -356,15 +419,16 @@ template <int DIM, bool DELTA> struct Walk {
 //   SUMS    add the warps' sums, in a fixed order, with U0 or O0 on top: u goes back by columns, o to memory
 //   1       copies the chunks ahead of them all
 // All numbers stay 32-bit: a product's operand enters as three bfloat16 numbers, the product as the six products of parts above 2^-24 of
-// it (product3); sums over more than 16 terms are 32-bit additions. An infinite entry of S makes its column's later results NaN.
+// it (product3); sums over more than 16 terms are 32-bit additions. A block that has found a u or a read-out that is not finite starts again
+// (walk_whole).
 // Bound by the chain of a chunk, 0.95 us: products (24 of mma.sync a scheduler, 9 cycles each), the meeting of the warps, u's sums, u
 // back to all of them, 64 multiply-adds of pairs a thread with their loads. With multiply-adds on S in shared memory for both products
 // the walk took 166 us for 2,048 tokens and 16 heads of 128 x 128, bound by shared memory's bandwidth; this form 121 (105 with both on
 // the tensor cores, see the errors above). What that took: no mbarrier on the chain, loads ahead of the waits, read-outs and
 // sums on warps of their own. HGRN2 with heads of 64 x 64, which has no u to wait for: 88 -> 49 us for 128 chunks. Where blocks are many
 // the workspace's bytes count: every block of columns reads its head's operands. HGRN2's values are fetched here, by the warps of the
-// sums, two chunks ahead. Vectors and walk of 32 portions of 100 tokens over 16 heads of 128 x 128: delta rule 387 us (multiply-adds 463),
-// HGRN2 202 (239); 16 portions of 1,000 tokens 1,479 (1,698) and 888 (1,026); heads of 64 x 64, 6 portions of 351 tokens, 77 (81) and 51 (53).
+// sums, two chunks ahead. Vectors and walk of 32 portions of 100 tokens over 16 heads of 128 x 128: delta rule 398 us (multiply-adds 463),
+// HGRN2 205 (239); 16 portions of 1,000 tokens 1,505 (1,699) and 906 (1,026); heads of 64 x 64, 6 portions of 351 tokens, 75 (81) and 45 (53).
 template <int DIM, bool DELTA>
 __global__ void __launch_bounds__(Walk<DIM, DELTA>::THREADS, DIM == 128 && DELTA ? 1 : 2)
 chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long long slot_stride, int n_slots, const ChunkArgs a,
@@ -378,15 +442,15 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     uint32_t* frags = reinterpret_cast<uint32_t*>(part + 3 * W::PART);        // [2][WARPS] S before even and before odd chunks
     float* u_cols = DELTA ? reinterpret_cast<float*>(frags + 2 * WARPS * L::OPERAND) : part + 2 * W::PART;        // [US][CB][UP]
     __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES];
-    __shared__ int abort_flag_;
-    volatile int* abort_flag = &abort_flag_;
+    __shared__ int abort_flag_, again_;
+    volatile int *abort_flag = &abort_flag_, *again = &again_;
     // the column blocks of a head, its request's heads, the requests: neighbours run through the same chunks at the same time (with
     // the requests' blocks in turn, two prompts of unequal lengths took 326 us through both mixers instead of 295)
     const int blocks = (a.vd + CB - 1) / CB, blk = blockIdx.x % blocks, h = blockIdx.x / blocks % a.heads, b = blockIdx.x / blocks / a.heads;
     const int tid = threadIdx.x, lane = tid & 31;
     if (tid == 0) {
         for (int i = 0; i < a.stages; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
-        abort_flag_ = 0;
+        abort_flag_ = again_ = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     pdl_trigger();
@@ -438,6 +502,7 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
     auto meet_later = []() { asm volatile("bar.arrive 1, %0;" ::"n"(W::MEET) : "memory"); };
     auto u_whole = []() { asm volatile("bar.arrive 2, %0;" ::"n"((WARPS + SUMS) * 32) : "memory"); };
     auto wait_u = []() { asm volatile("bar.sync 2, %0;" ::"n"((WARPS + SUMS) * 32) : "memory"); };
+    float* st = state + (size_t)slot * slot_stride + (size_t)h * a.dim * a.vd;
     if (tid >= W::MEET) {        // ------------------------------------------------ copies
         if (lane != 0) return;
         const float* ws = a.ws + ((size_t)(before + c0 - a.chunk0) * a.heads + h) * a.stride;
@@ -457,6 +522,7 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
         for (int c = max(0, issued - a.stages); c < issued; ++c) mbar_wait(&full[c % a.stages], (uint32_t)(c / a.stages) & 1u, &none);
         return;
     }
+    do {                                         // (one of three)
     if (tid >= (WARPS + W::READ) * 32) {                             // ------------------------------------------------ sums over the warps
         // a thread: one column of two neighbouring tokens, registers 2 half and 2 half + 1 of lane l's accumulator j
         const int r = tid - (WARPS + W::READ) * 32, l = (r >> 1) & 31, half = r & 1, j = r >> 6;
@@ -471,7 +537,8 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
                 for (int w = 0; w < n; ++w) y[w].x += y[w + n].x, y[w].y += y[w + n].y;
             return make_float2(x.x + y[0].x, x.y + y[0].y);
         };
-        bool ok = true;
+        bool ok = true, finite = true;
+        auto look = [&](float2 x) { finite = finite && fabsf(x.x + x.y) < INFINITY; };
         auto there = [&]() {
             if (mbar_wait(&full[at], lap & 1u, abort_flag)) return;
             ok = false;                          // bounded: every warp still runs through its chunks, and nothing is written
@@ -483,6 +550,7 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
         int left = col0 + col < a.vd ? len - c0 * CT - token : 0;        // tokens from the thread's first on
         auto read_out = [&](int c, float2 x) {
             x = add_up(part + (c & 1) * W::PART, x);
+            look(x);
             if (ok && left > 0) *o = x.x;
             if (ok && left > 1) o[o_ld] = x.y;
             o += CT * o_ld, left -= CT;
@@ -515,8 +583,10 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
             if (c + 1 < n_chunks) there();
             meet();
             if constexpr (DELTA) {
-                place(c, add_up(u_part, u0));
+                const float2 x = add_up(u_part, u0);
+                place(c, x);
                 u_whole();
+                look(x);
             }
             if (c > 0 && r == 0) mbar_arrive(&empty[last]);
             // the delta rule's read-outs are formed while u's sums are: they are there a chunk later
@@ -526,7 +596,9 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
         }
         meet();
         if constexpr (DELTA) read_out(n_chunks - 1, o0);
-        return;
+        if (!finite) *again = 1;
+        meet();
+        break;
     }
     Cols3 w;
     if (DELTA && tid >= WARPS * 32) {                             // ------------------------------------------------ read-outs
@@ -542,12 +614,12 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
             put(part + (c & 1) * W::PART);
         }
         meet();
-        return;
+        meet();
+        break;
     }
     // -------------------------------------------------------------------------------------------- the state
     // the lane's entries of S: accumulator j's register 2 c + e is channel row + 2 j + e, column g + 8 c of the block
     const int row = warp * 16 + t4 * 4;
-    float* st = state + (size_t)slot * slot_stride + (size_t)h * a.dim * a.vd;
     auto entry = [&](int j, int i) -> float* {
         const int r = row + 2 * j + (i & 1), c = col0 + g + 8 * (i >> 1);
         return (r < a.dim && c < a.vd) ? st + (size_t)r * a.vd + c : nullptr;
@@ -565,7 +637,7 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int c = 0; c < 2; ++c) split3(s.r[0][2 * j + c], s.r[1][2 * j + c], s.r[2][2 * j + c], S[j][2 * c], S[j][2 * c + 1]);
+            for (int c = 0; c < 2; ++c) split3<false>(s.r[0][2 * j + c], s.r[1][2 * j + c], s.r[2][2 * j + c], S[j][2 * c], S[j][2 * c + 1]);
     };
     split_state();
     meet();
@@ -608,12 +680,20 @@ chunk_walk_kernel(float* __restrict__ o_out, float* __restrict__ state, long lon
         split_state();
     }
     meet();
-    if (*abort_flag) return;     // the copies gave up: the state stays as it was
+    meet();
+    if (*again || *abort_flag) break;            // (the copies gave up: the state stays as it was)
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (float* p = entry(j, i)) *p = S[j][i];
+    } while (false);
+    // behind the second of the two last meetings: whether something was not finite
+    if (!*again || *abort_flag) return;
+    const size_t first = (size_t)start + (size_t)c0 * CT, at_col = (size_t)h * a.vd + col0;
+    walk_whole<DIM, DELTA>(sm, a.ws + ((size_t)(before + c0 - a.chunk0) * a.heads + h) * a.stride, (long long)a.heads * a.stride, blk, st, a.dim, a.vd,
+                           o_out + first * a.heads * a.vd + at_col, (long long)a.heads * a.vd, DELTA ? nullptr : a.v + first * a.ld_v + at_col, a.ld_v,
+                           len - c0 * CT, n_chunks);
 }
 
 template <int DIM, bool DELTA> int floats_a_chunk(int vd) {

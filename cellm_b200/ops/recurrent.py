@@ -211,7 +211,7 @@ def attention_flash_masked(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: i
 
 # Portions of this many tokens and more run the recurrences with a decay per channel in chunks (heads of up to 128
 # rows). One portion, 16 heads, token by token against in chunks: the delta rule with states of 128 x 128 32 against 21 us
-# at 64 tokens, 25 against 21 at 48, 12 against 20 at 24 (two kernels in place of one); 938 against 176 at 2,048. HGRN2 with
+# at 64 tokens, 25 against 21 at 48, 12 against 20 at 24 (two kernels in place of one); 938 against 178 at 2,048. HGRN2 with
 # 64 x 128 15 against 27 us at 64 tokens, 45 against 23 at 128; 627 against 89 at 2,048.
 DELTA_CHUNKS_FROM, HGRN2_CHUNKS_FROM = 48, 96
 _STATE_CHUNK = 16           # tokens a chunk of state_chunks.cu

@@ -574,6 +574,44 @@ def test_chunks_move_the_state_as_exactly_as_multiply_adds(dim, low, high):
 
 
 @pytest.mark.parametrize("kind", ["delta", "hgrn2"])
+@pytest.mark.parametrize("dim", [64, 112])
+def test_chunks_of_states_with_infinities_and_the_largest_numbers(kind, dim):
+    """States with infinite entries, entries that bfloat16 would round to infinity and one that is no number, against the walk
+    token by token: infinite where that is (the delta rule's column then is no number in either form), and the other columns as ever."""
+    from cellm_b200 import ops
+    heads, vd, n, g = 2, 40, 100, torch.Generator().manual_seed(dim)
+    unit = lambda: torch.nn.functional.normalize(torch.randn(n, heads, dim, generator=g), dim=-1).reshape(n, -1)
+    S0 = torch.randn(1, heads, dim, vd, generator=g)
+    S0[0, 0, 3, 5], S0[0, 0, 60, 17], S0[0, 1, 40, 1], S0[0, 1, 41, 1] = math.inf, -math.inf, math.inf, -math.inf
+    S0[0, 0, 7, 8], S0[0, 1, 33, 20], S0[0, 1, 1, 39] = 3.4e38, -3.4e38, math.nan
+    qk, v = torch.cat([unit(), unit()], 1).to(DEV).contiguous(), torch.randn(n, heads * vd, generator=g).to(DEV)
+    beta, decay = torch.rand(n, heads, generator=g).to(DEV), (0.8 + 0.2 * torch.rand(n, heads * dim, generator=g)).to(DEV)
+    proj = torch.cat([qk[:, :heads * dim], 1 + torch.rand(n, heads * dim, generator=g).to(DEV), v], 1).contiguous()
+    zero, ctx, got = torch.zeros(heads * dim, device=DEV), step_ctx([n], [0], [0]), []
+    for chunked in (False, True):
+        state = S0.to(DEV).clone()
+        if kind == "delta":
+            o = ops.delta_scan(qk, v, beta, decay, state, ctx, heads, heads, dim, vd, chunked=chunked)
+        else:
+            o = ops.hgrn2_scan(proj.clone(), 0, heads * dim, 2 * heads * dim, zero, zero, state, ctx, heads, dim, vd, chunked=chunked)
+        got.append((o.view(n, heads, vd).transpose(0, 1).cpu(), state[0].cpu()))
+    assert int(ctx.err.item()) == 0
+    off = torch.zeros(heads, vd, dtype=torch.bool)
+    for h, c in ((0, 5), (0, 17), (1, 1), (1, 39)):
+        off[h, c] = True
+    for a, b in zip(*got):          # [heads, rows, vd]
+        for h in range(heads):
+            for c in range(vd):
+                x, y = a[h, :, c], b[h, :, c]
+                if off[h, c] and kind == "delta":
+                    assert not x.isfinite().any() and not y.isfinite().any()
+                    continue
+                assert off[h, c] or x.isfinite().all()
+                finite = x[x.isfinite()].abs()
+                torch.testing.assert_close(y, x, rtol=2e-5, atol=2e-5 * float(finite.max()) if finite.numel() else 0.0, equal_nan=True)
+
+
+@pytest.mark.parametrize("kind", ["delta", "hgrn2"])
 @pytest.mark.parametrize("held", [1, 4, 7, 100])
 def test_chunks_go_through_a_small_workspace_in_runs(monkeypatch, kind, held):
     """Runs that end inside a request, at its end and behind several, of one chunk and of all: the same bits, states and read-outs."""
