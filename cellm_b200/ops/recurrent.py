@@ -137,19 +137,21 @@ def attention_plain_masked(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: i
 
 
 # Pieces of keys of the tensor-core attention below, of at least two blocks of 64 keys. Tiles of 64 rows (four warps) are cut only
-# where a step's tiles are few. Those of 16 rows are single warps that walk their keys alone, six of which an SM holds: what counts
-# is the blocks of keys a warp walks, and one more to begin with, times the rounds of 888 such warps, and the merge (8 kv heads, window
-# 1,024, both mixers of a layer: 8 requests 72 us in 4 pieces, 61 in 9; 16 95 in 2, 68 in 6, 76 in 9; 32 153 whole, 102 in 3; 64
-# 177 whole, 160 in 3).
-PIECES_FILL, PIECES_FILL_NARROW = 296, 888
+# where a step's tiles are few. Those of 16 rows are single warps that walk their keys alone; their queries and two stages of keys and
+# values take 544 bytes an entry of a head, so an SM holds twelve of them with heads of 32, six of 64, four of 96, three of 128. What counts is the
+# blocks of keys a warp walks, and one more to begin with, times the rounds of as many warps as the SMs hold, and the merge.
+# The attention alone behind a window of 1,024, 8 kv heads, uncut and cut: heads of 32, 16 requests 28 us in 2 pieces, 12 in 9; 32 39 whole, 17 in 6;
+# heads of 64, 8 requests 27 in 4, 15 in 9; 32 81 whole, 35 in 3; heads of 128, 8 requests 55 in 4, 39 in 6 (58 in 9: a second round); 48 178 whole, 182 in 2.
+PIECES_FILL = 296
 
 
-def _pieces(span: int, tiles: int, wide: bool) -> int:
+def _pieces(span: int, tiles: int, wide: bool, hd: int = 64) -> int:
     tiles, most = max(1, tiles), min(-(-span // 128), 32)
     if wide:
         return max(1, min(most, PIECES_FILL // tiles))
-    cost = lambda n: -(-tiles * n // PIECES_FILL_NARROW) * (-(-span // (64 * n)) + 1) + (1.5 if n > 1 else 0)
-    return min((max(1, min(most, rounds * PIECES_FILL_NARROW // tiles)) for rounds in (0, 1, 2)), key=cost)
+    fill = 148 * (228 * 1024 // ((16 + 4 * 64) * hd * 2 + 1024))
+    cost = lambda n: -(-tiles * n // fill) * (-(-span // (64 * n)) + 1) + (1.5 if n > 1 else 0)
+    return min((max(1, min(most, rounds * fill // tiles)) for rounds in (0, 1, 2)), key=cost)
 
 
 def attention_flash_sink(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: int, scale: float, window: int,
@@ -167,7 +169,7 @@ def attention_flash_sink(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: int
     n_tiles = sum(-(-n * G // rows) for n in ctx.q_lens)
     longest = ctx.max_total_len          # a captured step's bound: the width of its block tables
     span = min(longest, window + ctx.max_q_len) if window > 0 else longest
-    nsplit = _pieces(span, n_tiles * nkv, wide)
+    nsplit = _pieces(span, n_tiles * nkv, wide, hd)
     out = torch.empty((T, nh * hd), dtype=q.dtype, device=q.device)
     part_o = part_ml = None
     if nsplit > 1:
@@ -196,7 +198,7 @@ def attention_flash_masked(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: i
     n_tiles = sum(-(-n * G // rows) for n in ctx.q_lens)
     longest = ctx.max_total_len
     span = min(longest, window + keep_first + ctx.max_q_len) if window > 0 else longest
-    nsplit = _pieces(span, n_tiles * nkv, wide)
+    nsplit = _pieces(span, n_tiles * nkv, wide, hd)
     out = torch.empty((T, nh * hd), dtype=q.dtype, device=q.device)
     part_o = part_ml = None
     if nsplit > 1:
@@ -396,7 +398,7 @@ def attention_flash_chunked(q: torch.Tensor, cache, ctx, nh: int, nkv: int, hd: 
     n_tiles = sum(-(-n * G // rows) for n in ctx.q_lens)
     longest = ctx.max_total_len
     span = min(longest, chunk + ctx.max_q_len) if chunk > 0 else longest
-    nsplit = _pieces(span, n_tiles * nkv, wide)
+    nsplit = _pieces(span, n_tiles * nkv, wide, hd)
     out = torch.empty((T, nh * hd), dtype=q.dtype, device=q.device)
     part_o = part_ml = None
     if nsplit > 1:

@@ -234,3 +234,14 @@ def test_pieces_of_keys_where_an_attention_walks_them_alone(span, tiles, wide, p
     """Never more pieces than pairs of blocks of 64 keys, nor than 32; whole where the tiles fill the GPU anyway."""
     from cellm_b200.ops import recurrent
     assert recurrent._pieces(span, tiles, wide) == pieces
+
+
+@pytest.mark.parametrize("hd,held,cases", [(32, 12, {64: 9, 128: 9, 256: 6, 512: 3, 4000: 1}), (96, 4, {16: 9, 64: 9, 128: 4, 256: 2, 600: 1}),
+                                           (128, 3, {8: 9, 64: 6, 128: 3, 256: 3, 384: 1, 512: 1})])
+def test_pieces_of_keys_by_the_warps_an_sm_holds(hd, held, cases):
+    """Single-warp tiles of wider heads are fewer an SM: a step is cut into no more pieces than one round of them, or two, holds."""
+    from cellm_b200.ops import recurrent
+    for tiles, pieces in cases.items():
+        assert recurrent._pieces(1025, tiles, False, hd) == pieces
+        assert pieces == 1 or tiles * pieces <= 2 * 148 * held
+    assert recurrent._pieces(3000, 100, True, hd) == 2
