@@ -324,15 +324,16 @@ hgrn2_gates_kernel(float* __restrict__ proj, long long ld, int col_q, int col_f,
     }
 }
 
-// The same, a block a token, four columns a thread (everything on 16-byte borders): the same values. 1,775 tokens of 2 x 768 columns: 9.6 ->
-// 6.6 us; the other form divides a 64-bit index for every value.
+// The same, four columns a thread (everything on 16-byte borders), a block a token or, where the tokens are few, a part of one: the same
+// values. The other form divides a 64-bit index for every value: 2,048 tokens of 2 x 768 columns 10.3 -> 4.6 us, 96 of them 1.8 -> 1.7; 128
+// tokens of 2 x 2,048 columns 3.1 -> 2.0 (a block a token 3.5).
 __global__ void __launch_bounds__(256)
 hgrn2_gates_fours_kernel(float* __restrict__ proj, long long ld, int col_q, int col_f, const float* __restrict__ f_bias,
                          const float* __restrict__ lower, int n) {
     pdl_trigger();
     pdl_wait();
     float* row = proj + (size_t)blockIdx.x * ld;
-    for (int c = threadIdx.x * 4; c < 2 * n; c += blockDim.x * 4) {
+    for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4; c < 2 * n; c += gridDim.y * blockDim.x * 4) {
         if (c < n) {
             float4* at = reinterpret_cast<float4*>(row + col_q + c);
             const float4 x = *at;
@@ -403,7 +404,9 @@ CELLM_API int cellm_hgrn2_gates(float* proj, long long ld, int col_q, int col_f,
     const size_t total = (size_t)T * 2 * heads * dim;
     const int n = heads * dim;
     if (n % 4 == 0 && ld % 4 == 0 && col_q % 4 == 0 && col_f % 4 == 0 && aligned16(proj) && aligned16(f_bias) && aligned16(lower)) {
-        CELLM_RUN(hgrn2_gates_fours_kernel, T, std::min(256, (n / 4 + 31) / 32 * 32), 0, stream, proj, ld, col_q, col_f, f_bias, lower, n);
+        // as many parts as leave a thread one piece of four, while their blocks are resident at once (8 an SM)
+        const int threads = std::min(256, (n / 4 + 31) / 32 * 32), parts = std::min((n / 2 + threads - 1) / threads, std::max(1, 148 * 8 / T));
+        CELLM_RUN(hgrn2_gates_fours_kernel, dim3(T, parts), threads, 0, stream, proj, ld, col_q, col_f, f_bias, lower, n);
         return CELLM_OK;
     }
     CELLM_RUN(hgrn2_gates_kernel, (unsigned)std::min<size_t>((total + 255) / 256, 148 * 16), 256, 0, stream, proj, ld, col_q, col_f, f_bias,

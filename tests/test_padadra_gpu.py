@@ -894,7 +894,7 @@ def test_head_norms_by_fours_and_one_by_one(T, heads, vd, lead, act):
         torch.testing.assert_close(got.cpu().double().view(T, heads, vd), want, **tol)
 
 
-@pytest.mark.parametrize("T,heads,dim", [(1, 1, 4), (3, 5, 100), (7, 12, 64)])
+@pytest.mark.parametrize("T,heads,dim", [(1, 1, 4), (3, 5, 100), (7, 12, 64), (300, 32, 128), (1200, 2, 64)])
 def test_hgrn2_gates_by_fours_and_one_by_one(T, heads, dim):
     from cellm_b200.ops._lib import check, fn, ptr, stream_of
     n, g = heads * dim, torch.Generator().manual_seed(T * dim)
