@@ -51,6 +51,7 @@ gemm_runs_kernel(float* __restrict__ C, const float* __restrict__ A, const float
                  long long lda, long long ldw, long long ldc, int vec) {
     using T = RunTile<TM, TN, LY>;
     constexpr int BM = T::BM, BN = T::BN, GT = 8 * LY;
+    static_assert(BM % (GT / 4) == 0 && BN % (GT / 4) == 0, "a thread's copies are of whole tiles");
     static_assert(BM * BN <= 2 * T::STAGE, "a group's sums take the place of its stages");
     extern __shared__ __align__(16) float gp_smem[];
     const int groups = blockDim.x / GT, g = threadIdx.x / GT, tid = threadIdx.x % GT;
@@ -71,7 +72,6 @@ gemm_runs_kernel(float* __restrict__ C, const float* __restrict__ A, const float
             float* to = dst + r0 * GP_PITCH + kk;
 #pragma unroll
             for (int i = 0; i < BM; i += GT / 4) {
-                if (GT / 4 > BM && r0 >= BM) break;
                 const bool in = m0 + r0 + i < M && gk < K;
                 gp_copy(to + i * GP_PITCH, in ? a + (size_t)i * lda : A, 16, in);
             }
@@ -237,26 +237,37 @@ CELLM_API int cellm_gemm_plain(void* C, const void* A, const void* W, int M, int
     const long long few = M <= 16 ? 32 : vec ? (K / 4 < 32 ? K / 4 : 32) : 8;
     if (in_dtype == CELLM_F32 && out_dtype == CELLM_F32 && ((vec && K >= 2 * GP_RUN) || tiles64 <= few)) {
         const int n_runs = (K + GP_RUN - 1) / GP_RUN, rounds = (n_runs + 7) / 8, groups = (n_runs + rounds - 1) / rounds;
-        // The tile whose waves over the SMs take least. Microseconds of K = 1,536 measured for one tile an SM and for each
-        // wave of several: whole waves where a block fills an SM; the groups of one warp share it, so that their waves melt together (from
-        // four groups on, below which they are too few warps). 213 x 2,560 sums take 108 us in tiles of 64 x 64, 63 of 32 x 64, 77 of
-        // 32 x 32, 85 of 16 x 32, 64 and 63 of those by single warps; 261 x 2,560 111, 91, 95, 105, 92, 77; 16 x 1,536 55, 31, 20, 14,
-        // 21, 16; 2,048 x 2,048 (K 2,048) 468, 540, 657, 859, 519, 560.
-        struct Tile { int bm, bn; double alone, wave, first; };
-        static const Tile long_k[6] = {
-            {64, 64, 58., 52., 0.}, {32, 64, 32., 30., 0.}, {32, 32, 20.5, 19.3, 0.}, {16, 32, 14.3, 11.5, 0.}, {32, 32, 25., 14.3, 10.},
-            {16, 32, 16.5, 7.65, 5.}};
-        // (fewer groups: their own measured costs)
-        static const Tile short_k[4] = {{64, 64, 62.8, 60., 0.}, {32, 64, 34.4, 33., 0.}, {32, 32, 22.4, 21., 0.}, {16, 32, 18., 12., 0.}};
+        // The tile whose waves over the SMs take least: measured microseconds of one tile an SM (`alone`), else of each wave, behind
+        // `first` and no less than `least`; `step` waves start together (1: a block fills an SM; 2: two share it; 0: blocks so small
+        // that their waves melt together).
+        struct Tile { int bm, bn; double alone, wave, first, least; int step; };
+        // Five groups and more, K = 1,536. 213 x 2,560 sums take 108 us in tiles of 64 x 64, 63 of 32 x 64, 77 of 32 x 32, 85 of
+        // 16 x 32, 64 and 63 of those by single warps; 261 x 2,560 111, 91, 95, 105, 92, 77; 16 x 1,536 55, 31, 20, 14, 21, 16;
+        // 2,048 x 2,048 (K 2,048) 468, 540, 657, 859, 519, 560.
+        static const Tile long_k[6] = {{64, 64, 58., 52., 0., 0., 1}, {32, 64, 32., 30., 0., 0., 1}, {32, 32, 20.5, 19.3, 0., 0., 1},
+                                       {16, 32, 14.3, 11.5, 0., 0., 1}, {32, 32, 25., 14.3, 10., 33., 0}, {16, 32, 16.5, 7.65, 5., 33., 0}};
+        // Four, K = 1,024. 261 x 2,560: 74, 73, 68, 69, 58, 51 us; 400 x 1,536 74, 64, 66, 62, 57, 47; 64 x 2,560 44, 34, 25, 24, 31, 29;
+        // 700 x 2,560 113, 116, 139, 161, 114, 117; 2,048 x 1,536 214, 208, 244, 277, 196, 197.
+        static const Tile four[6] = {{64, 64, 44., 36., 0., 0., 1}, {32, 64, 26., 20.5, 0., 0., 1}, {32, 32, 18., 11.6, 12., 0., 0},
+                                     {16, 32, 14., 6.6, 8., 21., 0}, {32, 32, 23., 9.1, 9., 29., 0}, {16, 32, 13., 4.6, 8., 28., 0}};
+        // Three, K = 768. 261 x 2,560: 57, 60, 48, 53, 40, 43 us; 400 x 1,536 57, 59, 44, 48, 40, 39; 100 x 1,536 41, 28, 25, 23, 28, 25;
+        // 2,048 x 1,536 164, 173, 166, 210, 154, 151 (tiles of 32 x 32 by single warps win nowhere by more than 3 us, and lose 10 where
+        // nearly six an SM meet).
+        static const Tile three[6] = {{64, 64, 40., 27.4, 0., 0., 2}, {32, 64, 28., 14.8, 0., 0., 2}, {32, 32, 16.3, 8., 8., 24.6, 0},
+                                      {16, 32, 10.6, 5.1, 5., 17.7, 0}, {0}, {16, 32, 12., 3.3, 15., 15.6, 0}};
+        // Fewer (single warps are too few of them then), and rows off the 16-byte border.
+        static const Tile short_k[6] = {{64, 64, 62.8, 60., 0., 0., 1}, {32, 64, 34.4, 33., 0., 0., 1}, {32, 32, 22.4, 21., 0., 0., 1},
+                                        {16, 32, 18., 12., 0., 0., 1}, {0}, {0}};
+        const Tile* const tiles = !vec || groups < 3 ? short_k : groups == 3 ? three : groups == 4 ? four : long_k;
         int best = 0;
         double least = 0;
-        const bool many = groups >= 4 && vec;
-        for (int i = 0; i < (many ? 6 : 4); ++i) {
-            const Tile t = many ? long_k[i] : short_k[i];
-            if (i > 0 && (M + t.bm - 1) / t.bm > 65535) continue;      // as many rows as 64 x 64 tiles take, whatever their number
+        for (int i = 0; i < 6; ++i) {
+            const Tile& t = tiles[i];
+            if (!t.bm || (i > 0 && (M + t.bm - 1) / t.bm > 65535)) continue;      // as many rows as 64 x 64 tiles take, whatever their number
             const double waves = (double)((long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn)) / 148.;
-            double cost = waves <= 1. ? t.alone : i >= 4 ? std::max(33., t.first + waves * t.wave) : ceil(waves) * t.wave;
-            if (many && i == 3 && waves <= 1. && waves * 148. > 64.) cost = 19.6;           // (more than 64 of these wait for memory together)
+            double cost = t.alone;
+            if (waves > 1.) cost = std::max(t.least, t.first + (t.step ? ceil(waves / t.step) * t.step : waves) * t.wave);
+            else if (tiles == long_k && i == 3 && waves * 148. > 64.) cost = 19.6;          // (more than 64 of these wait for memory together)
             if (i == 0 || cost < least) best = i, least = cost;
         }
 #define RUNS(TM, TN, LY) return run_tiles<TM, TN, LY>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, groups, vec, stream)

@@ -783,7 +783,7 @@ def test_gemm_plain_in_32_bits_either_way(K):
         assert torch.equal(ops.gemm_plain(a[rows].contiguous(), w[cols].contiguous(), torch.float32), out[rows, cols])
 
 
-@pytest.mark.parametrize("M,N,K", [(261, 1500, 1100), (130, 2570, 1536), (410, 6100, 1028)])
+@pytest.mark.parametrize("M,N,K", [(261, 1500, 1100), (130, 2570, 1536), (410, 6100, 1028), (261, 2570, 768), (1100, 1540, 644)])
 def test_gemm_plain_in_32_bits_by_single_warps(M, N, K):
     """Sizes that tiles of 16 x 32 and of 32 x 32 by single warps take, with part-filled last tiles and runs: a corner of the product,
     which other tiles take, is the same bits."""
