@@ -64,7 +64,7 @@ __global__ void add_rmsnorm_vec8_kernel(float* __restrict__ x, const __nv_bfloat
     pdl_wait();
     const int i0 = threadIdx.x * 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool on = i0 < H;
-    const bool write_back = (rows == nullptr) && (delta != nullptr);
+    const bool write_back = rows == nullptr;
     float v[R][8];
     float4 a[R], b[R];
     uint4 d[R], e[R];
@@ -78,8 +78,8 @@ __global__ void add_rmsnorm_vec8_kernel(float* __restrict__ x, const __nv_bfloat
         if (!row_on[k]) continue;
         a[k] = *reinterpret_cast<const float4*>(x + at[k]);
         b[k] = *reinterpret_cast<const float4*>(x + at[k] + 4);
-        if (delta) d[k] = *reinterpret_cast<const uint4*>(delta + at[k]);
-        if (delta && delta2) e[k] = *reinterpret_cast<const uint4*>(delta2 + at[k]);
+        d[k] = *reinterpret_cast<const uint4*>(delta + at[k]);
+        if (delta2) e[k] = *reinterpret_cast<const uint4*>(delta2 + at[k]);
     }
     float wv[8];                 // the weights travel while the row's sum is taken
 #pragma unroll
@@ -91,20 +91,18 @@ __global__ void add_rmsnorm_vec8_kernel(float* __restrict__ x, const __nv_bfloat
         for (int j = 0; j < 8; ++j) v[k][j] = 0.f;
         if (row_on[k]) {
             v[k][0] = a[k].x; v[k][1] = a[k].y; v[k][2] = a[k].z; v[k][3] = a[k].w; v[k][4] = b[k].x; v[k][5] = b[k].y; v[k][6] = b[k].z; v[k][7] = b[k].w;
-            if (delta) {
-                const __nv_bfloat162* dp = reinterpret_cast<const __nv_bfloat162*>(&d[k]);
-                const __nv_bfloat162* ep = reinterpret_cast<const __nv_bfloat162*>(&e[k]);
+            const __nv_bfloat162* dp = reinterpret_cast<const __nv_bfloat162*>(&d[k]);
+            const __nv_bfloat162* ep = reinterpret_cast<const __nv_bfloat162*>(&e[k]);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float2 f = __bfloat1622float2(dp[j]);
-                    if (delta2) {
-                        const float2 g = __bfloat1622float2(ep[j]);
-                        v[k][2 * j] += f.x + g.x;
-                        v[k][2 * j + 1] += f.y + g.y;
-                    } else {
-                        v[k][2 * j] += f.x;
-                        v[k][2 * j + 1] += f.y;
-                    }
+            for (int j = 0; j < 4; ++j) {
+                const float2 f = __bfloat1622float2(dp[j]);
+                if (delta2) {
+                    const float2 g = __bfloat1622float2(ep[j]);
+                    v[k][2 * j] += f.x + g.x;
+                    v[k][2 * j + 1] += f.y + g.y;
+                } else {
+                    v[k][2 * j] += f.x;
+                    v[k][2 * j + 1] += f.y;
                 }
             }
             if (write_back) {
@@ -134,6 +132,70 @@ __global__ void add_rmsnorm_vec8_kernel(float* __restrict__ x, const __nv_bfloat
     }
 }
 
+// The same with 32 registers, with which an SM holds 2,048 threads, a row a block: without an addend, and for rows of more than 4,096
+// values, of whose blocks it holds one with more (300 rows of 8,192 values take 7.8 us, 8.6 in the form above; without an addend 1,200
+// rows of 2,048 4.4 and 4.7).
+template <typename TW>
+__global__ void add_rmsnorm_vec8_lean_kernel(float* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
+                                             const __nv_bfloat16* __restrict__ delta2, const TW* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                                             const int* __restrict__ rows, int H, float eps) {
+    __shared__ float scratch[32];
+    pdl_trigger();
+    pdl_wait();
+    const int r = blockIdx.x;
+    const int t = rows ? rows[r] : r;
+    const int i0 = threadIdx.x * 8;
+    const bool on = i0 < H;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+    if (on) {
+        const float4 a = *reinterpret_cast<const float4*>(x + (size_t)t * H + i0);
+        const float4 b = *reinterpret_cast<const float4*>(x + (size_t)t * H + i0 + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        if (delta) {
+            const uint4 d = *reinterpret_cast<const uint4*>(delta + (size_t)t * H + i0);
+            const __nv_bfloat162* dp = reinterpret_cast<const __nv_bfloat162*>(&d);
+            if (delta2) {
+                const uint4 e = *reinterpret_cast<const uint4*>(delta2 + (size_t)t * H + i0);
+                const __nv_bfloat162* ep = reinterpret_cast<const __nv_bfloat162*>(&e);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 f = __bfloat1622float2(dp[j]), g = __bfloat1622float2(ep[j]);
+                    v[2 * j] += f.x + g.x;
+                    v[2 * j + 1] += f.y + g.y;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 f = __bfloat1622float2(dp[j]);
+                    v[2 * j] += f.x;
+                    v[2 * j + 1] += f.y;
+                }
+            }
+            if (!rows) {
+                *reinterpret_cast<float4*>(x + (size_t)t * H + i0) = make_float4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<float4*>(x + (size_t)t * H + i0 + 4) = make_float4(v[4], v[5], v[6], v[7]);
+            }
+        }
+    }
+    float wv[8];                 // the weights travel while the row's sum is taken
+#pragma unroll
+    for (int j = 0; j < 8; ++j) wv[j] = on ? to_float(w[i0 + j]) : 0.f;
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+    const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)H + eps);
+    if (!on) return;
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        __nv_bfloat162 pk = __floats2bfloat162_rn(v[2 * j] * inv * wv[2 * j], v[2 * j + 1] * inv * wv[2 * j + 1]);
+        o[j] = *reinterpret_cast<uint32_t*>(&pk);
+    }
+    *reinterpret_cast<uint4*>(y + (size_t)r * H + i0) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // x: [*, H] float; delta, delta2: [*, H] act dtype or null (delta2 only beside delta); w: [H]; y: [n_rows, H] act dtype;
 // rows: null (all n_rows rows, x updated in place) or n_rows row indices (x left as is).
 static int add_rmsnorm_impl(float* x, const void* delta, const void* delta2, const void* w, int w_dtype, void* y,
@@ -144,14 +206,24 @@ static int add_rmsnorm_impl(float* x, const void* delta, const void* delta2, con
     if (groups < 1 || H % groups) return CELLM_ERR_SIZE;
     if (groups == 1 && act_dtype == CELLM_BF16 && (H & 7) == 0 && H <= 8192 && (((uintptr_t)x | (uintptr_t)delta | (uintptr_t)delta2 | (uintptr_t)y) & 15) == 0) {
         const int vthreads = ((H / 8 + 31) / 32) * 32;
-        // two rows a block where a row a block is more blocks than the SMs hold at once (2,048 threads each)
-        const bool two = !rows && (long long)n_rows * vthreads > 148LL * 2048;
+        // two rows a block where a row a block is more blocks than the SMs hold at once (46 registers a thread: 1,400 threads): 1,000
+        // rows of 2,048 values 5.0 us a row a block, 4.7 two; 600 rows 3.7 and 4.5
+        const bool lean = !delta || vthreads > 512, two = !rows && (long long)n_rows * vthreads > 148LL * 1400;
 #define VEC8(TW, R)                                                                                                        \
     CELLM_RUN((add_rmsnorm_vec8_kernel<TW, R>), (unsigned)((n_rows + R - 1) / R), vthreads, 0, stream, x, (const __nv_bfloat16*)delta, \
               (const __nv_bfloat16*)delta2, (const TW*)w, (__nv_bfloat16*)y, rows, n_rows, H, eps)
-        if (w_dtype == CELLM_BF16) { if (two) VEC8(__nv_bfloat16, 2); else VEC8(__nv_bfloat16, 1); }
-        else if (w_dtype == CELLM_F32) { if (two) VEC8(float, 2); else VEC8(float, 1); }
+#define VEC8_OF(TW)                                                                                                        \
+    do {                                                                                                                   \
+        if (lean)                                                                                                          \
+            CELLM_RUN(add_rmsnorm_vec8_lean_kernel<TW>, n_rows, vthreads, 0, stream, x, (const __nv_bfloat16*)delta,       \
+                      (const __nv_bfloat16*)delta2, (const TW*)w, (__nv_bfloat16*)y, rows, H, eps);                        \
+        else if (two) VEC8(TW, 2);                                                                                         \
+        else VEC8(TW, 1);                                                                                                  \
+    } while (0)
+        if (w_dtype == CELLM_BF16) VEC8_OF(__nv_bfloat16);
+        else if (w_dtype == CELLM_F32) VEC8_OF(float);
         else return CELLM_ERR_DTYPE;
+#undef VEC8_OF
 #undef VEC8
         return CELLM_OK;
     }

@@ -64,6 +64,22 @@ def test_add_rmsnorm(dtype, H):
     close(ops.add_rmsnorm(x, None, w.float(), 1e-6, dtype), plain.rms_norm(x1.double().cpu(), w.double().cpu(), 1e-6), dtype, "no addend, 32-bit weight")
 
 
+@pytest.mark.parametrize("T,H", [(3, 4096), (3, 4104), (2, 8192), (811, 2048), (1001, 1544)])
+def test_add_rmsnorm_of_wide_rows_and_of_many(T, H):
+    """bfloat16 rows of more than 4,096 values, two rows a block (an odd number of them), and rows without an addend, which take a form of
+    few registers: a row alone gives the same bits."""
+    from cellm_b200 import ops
+    x, delta, w = torch.randn(T, H, device=DEV), torch.randn(T, H, device=DEV).bfloat16(), torch.rand(H, device=DEV) + 0.5
+    for addend in (delta, None):
+        stream, alone = x.clone(), x[-1:].clone()
+        y = ops.add_rmsnorm(stream, addend, w, 1e-5, torch.bfloat16)
+        s = x.double() + (delta.double() if addend is not None else 0)
+        close(stream, s, torch.float32, "stream")
+        close(y, plain.rms_norm(s.cpu(), w.double().cpu(), 1e-5), torch.bfloat16, "normed")
+        one = ops.add_rmsnorm(alone, addend[-1:].contiguous() if addend is not None else None, w, 1e-5, torch.bfloat16)
+        assert torch.equal(y[-1:], one) and torch.equal(stream[-1:], alone)
+
+
 @pytest.mark.parametrize("dtype", DT)
 def test_swiglu_and_residual_add(dtype):
     from cellm_b200 import ops
