@@ -328,8 +328,9 @@ attention_flash_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part
 }
 
 // The same as below for at most 32 pieces: the pieces' values are under way together and before their maxima are looked at (one piece's
-// after the other's weight they cost a wait on L2 each); every warp forms the weights for itself, a lane a piece. The same sums in
-// the same order; values of a piece without weight (never written) are not used.
+// after the other's weight they cost a wait on L2 each); every warp forms the weights for itself, a lane a piece. The sums are taken in
+// the pieces' order, as there (fused multiply-adds, as the compiler may choose there); values of a piece without weight (never
+// written) are not used.
 __global__ void __launch_bounds__(64)
 attention_merge_few_kernel(__nv_bfloat16* out, const float* part_o, const float* part_ml, size_t n_rows, int hd, int nsplit,
                            const float* __restrict__ sinks, const float* __restrict__ unrot, int interleaved,

@@ -270,15 +270,15 @@ head_product_kernel(TA* __restrict__ out, long long ldo, long long out_hs, const
     }
 }
 
-// A few tokens (decoding, bfloat16): the matrices are what has to be read, once. A block takes 16 output rows of one
-// head; the tokens' inputs wait in shared memory; eight neighbouring threads share a row and take neighbouring 16-byte
+// A few tokens (decoding, bfloat16): the matrices are what has to be read, once. A block takes 128 / LANES output rows of one
+// head; the tokens' inputs wait in shared memory; LANES neighbouring threads share a row and take neighbouring 16-byte
 // pieces of it by turns (so a row's loads are whole 128-byte lines and the inputs' reads fall into different banks),
 // and add their sums by shuffles. K (a multiple of 64) is summed in the same order for every token count up to
-// HP_SMALL_T.
+// HP_SMALL_T (in another for 8 threads a row than for 16).
 #define HP_SMALL_T 16
 #define HP_SMALL_AHEAD 8        // pieces of a row asked for ahead: all of K up to 512
-// LANES threads share a row: 8, or 16 from K = 256 on, where a thread's products are what takes time (with the preparation's loads
-// ahead of its barrier and of its stores a layer that decodes 8 requests went from 52.3 to 48.2 us).
+// LANES is 8, or 16 from K = 256 on where a thread's products are what takes time: up to 4,096 rows over all heads. 8 tokens, K = 512:
+// 1,024 rows 8.2 us with 8 and 5.5 with 16, 4,096 9.8 and 7.8, 8,192 10.6 and 11.5; K = 256: 5.1 and 3.7, 6.1 and 5.2, 6.6 and 7.6.
 template <int LANES>
 __global__ void __launch_bounds__(128)
 head_product_small_kernel(__nv_bfloat16* __restrict__ out, long long ldo, long long out_hs, const __nv_bfloat16* in,
@@ -362,7 +362,7 @@ CELLM_API int cellm_head_product(void* out, long long ldo, long long out_hs, con
     CELLM_RUN(head_product_small_kernel<LANES>, dim3((unsigned)((N + 128 / LANES - 1) / (128 / LANES)), (unsigned)heads), 128, smem, stream, \
               (__nv_bfloat16*)out, ldo, out_hs, (const __nv_bfloat16*)in, ldi, in_hs, (const __nv_bfloat16*)w, T, N, K,         \
               (int)((((uintptr_t)in & 15) == 0) && (ldi & 7) == 0 && (in_hs & 7) == 0))
-        if (K >= 256) SMALL(16);
+        if (K >= 256 && (long long)heads * N <= 4096) SMALL(16);
         else SMALL(8);
 #undef SMALL
         return CELLM_OK;

@@ -378,6 +378,20 @@ def test_head_product_of_few_tokens(T, heads, N, K):
     torch.testing.assert_close(out.cpu().double(), want, rtol=2e-2, atol=8e-2)
 
 
+@pytest.mark.parametrize("heads,N,K", [(4, 1000, 256), (4, 1032, 256), (3, 37, 320), (2, 4, 1088), (5, 100, 192)])
+def test_head_product_of_few_tokens_by_eight_and_sixteen_threads_a_row(heads, N, K):
+    """Both numbers of threads a row, blocks that end inside a head, K that ends inside the threads' round: a token alone gives the bits of
+    16; 64 bits rounded once, and 32-bit sums of K terms (K * 2^-24 of their magnitudes' sum, below 2^-8 of a result of theirs)."""
+    from cellm_b200 import ops
+    g = torch.Generator().manual_seed(N)
+    x, w = _t(torch.randn(16, heads, K, generator=g), torch.bfloat16), _t(torch.randn(heads, N, K, generator=g), torch.bfloat16)
+    out = ops.head_product(x, w)
+    want = torch.einsum("thk,hnk->thn", x.cpu().double(), w.cpu().double())
+    torch.testing.assert_close(out.cpu().double(), want, rtol=2.0 ** -8, atol=2.0 ** -24 * K * K ** 0.5)
+    for t in (0, 7, 15):
+        assert torch.equal(ops.head_product(x[t:t + 1].contiguous(), w)[0], out[t])
+
+
 @pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
 def test_gated_act(act):
     from cellm_b200 import ops
