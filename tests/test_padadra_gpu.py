@@ -640,13 +640,15 @@ def test_chunks_go_through_a_small_workspace_in_runs(monkeypatch, kind, held):
 
 
 @pytest.mark.parametrize("kind", ["delta", "hgrn2"])
-@pytest.mark.parametrize("requests,dim,vd", [(3, 128, 128), (9, 128, 128), (40, 64, 128)])
+@pytest.mark.parametrize("requests,dim,vd", [(3, 128, 128), (9, 128, 128), (14, 128, 128), (3, 64, 128), (9, 64, 128), (13, 64, 128), (40, 64, 128)])
 def test_chunks_with_several_blocks_an_sm(kind, requests, dim, vd):
-    """1, 2 and 8 blocks of the walk an SM, with the stages that are left each: the walk's results, for every request (the bound is
-    that of the recurrences against 64 bits)."""
+    """Grids of the walk of up to one, two, three and more blocks an SM, by which the stages are chosen and by them and the threads what an SM
+    holds: one block of four stages each; then with heads of 64 rows two of four, HGRN2 three of four and four of three, the delta rule two of
+    three; with 128 HGRN2 two of four and two of three, the delta rule one of three. A portion of 26 chunks beside short ones: the walk's
+    results token by token, for every request (the bound is that of the recurrences against 64 bits)."""
     from cellm_b200 import ops
     heads, g = 4, torch.Generator().manual_seed(requests)
-    lens = [96 + 7 * (i % 5) for i in range(requests)]
+    lens = [401] + [96 + 7 * (i % 5) for i in range(1, requests)]
     T, ctx, got = sum(lens), step_ctx(lens, [0] * requests, list(range(requests))), []
     unit = lambda: torch.nn.functional.normalize(torch.randn(T, heads, dim, generator=g), dim=-1).reshape(T, -1)
     qk, v = torch.cat([unit(), unit()], 1).to(DEV).contiguous(), torch.randn(T, heads * vd, generator=g).to(DEV)
