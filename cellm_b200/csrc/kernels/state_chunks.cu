@@ -422,11 +422,11 @@ __device__ __forceinline__ void walk_whole(float* sm, const float* ws, long long
 // it (product3); sums over more than 16 terms are 32-bit additions. A block that has found a u or a read-out that is not finite starts again
 // (walk_whole).
 // Bound by the chain of a chunk, 0.95 us: products (24 of mma.sync a scheduler, 9 cycles each), the meeting of the warps, u's sums, u
-// back to all of them, 64 multiply-adds of pairs a thread with their loads. With multiply-adds on S in shared memory for both products
+// back to all of them, 64 multiply-adds of pairs a thread with their loads (which keep shared memory busy for 0.69 of the time). With multiply-adds on S in shared memory for both products
 // the walk took 166 us for 2,048 tokens and 16 heads of 128 x 128, bound by shared memory's bandwidth; this form 121 (105 with both on
 // the tensor cores, see the errors above). What that took: no mbarrier on the chain, loads ahead of the waits, read-outs and
-// sums on warps of their own. HGRN2 with heads of 64 x 64, which has no u to wait for: 88 -> 49 us for 128 chunks. Where blocks are many
-// the workspace's bytes count: every block of columns reads its head's operands. HGRN2's values are fetched here, by the warps of the
+// sums on warps of their own. HGRN2 with 12 heads of 64 x 128, which has no u to wait for: two prompts of 112 chunks 88 -> 58 us. Where blocks
+// are many the workspace's bytes count: every block of columns reads its head's operands. HGRN2's values are fetched here, by the warps of the
 // sums, two chunks ahead. Vectors and walk of 32 portions of 100 tokens over 16 heads of 128 x 128: delta rule 398 us (multiply-adds 463),
 // HGRN2 205 (239); 16 portions of 1,000 tokens 1,505 (1,699) and 906 (1,026); heads of 64 x 64, 6 portions of 351 tokens, 75 (81) and 45 (53).
 template <int DIM, bool DELTA>
